@@ -22,23 +22,19 @@
 // `decay_prepare`.
 //
 // Only differences L_i - L_j with i >= j are ever exponentiated, so nothing overflows however strong
-// the decay.  `chunk_prepare` makes W, Uv, B, Q * exp L, K * exp(L_end - L) and exp L_end for every
-// (chunk, head) in parallel.  What follows keeps the chain from chunk to chunk as short as it can be
-// and does everything else in parallel over chunks (see the two groups of kernels below): for the
-// decayed sum the chain is element-wise, for the delta rule it is one product S <- M S + N per chunk.
-// `chunk_apply` is the first, direct form (three products with the state per chunk inside the chain);
-// it stays for sizes whose operands the later kernels cannot hold.  All arithmetic is float on the
+// the decay.  A first launch (`delta_prepare`, `decay_prepare`, `wkv_prepare`) makes W, Uv, B, Q * exp L,
+// K * exp(L_end - L) and exp L_end for every (chunk, head) in parallel.  What follows keeps the chain from chunk to
+// chunk as short as it can be and does everything else in parallel over chunks: for the decayed sums the chain is
+// element-wise, for the delta rule two products with the state a chunk.  All arithmetic is float on the
 // CUDA cores: scores, decays, the triangular solve and the state stay 32-bit in both storage types.
 // Chunks start at the portion's first token; results do not depend on where a portion is cut beyond
 // rounding.
 #include "recurrence_rules.cuh"
-#include <utility>
 
 namespace pmm {
 
 constexpr int kChunk = 64;
-constexpr int kPrepThreads = 512;
-constexpr int kApplyThreads = 256;
+constexpr int kPrepThreads = 256;
 
 __device__ __forceinline__ float sigmoid_c(float x) { return 1.f / (1.f + expf(-x)); }
 
@@ -58,8 +54,7 @@ struct ChunkArgs {
   // per (chunk, head), chunk-major: W [C, d] (delta), Uv [C, dv], B [C, C], Qg [C, d], Ke [C, d], Eg [d]
   float *W, *Uv, *B, *Qg, *Ke, *Eg;
   int vec_in;                           // q, k, v (and a) rows and heads start on boundaries of four elements
-  int sub_blocks;                       // chunk_prepare scales rows once per sub-block of 16 tokens (its shared memory allows it)
-  float *N, *M;                         // [d, dv] and (delta) [d, d] per (chunk, head): see the kernels that use them
+  float* N;                             // [d, dv] per (chunk, head): see the kernels that use it
   float* state; const int* slots; float* out;
 };
 
@@ -81,15 +76,149 @@ __device__ __forceinline__ bool locate_chunk(const int* __restrict__ cu, int n_s
   return false;
 }
 
+// ----------------------------------------------------------------------------------------------
+// Four neighbouring elements of a row in the storage type (`vec`: the row starts on a boundary of four elements).
 template <typename S>
-__global__ void __launch_bounds__(kPrepThreads)
-    chunk_prepare_kernel(ChunkArgs p) {
-  extern __shared__ float sm[];
-  const int d = p.d, dv = p.dv, ds = d + 1;  // rows of stride d + 1: row i, column c sits in bank (i + c) mod 32
-  float* sK = sm;                         // [C][ds]
-  float* sQ = sK + kChunk * ds;           // [C][ds]   (later: the right-hand sides of the solve)
-  float* sL = sQ + kChunk * ds;           // [C][ds]
-  float* sA = sL + kChunk * ds;           // [C][C + 1]
+__device__ __forceinline__ float4 load4(const S* p, bool vec) {
+  if (!vec) return make_float4(ldf(p), ldf(p + 1), ldf(p + 2), ldf(p + 3));
+  return ldf4(p);
+}
+
+// ----------------------------------------------------------------------------------------------
+// Two floats in one register pair: one instruction for two multiply-adds, each rounded as by itself.
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair(float x, float y) {
+  Pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 halves(Pair v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+struct Quad { Pair lo, hi; };
+__device__ __forceinline__ Quad quad(const float* p) {  // sixteen bytes
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
+
+// ----------------------------------------------------------------------------------------------
+// The delta rule's operands W, Uv, B, Q * exp L, K * exp(L_end - L), exp L_end of one (chunk, head) per block.
+//
+// Sums of logarithms (to base 2) start anew every 8 tokens, and products across boundaries use two factors, each at most
+// one: with r the last row before i's half, exp(L_i - L_j) = exp(L_i - L_r) exp(L_r - L_j).  So only the pairs within 8
+// tokens take an exponential per channel; then q_i, k_i (weakened from their half's start) and k_j (weakened to its half's
+// end) lie in place as three matrices, pairs across halves of 8, 16 and 32 tokens are plain products in 4 x 4 tiles of A
+// and B at once, and between two levels the rows are weakened by one more half's total.  What is left at the end is
+// Q * exp L, K * exp L and K * exp(L_end - L).
+// The triangular solve takes a thread per column of [W | Uv], 16 rows at a time in registers: the rows solved before are
+// taken off first, then each row that becomes known is taken off those below, with A read as broadcast rows of its
+// transpose, which lies where q was (its entries wait in registers until q is done).
+// Rows from the chunk's end on are made as zeros, so that the chain kernel needs no count of rows.
+//
+// Bound by the issue of its own instructions; 256 threads and 109 KB at d = 128 put two blocks on an SM, so that one
+// block's barriers and shared-memory latencies are the other's turn and the 256 blocks of 2,048 tokens and 8 heads are one
+// wave.  That size, 128 x 128: first form (rows scaled per sub-block of 16 into copies, scalar shared-memory reads, a column
+// walking A in shared memory, 157 KB) 160 us, 4 x 4 tiles with the solve's whole column in registers (unrolled past the
+// instruction cache, one block an SM) 96 us, this form 64 us.
+constexpr float kLogDecayMin = -1e4f;  // a token's logarithm to base 2: the power is zero long before, and sums stay finite
+constexpr int kPrepRows = kChunk / 8;  // halves of 8 tokens
+
+inline size_t delta_prepare_smem(int d) {
+  const size_t row = static_cast<size_t>(d) + 4;
+  const size_t q = kChunk * row > kChunk * kChunk ? kChunk * row : kChunk * kChunk;
+  return sizeof(float) * (q + 2 * kChunk * row + 14 * static_cast<size_t>(d));
+}
+
+// v[32] summed over LANES neighbouring lanes; lane l keeps sums (l % LANES) * 32 / LANES .. in v[0 .. 32 / LANES - 1]
+template <int LANES>
+__device__ __forceinline__ void sum_scatter(float (&v)[32], int lane) {
+  int count = 32;
+#pragma unroll
+  for (int off = LANES / 2; off >= 1; off >>= 1) {
+    count >>= 1;
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (i < count) {
+        const float send = up ? v[i] : v[i + count], keep = up ? v[i + count] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+  }
+}
+
+// A and B of the pairs (i, j), i in the odd and j in the even half of HALF tokens of every span of 2 HALF tokens, in 4 x 4
+// tiles whose channels are shared by kSlices lanes.  B goes out, A stays with the threads: `keep` entry e is entry
+// slice * kKeep + e of its tile where that is below 16.
+template <int HALF>
+struct CrossPairs {
+  static constexpr int kSide = HALF / 4, kTiles = (kChunk / (2 * HALF)) * kSide * kSide;  // 16, 32 and 64 tiles
+  static constexpr int kSlices = kPrepThreads / kTiles, kKeep = 32 / kSlices;             // 16, 8 and 4 lanes
+  int slice, i0, j0;
+  float keep[kKeep];
+  __device__ __forceinline__ void run(const float* __restrict__ sQ, const float* __restrict__ sK, const float* __restrict__ sKd,
+                                      float* __restrict__ oB, int ds, int d4, int n, int tid) {
+    const int tile = tid / kSlices, g = tile / (kSide * kSide), in = tile % (kSide * kSide);
+    slice = tid % kSlices;
+    i0 = 2 * HALF * g + HALF + 4 * (in / kSide);
+    j0 = 2 * HALF * g + 4 * (in % kSide);
+    Pair acc[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) acc[e] = 0;
+    for (int c4 = slice; c4 < d4; c4 += kSlices) {
+      Quad kd[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) kd[s] = quad(sKd + (j0 + s) * ds + 4 * c4);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const Quad k = quad(sK + (i0 + r) * ds + 4 * c4), q = quad(sQ + (i0 + r) * ds + 4 * c4);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          acc[4 * r + s] = fma2(k.hi, kd[s].hi, fma2(k.lo, kd[s].lo, acc[4 * r + s]));
+          acc[16 + 4 * r + s] = fma2(q.hi, kd[s].hi, fma2(q.lo, kd[s].lo, acc[16 + 4 * r + s]));
+        }
+      }
+    }
+    float v[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) {
+      const float2 two = halves(acc[e]);
+      v[e] = two.x + two.y;
+    }
+    sum_scatter<kSlices>(v, slice);
+#pragma unroll
+    for (int e = 0; e < kKeep; ++e) {
+      const int at = slice * kKeep + e, i = i0 + (at % 16) / 4;
+      keep[e] = v[e];
+      if (at >= 16 && i < n) oB[i * kChunk + j0 + at % 4] = v[e];
+    }
+  }
+  __device__ __forceinline__ void leave(float* __restrict__ sAt) const {
+#pragma unroll
+    for (int e = 0; e < kKeep; ++e) {
+      const int at = slice * kKeep + e;
+      if (at < 16) sAt[(j0 + at % 4) * kChunk + i0 + at / 4] = keep[e];
+    }
+  }
+};
+
+template <typename S>
+__global__ void __launch_bounds__(kPrepThreads, 2)
+    delta_prepare_kernel(ChunkArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  const int d = p.d, d4 = d / 4, dv = p.dv, ds = d + 4;  // rows of stride d + 4: neighbouring rows' 16-byte reads fall into different banks
+  float* sQ = sm;                               // [C][ds]  q, then weakened from its half's start
+  float* sAt = sm;                              // [C][C]   A transposed: row j, entries i > j (once q is done)
+  float* sK = sQ + max(kChunk * ds, kChunk * kChunk);  // [C][ds]  k, then weakened from its half's start, then W
+  float* sL = sK + kChunk * ds;                 // [C][ds]  sums of logarithms, then k weakened to its half's end, then columns of Uv
+  float* sT = sL + kChunk * ds;                 // [8 + 4 + 2][d]  totals of 8 tokens, then powers of the totals of 8, 16 and 32
   __shared__ float s_beta[kChunk];
   pdl_launch_dependents();
   pdl_wait();
@@ -98,189 +227,214 @@ __global__ void __launch_bounds__(kPrepThreads)
   if (!locate_chunk(p.cu, p.n_seq, chunk, &seq, &t0, &n)) return;
   const int hk = h / (p.H / p.Hk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const S* gq = static_cast<const S*>(p.q);
-  const S* gk = static_cast<const S*>(p.k);
-  const S* gv = static_cast<const S*>(p.v);
+  constexpr int kWarps = kPrepThreads / 32;
   const size_t ch = static_cast<size_t>(chunk) * p.H + h;
-  float* oW = p.W + ch * kChunk * d;
-  float* oUv = p.Uv + ch * kChunk * dv;
   float* oB = p.B + ch * kChunk * kChunk;
+  const bool vec = p.vec_in != 0;
+  constexpr float kLog2E = 1.4426950408889634f;
+
+  // ---- unit-length q and k and the decays' logarithms: a warp per token
+  const float a_neg = -expf(p.a_log[h]) * kLog2E;
+#pragma unroll 2
+  for (int i = warp; i < kChunk; i += kWarps) {
+    float *rq = sQ + i * ds, *rk = sK + i * ds, *rl = sL + i * ds;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i >= n) {
+      for (int c4 = lane; c4 < d4; c4 += 32) {
+        *reinterpret_cast<float4*>(rq + 4 * c4) = zero;
+        *reinterpret_cast<float4*>(rk + 4 * c4) = zero;
+        *reinterpret_cast<float4*>(rl + 4 * c4) = zero;
+      }
+      continue;
+    }
+    const long long t = t0 + i;
+    float sq = 0.f, sk = 0.f;
+    for (int c4 = lane; c4 < d4; c4 += 32) {
+      const int c = 4 * c4;
+      const float4 q = load4(static_cast<const S*>(p.q) + t * p.ld_q + hk * d + c, vec);
+      const float4 k = load4(static_cast<const S*>(p.k) + t * p.ld_k + hk * d + c, vec);
+      const float4 a = load4(static_cast<const S*>(p.a) + t * p.ld_a + h * d + c, vec);
+      const float* b = p.dt_bias + h * d + c;
+      auto decay = [a_neg](float z) {
+        const float l = a_neg * softplus_f(z);
+        return l < kLogDecayMin ? kLogDecayMin : l;  // (NaN stays)
+      };
+      sq += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+      sk += k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w;
+      *reinterpret_cast<float4*>(rq + c) = q;
+      *reinterpret_cast<float4*>(rk + c) = k;
+      *reinterpret_cast<float4*>(rl + c) = make_float4(decay(a.x + b[0]), decay(a.y + b[1]), decay(a.z + b[2]), decay(a.w + b[3]));
+    }
+    const float fq = p.q_scale / sqrtf(warp_sum(sq) + p.unit_eps), fk = 1.f / sqrtf(warp_sum(sk) + p.unit_eps);
+    for (int c4 = lane; c4 < d4; c4 += 32) {
+      float4 q = *reinterpret_cast<float4*>(rq + 4 * c4), k = *reinterpret_cast<float4*>(rk + 4 * c4);
+      *reinterpret_cast<float4*>(rq + 4 * c4) = make_float4(q.x * fq, q.y * fq, q.z * fq, q.w * fq);
+      *reinterpret_cast<float4*>(rk + 4 * c4) = make_float4(k.x * fk, k.y * fk, k.z * fk, k.w * fk);
+    }
+  }
+  if (tid < kChunk)
+    s_beta[tid] = tid < n ? sigmoid_c(ldf(static_cast<const S*>(p.beta) + static_cast<long long>(t0 + tid) * p.ld_beta + h)) : 0.f;
+  __syncthreads();
+  for (int blk = warp; blk < kPrepRows; blk += kWarps) {  // running sums within 8 tokens
+    for (int c = lane; c < d; c += 32) {
+      float run = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        run += sL[(8 * blk + i) * ds + c];
+        sL[(8 * blk + i) * ds + c] = run;
+      }
+      sT[blk * d + c] = run;
+    }
+  }
+  __syncthreads();
+
+  // ---- pairs within 8 tokens: a thread per pair, the exponential per channel
+  float own_a[kChunk * 8 / kPrepThreads];
+#pragma unroll
+  for (int u = 0; u < kChunk * 8 / kPrepThreads; ++u) {
+    const int e = tid + kPrepThreads * u, i = e >> 3, j = (i & ~7) + (e & 7);
+    own_a[u] = 0.f;
+    if (j <= i) {
+      const float *qi = sQ + i * ds, *ki = sK + i * ds, *li = sL + i * ds, *kj = sK + j * ds, *lj = sL + j * ds;
+      Pair accA = 0, accB = 0;
+#pragma unroll 2
+      for (int c = 0; c < d; c += 4) {
+        const Quad q = quad(qi + c), k = quad(ki + c);
+        const float4 o = *reinterpret_cast<const float4*>(kj + c), l = *reinterpret_cast<const float4*>(li + c), m = *reinterpret_cast<const float4*>(lj + c);
+        const Pair lo = pair(o.x * exp2f(l.x - m.x), o.y * exp2f(l.y - m.y)), hi = pair(o.z * exp2f(l.z - m.z), o.w * exp2f(l.w - m.w));
+        accA = fma2(k.hi, hi, fma2(k.lo, lo, accA));
+        accB = fma2(q.hi, hi, fma2(q.lo, lo, accB));
+      }
+      const float2 two_a = halves(accA), two_b = halves(accB);
+      own_a[u] = two_a.x + two_a.y;
+      if (i < n) oB[i * kChunk + j] = two_b.x + two_b.y;
+    }
+  }
+  __syncthreads();
+  auto times = [](float* at, const float4& f) {
+    float4 v = *reinterpret_cast<float4*>(at);
+    *reinterpret_cast<float4*>(at) = make_float4(v.x * f.x, v.y * f.y, v.z * f.z, v.w * f.w);
+  };
+  auto power = [](const float4& l) { return make_float4(exp2f(l.x), exp2f(l.y), exp2f(l.z), exp2f(l.w)); };
+  for (int i = warp; i < kChunk; i += kWarps) {
+    for (int c = 4 * lane; c < d; c += 128) {
+      const float4 l = *reinterpret_cast<const float4*>(sL + i * ds + c), t = *reinterpret_cast<const float4*>(sT + (i >> 3) * d + c);
+      const float4 k = *reinterpret_cast<const float4*>(sK + i * ds + c);
+      const float4 up = power(l), down = power(make_float4(t.x - l.x, t.y - l.y, t.z - l.z, t.w - l.w));
+      *reinterpret_cast<float4*>(sL + i * ds + c) = make_float4(k.x * down.x, k.y * down.y, k.z * down.z, k.w * down.w);
+      *reinterpret_cast<float4*>(sK + i * ds + c) = make_float4(k.x * up.x, k.y * up.y, k.z * up.z, k.w * up.w);
+      times(sQ + i * ds + c, up);
+    }
+  }
+  __syncthreads();
+  for (int c = tid; c < d; c += kPrepThreads) {  // the totals' powers, from the sums
+    float t[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) t[b] = sT[b * d + c];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) sT[b * d + c] = exp2f(t[b]);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) sT[(8 + b) * d + c] = exp2f(t[2 * b] + t[2 * b + 1]);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) sT[(12 + b) * d + c] = exp2f((t[4 * b] + t[4 * b + 1]) + (t[4 * b + 2] + t[4 * b + 3]));
+    p.Eg[ch * d + c] = exp2f(((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7])));
+  }
+  // ---- pairs across halves of 8, 16 and 32 tokens; after each, rows reach through the neighbouring half
+  auto widen = [&](int half, int first_total) {
+    __syncthreads();
+    for (int i = warp; i < kChunk; i += kWarps) {
+      const int b = i / half;
+      for (int c = 4 * lane; c < d; c += 128) {
+        const float4 f = *reinterpret_cast<const float4*>(sT + (first_total + (b ^ 1)) * d + c);
+        if (b & 1) {
+          times(sQ + i * ds + c, f);
+          times(sK + i * ds + c, f);
+        } else {
+          times(sL + i * ds + c, f);
+        }
+      }
+    }
+    __syncthreads();
+  };
+  CrossPairs<8> by8;
+  by8.run(sQ, sK, sL, oB, ds, d4, n, tid);
+  widen(8, 0);
+  CrossPairs<16> by16;
+  by16.run(sQ, sK, sL, oB, ds, d4, n, tid);
+  widen(16, 8);
+  CrossPairs<32> by32;
+  by32.run(sQ, sK, sL, oB, ds, d4, n, tid);
+  widen(32, 12);
+
+  // ---- what the other launches read; V takes the place of K * exp(L_end - L), A that of q
   float* oQg = p.Qg + ch * kChunk * d;
   float* oKe = p.Ke + ch * kChunk * d;
-  float* oEg = p.Eg + ch * d;
-
-  // ---- q, k (and the logarithms of the decays) of the chunk's tokens
-  const float a_neg = -expf(p.a_log[h]);
-  for (int e = tid; e < n * d; e += kPrepThreads) {
-    const int i = e / d, c = e - i * d;
-    const long long t = t0 + i;
-    const float qv = ldf(gq + t * p.ld_q + hk * d + c), kv = ldf(gk + t * p.ld_k + hk * d + c);
-    sQ[i * ds + c] = qv;
-    sK[i * ds + c] = kv;
-    const float av = ldf(static_cast<const S*>(p.a) + t * p.ld_a + h * d + c) + p.dt_bias[h * d + c];
-    sL[i * ds + c] = a_neg * softplus_f(av);
-  }
-  if (tid < n) s_beta[tid] = sigmoid_c(ldf(static_cast<const S*>(p.beta) + static_cast<long long>(t0 + tid) * p.ld_beta + h));
-  __syncthreads();
-  for (int i = warp; i < n; i += kPrepThreads / 32) {  // unit length per token
-    float sq = 0.f, sk = 0.f;
-    for (int c = lane; c < d; c += 32) {
-      sq += sQ[i * ds + c] * sQ[i * ds + c];
-      sk += sK[i * ds + c] * sK[i * ds + c];
-    }
-    sq = warp_sum(sq);
-    sk = warp_sum(sk);
-    const float fq = p.q_scale / sqrtf(sq + p.unit_eps), fk = 1.f / sqrtf(sk + p.unit_eps);
-    for (int c = lane; c < d; c += 32) {
-      sQ[i * ds + c] *= fq;
-      sK[i * ds + c] *= fk;
-    }
-  }
-  for (int c = tid; c < d; c += kPrepThreads) {  // running sums of the logarithms
-    float run = 0.f;
-    for (int i = 0; i < n; ++i) {
-      run += sL[i * ds + c];
-      sL[i * ds + c] = run;
+  for (int i = warp; i < kChunk; i += kWarps) {
+    for (int c = 4 * lane; c < d; c += 128) {
+      *reinterpret_cast<float4*>(oQg + i * d + c) = *reinterpret_cast<const float4*>(sQ + i * ds + c);
+      *reinterpret_cast<float4*>(oKe + i * d + c) = *reinterpret_cast<const float4*>(sL + i * ds + c);
     }
   }
   __syncthreads();
-
-  // ---- A (delta) and B
-  if (p.sub_blocks) {
-    // Pairs inside one sub-block of 16 tokens: the exponential per channel.  A warp takes two rows,
-    // 16 lanes each, a lane one column of the row's sub-block.
-    for (int i2 = 2 * warp; i2 < n; i2 += 2 * (kPrepThreads / 32)) {
-      const int i = i2 + (lane >> 4), j = (i & ~15) + (lane & 15);
-      if (i < n && j <= i) {
-        const float *qi = sQ + i * ds, *ki = sK + i * ds, *li = sL + i * ds, *kj = sK + j * ds, *lj = sL + j * ds;
-        float accA = 0.f, accB = 0.f;
-        for (int c = 0; c < d; ++c) {
-          const float w = expf(li[c] - lj[c]) * kj[c];
-          accA += ki[c] * w;
-          accB += qi[c] * w;
-        }
-        sA[i * (kChunk + 1) + j] = accA;
-        oB[i * kChunk + j] = accB;
-      }
-    }
-    // Pairs across sub-blocks: with r the last row before i's sub-block, exp(L_i - L_j) = exp(L_i - L_r) exp(L_r - L_j),
-    // both factors at most one, so the rows are scaled once per sub-block and the pairs are plain dot products.
-    float* sKd = sA + kChunk * (kChunk + 1);   // [48][ds]  k_j exp(L_r - L_j), j before the sub-block
-    float* sKp = sKd + 48 * ds;                // [16][ds]  k_i exp(L_i - L_r), i in the sub-block
-    float* sQp = sKp + 16 * ds;                // [16][ds]  q_i exp(L_i - L_r)
-    for (int blk = 1; 16 * blk < n; ++blk) {
-      const int r = 16 * blk - 1, rows = min(16, n - 16 * blk);
-      __syncthreads();  // the sub-block before is done with the scaled rows
-      for (int e = tid; e < 16 * blk * d; e += kPrepThreads) {
-        const int j = e / d, c = e - j * d;
-        sKd[j * ds + c] = sK[j * ds + c] * expf(sL[r * ds + c] - sL[j * ds + c]);
-      }
-      for (int e = tid; e < rows * d; e += kPrepThreads) {
-        const int ii = e / d, c = e - ii * d, i = 16 * blk + ii;
-        const float pw = expf(sL[i * ds + c] - sL[r * ds + c]);
-        sKp[ii * ds + c] = sK[i * ds + c] * pw;
-        sQp[ii * ds + c] = sQ[i * ds + c] * pw;
-      }
-      __syncthreads();
-      if (warp < rows) {  // a warp per row of the sub-block, a lane the columns j = lane and lane + 32
-        const int i = 16 * blk + warp;
-        const float *kp = sKp + warp * ds, *qp = sQp + warp * ds;
+  by8.leave(sAt);
+  by16.leave(sAt);
+  by32.leave(sAt);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int j = lane + 32 * half;
-          if (j < 16 * blk) {
-            const float* kd = sKd + j * ds;
-            float accA = 0.f, accB = 0.f;
-            for (int c = 0; c < d; ++c) {
-              accA += kp[c] * kd[c];
-              accB += qp[c] * kd[c];
-            }
-            sA[i * (kChunk + 1) + j] = accA;
-            oB[i * kChunk + j] = accB;
+  for (int u = 0; u < kChunk * 8 / kPrepThreads; ++u) {
+    const int e = tid + kPrepThreads * u, i = e >> 3, j = (i & ~7) + (e & 7);
+    if (j <= i) sAt[j * kChunk + i] = own_a[u];  // (the diagonal's is not read for a result)
+  }
+
+  // ---- T X = diag(beta) [K * exp L | V] by forward substitution, V's columns d at a time
+  const S* gv = static_cast<const S*>(p.v) + static_cast<long long>(t0) * p.ld_v + h * dv;
+  for (int v0 = 0; v0 < dv; v0 += d) {
+    const int vw = min(d, dv - v0);
+    for (int i = warp; i < kChunk; i += kWarps)
+      for (int c = lane; c < vw; c += 32) sL[i * ds + c] = i < n ? ldf(gv + static_cast<long long>(i) * p.ld_v + v0 + c) : 0.f;
+    __syncthreads();
+    const int n_w = v0 == 0 ? d : 0;  // the first pass also solves for W
+    for (int col = tid; col < n_w + vw; col += kPrepThreads) {
+      const bool is_w = col < n_w;
+      const int c = is_w ? col : col - n_w;
+      float* x = (is_w ? sK : sL) + c;
+      float* to = is_w ? p.W + ch * kChunk * d + c : p.Uv + ch * kChunk * dv + v0 + c;
+      const int ld = is_w ? d : dv;
+#pragma unroll 1
+      for (int b0 = 0; b0 < kChunk; b0 += 16) {
+        Pair r[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) r[u] = pair(x[(b0 + 2 * u) * ds], x[(b0 + 2 * u + 1) * ds]);
+        const float* at = sAt + b0;
+#pragma unroll 4
+        for (int m = 0; m < b0; ++m) {
+          const float xm = -x[m * ds];
+          const Pair xx = pair(xm, xm);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const Quad a = quad(at + m * kChunk + 4 * u);
+            r[2 * u] = fma2(a.lo, xx, r[2 * u]);
+            r[2 * u + 1] = fma2(a.hi, xx, r[2 * u + 1]);
+          }
+        }
+        at += b0 * kChunk;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float2 two = halves(r[j / 2]);
+          const float xj = ((j & 1) ? two.y : two.x) * s_beta[b0 + j];
+          x[(b0 + j) * ds] = xj;
+          to[(b0 + j) * ld] = xj;
+          const Pair xx = pair(-xj, -xj);
+#pragma unroll
+          for (int u = (j + 1) / 4; u < 4; ++u) {  // (a pair of rows that is not all below row j: what its done half becomes is not read)
+            const Quad a = quad(at + j * kChunk + 4 * u);
+            if (4 * u + 1 > j) r[2 * u] = fma2(a.lo, xx, r[2 * u]);
+            r[2 * u + 1] = fma2(a.hi, xx, r[2 * u + 1]);
           }
         }
       }
     }
-  } else {
-  // a warp takes rows i, a lane the columns j = lane and lane + 32
-  for (int i = warp; i < n; i += kPrepThreads / 32) {
-    const float* qi = sQ + i * ds;
-    const float* ki = sK + i * ds;
-    const float* li = sL + i * ds;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int j = lane + 32 * half;
-      if (j > i) continue;
-      const float* kj = sK + j * ds;
-      float accA = 0.f, accB = 0.f;
-      const float* lj = sL + j * ds;
-      for (int c = 0; c < d; ++c) {
-        const float w = expf(li[c] - lj[c]) * kj[c];
-        accA += ki[c] * w;
-        accB += qi[c] * w;
-      }
-      sA[i * (kChunk + 1) + j] = accA;
-      oB[i * kChunk + j] = accB;
-    }
-  }
-  }
-  // ---- q * exp L, k * exp(L_end - L), exp L_end
-  for (int e = tid; e < n * d; e += kPrepThreads) {
-    const int i = e / d, c = e - i * d;
-    const float up = sL[i * ds + c], end = sL[(n - 1) * ds + c];
-    oQg[i * d + c] = sQ[i * ds + c] * expf(up);
-    oKe[i * d + c] = sK[i * ds + c] * expf(end - up);
-  }
-  for (int c = tid; c < d; c += kPrepThreads) oEg[c] = expf(sL[(n - 1) * ds + c]);
-  __syncthreads();  // A is whole; q is no longer needed: its rows become the right-hand sides
-
-  // ---- T X = diag(beta) R by forward substitution in place, a thread per column.  R = K * exp L
-  //      (X = W) lies where q was; R = V (X = Uv), d columns at a time, where the logarithms were:
-  //      they are no longer needed once K * exp L is made.
-  float* sXw = sQ;
-  float* sXv = sL;
-  for (int e = tid; e < n * d; e += kPrepThreads) {
-    const int i = e / d, c = e - i * d;
-    sXw[i * ds + c] = sK[i * ds + c] * expf(sL[i * ds + c]);
-  }
-  __syncthreads();
-  for (int v0 = 0; v0 < dv; v0 += d) {
-    const int vw = min(d, dv - v0);
-    for (int e = tid; e < n * vw; e += kPrepThreads) {
-      const int i = e / vw, c = e - i * vw;
-      sXv[i * ds + c] = ldf(gv + static_cast<long long>(t0 + i) * p.ld_v + h * dv + v0 + c);
-    }
-    __syncthreads();
-    const int n_cols = (v0 == 0 ? d : 0) + vw;  // the first pass also solves for W
-    for (int col = tid; col < n_cols; col += kPrepThreads) {
-      const bool is_w = v0 == 0 && col < d;
-      const int c = is_w ? col : col - (v0 == 0 ? d : 0);
-      float* x = (is_w ? sXw : sXv) + c;
-      for (int j = 0; j < n; ++j) {
-        const float* arow = sA + j * (kChunk + 1);
-        float acc0 = 0.f, acc1 = 0.f;
-        int m = 0;
-        for (; m + 1 < j; m += 2) {
-          acc0 += arow[m] * x[m * ds];
-          acc1 += arow[m + 1] * x[(m + 1) * ds];
-        }
-        if (m < j) acc0 += arow[m] * x[m * ds];
-        const float xj = s_beta[j] * (x[j * ds] - (acc0 + acc1));
-        x[j * ds] = xj;
-        if (is_w) oW[j * d + c] = xj;
-        else oUv[j * dv + v0 + c] = xj;
-      }
-    }
     __syncthreads();  // the next pass loads further columns of V over these
   }
-}
-
-// ----------------------------------------------------------------------------------------------
-// Four neighbouring elements of a row in the storage type (`vec`: the row starts on a boundary of four elements).
-template <typename S>
-__device__ __forceinline__ float4 load4(const S* p, bool vec) {
-  if (!vec) return make_float4(ldf(p), ldf(p + 1), ldf(p + 2), ldf(p + 3));
-  return ldf4(p);
 }
 
 // The values of the chunk's tokens as floats (silu of them for kRuleDecay), eight or four bytes at a time where they lie so
@@ -539,167 +693,10 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// A block owns NC (16, or 8 where that is needed to fill the GPU) columns of one head's state for one
-// sequence and walks the sequence's chunks in order.  Thread (column c, row group rg of 256 / NC): rows
-// rg * NC/4 .. of the chunk in the products with S, rows rg * RPT .. + RPT - 1 of S in the state update
-// (d <= RPT * 256 / NC).  The next chunk's
-// operands come by asynchronous copies while this chunk is computed: Q * exp L and W as soon as the
-// products with S are done, B, K * exp(L_end - L) and Uv once the state update has read them.
-template <int NC, int RPT, bool DELTA>
-__global__ void __launch_bounds__(kApplyThreads)
-    chunk_apply_kernel(ChunkArgs p) {
-  constexpr int kRows = kChunk / (kApplyThreads / NC);  // rows of a chunk per thread in the products with S
-  extern __shared__ __align__(16) float sm[];
-  const int d = p.d, dv = p.dv;
-  float* sW = sm;                          // [C][d]   (delta)
-  float* sKe = sW + (DELTA ? kChunk * d : 0);  // [C][d]
-  float* sQg = sKe + kChunk * d;           // [C][d]
-  float* sB = sQg + kChunk * d;            // [C][C]
-  float* sU = sB + kChunk * kChunk;        // [C][NC]
-  float* sS = sU + kChunk * NC;    // [d][NC]
-  float* sEg = sS + d * NC;        // [d]
-  pdl_launch_dependents();
-  pdl_wait();
-  const int seq = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * NC;
-  const int tid = threadIdx.x;
-  const int c = tid % NC, rg = tid / NC;
-  const int first = p.cu[seq], len = p.cu[seq + 1] - first;
-  if (len <= 0) return;
-  int chunk0 = 0;
-  for (int s = 0; s < seq; ++s) chunk0 += (p.cu[s + 1] - p.cu[s] + kChunk - 1) / kChunk;
-  const bool col_ok = j0 + c < dv;
-  const bool tile_async = dv % 4 == 0;
-  const int d4 = d / 4;
-  float* st = p.state + ((static_cast<size_t>(p.slots[seq]) * p.H + h) * d) * dv;
-
-  auto fetch_early = [&](int chunk, int n) {   // operands of the products with S
-    const size_t ch = static_cast<size_t>(chunk) * p.H + h;
-    const float* gQg = p.Qg + ch * kChunk * d;
-    for (int e = tid; e < n * d4; e += kApplyThreads) cp_async16(sQg + 4 * e, gQg + 4 * e);
-    if (DELTA) {
-      const float* gW = p.W + ch * kChunk * d;
-      for (int e = tid; e < n * d4; e += kApplyThreads) cp_async16(sW + 4 * e, gW + 4 * e);
-    }
-    cp_async_commit();
-  };
-  auto fetch_late = [&](int chunk, int n) {    // the rest
-    const size_t ch = static_cast<size_t>(chunk) * p.H + h;
-    const float* gKe = p.Ke + ch * kChunk * d;
-    for (int e = tid; e < n * d4; e += kApplyThreads) cp_async16(sKe + 4 * e, gKe + 4 * e);
-    const float* gB = p.B + ch * kChunk * kChunk;
-    for (int e = tid; e < n * (kChunk / 4); e += kApplyThreads) cp_async16(sB + 4 * e, gB + 4 * e);
-    const float* gU = p.Uv + ch * kChunk * dv;
-    if (tile_async) {
-      for (int e = tid; e < n * (NC / 4); e += kApplyThreads) {
-        const int i = e / (NC / 4), g = e % (NC / 4);
-        if (j0 + 4 * g < dv) cp_async16(sU + i * NC + 4 * g, gU + static_cast<size_t>(i) * dv + j0 + 4 * g);
-        else *reinterpret_cast<float4*>(sU + i * NC + 4 * g) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    } else {
-      for (int e = tid; e < n * NC; e += kApplyThreads) {
-        const int i = e / NC, cc = e % NC;
-        sU[e] = (j0 + cc < dv) ? gU[static_cast<size_t>(i) * dv + j0 + cc] : 0.f;
-      }
-    }
-    for (int e = tid; e < d4; e += kApplyThreads) cp_async16(sEg + 4 * e, p.Eg + ch * d + 4 * e);
-    cp_async_commit();
-  };
-
-  fetch_early(chunk0, min(kChunk, len));
-  fetch_late(chunk0, min(kChunk, len));
-  for (int e = tid; e < d * NC; e += kApplyThreads) {
-    const int r = e / NC, cc = e % NC;
-    sS[e] = (j0 + cc < dv) ? st[static_cast<size_t>(r) * dv + j0 + cc] : 0.f;
-  }
-  int chunk = chunk0;
-  for (int t0 = 0; t0 < len; t0 += kChunk, ++chunk) {
-    const int n = min(kChunk, len - t0);
-    const bool more = t0 + kChunk < len;
-    const int n_next = more ? min(kChunk, len - t0 - kChunk) : 0;
-    cp_async_wait<1>();  // Q * exp L and W of this chunk have landed (the later group may still fly)
-    __syncthreads();     // ... for every thread, and everyone's rows of S are written
-    // ---- rows i = rg * 4 .. + 3 of W S and of the read-out's first term (Q * exp L) S
-    float o[kRows], u[kRows];
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) o[r] = u[r] = 0.f;
-    for (int k4 = 0; k4 < d4; ++k4) {
-      const float s0 = sS[(4 * k4 + 0) * NC + c], s1 = sS[(4 * k4 + 1) * NC + c];
-      const float s2 = sS[(4 * k4 + 2) * NC + c], s3 = sS[(4 * k4 + 3) * NC + c];
-#pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        const int i = rg * kRows + r;
-        if (i < n) {
-          const float4 qv = reinterpret_cast<const float4*>(sQg + i * d)[k4];
-          o[r] += qv.x * s0 + qv.y * s1 + qv.z * s2 + qv.w * s3;
-          if (DELTA) {
-            const float4 wv = reinterpret_cast<const float4*>(sW + i * d)[k4];
-            u[r] += wv.x * s0 + wv.y * s1 + wv.z * s2 + wv.w * s3;
-          }
-        }
-      }
-    }
-    cp_async_wait<0>();  // B, K * exp(L_end - L) and Uv
-    __syncthreads();     // ... for every thread; everyone is done with Q * exp L and W
-    if (more) fetch_early(chunk + 1, n_next);
-    if (DELTA) {
-#pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        const int i = rg * kRows + r;
-        if (i < n) sU[i * NC + c] -= u[r];  // U = Uv - W S
-      }
-      __syncthreads();  // U is whole
-    }
-    // ---- o_i += sum_{j <= i} B_ij u_j, rows out
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      const int i = rg * kRows + r;
-      if (i < n) {
-        float acc = o[r];
-        const float* brow = sB + i * kChunk;
-        for (int j = 0; j <= i; ++j) acc += brow[j] * sU[j * NC + c];
-        if (col_ok) p.out[static_cast<size_t>(first + t0 + i) * (p.H * dv) + h * dv + j0 + c] = acc;
-      }
-    }
-    // ---- S <- diag(exp L_end) S + (K * exp(L_end - L))^T U: rows k = rg * RPT .. + RPT - 1 of column c
-    float acc[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) acc[r] = 0.f;
-    const int k_base = rg * RPT;
-    for (int j = 0; j < n; ++j) {
-      const float uj = sU[j * NC + c];
-      const float* krow = sKe + j * d + k_base;
-#pragma unroll
-      for (int r4 = 0; r4 < RPT / 4; ++r4) {
-        if (k_base + 4 * r4 < d) {
-          const float4 kv = *reinterpret_cast<const float4*>(krow + 4 * r4);
-          acc[4 * r4 + 0] += kv.x * uj;
-          acc[4 * r4 + 1] += kv.y * uj;
-          acc[4 * r4 + 2] += kv.z * uj;
-          acc[4 * r4 + 3] += kv.w * uj;
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int k = k_base + r;
-      if (k < d) sS[k * NC + c] = sEg[k] * sS[k * NC + c] + acc[r];  // own entries only
-    }
-    __syncthreads();  // everyone is done with B, K * exp(L_end - L), U and exp L_end
-    if (more) fetch_late(chunk + 1, n_next);
-    else cp_async_commit();  // keeps the count of groups in flight the same on the last round
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-  for (int e = tid; e < d * NC; e += kApplyThreads) {
-    const int r = e / NC, cc = e % NC;
-    if (j0 + cc < dv) st[static_cast<size_t>(r) * dv + j0 + cc] = sS[e];
-  }
-}
-
 // ----------------------------------------------------------------------------------------------
 // The decayed sum has no product with the state inside its chain: S_end = a^n S_0 + N with
 // N = (K * a^(n-1-j))^T V, so the chain over a sequence's chunks is element-wise.  Three launches after
-// chunk_prepare, all but the middle one parallel over chunks: (1) N of every chunk; (2) a running
+// the operands', all but the middle one parallel over chunks: (1) N of every chunk; (2) a running
 // pass per state element that leaves every chunk's starting state where its N was; (3) the rows
 // o_i = (q_i a^(i+1))^T S_0 + sum_{j<=i} B_ij v_j of every chunk.
 constexpr int kDecayTile = 64;      // state columns per block in (1) and (3)
@@ -891,296 +888,246 @@ __global__ void __launch_bounds__(kDecayThreads)
 }
 
 // ----------------------------------------------------------------------------------------------
-// The delta rule's link from chunk to chunk, S_end = diag(exp L_end) S_0 + Ke^T (Uv - W S_0) with
-// Ke = K * exp(L_end - L), is one product with the state once it is written as
-//   S_end = M S_0 + N,    M = diag(exp L_end) - Ke^T W  [d, d],    N = Ke^T Uv  [d, dv],
-// and M and N do not depend on the state.  Three launches after chunk_prepare: (1) M and N of every
-// chunk in parallel; (2) the chain, a block per (sequence, head, 8 state columns), one product a chunk,
-// the next chunk's M fetched meanwhile, every chunk's starting state left where its N was; (3) the
-// rows o_i = (q_i * exp L_i)^T S_0 + sum_{j<=i} B_ij u_j, U = Uv - W S_0, of every chunk in parallel.
+// The delta rule's link from chunk to chunk:  U = Uv - W S_0,  S_end = diag(exp L_end) S_0 + Ke^T U  with
+// Ke = K * exp(L_end - L).  A block owns 8 columns of one head's state for one sequence and walks the sequence's chunks;
+// U goes where Uv was and every chunk's starting state to N, so that the read-out o_i = (q_i * exp L_i)^T S_0 +
+// sum_{j<=i} B_ij u_j of all chunks at once is the decayed sum's (decay_chunk_output_kernel with U as its values).
+// Both products are made in 4 x 4 tiles with the summed index shared by 8 (4) lanes, two multiply-adds an instruction;
+// the next chunk's W and Ke come by asynchronous copies meanwhile.  Bound by the latency of a link (barriers, reads, sums
+// over lanes) on two warps a scheduler.  Measured at 2,048 tokens and 8 heads of 128 x 128 (32 links): 72 us; with
+// the summed index shared by 16 (8) lanes of 512 threads 95 us, in 2 x 2 (4 x 2) tiles shared by two lanes 99 us.
+// (The form S_end = M S_0 + N with M = diag(exp L_end) - Ke^T W reads as many bytes a link, needs a launch of its own for M
+// and N and leaves W S_0 to the read-out: its three launches took 50, 130 and 74 us behind the operands'.)
 constexpr int kChainCols = 8;
+constexpr int kChainThreads = 256;
 
-// X = Ke^T [-W | Uv]: columns below d go to M (with exp L_end on the diagonal), the others to N
-__global__ void __launch_bounds__(kDecayThreads)
-    delta_chunk_compose_kernel(ChunkArgs p, float* __restrict__ gM_all) {
-  extern __shared__ __align__(16) float sm[];
-  const int d = p.d, dv = p.dv;
-  float* sKe = sm;                    // [C][d]
-  float* sR = sKe + kChunk * d;       // [C][tile]
-  pdl_launch_dependents();
-  pdl_wait();
-  const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kDecayTile;
-  int seq, t0, n;
-  if (!locate_chunk(p.cu, p.n_seq, chunk, &seq, &t0, &n)) return;
-  const int tid = threadIdx.x;
-  const size_t ch = static_cast<size_t>(chunk) * p.H + h;
-  const float* gKe = p.Ke + ch * kChunk * d;
-  const float* gW = p.W + ch * kChunk * d;
-  const float* gUv = p.Uv + ch * kChunk * dv;
-  for (int e = tid; e < n * d; e += kDecayThreads) sKe[e] = gKe[e];
-  for (int e = tid; e < n * kDecayTile; e += kDecayThreads) {
-    const int j = e / kDecayTile, col = c0 + e % kDecayTile;
-    float v = 0.f;
-    if (col < d) v = -gW[static_cast<size_t>(j) * d + col];
-    else if (col < d + dv) v = gUv[static_cast<size_t>(j) * dv + col - d];
-    sR[e] = v;
-  }
-  __syncthreads();
-  float* gM = gM_all + ch * static_cast<size_t>(d) * d;
-  float* gN = p.N + ch * static_cast<size_t>(d) * dv;
-  const int cc = 4 * (tid % 16);
-  for (int k0 = 4 * (tid / 16); k0 < d; k0 += 4 * (kDecayThreads / 16)) {
-    float acc[4][4];
-    product_tn(acc, sKe, d, k0, sR, cc, n);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int k = k0 + r, col = c0 + cc + c;
-        if (col < d) gM[static_cast<size_t>(k) * d + col] = acc[r][c] + (k == col ? p.Eg[ch * d + k] : 0.f);
-        else if (col < d + dv) gN[static_cast<size_t>(k) * dv + col - d] = acc[r][c];
-      }
-    }
-  }
+inline size_t delta_chain_smem(int d, int n_buf) {
+  return sizeof(float) * (static_cast<size_t>(n_buf) * 2 * kChunk * d + static_cast<size_t>(d + 4) * kChainCols + 2 * kChunk * kChainCols);
 }
 
-template <int RPT>  // rows of S per thread: d <= 32 * RPT
-__global__ void __launch_bounds__(kDecayThreads)
-    delta_chunk_chain_kernel(ChunkArgs p, const float* __restrict__ gM_all, int n_buf) {
+// D: the key size where it is known when compiling (the loops unroll and their addresses are constants), 0: p.d.
+template <int D>
+__global__ void __launch_bounds__(kChainThreads)
+    delta_chunk_chain_kernel(ChunkArgs p, int n_buf) {
   extern __shared__ __align__(16) float sm[];
-  const int d = p.d, dv = p.dv;
-  float* sM = sm;                                   // [n_buf][d][d]
-  float* sS = sM + static_cast<size_t>(n_buf) * d * d;  // [d][NC]
+  constexpr int KT = D == 0 ? 2 : 1;      // 4-row tiles of S per thread (128 rows a pass; d <= 244)
+  const int d = D ? D : p.d, dv = p.dv, d4 = d / 4;
+  float* sIn = sm;                                                  // [n_buf][W: C x d | Ke: C x d]
+  float* sS = sIn + static_cast<size_t>(n_buf) * 2 * kChunk * d;    // [8][ss]: the columns of S
+  const int ss = d + 4;                                             // (a stride at which 4 slices of 2 columns fall into different banks)
+  float* sU = sS + kChainCols * ss;                                 // [C][8][2]: every entry twice, as a pair
   pdl_launch_dependents();
   pdl_wait();
   const int seq = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kChainCols;
-  const int tid = threadIdx.x;
-  const int c = tid % kChainCols, kg = tid / kChainCols;  // 32 row groups
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int first = p.cu[seq], len = p.cu[seq + 1] - first;
   if (len <= 0) return;
   int chunk0 = 0;
   for (int s = 0; s < seq; ++s) chunk0 += (p.cu[s + 1] - p.cu[s] + kChunk - 1) / kChunk;
   const int n_chunks = (len + kChunk - 1) / kChunk;
-  const bool col_ok = j0 + c < dv;
-  const int dd4 = d * d / 4, d4 = d / 4;
   float* st = p.state + ((static_cast<size_t>(p.slots[seq]) * p.H + h) * d) * dv;
+  auto unit = [&](int ci) { return static_cast<size_t>(chunk0 + ci) * p.H + h; };
   auto fetch = [&](int ci) {
-    const float* gM = gM_all + (static_cast<size_t>(chunk0 + ci) * p.H + h) * static_cast<size_t>(d) * d;
-    float* dst = sM + static_cast<size_t>(ci % n_buf) * d * d;
-    for (int e = tid; e < dd4; e += kDecayThreads) cp_async16(dst + 4 * e, gM + 4 * e);
+    const float *gW = p.W + unit(ci) * kChunk * d, *gKe = p.Ke + unit(ci) * kChunk * d;
+    float* dst = sIn + static_cast<size_t>(ci % n_buf) * 2 * kChunk * d;
+#pragma unroll 4
+    for (int e = tid; e < kChunk * d4; e += kChainThreads) {
+      cp_async16(dst + 4 * e, gW + 4 * e);
+      cp_async16(dst + kChunk * d + 4 * e, gKe + 4 * e);
+    }
     cp_async_commit();
   };
   fetch(0);
-  for (int e = tid; e < d * kChainCols; e += kDecayThreads) {
-    const int r = e / kChainCols, cc = e % kChainCols;
-    sS[e] = (j0 + cc < dv) ? st[static_cast<size_t>(r) * dv + j0 + cc] : 0.f;
+  // product with W: rows u_row .., columns u_col .., the state's rows 4 m .. with m = slice mod 8; this thread keeps the
+  // sums of row u_at, columns u_c and the next
+  const int u_col = 4 * (lane & 1), u_slice = (lane >> 1) & 7, u_row = 4 * (2 * warp + (lane >> 4));
+  const int u_at = u_row + (u_slice >> 1), u_c = u_col + 2 * (u_slice & 1);
+  // state update: rows 4 s_tile .., columns s_col .., the chunk's rows j = slice mod 4; kept: row s_slice
+  const int s_col = 4 * (warp & 1), s_slice = lane >> 3, s_tile = (warp >> 1) * 8 + (lane & 7);
+  for (int e = tid; e < d * kChainCols; e += kChainThreads) {
+    const int r = e / kChainCols, c = e % kChainCols;
+    sS[c * ss + r] = (j0 + c < dv) ? st[static_cast<size_t>(r) * dv + j0 + c] : 0.f;
   }
+  float uv[2] = {0.f, 0.f}, eg[KT];
+  const bool col0 = j0 + u_c < dv, col1 = j0 + u_c + 1 < dv;
+  auto read_ahead = [&](int ci) {   // the small operands of a chunk, a link ahead of their use
+    const float* gU = p.Uv + unit(ci) * kChunk * dv + static_cast<size_t>(u_at) * dv + j0 + u_c;
+    if (col0) uv[0] = gU[0];
+    if (col1) uv[1] = gU[1];
+#pragma unroll
+    for (int t = 0; t < KT; ++t) {
+      const int k = 4 * (s_tile + 32 * t) + s_slice;
+      eg[t] = k < d ? p.Eg[unit(ci) * d + k] : 0.f;
+    }
+  };
+  read_ahead(0);
   for (int ci = 0; ci < n_chunks; ++ci) {
-    if (n_buf > 1 && ci + 1 < n_chunks) {
-      fetch(ci + 1);        // into the other buffer, whose product ended before the barrier below
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();        // M of this chunk and everyone's rows of S are there
-    const float* M = sM + static_cast<size_t>(ci % n_buf) * d * d;
-    float* gN = p.N + (static_cast<size_t>(chunk0 + ci) * p.H + h) * static_cast<size_t>(d) * dv;
-    float acc[RPT], nv[RPT];
+    cp_async_wait<0>();
+    __syncthreads();        // W and Ke of this chunk and everyone's rows of S are there; everyone is done with the chunk before
+    if (n_buf > 1 && ci + 1 < n_chunks) fetch(ci + 1);
+    const float* W = sIn + static_cast<size_t>(ci % n_buf) * 2 * kChunk * d;
+    const float* Ke = W + kChunk * d;
+    {
+      Pair acc[4][4];
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) {  // N comes from global memory while the product runs
-      const int k = kg + 32 * r;
-      nv[r] = (k < d && col_ok) ? gN[static_cast<size_t>(k) * dv + j0 + c] : 0.f;
-      acc[r] = 0.f;
-    }
-    for (int q4 = 0; q4 < d4; ++q4) {
-      const float s0 = sS[(4 * q4 + 0) * kChainCols + c], s1 = sS[(4 * q4 + 1) * kChainCols + c];
-      const float s2 = sS[(4 * q4 + 2) * kChainCols + c], s3 = sS[(4 * q4 + 3) * kChainCols + c];
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) {
-        const int k = kg + 32 * r;
-        if (k < d) {
-          const float4 m = reinterpret_cast<const float4*>(M + static_cast<size_t>(k) * d)[q4];
-          acc[r] += m.x * s0 + m.y * s1 + m.z * s2 + m.w * s3;
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0;
+#pragma unroll 4
+      for (int m = u_slice; m < d4; m += 8) {
+        Quad w[4], s[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) w[r] = quad(W + (u_row + r) * d + 4 * m);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[c] = quad(sS + (u_col + c) * ss + 4 * m);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[r][c] = fma2(w[r].lo, s[c].lo, acc[r][c]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[r][c] = fma2(w[r].hi, s[c].hi, acc[r][c]);
+      }
+      float v[4][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 two = halves(acc[r][c]);
+          v[r][c] = two.x + two.y;
+        }
+      // summed over the 8 slices (lane bits 1 to 3); a lane keeps row slice >> 1, columns 2 (slice & 1) and the next
+      float x[8], y[4], z[2];
+      const bool b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        x[e] = (b3 ? v[2 + e / 4][e % 4] : v[e / 4][e % 4]) + __shfl_xor_sync(0xffffffffu, b3 ? v[e / 4][e % 4] : v[2 + e / 4][e % 4], 8);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = (b2 ? x[4 + e] : x[e]) + __shfl_xor_sync(0xffffffffu, b2 ? x[e] : x[4 + e], 4);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) z[e] = (b1 ? y[2 + e] : y[e]) + __shfl_xor_sync(0xffffffffu, b1 ? y[e] : y[2 + e], 2);
+      const float u0 = uv[0] - z[0], u1 = uv[1] - z[1];
+      *reinterpret_cast<float4*>(sU + 2 * (u_at * kChainCols + u_c)) = make_float4(u0, u0, u1, u1);
+      float* gU = p.Uv + unit(ci) * kChunk * dv + static_cast<size_t>(u_at) * dv + j0 + u_c;
+      if (col0) gU[0] = u0;
+      if (col1) gU[1] = u1;
+    }
+    float eg_now[KT];
+#pragma unroll
+    for (int t = 0; t < KT; ++t) eg_now[t] = eg[t];
+    __syncthreads();        // U is whole; everyone has read S
+    if (ci + 1 < n_chunks) read_ahead(ci + 1);
+    float* gN = p.N + unit(ci) * static_cast<size_t>(d) * dv;
+#pragma unroll
+    for (int t = 0; t < KT; ++t) {
+      const int m = s_tile + 32 * t;
+      const bool mine = D == 128 || m < d4;
+      Pair acc[2][4];   // rows 4 m, 4 m + 1 and 4 m + 2, 4 m + 3
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[0][c] = acc[1][c] = 0;
+      if (mine) {
+#pragma unroll 8
+        for (int j = s_slice; j < kChunk; j += 4) {
+          const Quad k = quad(Ke + j * d + 4 * m);
+          const float* u = sU + 2 * (j * kChainCols + s_col);
+          const Quad u01 = quad(u), u23 = quad(u + 4);
+          const Pair uu[4] = {u01.lo, u01.hi, u23.lo, u23.hi};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            acc[0][c] = fma2(k.lo, uu[c], acc[0][c]);
+            acc[1][c] = fma2(k.hi, uu[c], acc[1][c]);
+          }
+        }
+      }
+      float v[4][4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float2 top = halves(acc[0][c]), low = halves(acc[1][c]);
+        v[0][c] = top.x;
+        v[1][c] = top.y;
+        v[2][c] = low.x;
+        v[3][c] = low.y;
+      }
+      // summed over the 4 slices (lane bits 3 and 4); a lane keeps row 4 m + slice
+      float x[8], y[4];
+      const bool b4 = lane & 16, b3 = lane & 8;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        x[e] = (b4 ? v[2 + e / 4][e % 4] : v[e / 4][e % 4]) + __shfl_xor_sync(0xffffffffu, b4 ? v[e / 4][e % 4] : v[2 + e / 4][e % 4], 16);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = (b3 ? x[4 + e] : x[e]) + __shfl_xor_sync(0xffffffffu, b3 ? x[e] : x[4 + e], 8);
+      if (mine) {
+        float* at = sS + s_col * ss + 4 * m + s_slice;
+        const float4 old = make_float4(at[0], at[ss], at[2 * ss], at[3 * ss]);
+        at[0] = eg_now[t] * old.x + y[0];
+        at[ss] = eg_now[t] * old.y + y[1];
+        at[2 * ss] = eg_now[t] * old.z + y[2];
+        at[3 * ss] = eg_now[t] * old.w + y[3];
+        float* to = gN + static_cast<size_t>(4 * m + s_slice) * dv + j0 + s_col;  // the chunk's starting state
+        if (dv % 4 == 0) {
+          if (j0 + s_col < dv) *reinterpret_cast<float4*>(to) = old;
+        } else {
+          const float o[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (j0 + s_col + c < dv) to[c] = o[c];
         }
       }
     }
-    __syncthreads();        // everyone has read S (and this chunk's M)
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int k = kg + 32 * r;
-      if (k < d) {
-        if (col_ok) gN[static_cast<size_t>(k) * dv + j0 + c] = sS[k * kChainCols + c];  // the chunk's starting state
-        sS[k * kChainCols + c] = acc[r] + nv[r];
-      }
+    if (n_buf == 1 && ci + 1 < n_chunks) {
+      __syncthreads();      // everyone is done with the one buffer
+      fetch(ci + 1);
     }
-    if (n_buf == 1 && ci + 1 < n_chunks) fetch(ci + 1);
   }
   __syncthreads();
-  for (int e = tid; e < d * kChainCols; e += kDecayThreads) {
-    const int r = e / kChainCols, cc = e % kChainCols;
-    if (j0 + cc < dv) st[static_cast<size_t>(r) * dv + j0 + cc] = sS[e];
+  for (int e = tid; e < d * kChainCols; e += kChainThreads) {
+    const int r = e / kChainCols, c = e % kChainCols;
+    if (j0 + c < dv) st[static_cast<size_t>(r) * dv + j0 + c] = sS[c * ss + r];
   }
 }
 
-__global__ void __launch_bounds__(kDecayThreads)
-    delta_chunk_output_kernel(ChunkArgs p) {
-  extern __shared__ __align__(16) float sm[];
-  const int d = p.d, dv = p.dv;
-  float* sQg = sm;                          // [C][d]
-  float* sW = sQg + kChunk * d;             // [C][d]
-  float* sB = sW + kChunk * d;              // [C][C]
-  float* sS = sB + kChunk * kChunk;         // [d][tile]
-  float* sU = sS + d * kDecayTile;          // [C][tile]
-  pdl_launch_dependents();
-  pdl_wait();
-  const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kDecayTile;
-  int seq, t0, n;
-  if (!locate_chunk(p.cu, p.n_seq, chunk, &seq, &t0, &n)) return;
-  const int tid = threadIdx.x;
-  const size_t ch = static_cast<size_t>(chunk) * p.H + h;
-  const float* gQg = p.Qg + ch * kChunk * d;
-  const float* gW = p.W + ch * kChunk * d;
-  const float* gB = p.B + ch * kChunk * kChunk;
-  const float* gS = p.N + ch * static_cast<size_t>(d) * dv;
-  const float* gUv = p.Uv + ch * kChunk * dv;
-  const int d4 = d / 4;
-  for (int e = tid; e < n * d4; e += kDecayThreads) {
-    reinterpret_cast<float4*>(sQg)[e] = reinterpret_cast<const float4*>(gQg)[e];
-    reinterpret_cast<float4*>(sW)[e] = reinterpret_cast<const float4*>(gW)[e];
-  }
-  for (int e = tid; e < n * kChunk; e += kDecayThreads) sB[e] = gB[e];
-  for (int e = tid; e < d * kDecayTile; e += kDecayThreads) {
-    const int k = e / kDecayTile, c = e % kDecayTile;
-    sS[e] = (c0 + c < dv) ? gS[static_cast<size_t>(k) * dv + c0 + c] : 0.f;
-  }
-  for (int e = tid; e < n * kDecayTile; e += kDecayThreads) {
-    const int j = e / kDecayTile, c = e % kDecayTile;
-    sU[e] = (c0 + c < dv) ? gUv[static_cast<size_t>(j) * dv + c0 + c] : 0.f;
-  }
-  __syncthreads();
-  // thread: rows i0 .. i0 + 3, columns cc .. cc + 3
-  const int cc = 4 * (tid % 16), i0 = 4 * (tid / 16);
-  float o[4][4], u[4][4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) o[r][c] = u[r][c] = 0.f;
-  if (i0 < n) {
-    product_nn(o, sQg, d, i0, sS, cc, d, false);
-    product_nn(u, sW, d, i0, sS, cc, d, false);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) sU[(i0 + r) * kDecayTile + cc + c] -= u[r][c];  // U = Uv - W S_0 (own entries)
-  }
-  __syncthreads();
-  if (i0 < n) {
-    product_nn(o, sB, kChunk, i0, sU, cc, i0 + 4, true);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (i0 + r < n && c0 + cc + c < dv)
-          p.out[static_cast<size_t>(t0 + i0 + r) * (p.H * dv) + h * dv + c0 + cc + c] = o[r][c];
-  }
-}
+// Largest key sizes: what the blocks that hold a chunk's operands take of shared memory (200 KB and more).
+inline int largest_key(int rule) { return rule == kRuleDelta ? 244 : rule == kRuleWkv ? 280 : 352; }
 
-inline size_t prepare_smem(int d, int rule, bool sub_blocks = false) {
-  if (rule == kRuleWkv) return wkv_prepare_smem(d);
-  if (rule != kRuleDelta) return decay_prepare_smem(d);
-  return sizeof(float) * (static_cast<size_t>(kChunk) * (d + 1) * 3 + kChunk * (kChunk + 1) +
-                          (sub_blocks ? static_cast<size_t>(48 + 32) * (d + 1) : 0));
-}
-inline size_t apply_smem(int d, bool delta, int nc = 16) {
-  return sizeof(float) * (static_cast<size_t>(kChunk) * d * (delta ? 3 : 2) + kChunk * kChunk + kChunk * nc +
-                          static_cast<size_t>(d) * nc + d);
+inline size_t prepare_smem(int d, int rule) {
+  return rule == kRuleWkv ? wkv_prepare_smem(d) : rule == kRuleDelta ? delta_prepare_smem(d) : decay_prepare_smem(d);
 }
 
 template <typename S, int RULE>
 int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   constexpr bool DELTA = RULE == kRuleDelta;
-  a.sub_blocks = DELTA && prepare_smem(a.d, RULE, true) <= 220 * 1024;
-  const size_t sp = prepare_smem(a.d, RULE, a.sub_blocks != 0);
+  const int d = a.d, tiles = (a.dv + kDecayTile - 1) / kDecayTile;
+  if (tiles > 65535) return PMM_ERR_BAD_ARGUMENT;
   void (*prep)(ChunkArgs) = nullptr;
   if constexpr (RULE == kRuleWkv) prep = wkv_prepare_kernel<S>;
-  else if constexpr (DELTA) prep = chunk_prepare_kernel<S>;
+  else if constexpr (DELTA) prep = delta_prepare_kernel<S>;
   else prep = decay_prepare_kernel<S, RULE>;
   const size_t unit = 4 * sizeof(S);
   auto whole = [&](const void* ptr, long long ld) { return reinterpret_cast<uintptr_t>(ptr) % unit == 0 && ld % 4 == 0; };
-  a.vec_in = whole(a.q, a.ld_q) && whole(a.k, a.ld_k) && whole(a.v, a.ld_v) &&
+  a.vec_in = whole(a.q, a.ld_q) && whole(a.k, a.ld_k) && whole(a.v, a.ld_v) && (!DELTA || whole(a.a, a.ld_a)) &&
              (RULE != kRuleWkv || (reinterpret_cast<uintptr_t>(a.a) % 16 == 0 && a.ld_a % 4 == 0 && reinterpret_cast<uintptr_t>(a.dt_bias) % 16 == 0));
-  if (sp > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sp));
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  auto allow = [](auto kernel, size_t bytes) {
+    return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  };
+  const size_t sp = prepare_smem(d, RULE), s1 = sizeof(float) * kChunk * (static_cast<size_t>(d) + kDecayTile);
+  const size_t s3 = sizeof(float) * (static_cast<size_t>(kChunk) * d + static_cast<size_t>(d) * kDecayTile + kChunk * kDecayTile);
+  const int n_buf = delta_chain_smem(d, 2) <= 200 * 1024 ? 2 : 1;
+  const size_t s2 = delta_chain_smem(d, n_buf);
+  auto chain = d == 128 ? delta_chunk_chain_kernel<128> : d == 64 ? delta_chunk_chain_kernel<64> : delta_chunk_chain_kernel<0>;
+  cudaError_t e = allow(prep, sp);
+  if (e == cudaSuccess) e = DELTA ? allow(chain, s2) : allow(decay_chunk_state_kernel, s1);
+  if (e == cudaSuccess) e = allow(decay_chunk_output_kernel, s3);
+  if (e != cudaSuccess) return static_cast<int>(e);
   launch_pdl(prep, dim3(n_chunks, a.H), dim3(DELTA ? kPrepThreads : RULE == kRuleWkv ? kWkvThreads : kDecayPrepThreads), sp, stream, a);
   if (DELTA) {
-    const int d = a.d;
-    const int tiles_c = (d + a.dv + kDecayTile - 1) / kDecayTile, tiles_o = (a.dv + kDecayTile - 1) / kDecayTile;
-    const size_t s1 = sizeof(float) * kChunk * (static_cast<size_t>(d) + kDecayTile);
-    const size_t m_bytes = sizeof(float) * static_cast<size_t>(d) * d, s_bytes = sizeof(float) * d * kChainCols;
-    const int n_buf = 2 * m_bytes + s_bytes <= 200 * 1024 ? 2 : 1;
-    const size_t s2 = n_buf * m_bytes + s_bytes;
-    const size_t s3 = sizeof(float) * (2 * static_cast<size_t>(kChunk) * d + kChunk * kChunk +
-                                       static_cast<size_t>(d) * kDecayTile + kChunk * kDecayTile);
-    if (s2 <= 200 * 1024 && s3 <= 200 * 1024) {
-      auto chain = d <= 64 ? delta_chunk_chain_kernel<2> : d <= 128 ? delta_chunk_chain_kernel<4> : delta_chunk_chain_kernel<8>;
-      cudaError_t e = cudaSuccess;
-      if (s1 > 48 * 1024) e = cudaFuncSetAttribute(delta_chunk_compose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(s1));
-      if (e == cudaSuccess && s2 > 48 * 1024) e = cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(s2));
-      if (e == cudaSuccess && s3 > 48 * 1024) e = cudaFuncSetAttribute(delta_chunk_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(s3));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      launch_pdl(delta_chunk_compose_kernel, dim3(n_chunks, a.H, tiles_c), dim3(kDecayThreads), s1, stream, a, a.M);
-      launch_pdl(chain, dim3((a.dv + kChainCols - 1) / kChainCols, a.H, a.n_seq), dim3(kDecayThreads), s2, stream, a,
-                 static_cast<const float*>(a.M), n_buf);
-      launch_pdl(delta_chunk_output_kernel, dim3(n_chunks, a.H, tiles_o), dim3(kDecayThreads), s3, stream, a);
-      return launch_status();
-    }
-  }
-  if (!DELTA) {
-    const int tiles = (a.dv + kDecayTile - 1) / kDecayTile;
-    const size_t s1 = sizeof(float) * kChunk * (static_cast<size_t>(a.d) + kDecayTile);
-    const size_t s3 = sizeof(float) * (static_cast<size_t>(kChunk) * a.d + static_cast<size_t>(a.d) * kDecayTile + kChunk * kDecayTile);
-    if (s3 <= 200 * 1024 && tiles <= 65535) {
-      for (auto pair : {std::make_pair(decay_chunk_state_kernel, s1), std::make_pair(decay_chunk_output_kernel, s3)}) {
-        if (pair.second > 48 * 1024) {
-          cudaError_t e = cudaFuncSetAttribute(pair.first, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(pair.second));
-          if (e != cudaSuccess) return static_cast<int>(e);
-        }
-      }
-      launch_pdl(decay_chunk_state_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s1, stream, a);
-      launch_pdl(decay_chunk_scan_kernel, dim3((a.d * a.dv + kDecayThreads - 1) / kDecayThreads, a.H, a.n_seq),
-                 dim3(kDecayThreads), 0, stream, a);
-      launch_pdl(decay_chunk_output_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s3, stream, a);
-      return launch_status();
-    }
-  }
-  // 16 state columns a block; 8 where 16 would leave most of the GPU without a block
-  const bool narrow = static_cast<long long>((a.dv + 15) / 16) * a.H * a.n_seq < 100;
-  const int nc = narrow ? 8 : 16;
-  const size_t sa = apply_smem(a.d, DELTA, nc);
-  dim3 grid((a.dv + nc - 1) / nc, a.H, a.n_seq);
-#define PMM_APPLY_CASE(NC, RPT)                                                                               \
-  do {                                                                                                        \
-    auto kern = chunk_apply_kernel<NC, RPT, DELTA>;                                                           \
-    if (sa > 48 * 1024) {                                                                                     \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,                 \
-                                           static_cast<int>(sa));                                             \
-      if (e != cudaSuccess) return static_cast<int>(e);                                                       \
-    }                                                                                                         \
-    launch_pdl(kern, grid, dim3(kApplyThreads), sa, stream, a);                                               \
-  } while (0)
-  if (narrow) {
-    if (a.d <= 128) PMM_APPLY_CASE(8, 4);
-    else PMM_APPLY_CASE(8, 8);
+    launch_pdl(chain, dim3((a.dv + kChainCols - 1) / kChainCols, a.H, a.n_seq), dim3(kChainThreads), s2, stream, a, n_buf);
   } else {
-    if (a.d <= 64) PMM_APPLY_CASE(16, 4);
-    else if (a.d <= 128) PMM_APPLY_CASE(16, 8);
-    else if (a.d <= 192) PMM_APPLY_CASE(16, 12);
-    else PMM_APPLY_CASE(16, 16);
+    launch_pdl(decay_chunk_state_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s1, stream, a);
+    launch_pdl(decay_chunk_scan_kernel, dim3((d * a.dv + kDecayThreads - 1) / kDecayThreads, a.H, a.n_seq),
+               dim3(kDecayThreads), 0, stream, a);
   }
-#undef PMM_APPLY_CASE
+  launch_pdl(decay_chunk_output_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s3, stream, a);
   return launch_status();
 }
 
@@ -1190,16 +1137,13 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
 // shared memory).
 // rule: kRuleDecay .. kRuleWkv (0: the decayed sum, 1: the delta rule, 2: retention, 3: time mixing).
 PMM_EXPORT int pmm_recurrent_chunked_supported(int d, int rule) {
-  if (d <= 0 || d % 4) return 0;
-  const bool delta = rule == pmm::kRuleDelta;
-  return pmm::prepare_smem(d, rule) <= 220 * 1024 && pmm::apply_smem(d, delta) <= 220 * 1024 ? 1 : 0;
+  return d > 0 && d % 4 == 0 && d <= pmm::largest_key(rule) ? 1 : 0;
 }
 
 // Floats of scratch per (chunk, head).
 PMM_EXPORT long long pmm_recurrent_chunked_scratch(int d, int dv, int rule) {
-  const bool delta = rule == pmm::kRuleDelta;
-  // Ke, Qg, Uv, B, Eg; N (then every chunk's starting state); for the delta rule also W and M
-  const long long w = delta ? static_cast<long long>(pmm::kChunk) * d + static_cast<long long>(d) * d : 0;
+  // Ke, Qg, Uv, B, Eg; N (then every chunk's starting state); for the delta rule also W
+  const long long w = rule == pmm::kRuleDelta ? static_cast<long long>(pmm::kChunk) * d : 0;
   return static_cast<long long>(pmm::kChunk) * (2 * d + dv + pmm::kChunk) + static_cast<long long>(d) * dv + w + d;
 }
 
@@ -1214,7 +1158,6 @@ inline void place_scratch(ChunkArgs& p, float* s, size_t ch, bool delta) {
   p.N = s; s += ch * static_cast<size_t>(d) * dv;
   if (delta) {
     p.W = s; s += ch * kChunk * d;
-    p.M = s; s += ch * static_cast<size_t>(d) * d;
   }
   p.Uv = s; s += ch * kChunk * dv;
   p.Eg = s;

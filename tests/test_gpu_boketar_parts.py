@@ -199,6 +199,35 @@ def test_gated_delta_rule_in_chunks(dtype, H, G, d, dv):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d,dv,shift", [(64, 64, 0), (64, 61, 1), (128, 8, 0), (128, 130, 3), (244, 17, 2), (4, 4, 0)])
+def test_gated_delta_rule_in_chunks_of_views(dtype, d, dv, shift):
+    """Every form of the chunked delta rule (key sizes known when compiling and others, one and two buffers in the chain,
+    rows on and off boundaries of four elements, value columns that are no whole tile, more values than keys) on both sides
+    of a chunk's edge against the token-serial kernel.  Tolerance: float sums of up to 130 tokens and 244 channels in another
+    order, relative to the largest entry."""
+    H, G = 2, 1
+    for n in (1, 2, 7, 8, 9, 64, 129):
+        width = 2 * G * d + H * dv + H * d + H
+        rows = (rnd(n, width + 8, seed=n) * torch.linspace(0.5, 2.0, n)[:, None]).to(DEV, dtype)[:, shift:shift + width]
+        q, k, v, a, beta = rows.split([G * d, G * d, H * dv, H * d, H], dim=1)
+        dt_bias, a_log = (rnd(H * d, seed=6) * 4.0 - 1.0).to(DEV), (rnd(H, seed=7) + 1.0).to(DEV)
+        got = {}
+        for kind in ("chunked", "serial"):
+            state = (rnd(2, H, d, dv, seed=8) * 0.1).to(DEV)
+            out = torch.empty(n, H * dv, device=DEV)
+            cu, _, sl = batch_index([n], [1])
+            if kind == "chunked":
+                scratch = torch.full((K.recurrent_chunked_scratch_floats([n], H, d, dv, True),), float("nan"), device=DEV)
+                K.recurrent_chunked(q, k, v, state, cu, sl, [n], out, scratch, H, G, d, dv, beta=beta, a=a, dt_bias=dt_bias,
+                                    a_log=a_log, unit_eps=1e-6, q_scale=d ** -0.5)
+            else:
+                K.delta_scan(q, k, v, beta, a, dt_bias, a_log, state, cu, sl, 1, out, H, G, d, dv, 1e-6, d ** -0.5)
+            got[kind] = (out, state)
+        for x, y in zip(got["chunked"], got["serial"]):
+            assert float((x - y).abs().max()) <= 2e-5 * max(1.0, float(y.abs().max())), (n, float((x - y).abs().max()))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,d,dv", [(2, 16, 24), (4, 32, 32), (1, 100, 7), (3, 4, 130)])
 def test_decayed_linear_attention_in_chunks(dtype, H, d, dv):
     T = 600
