@@ -14,16 +14,39 @@
 // last tile leaves.  A row's result does not depend on which other rows share its tile.
 #include "common.cuh"
 #include "mma_helpers.cuh"
+#include "moe_tile.cuh"
 
 namespace pmm {
 
-// A block routes TOK tokens: their rows wait in shared memory as floats, every warp takes the experts
-// e = warp, warp + 8, ... and reads a router row once (16 bytes a lane and access) for all TOK dot
+// A block routes TOK tokens: their rows wait in shared memory as floats, every warp takes one expert (one token) or two
+// (several tokens) at a time and reads a router row once (16 bytes a lane and access) for all TOK dot
 // products; then a warp per token picks the `top` largest logits and norms their exponentials.
-constexpr int kRouteWarps = 8;
+// A chain of reads and reductions, bound by their latency: a warp's first router rows are read before the wait for the
+// kernel before this one (they are weights), and up to 32 experts are ranked by one lane each against all others at once
+// (`ranked`) where picking them one after the other takes ten exchanges between lanes apiece.  16 experts, 4 chosen in 2
+// of 4 groups, width 1,024, inside a step: 8 tokens 11 -> 4.5 us.
+constexpr int kRouteAhead = 8;   // sixteen-byte pieces of a router row a lane holds before the wait (128 columns each)
+template <int TOK>
+struct RouteShape {
+  static constexpr int kPer = TOK == 1 ? 1 : 2;      // experts a warp makes at a time: several tokens' rows are read once for both
+  static constexpr int kWarps = TOK == 1 ? 16 : 8;
+};
+
+// This lane's place (0: the largest; the lower index wins a tie) among values v[0 .. n - 1], n <= 32, none of them NaN.
+__device__ __forceinline__ int ranked(const float* v, int n, int lane) {
+  const float mine = lane < n ? v[lane] : -INFINITY;
+  int rank = 0;
+#pragma unroll 8
+  for (int e = 0; e < n; ++e) rank += (v[e] > mine || (v[e] == mine && e < lane)) ? 1 : 0;
+  return rank;
+}
+// Whether one lane an expert can rank them: the picks of a row with NaN or infinite entries are left to the serial form.
+__device__ __forceinline__ bool all_finite(const float* v, int n, int lane) {
+  return n <= 32 && __all_sync(0xffffffffu, lane >= n || fabsf(v[lane]) < INFINITY);
+}
 
 template <typename S, int TOK>
-__global__ void __launch_bounds__(kRouteWarps * 32)
+__global__ void __launch_bounds__(RouteShape<TOK>::kWarps * 32)
     moe_route_kernel(const S* __restrict__ x, long long ld_x, const float* __restrict__ w,
                      const float* __restrict__ bias, int* __restrict__ ids, float* __restrict__ weights, int T, int D,
                      int E, int top, int scored, const float* __restrict__ correction, int groups, int keep,
@@ -33,45 +56,95 @@ __global__ void __launch_bounds__(kRouteWarps * 32)
   float* rows = route_smem;
   float* logits = route_smem + TOK * Dpad;
   pdl_launch_dependents();
-  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t0 = blockIdx.x * TOK;
   const int nt = min(TOK, T - t0);
-  for (int r = 0; r < TOK; ++r)
-    for (int i = threadIdx.x; i < Dpad; i += blockDim.x)
-      rows[r * Dpad + i] = (r < nt && i < D) ? ldf(x + static_cast<long long>(t0 + r) * ld_x + i) : 0.f;
-  __syncthreads();
   const bool vec = (D & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(gate_w) & 15) == 0;
   // (gate_w: one more row, whose product goes through a sigmoid into gate_out[t]: a gate per token that reads the
   // router's input, such as a shared expert's)
   const int n_rows = E + (gate_w ? 1 : 0);
-  for (int e = warp; e < n_rows; e += kRouteWarps) {
-    float acc[TOK];
+  constexpr int kPer = RouteShape<TOK>::kPer, kRouteWarps = RouteShape<TOK>::kWarps;
+  auto router_row = [&](int e) { return e < E ? w + static_cast<size_t>(e) * D : gate_w; };
+  float4 ahead[kPer][kRouteAhead];
+  if (vec) {
 #pragma unroll
-    for (int r = 0; r < TOK; ++r) acc[r] = 0.f;
-    const float* wr = e < E ? w + static_cast<size_t>(e) * D : gate_w;
+    for (int q = 0; q < kPer; ++q)
+#pragma unroll
+      for (int k = 0; k < kRouteAhead; ++k)
+        if (warp * kPer + q < n_rows && lane * 4 + 128 * k < D)
+          ahead[q][k] = *reinterpret_cast<const float4*>(router_row(warp * kPer + q) + lane * 4 + 128 * k);
+  }
+  pdl_wait();
+  if ((D & 3) == 0 && ld_x % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (4 * sizeof(S)) == 0) {
+    const int D4 = D / 4;
+    for (int i = threadIdx.x; i < TOK * D4; i += blockDim.x) {
+      const int r = i / D4, c = 4 * (i - r * D4);
+      *reinterpret_cast<float4*>(rows + r * Dpad + c) =
+          r < nt ? ldf4(x + static_cast<long long>(t0 + r) * ld_x + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
+    for (int r = 0; r < TOK; ++r)
+      for (int i = threadIdx.x; i < Dpad; i += blockDim.x)
+        rows[r * Dpad + i] = (r < nt && i < D) ? ldf(x + static_cast<long long>(t0 + r) * ld_x + i) : 0.f;
+  }
+  __syncthreads();
+  for (int e0 = warp * kPer; e0 < n_rows; e0 += kRouteWarps * kPer) {
+    const int n_here = min(kPer, n_rows - e0);
+    float acc[kPer][TOK];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+#pragma unroll
+      for (int r = 0; r < TOK; ++r) acc[q][r] = 0.f;
     if (vec) {
-      for (int i = lane * 4; i < D; i += 128) {
-        const float4 wv = *reinterpret_cast<const float4*>(wr + i);
+      auto piece = [&](int i, const float4 (&wv)[kPer]) {
 #pragma unroll
         for (int r = 0; r < TOK; ++r) {
           const float4 xv = *reinterpret_cast<const float4*>(rows + r * Dpad + i);
-          acc[r] += xv.x * wv.x + xv.y * wv.y + xv.z * wv.z + xv.w * wv.w;
+#pragma unroll
+          for (int q = 0; q < kPer; ++q) acc[q][r] += xv.x * wv[q].x + xv.y * wv[q].y + xv.z * wv[q].z + xv.w * wv[q].w;
         }
+      };
+      int done = lane * 4;
+      if (e0 == warp * kPer) {
+#pragma unroll
+        for (int k = 0; k < kRouteAhead; ++k)
+          if (lane * 4 + 128 * k < D) {
+            float4 wv[kPer];
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) wv[q] = q < n_here ? ahead[q][k] : make_float4(0.f, 0.f, 0.f, 0.f);
+            piece(lane * 4 + 128 * k, wv);
+          }
+        done += 128 * kRouteAhead;
+      }
+#pragma unroll 4
+      for (int i = done; i < D; i += 128) {
+        float4 wv[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+          wv[q] = q < n_here ? *reinterpret_cast<const float4*>(router_row(e0 + q) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        piece(i, wv);
       }
     } else {
       for (int i = lane; i < D; i += 32) {
-        const float wv = wr[i];
 #pragma unroll
-        for (int r = 0; r < TOK; ++r) acc[r] += rows[r * Dpad + i] * wv;
+        for (int q = 0; q < kPer; ++q) {
+          const float wv = q < n_here ? router_row(e0 + q)[i] : 0.f;
+#pragma unroll
+          for (int r = 0; r < TOK; ++r) acc[q][r] += rows[r * Dpad + i] * wv;
+        }
       }
     }
 #pragma unroll
-    for (int r = 0; r < TOK; ++r) {
-      const float sum = warp_sum(acc[r]);
-      if (lane == 0) {
-        if (e < E) logits[r * E + e] = sum + (bias ? bias[e] : 0.f);
-        else if (r < nt) gate_out[t0 + r] = 1.f / (1.f + expf(-sum));
+    for (int q = 0; q < kPer; ++q) {
+      const int e = e0 + q;
+      if (q >= n_here) break;
+#pragma unroll
+      for (int r = 0; r < TOK; ++r) {
+        const float sum = warp_sum(acc[q][r]);
+        if (lane == 0) {
+          if (e < E) logits[r * E + e] = sum + (bias ? bias[e] : 0.f);
+          else if (r < nt) gate_out[t0 + r] = 1.f / (1.f + expf(-sum));
+        }
       }
     }
   }
@@ -112,6 +185,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32)
         }
       }
       __syncwarp();
+      const bool at_once = all_finite(z, E, lane);
       if (groups > 1) {
         const int per = E / groups;
         for (int g = lane; g < groups; g += 32) {
@@ -124,7 +198,14 @@ __global__ void __launch_bounds__(kRouteWarps * 32)
         }
         __syncwarp();
         // the `keep` best groups are marked by +inf in gs; then the others' experts drop out
-        for (int j = 0; j < keep; ++j) {
+        const bool groups_at_once = at_once && all_finite(gs, groups, lane);
+        if (groups_at_once) {
+          const bool kept = ranked(gs, groups, lane) < keep;
+          __syncwarp();
+          if (lane < groups && kept) gs[lane] = INFINITY;
+          __syncwarp();
+        }
+        for (int j = groups_at_once ? keep : 0; j < keep; ++j) {
           float best = -INFINITY;
           int arg = 0x7fffffff;
           for (int g = lane; g < groups; g += 32) {
@@ -143,6 +224,21 @@ __global__ void __launch_bounds__(kRouteWarps * 32)
         for (int e = lane; e < E; e += 32)
           if (gs[e / per] != INFINITY) z[e] = -INFINITY;
         __syncwarp();
+      }
+      if (at_once) {
+        const int place = ranked(z, E, lane);
+        const bool chosen = lane < E && place < top;
+        __syncwarp();
+        if (chosen) z[place] = sc[lane];  // the chosen scores in their order
+        __syncwarp();
+        float denom = 0.f;
+        for (int j = 0; j < top; ++j) denom += z[j];
+        const float inv = scored >= 2 ? scale : scale / (denom + 1e-20f);
+        if (chosen) {
+          ids[static_cast<size_t>(t0 + r) * top + place] = lane;
+          weights[static_cast<size_t>(t0 + r) * top + place] = sc[lane] * inv;
+        }
+        continue;
       }
       float denom = 0.f;
       for (int j = 0; j < top; ++j) {
@@ -175,6 +271,24 @@ __global__ void __launch_bounds__(kRouteWarps * 32)
   }
   for (int r = warp; r < nt; r += kRouteWarps) {
     float* z = logits + r * E;
+    if (all_finite(z, E, lane)) {
+      const int place = ranked(z, E, lane);
+      const float mine = lane < E ? z[lane] : -INFINITY;
+      const unsigned top_lane = __ballot_sync(0xffffffffu, lane < E && place == 0);
+      const float p = expf(mine - z[__ffs(top_lane) - 1]);
+      const bool chosen = lane < E && place < top;
+      __syncwarp();
+      if (chosen) z[place] = p;
+      __syncwarp();
+      float denom = 0.f;
+      for (int j = 0; j < top; ++j) denom += z[j];
+      const float inv = 1.f / denom;
+      if (chosen) {
+        ids[static_cast<size_t>(t0 + r) * top + place] = lane;
+        weights[static_cast<size_t>(t0 + r) * top + place] = p * inv;
+      }
+      continue;
+    }
     float first = 0.f, denom = 0.f;
     for (int j = 0; j < top; ++j) {
       float best = -INFINITY;
@@ -262,6 +376,64 @@ __global__ void __launch_bounds__(1024)
     if (ids[i] == e) perm[before++] = i;
 }
 
+// Plan and fill in one launch for up to kPlanExperts experts: a block per expert counts all pairs (a histogram a warp, so that
+// few threads meet on a counter), sums the experts before its own, and writes its pairs in their order; block 0 writes the
+// offsets.  At 8,192 pairs of 16 experts, inside a step: 4.8 us, the two launches 8.
+constexpr int kPlanExperts = 128;
+
+__global__ void __launch_bounds__(1024)
+    moe_plan_fill_kernel(const int* __restrict__ ids, int A, int E, int tile_rows, int* __restrict__ offsets,
+                         int* __restrict__ tile_start, int* __restrict__ perm) {
+  extern __shared__ int plan_hist[];  // [32 warps][E] | counts [E]
+  __shared__ int warp_total[32];
+  int* counts = plan_hist + 32 * E;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_launch_dependents();
+  for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) plan_hist[i] = 0;
+  __syncthreads();
+  pdl_wait();
+  const int e = blockIdx.x;
+  const int run = (A + 1023) / 1024;  // a thread owns a run of consecutive pairs
+  const int i0 = min(A, static_cast<int>(threadIdx.x) * run), i1 = min(A, i0 + run);
+  int mine = 0;
+  for (int i = i0; i < i1; ++i) {
+    const int id = ids[i];
+    if (id >= 0 && id < E) atomicAdd(&plan_hist[warp * E + id], 1);
+    mine += id == e;
+  }
+  int incl = mine;  // inclusive sum over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_total[warp] = incl;
+  __syncthreads();
+  for (int i = threadIdx.x; i < E; i += blockDim.x) {
+    int c = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) c += plan_hist[w * E + i];
+    counts[i] = c;
+  }
+  __syncthreads();
+  if (e == 0)
+    for (int i = threadIdx.x; i <= E; i += blockDim.x) {
+      int rows = 0, tiles = 0;
+      for (int o = 0; o < i; ++o) {
+        rows += counts[o];
+        tiles += (counts[o] + tile_rows - 1) / tile_rows;
+      }
+      offsets[i] = rows;
+      tile_start[i] = tiles;
+    }
+  if (counts[e] == 0) return;
+  int before = incl - mine;
+  for (int o = 0; o < e; ++o) before += counts[o];
+  for (int w = 0; w < warp; ++w) before += warp_total[w];
+  for (int i = i0; i < i1; ++i)
+    if (ids[i] == e) perm[before++] = i;
+}
+
 // The whole plan of a step with few pairs (a decode step) in one block and one launch: a thread per expert
 // counts its pairs, one thread sums, then every expert's thread writes its pairs in their order.
 constexpr int kPlanSmallPairs = 512;
@@ -313,21 +485,6 @@ __device__ __forceinline__ float clamped_glu(float g, float u, float limit, floa
 __device__ __forceinline__ float relu_squared(float z) {
   z = fmaxf(z, 0.f);
   return z * z;
-}
-
-// Finds the expert and the rows of row tile `tile`; false when there is no such tile.
-__device__ __forceinline__ bool moe_tile(int tile, const int* __restrict__ offsets, const int* __restrict__ tile_start,
-                                         int E, int tile_rows, int& e, int& row0, int& row1) {
-  if (tile >= tile_start[E]) return false;
-  int lo = 0, hi = E - 1;  // the last e with tile_start[e] <= tile (experts without rows share a start)
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tile_start[mid] <= tile) lo = mid; else hi = mid - 1;
-  }
-  e = lo;
-  row0 = offsets[e] + (tile - tile_start[e]) * tile_rows;
-  row1 = min(offsets[e + 1], row0 + tile_rows);
-  return true;
 }
 
 // The grouped product in float arithmetic on the CUDA cores, for any sizes and both storage types.
@@ -516,9 +673,17 @@ __global__ void __launch_bounds__(128)
 }
 
 // The same product for steps of few pairs (decode steps), where an expert has a handful of rows and the
-// launch is a read of the chosen experts' matrices: tiles of 16 rows x 64 columns, the four warps share the
-// columns, K in slices of 64 through a four-stage ring, so that a block keeps three slices in flight.
-constexpr int kFewRows = 16, kFewCols = 64, kFewK = 64, kFewStages = 4, kFewLd = kFewK + 8;
+// launch is a read of the chosen experts' matrices: tiles of 16 rows, the four warps share the
+// columns, K in slices through a four-stage ring, so that a block keeps three slices in flight.  What it takes is a block's
+// walk along K: 64 columns and slices of 64 for the down product (K is an expert's width); 32 gate and 32 up columns and
+// slices of 128 for the up product, whose K is the model's width: twice the blocks, half the steps (8 tokens, 4 of 16 experts
+// of 256, width 1,024, inside a step: 14.5 us with 64 + 64 columns and slices of 64, 10 us so).
+constexpr int kFewRows = 16, kFewStages = 4;
+template <bool UP>
+struct FewTile {
+  static constexpr int kCols = UP ? 32 : 64, kK = UP ? 128 : 64, kLd = kK + 8, kBRows = UP ? 2 * kCols : kCols;
+  static constexpr int kStageElems = (kFewRows + kBRows) * kLd;
+};
 
 template <bool UP>
 __global__ void __launch_bounds__(128)
@@ -526,8 +691,8 @@ __global__ void __launch_bounds__(128)
                         const int* __restrict__ perm, const int* __restrict__ offsets,
                         const int* __restrict__ tile_start, int E, int top, int K, int N, float limit, float alpha,
                         float shift, int ungated, const float* __restrict__ row_w, bf16* __restrict__ out) {
-  constexpr int BROWS = UP ? 2 * kFewCols : kFewCols;
-  constexpr int kStageElems = (kFewRows + BROWS) * kFewLd;
+  constexpr int kCols = FewTile<UP>::kCols, kK = FewTile<UP>::kK, kLd = FewTile<UP>::kLd, BROWS = FewTile<UP>::kBRows;
+  constexpr int kStageElems = FewTile<UP>::kStageElems;
   extern __shared__ __align__(16) unsigned char few_smem[];
   bf16* ring = reinterpret_cast<bf16*>(few_smem);
   __shared__ int src_row[kFewRows];
@@ -536,7 +701,7 @@ __global__ void __launch_bounds__(128)
   pdl_wait();
   int e, row0, row1;
   if (!moe_tile(blockIdx.y, offsets, tile_start, E, kFewRows, e, row0, row1)) return;
-  const int n0 = blockIdx.x * kFewCols;
+  const int n0 = blockIdx.x * kCols;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < kFewRows) {
     const int i = row0 + threadIdx.x;
@@ -549,53 +714,62 @@ __global__ void __launch_bounds__(128)
 
   auto stage = [&](int buf, int k0) {
     bf16* As = ring + static_cast<size_t>(buf) * kStageElems;
-    bf16* Bs = As + kFewRows * kFewLd;
-    {  // 16 rows x 8 pieces of 8 elements: one a thread
-      const int r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 8;
+    bf16* Bs = As + kFewRows * kLd;
+    constexpr int kPieces = kK / 8;  // of 8 elements in a row of the slice
+    for (int idx = threadIdx.x; idx < kFewRows * kPieces; idx += 128) {
+      const int r = idx / kPieces, c = (idx % kPieces) * 8;
       const int src = src_row[r];
       const bool ok = src >= 0 && k0 + c < K;
-      cp_async16(As + r * kFewLd + c, ok ? a + static_cast<long long>(src) * ld_a + k0 + c : a, ok);
+      cp_async16(As + r * kLd + c, ok ? a + static_cast<long long>(src) * ld_a + k0 + c : a, ok);
     }
-    for (int idx = threadIdx.x; idx < BROWS * 8; idx += 128) {
-      const int r = idx >> 3, c = (idx & 7) * 8;
-      const int col = UP ? (r < kFewCols ? n0 + r : n0 + r - kFewCols) : n0 + r;
+#pragma unroll
+    for (int idx = threadIdx.x; idx < BROWS * kPieces; idx += 128) {
+      const int r = idx / kPieces, c = (idx % kPieces) * 8;
+      const int col = UP ? (r < kCols ? n0 + r : n0 + r - kCols) : n0 + r;
       const bool ok = col < N && k0 + c < K;
-      const size_t wrow = UP && r >= kFewCols ? static_cast<size_t>(N) + col : col;
-      cp_async16(Bs + r * kFewLd + c, ok ? we + wrow * K + k0 + c : we, ok);
+      const size_t wrow = UP && r >= kCols ? static_cast<size_t>(N) + col : col;
+      cp_async16(Bs + r * kLd + c, ok ? we + wrow * K + k0 + c : we, ok);
     }
     cp_async_commit();
   };
 
-  float acc[UP ? 4 : 2][4];
+  float acc[2][4];   // UP: the warp's 8 gate and 8 up columns; else its 16 columns
 #pragma unroll
-  for (int j = 0; j < (UP ? 4 : 2); ++j)
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
 
-  const int n_slices = (K + kFewK - 1) / kFewK;
+  const int n_slices = (K + kK - 1) / kK;
 #pragma unroll
   for (int s = 0; s < kFewStages - 1; ++s) {
-    if (s < n_slices) stage(s, s * kFewK);
+    if (s < n_slices) stage(s, s * kK);
     else cp_async_commit();
   }
   for (int s = 0; s < n_slices; ++s) {
     cp_async_wait<kFewStages - 2>();  // slice s has landed
     __syncthreads();                  // ... for every thread, and slice s - 1's buffer is free
-    if (s + kFewStages - 1 < n_slices) stage((s + kFewStages - 1) % kFewStages, (s + kFewStages - 1) * kFewK);
+    if (s + kFewStages - 1 < n_slices) stage((s + kFewStages - 1) % kFewStages, (s + kFewStages - 1) * kK);
     else cp_async_commit();
     const bf16* As = ring + static_cast<size_t>(s % kFewStages) * kStageElems;
-    const bf16* Bs = As + kFewRows * kFewLd;
+    const bf16* Bs = As + kFewRows * kLd;
 #pragma unroll
-    for (int kk = 0; kk < kFewK; kk += 16) {
-      unsigned af[4];
-      ldmatrix_x4(af[0], af[1], af[2], af[3], As + (lane & 15) * kFewLd + kk + ((lane >> 4) << 3));
-#pragma unroll
-      for (int part = 0; part < (UP ? 2 : 1); ++part) {
-        unsigned b0, b1, b2, b3;
-        ldmatrix_x4(b0, b1, b2, b3,
-                    Bs + (part * kFewCols + warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * kFewLd + kk + (((lane >> 3) & 1) << 3));
-        mma_bf16(acc[2 * part], af, b0, b1);
-        mma_bf16(acc[2 * part + 1], af, b2, b3);
+    for (int kk = 0; kk < kK; kk += UP ? 32 : 16) {
+      unsigned af[4], b0, b1, b2, b3;
+      ldmatrix_x4(af[0], af[1], af[2], af[3], As + (lane & 15) * kLd + kk + ((lane >> 4) << 3));
+      if (UP) {
+        // 8 rows of the gate's (the up) matrix x 32 k, in two steps of 16
+        unsigned ag[4], c0, c1, c2, c3;
+        ldmatrix_x4(ag[0], ag[1], ag[2], ag[3], As + (lane & 15) * kLd + kk + 16 + ((lane >> 4) << 3));
+        ldmatrix_x4(b0, b1, b2, b3, Bs + (warp * 8 + (lane & 7)) * kLd + kk + ((lane >> 3) << 3));
+        ldmatrix_x4(c0, c1, c2, c3, Bs + (kCols + warp * 8 + (lane & 7)) * kLd + kk + ((lane >> 3) << 3));
+        mma_bf16(acc[0], af, b0, b1);
+        mma_bf16(acc[1], af, c0, c1);
+        mma_bf16(acc[0], ag, b2, b3);
+        mma_bf16(acc[1], ag, c2, c3);
+      } else {
+        ldmatrix_x4(b0, b1, b2, b3, Bs + (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * kLd + kk + (((lane >> 3) & 1) << 3));
+        mma_bf16(acc[0], af, b0, b1);
+        mma_bf16(acc[1], af, b2, b3);
       }
     }
   }
@@ -608,14 +782,14 @@ __global__ void __launch_bounds__(128)
     if (i >= row1) continue;
     const float rw = (UP && row_w) ? row_w[dst_row[r]] : 1.f;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < (UP ? 1 : 2); ++j) {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const int col = n0 + warp * 16 + j * 8 + c_in + q;
+        const int col = n0 + (UP ? warp * 8 : warp * 16 + j * 8) + c_in + q;
         if (col >= N) continue;
         if (UP) {
           out[static_cast<size_t>(i) * N + col] =
-              __float2bfloat16_rn(clamped_glu(rw * acc[j][half * 2 + q], rw * acc[UP ? 2 + j : j][half * 2 + q], limit, alpha, shift));
+              __float2bfloat16_rn(clamped_glu(rw * acc[0][half * 2 + q], rw * acc[1][half * 2 + q], limit, alpha, shift));
         } else {
           const float val = acc[j][half * 2 + q];
           out[static_cast<size_t>(ungated ? i : dst_row[r]) * N + col] = __float2bfloat16_rn(ungated ? relu_squared(val) : val);
@@ -642,6 +816,41 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The same sums for rows of whole sixteen-byte pieces: a thread makes one piece (8 values in bfloat16, 4 in float) of one
+// token, so that all of its reads are in flight together.  2,048 tokens of 4 experts, width 1,024, inside a step: 4.4 us,
+// a value a thread and read 8.2.
+template <typename S>
+__global__ void __launch_bounds__(256)
+    moe_combine_vec_kernel(const S* __restrict__ y, const float* __restrict__ weights, const S* __restrict__ shared,
+                           const float* __restrict__ shared_gate, S* __restrict__ out, int T, int D, int top) {
+  constexpr int V = 16 / sizeof(S);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int per_row = D / V;
+  const long long at = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int t = static_cast<int>(at / per_row), c = static_cast<int>(at - static_cast<long long>(t) * per_row) * V;
+  if (t >= T) return;
+  float acc[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) acc[v] = 0.f;
+  auto add = [&](const S* row, float p) {
+    float x[V];
+#pragma unroll
+    for (int v = 0; v < V; v += 4) {
+      const float4 q = ldf4(row + v);
+      x[v] = q.x, x[v + 1] = q.y, x[v + 2] = q.z, x[v + 3] = q.w;
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] += p * x[v];
+  };
+#pragma unroll 4
+  for (int j = 0; j < top; ++j)
+    add(y + (static_cast<size_t>(t) * top + j) * D + c, weights ? weights[static_cast<size_t>(t) * top + j] : 1.f);
+  if (shared) add(shared + static_cast<size_t>(t) * D + c, shared_gate ? shared_gate[t] : 1.f);
+#pragma unroll
+  for (int v = 0; v < V; v += 4) stf4(out + static_cast<size_t>(t) * D + c + v, make_float4(acc[v], acc[v + 1], acc[v + 2], acc[v + 3]));
+}
+
 }  // namespace pmm
 
 namespace pmm {
@@ -656,7 +865,7 @@ int launch_route(const void* x, long long ld_x, const float* w, const float* bia
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
   }
-  launch_pdl(kern, dim3((T + TOK - 1) / TOK), dim3(kRouteWarps * 32), smem, stream, static_cast<const S*>(x), ld_x, w, bias,
+  launch_pdl(kern, dim3((T + TOK - 1) / TOK), dim3(RouteShape<TOK>::kWarps * 32), smem, stream, static_cast<const S*>(x), ld_x, w, bias,
              ids, weights, T, D, E, top, scored, correction, groups, keep, scale, gate_w, gate_out);
   return launch_status();
 }
@@ -673,11 +882,14 @@ PMM_EXPORT int pmm_moe_route(const void* x, long long ld_x, const float* w, cons
   if (D <= 0 || E <= 0 || top <= 0 || top > E || (gate_w && !gate_out)) return PMM_ERR_BAD_ARGUMENT;
   if (scored && (groups <= 0 || E % groups || keep <= 0 || keep > groups || top > keep * (E / groups)))
     return PMM_ERR_BAD_ARGUMENT;
-  // few tokens: a block each, so that the step's few rows still spread over the GPU; many: four a block, which
-  // reads the router a quarter as often
-  const bool four = T >= 512 && (static_cast<size_t>(4) * (((D + 3) & ~3) + 3 * E)) * sizeof(float) <= 96 * 1024;
+  // few tokens: a block each, so that the step's few rows still spread over the GPU; many: four or eight a block (a
+  // block an SM is left), which read the router a quarter or an eighth as often
+  auto room = [&](int tok) { return (static_cast<size_t>(tok) * (((D + 3) & ~3) + 3 * E)) * sizeof(float) <= 96 * 1024; };
   PMM_DISPATCH_DTYPE(dtype, S, {
-    if (four)
+    if (T >= 1024 && room(8))
+      return pmm::launch_route<S, 8>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
+                                     gate_w, gate_out, stream);
+    if (T >= 512 && room(4))
       return pmm::launch_route<S, 4>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
                                      gate_w, gate_out, stream);
     return pmm::launch_route<S, 1>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
@@ -687,7 +899,7 @@ PMM_EXPORT int pmm_moe_route(const void* x, long long ld_x, const float* w, cons
 }
 
 // ids [A] -> offsets [E + 1], tile_start [E + 1] (row tiles of `tile_rows`), perm [A].  One launch for up to
-// kPlanSmallPairs pairs, else two.
+// kPlanSmallPairs pairs or kPlanExperts experts, else two.
 PMM_EXPORT int pmm_moe_plan(const int* ids, int A, int E, int tile_rows, int* offsets, int* tile_start, int* perm,
                             cudaStream_t stream) {
   if (A <= 0) return 0;
@@ -695,6 +907,11 @@ PMM_EXPORT int pmm_moe_plan(const int* ids, int A, int E, int tile_rows, int* of
   if (A <= pmm::kPlanSmallPairs) {
     pmm::launch_pdl(pmm::moe_plan_small_kernel, dim3(1), dim3(256), static_cast<size_t>(A + E) * sizeof(int), stream, ids,
                     A, E, tile_rows, offsets, tile_start, perm);
+    return pmm::launch_status();
+  }
+  if (E <= pmm::kPlanExperts) {
+    pmm::launch_pdl(pmm::moe_plan_fill_kernel, dim3(E), dim3(1024), static_cast<size_t>(33) * E * sizeof(int), stream, ids, A, E,
+                    tile_rows, offsets, tile_start, perm);
     return pmm::launch_status();
   }
   pmm::launch_pdl(pmm::moe_plan_kernel, dim3(1), dim3(1024), static_cast<size_t>(E) * sizeof(int), stream, ids, A, E,
@@ -731,9 +948,10 @@ PMM_EXPORT int pmm_moe_gemm(const void* a, long long ld_a, const void* w, const 
         reinterpret_cast<uintptr_t>(w) % 16)
       return PMM_ERR_BAD_ARGUMENT;
     if (tensor_cores == 2) {
-      const dim3 grid((N + pmm::kFewCols - 1) / pmm::kFewCols, row_tiles);
-      const size_t smem = static_cast<size_t>(pmm::kFewStages) * (pmm::kFewRows + (up ? 2 : 1) * pmm::kFewCols) *
-                          pmm::kFewLd * sizeof(pmm::bf16);
+      const int cols = up ? pmm::FewTile<true>::kCols : pmm::FewTile<false>::kCols;
+      const dim3 grid((N + cols - 1) / cols, row_tiles);
+      const size_t smem = static_cast<size_t>(pmm::kFewStages) * sizeof(pmm::bf16) *
+                          (up ? pmm::FewTile<true>::kStageElems : pmm::FewTile<false>::kStageElems);
       cudaError_t err;
       if (up) {
         auto kern = pmm::moe_gemm_few_kernel<true>;
@@ -777,6 +995,15 @@ PMM_EXPORT int pmm_moe_combine(const void* y, const float* weights, const void* 
                                int T, int D, int top, int dtype, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (D <= 0 || top <= 0) return PMM_ERR_BAD_ARGUMENT;
+  const int v = dtype == PMM_DTYPE_BF16 ? 8 : 4;
+  auto whole = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  if (D % v == 0 && whole(y) && whole(out) && (!shared || whole(shared))) {
+    const long long blocks = (static_cast<long long>(T) * (D / v) + 255) / 256;
+    PMM_DISPATCH_DTYPE(dtype, S, pmm::launch_pdl(pmm::moe_combine_vec_kernel<S>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0,
+                                                 stream, static_cast<const S*>(y), weights, static_cast<const S*>(shared),
+                                                 shared_gate, static_cast<S*>(out), T, D, top));
+    return pmm::launch_status();
+  }
   int ytiles = (D + 1023) / 1024;
   if (ytiles > 64) ytiles = 64;
   PMM_DISPATCH_DTYPE(dtype, S, pmm::launch_pdl(pmm::moe_combine_kernel<S>, dim3(T, ytiles), dim3(256), 0, stream,

@@ -2083,9 +2083,9 @@ def moe_plan(ids: Tensor, n_experts: int, form: str, offsets: Tensor, tile_start
     _i32(ids, "moe_plan: ids")
     _call("pmm_moe_plan", ids.data_ptr(), A, int(n_experts), moe_tile_rows(form), offsets.data_ptr(),
           tile_start.data_ptr(), perm.data_ptr(), _stream())
-    if A > 512:
+    if A > 512 and n_experts > 128:
         global launch_count
-        launch_count += 1  # two launches for many pairs
+        launch_count += 1  # two launches for many pairs of many experts
 
 
 def moe_tc_supported(a: Tensor, w: Tensor, n_out: int) -> bool:

@@ -214,3 +214,53 @@ def test_routed_experts_against_the_plain_sum(dtype, D, E, top, F, Fs, T, starve
             mine = perm.cpu()[off[e]:off[e + 1]].long()
             assert bool((flat[mine] == e).all()) and mine.tolist() == sorted(mine.tolist())
         assert tiles.cpu().tolist() == [sum(-(-(off[j + 1] - off[j]) // rows) for j in range(e)) for e in range(E + 1)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,E,top,D", [(1, 1, 1, 4), (3, 5, 5, 7), (9, 16, 4, 1028), (5, 31, 31, 132), (6, 32, 3, 128), (6, 33, 3, 128),
+                                       (515, 16, 4, 36), (513, 40, 2, 30), (1027, 17, 3, 68)])
+def test_ranked_and_picked_experts(dtype, T, E, top, D):
+    """One lane an expert (up to 32) and the serial picks, one, four and eight tokens a block, widths on and off whole pieces:
+    small whole numbers, so that the logits are exact and full of ties, which the lower index wins.  A row that is not a
+    number picks valid indices."""
+    g = torch.Generator().manual_seed(E)
+    x = torch.randint(-2, 3, (T, D), generator=g).float() * (torch.rand(T, D, generator=g) < 4.0 / D)
+    w = torch.randint(-2, 3, (E, D), generator=g).float()
+    if E > 3:
+        w[E - 1] = w[1]   # a tie in every row
+    z = x @ w.t()
+    want = torch.tensor([sorted(range(E), key=lambda e: (-z[t, e].item(), e))[:top] for t in range(T)])
+    chosen = torch.gather(z.double(), 1, want)
+    sig = torch.sigmoid(chosen)
+    weights_of = {False: torch.softmax(chosen, 1), "softmax": 2.0 * torch.gather(torch.softmax(z.double(), 1), 1, want)}
+    if float(z.abs().max()) < 10:   # (beyond, float sigmoids of different logits meet at one)
+        weights_of.update({True: 2.0 * sig / sig.sum(1, keepdim=True), "sigmoid": 2.0 * sig})
+    for scored, pw in weights_of.items():
+        ids = torch.full((T, top), -7, dtype=torch.int32, device=DEV)
+        weights = torch.empty(T, top, device=DEV)
+        K.moe_route(x.to(DEV, dtype), w.to(DEV), None, top, ids, weights, scored=scored, scale=2.0)
+        assert torch.equal(ids.cpu().long(), want), scored
+        close(weights, pw, torch.float32, f"weights {scored}", f32=1e-5)
+    bad = x.clone()
+    bad[0, 0] = float("nan")
+    for scored in weights_of:
+        K.moe_route(bad.to(DEV, dtype), w.to(DEV), None, top, ids, weights, scored=scored)
+        assert int(ids[0].min()) >= 0 and int(ids[0].max()) < E
+        if T > 1:
+            assert torch.equal(ids[1:].cpu().long(), want[1:])
+
+
+@pytest.mark.parametrize("A,E", [(513, 1), (1024, 16), (1025, 128), (3000, 129), (8192, 7)])
+def test_plan_of_many_pairs(A, E):
+    """One launch for up to 128 experts, two beyond: every expert's pairs in their order, experts without pairs among them."""
+    g = torch.Generator().manual_seed(A)
+    ids = (torch.randint(0, E, (A,), generator=g) // 2 * 2 % E).to(torch.int32)
+    offsets, tiles = (torch.empty(E + 1, dtype=torch.int32, device=DEV) for _ in range(2))
+    perm = torch.empty(A, dtype=torch.int32, device=DEV)
+    for form in ("mma", "tcgen05"):
+        K.moe_plan(ids.to(DEV), E, form, offsets, tiles, perm)
+        count = torch.bincount(ids.long(), minlength=E)
+        rows = K.moe_tile_rows(form)
+        assert torch.equal(perm.cpu().long(), torch.sort(ids.long(), stable=True).indices)
+        assert offsets.cpu().tolist() == [0] + count.cumsum(0).tolist()
+        assert tiles.cpu().tolist() == [0] + ((count + rows - 1) // rows).cumsum(0).tolist()
