@@ -803,6 +803,32 @@ def test_skinny_product_with_float32_output_for_the_head(M, N, Kd):
     assert bool(torch.isnan(out[:, N:]).all())
 
 
+@pytest.mark.parametrize("T,N,Kd", [(16, 127, 64), (33, 129, 8), (48, 256, 1024), (49, 136, 328), (63, 8, 1016), (64, 4, 2056), (3, 1, 6152)])
+def test_tcgen05_product_in_clusters(T, N, Kd):
+    """Blocks of a cluster share K: none of its boxes for some of them, one, four; tiles of 128 rows (64 + 64) and one beside;
+    tokens on and off 16; products longer than a cluster in several.  Small whole numbers, so that the sums are exact
+    however K is cut and a store differs by its own rounding alone."""
+    ops = K()
+    bf = torch.bfloat16
+    g = torch.Generator().manual_seed(T + N + Kd)
+    x = torch.randint(-3, 4, (T, Kd), generator=g).to(bf).to(DEV)
+    w = torch.randint(-3, 4, (N, Kd), generator=g).to(bf).to(DEV)
+    ref = x.double().cpu() @ w.double().cpu().t()      # |sums| <= 9 * 6152 < 2^24
+    h = torch.randint(-8, 9, (T, N), generator=g).float()
+    hd = h.to(DEV)
+    ops.skinny_tc_residual(hd, [(x, w, 2.0)])
+    assert torch.equal(hd.cpu().double(), h.double() + 2.0 * ref)
+    ops.skinny_tc_residual(hd, [(x, w, -1.0), (x[:, :8], w[:, :8].contiguous(), 4.0)])
+    assert torch.equal(hd.cpu().double(), h.double() + ref + 4.0 * (x.double().cpu()[:, :8] @ w.double().cpu()[:, :8].t()))
+    if Kd <= 1024:
+        out = torch.full((T, (N + 7) // 8 * 8), float("nan"), dtype=bf, device=DEV)
+        ops.skinny_tc_linear(x, w, out[:, :N])
+        assert torch.equal(out[:, :N].cpu(), ref.to(bf))
+        assert bool(torch.isnan(out[:, N:]).all())
+    torch.cuda.synchronize()
+    assert ops.tc_gemm_status(DEV) == 0
+
+
 @pytest.mark.parametrize("T", [1, 17, 40, 64])
 @pytest.mark.parametrize("N,Kd", [(50, 96), (1024, 1000), (4120, 1024), (6000, 512), (304, 72)])
 def test_tcgen05_weight_streaming_product(T, N, Kd):
