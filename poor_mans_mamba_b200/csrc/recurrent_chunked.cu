@@ -53,6 +53,7 @@ struct ChunkArgs {
   float unit_eps, q_scale;
   // per (chunk, head), chunk-major: W [C, d] (delta), Uv [C, dv], B [C, C], Qg [C, d], Ke [C, d], Eg [d]
   float *W, *Uv, *B, *Qg, *Ke, *Eg;
+  int with_state;                       // the prepare kernel makes N too (see chunk_state)
   int vec_in;                           // q, k, v (and a) rows and heads start on boundaries of four elements
   float* N;                             // [d, dv] per (chunk, head): see the kernels that use it
   float* state; const int* slots; float* out;
@@ -439,15 +440,17 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
 
 // The values of the chunk's tokens as floats (silu of them for kRuleDecay), eight or four bytes at a time where they lie so
 template <typename S, bool SILU>
-__device__ __forceinline__ void widen_values(const ChunkArgs& p, float* __restrict__ oUv, int h, int t0, int n, int tid, int n_threads) {
+__device__ __forceinline__ void widen_values(const ChunkArgs& p, float* __restrict__ oUv, float* __restrict__ sV, int h, int t0, int n, int tid, int n_threads) {
   const int dv = p.dv;
   const S* gv = static_cast<const S*>(p.v) + static_cast<long long>(t0) * p.ld_v + h * dv;
   if (dv % 4 == 0) {
+#pragma unroll 4
     for (int e = tid; e < n * (dv / 4); e += n_threads) {
       const int i = e / (dv / 4), c = 4 * (e - i * (dv / 4));
       float4 v = load4(gv + static_cast<long long>(i) * p.ld_v + c, p.vec_in != 0);
       if (SILU) v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
       *reinterpret_cast<float4*>(oUv + static_cast<size_t>(i) * dv + c) = v;
+      if (sV) *reinterpret_cast<float4*>(sV + i * dv + c) = v;  // (asked for with dv a multiple of 8 only)
     }
     return;
   }
@@ -458,9 +461,55 @@ __device__ __forceinline__ void widen_values(const ChunkArgs& p, float* __restri
   }
 }
 
+// N [d, dv] = Ke^T V of a chunk whose weakened keys and values lie in shared memory: 8 x (4 or 8) results a thread, two
+// multiply-adds an instruction, every sum in the order of the tokens.  d and dv are multiples of 8.  The prepare kernels end with it where their
+// blocks still share an SM: a launch, the keys' way out to memory and back and eight (instead of twelve or sixteen) sixteen-byte reads
+// for every 128 multiply-adds less.  Us inside a step, prepare and state: the decayed sum at 2,048 tokens, 8 heads, 128 x 128 20 + 16 -> 25, retention
+// at 1,501, 8 heads, 64 x 128 26 + 15 -> 23, time mixing at 1,501, 16 heads, 64 x 64 33 + 15 -> 39.
+template <int COLS>
+__device__ __forceinline__ void chunk_state(float* __restrict__ gN, const float* __restrict__ sKe, int ds, const float* __restrict__ sV,
+                                            int d, int dv, int n, int tid, int n_threads) {
+  constexpr int P = COLS / 2;   // pairs of columns: four neighbours, and with 8 columns four more half a row further
+  const int per_row = dv / COLS, tiles = (d / 8) * per_row;
+  for (int tile = tid; tile < tiles; tile += n_threads) {
+    const int c = 4 * (tile % per_row), k0 = 8 * (tile / per_row);
+    Pair acc[8][P];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int q = 0; q < P; ++q) acc[r][q] = 0ull;
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+      const float4 a0 = *reinterpret_cast<const float4*>(sKe + j * ds + k0), a1 = *reinterpret_cast<const float4*>(sKe + j * ds + k0 + 4);
+      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      Pair b[P];
+#pragma unroll
+      for (int q = 0; q < P; q += 2) {
+        const Quad v = quad(sV + j * dv + c + (q ? dv / 2 : 0));
+        b[q] = v.lo;
+        b[q + 1] = v.hi;
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const Pair a2 = pair(a[r], a[r]);
+#pragma unroll
+        for (int q = 0; q < P; ++q) acc[r][q] = fma2(a2, b[q], acc[r][q]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int q = 0; q < P; q += 2) {
+        const float2 lo = halves(acc[r][q]), hi = halves(acc[r][q + 1]);
+        *reinterpret_cast<float4*>(gN + static_cast<size_t>(k0 + r) * dv + c + (q ? dv / 2 : 0)) = make_float4(lo.x, lo.y, hi.x, hi.y);
+      }
+  }
+}
+
 // The operands of the decayed sum (kRuleDecay, kRuleRetention): B_ij = (q_i . k_j) a^(i-j), Q * a^(i+1), K * a^(n-1-i), a^n.
-// Rows of stride d + 4: sixteen-byte reads of neighbouring rows fall into different banks.  A thread makes a 4 x 4
-// piece of B.
+// Rows of stride d + 4: sixteen-byte reads of neighbouring rows fall into different banks.  A thread makes the entries of B of
+// four neighbouring rows and of every sixteenth column (16 threads read 16 neighbouring rows of k; with four
+// neighbouring columns a thread their reads fell into the same banks four by four).
 constexpr int kDecayPrepThreads = 256;
 
 inline size_t decay_prepare_smem(int d) { return sizeof(float) * (static_cast<size_t>(2 * kChunk) * (d + 4)); }
@@ -482,6 +531,7 @@ __global__ void __launch_bounds__(kDecayPrepThreads)
   const int tid = threadIdx.x;
   const size_t ch = static_cast<size_t>(chunk) * p.H + h;
   if (tid <= kChunk) s_pow[tid] = expf(logf(fmaxf(p.decay[h], 1e-38f)) * static_cast<float>(tid));
+#pragma unroll 4
   for (int e = tid; e < n * d4; e += kDecayPrepThreads) {
     const int i = e / d4, c = 4 * (e - i * d4);
     const long long t = t0 + i;
@@ -496,7 +546,8 @@ __global__ void __launch_bounds__(kDecayPrepThreads)
     *reinterpret_cast<float4*>(sQ + i * ds + c) = q;
     *reinterpret_cast<float4*>(sK + i * ds + c) = k;
   }
-  widen_values<S, SILU>(p, p.Uv + ch * kChunk * p.dv, h, t0, n, tid, kDecayPrepThreads);
+  float* sV = p.with_state ? sQ + kChunk * ds : nullptr;  // [C][dv]
+  widen_values<S, SILU>(p, p.Uv + ch * kChunk * p.dv, sV, h, t0, n, tid, kDecayPrepThreads);
   __syncthreads();
   if (RULE == kRuleRetention && p.rot.rot_dims > 0) {
     rotate_rows(sQ, sK, ds, n, t0, p.rot, tid, kDecayPrepThreads);
@@ -504,27 +555,30 @@ __global__ void __launch_bounds__(kDecayPrepThreads)
   }
   float* oB = p.B + ch * kChunk * kChunk;
   // (rows at and beyond n hold stale values whose results are not stored)
-  const int i0 = 4 * (tid / 16), j0 = 4 * (tid % 16);
-  if (j0 <= i0 && i0 < n) {
+  const int i0 = 4 * (tid / 16), j0 = tid % 16, spans = i0 / 16;  // columns j0, j0 + 16 .. up to the rows' own sixteen
+  if (i0 < n) {
     float acc[4][4] = {};
     for (int c = 0; c < d; c += 4) {
-      float4 q[4], k[4];
+      float4 q[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        q[r] = *reinterpret_cast<const float4*>(sQ + (i0 + r) * ds + c);
-        k[r] = *reinterpret_cast<const float4*>(sK + (j0 + r) * ds + c);
+      for (int r = 0; r < 4; ++r) q[r] = *reinterpret_cast<const float4*>(sQ + (i0 + r) * ds + c);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        if (s > spans) break;
+        const float4 k = *reinterpret_cast<const float4*>(sK + (j0 + 16 * s) * ds + c);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r][s] += q[r].x * k.x + q[r].y * k.y + q[r].z * k.z + q[r].w * k.w;
       }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int s = 0; s < 4; ++s) acc[r][s] += q[r].x * k[s].x + q[r].y * k[s].y + q[r].z * k[s].z + q[r].w * k[s].w;
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int s = 0; s < 4; ++s)
-        if (i0 + r < n && j0 + s <= i0 + r) oB[(i0 + r) * kChunk + j0 + s] = acc[r][s] * s_pow[i0 + r - j0 - s];
+      for (int s = 0; s < 4; ++s) {
+        const int i = i0 + r, j = j0 + 16 * s;
+        if (i < n && j <= i) oB[i * kChunk + j] = acc[r][s] * s_pow[i - j];
+      }
   }
+  if (p.with_state) __syncthreads();  // the keys are weakened in place
   float* oQg = p.Qg + ch * kChunk * d;
   float* oKe = p.Ke + ch * kChunk * d;
   for (int e = tid; e < n * d4; e += kDecayPrepThreads) {
@@ -532,9 +586,13 @@ __global__ void __launch_bounds__(kDecayPrepThreads)
     const float up = s_pow[i + 1], down = s_pow[n - 1 - i];
     const float4 q = *reinterpret_cast<const float4*>(sQ + i * ds + c), k = *reinterpret_cast<const float4*>(sK + i * ds + c);
     *reinterpret_cast<float4*>(oQg + i * d + c) = make_float4(q.x * up, q.y * up, q.z * up, q.w * up);
-    *reinterpret_cast<float4*>(oKe + i * d + c) = make_float4(k.x * down, k.y * down, k.z * down, k.w * down);
+    *reinterpret_cast<float4*>(p.with_state ? sK + i * ds + c : oKe + i * d + c) = make_float4(k.x * down, k.y * down, k.z * down, k.w * down);
   }
   for (int c = tid; c < d; c += kDecayPrepThreads) p.Eg[ch * d + c] = s_pow[n];
+  if (p.with_state) {
+    __syncthreads();
+    chunk_state<8>(p.N + ch * static_cast<size_t>(d) * p.dv, sK, ds, sV, d, p.dv, n, tid, kDecayPrepThreads);
+  }
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -577,7 +635,7 @@ __global__ void __launch_bounds__(kWkvThreads)
   const int nb = (n + 15) >> 4;
 
   const bool vec = p.vec_in != 0;
-#pragma unroll 2
+#pragma unroll 4
   for (int e = tid; e < n * d4; e += kWkvThreads) {
     const int i = e / d4, c = 4 * (e - i * d4);
     const long long t = t0 + i;
@@ -590,7 +648,8 @@ __global__ void __launch_bounds__(kWkvThreads)
     *reinterpret_cast<float4*>(sK + i * ds + c) = k;
     *reinterpret_cast<float4*>(sL + i * ds + c) = make_float4(decay(a.x + b.x), decay(a.y + b.y), decay(a.z + b.z), decay(a.w + b.w));
   }
-  widen_values<S, false>(p, oUv, h, t0, n, tid, kWkvThreads);
+  float* sV = p.with_state ? sT + 4 * d : nullptr;  // [C][dv]
+  widen_values<S, false>(p, oUv, sV, h, t0, n, tid, kWkvThreads);
   __syncthreads();
   for (int e = tid; e < nb * d; e += kWkvThreads) {
     const int blk = e / d, c = e - blk * d;
@@ -675,13 +734,17 @@ __global__ void __launch_bounds__(kWkvThreads)
     const float4 q = *reinterpret_cast<const float4*>(sQ + i * ds + c);
     *reinterpret_cast<float4*>(oQg + i * d + c) = make_float4(q.x * exp2f(l.x), q.y * exp2f(l.y), q.z * exp2f(l.z), q.w * exp2f(l.w));
     if (blk < nb - 1) weaken(sK + i * ds + c, *reinterpret_cast<const float4*>(sT + (nb - 1) * d + c));
-    *reinterpret_cast<float4*>(oKe + i * d + c) = *reinterpret_cast<const float4*>(sK + i * ds + c);
+    if (!p.with_state) *reinterpret_cast<float4*>(oKe + i * d + c) = *reinterpret_cast<const float4*>(sK + i * ds + c);
   }
   float* oEg = p.Eg + ch * d;
   for (int c = tid; c < d; c += kWkvThreads) {
     float all = 0.f;
     for (int b = 0; b < nb; ++b) all += sT[b * d + c];
     oEg[c] = exp2f(all);
+  }
+  if (p.with_state) {
+    __syncthreads();
+    chunk_state<4>(p.N + ch * static_cast<size_t>(d) * dv, sK, ds, sV, d, dv, n, tid, kWkvThreads);
   }
 }
 
@@ -723,40 +786,16 @@ __device__ __forceinline__ void product_tn(float (&acc)[4][4], const float* __re
     fma4x4(acc, *reinterpret_cast<const float4*>(A + j * lda + k0), *reinterpret_cast<const float4*>(R + j * kDecayTile + c0));
 }
 
-// acc[r][c] += sum_{k < kn} A[i0 + r][k] * R[k][c0 + c], kn a multiple of 4; with `tri`, only k <= i0 + r
-__device__ __forceinline__ void product_nn(float (&acc)[4][4], const float* __restrict__ A, int lda, int i0,
-                                           const float* __restrict__ R, int c0, int kn, bool tri) {
-  for (int k4 = 0; k4 < kn; k4 += 4) {
-    float4 a[4], b[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + (i0 + r) * lda + k4);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) b[q] = *reinterpret_cast<const float4*>(R + (k4 + q) * kDecayTile + c0);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const float av[4] = {a[r].x, a[r].y, a[r].z, a[r].w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (!tri || k4 + q <= i0 + r) {
-          acc[r][0] += av[q] * b[q].x;
-          acc[r][1] += av[q] * b[q].y;
-          acc[r][2] += av[q] * b[q].z;
-          acc[r][3] += av[q] * b[q].w;
-        }
-      }
-    }
-  }
-}
-
 // `count` floats (a multiple of 4, 16-byte aligned at both ends) by asynchronous copies
 __device__ __forceinline__ void copy_rows(float* __restrict__ dst, const float* __restrict__ src, int count, int tid) {
   for (int e = 4 * tid; e < count; e += 4 * kDecayThreads) cp_async16(dst + e, src + e);
 }
 
 // Columns c0 .. c0 + 63 of `rows` rows of a [rows, dv] matrix, zeros beyond dv
+template <int THREADS = kDecayThreads>
 __device__ __forceinline__ void copy_tile(float* __restrict__ dst, const float* __restrict__ src, int rows, int dv, int c0, int tid) {
   if (dv % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0) {
-    for (int e = tid; e < rows * (kDecayTile / 4); e += kDecayThreads) {
+    for (int e = tid; e < rows * (kDecayTile / 4); e += THREADS) {
       const int j = e / (kDecayTile / 4), c = 4 * (e % (kDecayTile / 4));
       float* to = dst + j * kDecayTile + c;
       if (c0 + c < dv) cp_async16(to, src + static_cast<size_t>(j) * dv + c0 + c);
@@ -764,7 +803,7 @@ __device__ __forceinline__ void copy_tile(float* __restrict__ dst, const float* 
     }
     return;
   }
-  for (int e = tid; e < rows * kDecayTile; e += kDecayThreads) {
+  for (int e = tid; e < rows * kDecayTile; e += THREADS) {
     const int j = e / kDecayTile, c = e % kDecayTile;
     dst[e] = (c0 + c < dv) ? src[static_cast<size_t>(j) * dv + c0 + c] : 0.f;
   }
@@ -844,13 +883,20 @@ __global__ void __launch_bounds__(kDecayThreads)
   *st = s;
 }
 
-__global__ void __launch_bounds__(kDecayThreads)
+// The rows of every chunk: [Q * a^(i+1) | B] times [S_0; V], one product whose inner index runs over the d state rows and then
+// the chunk's tokens up to the row's own, 64 rows x 64 columns a block.
+// Bound by the float units and the latency in front of them: a thread makes 8 x 4 results, twelve sixteen-byte reads for four
+// inner indices and 128 multiply-adds (4 x 4: eight for 64), two multiply-adds an instruction, every sum in the order of
+// the inner index.  The operands come in slices of 32 through a ring of three, 48 KB a block, so that four blocks share an SM
+// and the 512 blocks of 2,048 tokens, 8 heads and 128 x 128 states are one wave (whole operands: 80 KB, two blocks, two waves).
+// That size inside a step: 30 -> 27 us (8 x 8 results on two warps a block 29.5: too few warps in flight).
+constexpr int kOutThreads = 128, kOutK = 32, kOutStages = 3;
+constexpr int kOutStage = kChunk * kOutK + kOutK * kDecayTile;  // floats
+
+__global__ void __launch_bounds__(kOutThreads)
     decay_chunk_output_kernel(ChunkArgs p) {
   extern __shared__ __align__(16) float sm[];
   const int d = p.d, dv = p.dv;
-  float* sQg = sm;                          // [C][d]
-  float* sS = sQg + kChunk * d;             // [d][tile]
-  float* sV = sS + d * kDecayTile;          // [C][tile]
   pdl_launch_dependents();
   pdl_wait();
   const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kDecayTile;
@@ -862,28 +908,81 @@ __global__ void __launch_bounds__(kDecayThreads)
   const float* gB = p.B + ch * kChunk * kChunk;
   const float* gS = p.N + ch * static_cast<size_t>(d) * dv;
   const float* gV = p.Uv + ch * kChunk * dv;
-  copy_rows(sQg, gQg, n * d, tid);
-  copy_tile(sS, gS, d, dv, c0, tid);
-  copy_tile(sV, gV, n, dv, c0, tid);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  // thread: rows i0 .. i0 + 3, columns cc .. cc + 3 (rows at and beyond n hold stale values that are not stored)
-  const int cc = 4 * (tid % 16), i0 = 4 * (tid / 16);
-  if (i0 < n) {
-    float acc[4][4];
+  const int n_state = (d + kOutK - 1) / kOutK, n_slices = n_state + (n + kOutK - 1) / kOutK;
+
+  auto stage = [&](int s) {
+    if (s < n_slices) {
+      float* sA = sm + (s % kOutStages) * kOutStage;  // [C][32]
+      float* sR = sA + kChunk * kOutK;                // [32][64]
+      const bool own = s >= n_state;
+      const int k0 = (own ? s - n_state : s) * kOutK, kn = min(kOutK, (own ? n : d) - k0);
+      const float* a = own ? gB + k0 : gQg + k0;
+      const int lda = own ? kChunk : d, ka = own ? kOutK : kn;  // (B's rows are whole: entries past the diagonal are not read)
+      for (int e = tid; e < n * (kOutK / 4); e += kOutThreads) {
+        const int i = e / (kOutK / 4), c = 4 * (e % (kOutK / 4));
+        if (c < ka) cp_async16(sA + i * kOutK + c, a + static_cast<size_t>(i) * lda + c);
+      }
+      copy_tile<kOutThreads>(sR, (own ? gV : gS) + static_cast<size_t>(k0) * dv, kn, dv, c0, tid);
+    }
+    cp_async_commit();
+  };
+
+  // thread: rows i0 .. i0 + 7, columns cc .. cc + 3 (rows at and beyond n hold stale values that are not stored)
+  const int cc = 4 * (tid % 16), i0 = 8 * (tid / 16);
+  Pair acc[8][2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0ull;
+  // four inner indices from `k` of the slice; with `last`, only those up to last + r enter row r
+  auto four = [&](const float* sA, const float* sR, int k, bool whole, int last) {
+    float4 a[8];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-    product_nn(acc, sQg, d, i0, sS, cc, d, false);
-    product_nn(acc, gB, kChunk, i0, sV, cc, i0 + 4, true);  // (B from the L1 cache: one more block fits an SM)
+    for (int r = 0; r < 8; ++r) a[r] = *reinterpret_cast<const float4*>(sA + (i0 + r) * kOutK + k);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int q = 0; q < 4; ++q) {
+      const Quad b = quad(sR + (k + q) * kDecayTile + cc);
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (i0 + r < n && c0 + cc + c < dv)
-          p.out[static_cast<size_t>(t0 + i0 + r) * (p.H * dv) + h * dv + c0 + cc + c] = acc[r][c];
+      for (int r = 0; r < 8; ++r) {
+        if (!whole && k + q > last + r) continue;
+        const float av = q == 0 ? a[r].x : q == 1 ? a[r].y : q == 2 ? a[r].z : a[r].w;
+        const Pair a2 = pair(av, av);
+        acc[r][0] = fma2(a2, b.lo, acc[r][0]);
+        acc[r][1] = fma2(a2, b.hi, acc[r][1]);
+      }
+    }
+  };
+  for (int s = 0; s < kOutStages - 1; ++s) stage(s);
+  for (int s = 0; s < n_slices; ++s) {
+    cp_async_wait<kOutStages - 2>();
+    __syncthreads();  // slice s has landed for every thread, and slice s - 1's buffer is free
+    stage(s + kOutStages - 1);
+    const float* sA = sm + (s % kOutStages) * kOutStage;
+    const float* sR = sA + kChunk * kOutK;
+    if (i0 >= n) continue;
+    if (s < n_state) {
+      const int kn = min(kOutK, d - s * kOutK);
+      for (int k = 0; k < kn; k += 4) four(sA, sR, k, true, 0);
+    } else {
+      const int last = i0 - (s - n_state) * kOutK;  // of the slice's tokens, the row i0's own
+      int k = 0;
+      for (; k + 3 <= last && k < kOutK; k += 4) four(sA, sR, k, true, 0);
+      for (; k <= last + 7 && k < kOutK; k += 4) four(sA, sR, k, false, last);
+    }
+  }
+  if (i0 >= n) return;
+  const bool pieces = dv % 4 == 0 && reinterpret_cast<uintptr_t>(p.out) % 16 == 0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    if (i0 + r >= n) break;
+    float* o = p.out + static_cast<size_t>(t0 + i0 + r) * (p.H * dv) + h * dv + c0 + cc;
+    const float2 lo = halves(acc[r][0]), hi = halves(acc[r][1]);
+    if (pieces) {
+      if (c0 + cc < dv) *reinterpret_cast<float4*>(o) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    } else {
+      const float v[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (c0 + cc + e < dv) o[e] = v[e];
+    }
   }
 }
 
@@ -1110,8 +1209,14 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   auto allow = [](auto kernel, size_t bytes) {
     return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
-  const size_t sp = prepare_smem(d, RULE), s1 = sizeof(float) * kChunk * (static_cast<size_t>(d) + kDecayTile);
-  const size_t s3 = sizeof(float) * (static_cast<size_t>(kChunk) * d + static_cast<size_t>(d) * kDecayTile + kChunk * kDecayTile);
+  size_t sp = prepare_smem(d, RULE);
+  const size_t with_v = sp + sizeof(float) * kChunk * static_cast<size_t>(a.dv);
+  // (the prepare kernel makes the state's part too where at least two of its blocks share an SM with the values beside the
+  // keys; larger sizes keep the launch of its own, whose blocks split the columns)
+  a.with_state = !DELTA && d % 8 == 0 && a.dv % 8 == 0 && with_v <= 110 * 1024;
+  if (a.with_state) sp = with_v;
+  const size_t s1 = sizeof(float) * kChunk * (static_cast<size_t>(d) + kDecayTile);
+  const size_t s3 = sizeof(float) * kOutStages * kOutStage;
   const int n_buf = delta_chain_smem(d, 2) <= 200 * 1024 ? 2 : 1;
   const size_t s2 = delta_chain_smem(d, n_buf);
   auto chain = d == 128 ? delta_chunk_chain_kernel<128> : d == 64 ? delta_chunk_chain_kernel<64> : delta_chunk_chain_kernel<0>;
@@ -1123,11 +1228,12 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   if (DELTA) {
     launch_pdl(chain, dim3((a.dv + kChainCols - 1) / kChainCols, a.H, a.n_seq), dim3(kChainThreads), s2, stream, a, n_buf);
   } else {
-    launch_pdl(decay_chunk_state_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s1, stream, a);
+    if (!a.with_state)
+      launch_pdl(decay_chunk_state_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s1, stream, a);
     launch_pdl(decay_chunk_scan_kernel, dim3((d * a.dv + kDecayThreads - 1) / kDecayThreads, a.H, a.n_seq),
                dim3(kDecayThreads), 0, stream, a);
   }
-  launch_pdl(decay_chunk_output_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s3, stream, a);
+  launch_pdl(decay_chunk_output_kernel, dim3(n_chunks, a.H, tiles), dim3(kOutThreads), s3, stream, a);
   return launch_status();
 }
 

@@ -248,6 +248,33 @@ def test_decayed_linear_attention_in_chunks(dtype, H, d, dv):
     assert float(state[0].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("d,dv", [(8, 8), (64, 72), (64, 76), (72, 64), (128, 128), (136, 128), (128, 200)])
+def test_chunk_states_in_the_prepare_launch_and_beside_it(d, dv):
+    """The state's part made by the prepare kernel (sizes in whole eights whose operands leave room for two blocks an SM) and by
+    its own launch, column tiles of 64 and what is left of them, inner slices of 32 and what is left, portions that end anywhere
+    in a chunk; values that are infinite after a portion's last token of the chunk reach nothing."""
+    H, T = 2, 230
+    q, k, v = rnd(T, H * d, seed=1), rnd(T, H * d, seed=2), rnd(T, H * dv, seed=3)
+    decay = [0.97, 0.5]
+    want = P.decayed_linear_attention(P.silu(q.double()).view(T, H, d), P.silu(k.double()).view(T, H, d),
+                                      P.silu(v.double()).view(T, H, dv), decay).reshape(T, H * dv)
+    state = torch.zeros(2, H, d, dv, device=DEV)
+    out = torch.full((T, H * dv), float("nan"), device=DEV)
+    t0 = 0
+    for n in [1, 64, 129, 36]:
+        cu, _, sl = batch_index([n], [1])
+        scratch = torch.full((K.recurrent_chunked_scratch_floats([n], H, d, dv, False),), float("inf"), device=DEV)
+        K.recurrent_chunked(q[t0:t0 + n].to(DEV), k[t0:t0 + n].to(DEV), v[t0:t0 + n].to(DEV), state, cu, sl, [n],
+                            out[t0:t0 + n], scratch, H, H, d, dv, decay=torch.tensor(decay, device=DEV))
+        t0 += n
+    close(out, want, torch.float32, "rows", f32=1e-4)
+    s64 = torch.zeros(H, d, dv, dtype=torch.float64)
+    for t in range(T):
+        kk, vv = P.silu(k[t].double()).view(H, d), P.silu(v[t].double()).view(H, dv)
+        s64 = torch.tensor(decay, dtype=torch.float64).view(H, 1, 1) * s64 + kk.unsqueeze(2) * vv.unsqueeze(1)
+    close(state[1], s64, torch.float32, "state", f32=1e-4)
+
+
 # ----------------------------------------------------------------------------- window attention pieces
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,G,d,dv,rot", [(4, 2, 16, 32, 8), (2, 2, 48, 48, 48), (3, 1, 64, 16, 0), (8, 4, 64, 48, 64)])
