@@ -29,8 +29,9 @@ using bf16 = __nv_bfloat16;
 constexpr int kSgRows = 32;     // weight rows per block
 constexpr int kSgChunk = 256;   // columns per pipeline stage
 // Pipeline stages: five for up to 32 tokens (K = 1024 is four chunks: all of a block's weights are
-// requested at once); three for 33..64 tokens, whose activations take most of the shared memory.
-__host__ __device__ constexpr int sg_stages(int mt) { return mt > 4 ? 3 : 5; }
+// requested at once); three for 33..64 tokens, whose activations take most of the shared memory; four for the output head of
+// 9..16 rows, where a block walks many tiles and what counts is a second block on the SM (see skinny_smem).
+__host__ __device__ constexpr int sg_stages(int mt, bool head) { return mt > 4 ? 3 : mt == 2 && head ? 4 : 5; }
 constexpr int kSgWStride = kSgChunk + 8;
 constexpr int kSgThreads = 256;
 constexpr int kSgPieces = kSgRows * (kSgChunk / 8) / kSgThreads;  // 16-byte pieces per thread and chunk
@@ -100,7 +101,8 @@ __device__ __forceinline__ void sg_mma(float* d, const unsigned* a, unsigned b0,
 template <int MT, int MODE>
 struct SkinnyBlock {
   static constexpr int MP = MT * 8;  // padded tokens
-  static constexpr int kSgStages = sg_stages(MT);
+  static constexpr bool kHead = MODE == kSgStoreF32;  // the output head: only the M rows that hold tokens are kept
+  static constexpr int kSgStages = sg_stages(MT, kHead);
   static constexpr int kTileCols = MODE == kSgSwiglu ? 16 : kSgRows;  // output columns of a row tile
   using Args = SkinnyArgsOf<MODE>;
   const Args& args;
@@ -109,7 +111,7 @@ struct SkinnyBlock {
   int K, k0, k1, kx, xs, n_chunks;
   int t0, t_step, my_tiles, total;  // row tiles t0, t0 + t_step, ...; total = my_tiles * n_chunks copies
   bf16* sW;     // [stages][32][264]
-  bf16* sX;     // [MP][xs]
+  bf16* sX;     // [MP][xs]; the head's: [M][xs]
   float* sRed;  // [3][32][MP] column quarters, then up rows
   float* sNw;   // [kx] norm weights of the slice (norm prologue)
   float* sInv;  // [MP] rsqrt(mean(h^2) + eps) of each row (norm prologue): applied to the sums in the epilogue
@@ -126,7 +128,7 @@ struct SkinnyBlock {
     xs = kx + 8;                                                       // row stride of x in shared memory
     sW = reinterpret_cast<bf16*>(smem_raw);
     sX = sW + kSgStages * kSgRows * kSgWStride;
-    sRed = reinterpret_cast<float*>(sX + MP * xs);
+    sRed = reinterpret_cast<float*>(sX + (kHead ? a.M : MP) * xs);
     sNw = sRed + 3 * 32 * MP;
     sInv = sNw + kx;
     n_chunks = kx / kSgChunk;
@@ -193,7 +195,7 @@ __device__ void SkinnyBlock<MT, MODE>::run() const {
   if (total == 0) return;
   // next group: the activations when they are read as bfloat16, else the norm weights
   if (pr.h_in == nullptr) {
-    for (int i = tid; i < MP * (kx / 8); i += kSgThreads) {
+    for (int i = tid; i < (kHead ? M : MP) * (kx / 8); i += kSgThreads) {
       const int m = i / (kx / 8), k = k0 + (i % (kx / 8)) * 8;
       const bool ok = m < M && k < k1;
       sg_cp16(sX + m * xs + (k - k0), pr.x + (ok ? static_cast<size_t>(m) * pr.ldx + k : 0), ok);
@@ -275,6 +277,8 @@ __device__ void SkinnyBlock<MT, MODE>::run() const {
   }
 
   const int ft = warp & 1, kh = warp >> 1;  // row half, column quarter of a chunk
+  // row of x behind token column m: the head's columns beyond its last token repeat that token, nobody reads their sums
+  auto row_of = [&](int m) { return kHead ? min(m, M - 1) : m; };
   float acc[MT][4];
   int c = 0, tile_i = 0;                                                       // chunk and tile being multiplied
   int ld_tile = 0, ld_chunk = 0;                                               // ... and being requested
@@ -316,13 +320,13 @@ __device__ void SkinnyBlock<MT, MODE>::run() const {
       const int kx_col = c * kSgChunk + kcol;
       if (MT == 1) {  // up to 8 tokens: one 8-column operand
         unsigned b0, b1;
-        sg_ldm2(b0, b1, sX + (lane & 7) * xs + kx_col + ((lane >> 3) & 1) * 8);
+        sg_ldm2(b0, b1, sX + row_of(lane & 7) * xs + kx_col + ((lane >> 3) & 1) * 8);
         sg_mma(acc[0], a, b0, b1);
       }
 #pragma unroll
       for (int np = 0; np < MT / 2; ++np) {
         unsigned b0, b1, b2, b3;
-        sg_ldm(b0, b1, b2, b3, sX + (np * 16 + (lane & 7) + (lane >> 4) * 8) * xs + kx_col + ((lane >> 3) & 1) * 8);
+        sg_ldm(b0, b1, b2, b3, sX + row_of(np * 16 + (lane & 7) + (lane >> 4) * 8) * xs + kx_col + ((lane >> 3) & 1) * 8);
         sg_mma(acc[2 * np], a, b0, b1);
         sg_mma(acc[2 * np + 1], a, b2, b3);
       }
@@ -531,17 +535,26 @@ __global__ void __launch_bounds__(kSgThreads) skinny_chain_kernel(const SkinnyCh
     atomicAdd(ch.counter, kChainPerLaunch - static_cast<unsigned long long>(ch.n_phases - 1) * G);
 }
 
+// The head keeps only the M rows that hold tokens and has no norm weights: a block of up to 8 rows whose K is 3,072 takes
+// 93 KB instead of 149 and one of 16 rows whose K is 1,024 (four stages) 107 instead of 128, so that two share an SM and one
+// copies while the other waits at its barriers.  Inside a step, us: one row of 130,049 x 3,072 156 -> 139, 16 rows of
+// 32,784 x 1,024 22 -> 18.  (The layers' products keep whole tiles of rows: blocks as small as one token's let the next
+// launch's blocks in earlier, and a decode step of one request grew from 199 to 204 us, of eight from 909 to 927.)
 inline size_t skinny_smem(int MP, int kx) {
-  return static_cast<size_t>(sg_stages(MP / 8)) * kSgRows * kSgWStride * sizeof(bf16) +
+  return static_cast<size_t>(sg_stages(MP / 8, false)) * kSgRows * kSgWStride * sizeof(bf16) +
          static_cast<size_t>(MP) * (kx + 8) * sizeof(bf16) + 3 * 32 * MP * sizeof(float) +
          static_cast<size_t>(kx + MP) * sizeof(float);
+}
+inline size_t skinny_head_smem(int MP, int M, int kx) {
+  return static_cast<size_t>(sg_stages(MP / 8, true)) * kSgRows * kSgWStride * sizeof(bf16) +
+         static_cast<size_t>(M) * (kx + 8) * sizeof(bf16) + 3 * 32 * MP * sizeof(float);
 }
 
 template <int MT, int MODE>
 int launch_skinny(const SkinnyArgsOf<MODE>& a, int k_max, cudaStream_t stream) {
   constexpr int MP = MT * 8;
   const int kx = (min(a.k_slice, k_max) + kSgChunk - 1) / kSgChunk * kSgChunk;
-  const size_t smem = skinny_smem(MP, kx);
+  const size_t smem = MODE == kSgStoreF32 ? skinny_head_smem(MP, a.M, kx) : skinny_smem(MP, kx);
   if (smem > 220 * 1024) return PMM_ERR_BAD_ARGUMENT;
   auto kern = skinny_gemm_kernel<MT, MODE, false>;
   auto kern_one = skinny_gemm_kernel<MT, MODE, true>;
