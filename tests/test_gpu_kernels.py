@@ -803,6 +803,21 @@ def test_skinny_product_with_float32_output_for_the_head(M, N, Kd):
     assert bool(torch.isnan(out[:, N:]).all())
 
 
+@pytest.mark.parametrize("M,N,Kd", [(1, 12001, 3072), (2, 9601, 1024), (7, 31, 8), (9, 9601, 1024), (11, 70, 1032), (15, 9601, 264), (16, 33, 2048)])
+def test_head_keeps_only_the_rows_that_hold_tokens(M, N, Kd):
+    """Rows on and off whole tiles of 8 and 16, blocks with one tile of weights and with several, K on and off the chunks of
+    256: small whole numbers, so that the sums are exact, and rows whose neighbours hold infinities."""
+    ops = K()
+    g = torch.Generator().manual_seed(M + N + Kd)
+    xw = torch.full((M + 2, Kd), float("inf"), dtype=torch.bfloat16)
+    xw[1:M + 1] = torch.randint(-3, 4, (M, Kd), generator=g).to(torch.bfloat16)
+    w = torch.randint(-3, 4, (N, Kd), generator=g).to(torch.bfloat16)
+    out = torch.full((M, N + 3), float("nan"), device=DEV)
+    ops.skinny_linear_f32(xw.to(DEV)[1:M + 1], w.to(DEV), out[:, :N], 0.5)
+    assert torch.equal(out[:, :N].cpu().double(), 0.5 * (xw[1:M + 1].double() @ w.double().t()))
+    assert bool(torch.isnan(out[:, N:]).all())
+
+
 @pytest.mark.parametrize("T,N,Kd", [(16, 127, 64), (33, 129, 8), (48, 256, 1024), (49, 136, 328), (63, 8, 1016), (64, 4, 2056), (3, 1, 6152)])
 def test_tcgen05_product_in_clusters(T, N, Kd):
     """Blocks of a cluster share K: none of its boxes for some of them, one, four; tiles of 128 rows (64 + 64) and one beside;
