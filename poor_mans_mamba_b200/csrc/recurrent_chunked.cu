@@ -895,9 +895,13 @@ __global__ void __launch_bounds__(kDecayThreads)
 // the inner index.  The operands come in slices of 32 through a ring of three, 48 KB a block, so that four blocks share an SM
 // and the 512 blocks of 2,048 tokens, 8 heads and 128 x 128 states are one wave (whole operands: 80 KB, two blocks, two waves).
 // That size inside a step: 30 -> 27 us (8 x 8 results on two warps a block 29.5: too few warps in flight).
-constexpr int kOutThreads = 128, kOutK = 32, kOutStages = 3;
+// FOURS: four inner indices are summed by themselves before they enter a result, a quarter more instructions and a quarter
+// of the long sum's roundings (the rows' error against float64 at d = 244 behind a given state 2.8e-7 -> 1.7e-7); chosen for the
+// delta rule's keys from kFoursFrom entries on, which were always summed so.
+constexpr int kOutThreads = 128, kOutK = 32, kOutStages = 3, kFoursFrom = 224;
 constexpr int kOutStage = kChunk * kOutK + kOutK * kDecayTile;  // floats
 
+template <bool FOURS>
 __global__ void __launch_bounds__(kOutThreads)
     decay_chunk_output_kernel(ChunkArgs p) {
   extern __shared__ __align__(16) float sm[];
@@ -942,6 +946,27 @@ __global__ void __launch_bounds__(kOutThreads)
     float4 a[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) a[r] = *reinterpret_cast<const float4*>(sA + (i0 + r) * kOutK + k);
+    if constexpr (FOURS) {
+      if (whole) {
+        Quad b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) b[q] = quad(sR + (k + q) * kDecayTile + cc);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float av[4] = {a[r].x, a[r].y, a[r].z, a[r].w};
+          Pair lo = 0ull, hi = 0ull;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const Pair a2 = pair(av[q], av[q]);
+            lo = fma2(a2, b[q].lo, lo);
+            hi = fma2(a2, b[q].hi, hi);
+          }
+          acc[r][0] = fma2(pair(1.f, 1.f), lo, acc[r][0]);
+          acc[r][1] = fma2(pair(1.f, 1.f), hi, acc[r][1]);
+        }
+        return;
+      }
+    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const Quad b = quad(sR + (k + q) * kDecayTile + cc);
@@ -1224,10 +1249,11 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   const size_t s3 = sizeof(float) * kOutStages * kOutStage;
   const int n_buf = delta_chain_smem(d, 2) <= 200 * 1024 ? 2 : 1;
   const size_t s2 = delta_chain_smem(d, n_buf);
+  auto output = DELTA && d >= kFoursFrom ? decay_chunk_output_kernel<true> : decay_chunk_output_kernel<false>;
   auto chain = d == 128 ? delta_chunk_chain_kernel<128> : d == 64 ? delta_chunk_chain_kernel<64> : delta_chunk_chain_kernel<0>;
   cudaError_t e = allow(prep, sp);
   if (e == cudaSuccess) e = DELTA ? allow(chain, s2) : allow(decay_chunk_state_kernel, s1);
-  if (e == cudaSuccess) e = allow(decay_chunk_output_kernel, s3);
+  if (e == cudaSuccess) e = allow(output, s3);
   if (e != cudaSuccess) return static_cast<int>(e);
   launch_pdl(prep, dim3(n_chunks, a.H), dim3(DELTA ? kPrepThreads : RULE == kRuleWkv ? kWkvThreads : kDecayPrepThreads), sp, stream, a);
   if (DELTA) {
@@ -1238,7 +1264,7 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
     launch_pdl(decay_chunk_scan_kernel, dim3((d * a.dv + kDecayThreads - 1) / kDecayThreads, a.H, a.n_seq),
                dim3(kDecayThreads), 0, stream, a);
   }
-  launch_pdl(decay_chunk_output_kernel, dim3(n_chunks, a.H, tiles), dim3(kOutThreads), s3, stream, a);
+  launch_pdl(output, dim3(n_chunks, a.H, tiles), dim3(kOutThreads), s3, stream, a);
   return launch_status();
 }
 

@@ -252,6 +252,23 @@ def test_gated_delta_rule_solve_rounds_a_row_once(d):
     assert float((state[1].cpu().double() - s64).norm() / s64.norm()) < 2.2 * 2.0 ** -24
 
 
+@pytest.mark.parametrize("d", [224, 244])
+def test_gated_delta_rule_read_out_of_long_keys(d):
+    """A given state read out by keys of 224 entries and more, no decay, no writes (beta zero, values zero): a sum of d random
+    terms.  One after the other they measured 2.8e-7, in fours 1.7e-7; the bound lies between, at 3.7 half units in the last place."""
+    H, n, dv = 4, 64, 64
+    q, s0 = rnd(n, H * d, seed=d), torch.randn(2, H, d, dv, generator=torch.Generator().manual_seed(d + 1))
+    state, out = s0.to(DEV), torch.empty(n, H * dv, device=DEV)
+    cu, _, sl = batch_index([n], [1])
+    scratch = torch.empty(K.recurrent_chunked_scratch_floats([n], H, d, dv, True), device=DEV)
+    K.recurrent_chunked(q.to(DEV), q.to(DEV), torch.zeros(n, H * dv, device=DEV), state, cu, sl, [n], out, scratch, H, H, d, dv,
+                        beta=torch.full((n, H), -200.0, device=DEV), a=torch.zeros(n, H * d, device=DEV),
+                        dt_bias=torch.full((H * d,), -30.0, device=DEV), a_log=torch.zeros(H, device=DEV))
+    qq = q.double().view(n, H, d)
+    want = torch.einsum("nhd,hdv->nhv", qq / qq.norm(dim=-1, keepdim=True), s0[1].double()).reshape(n, H * dv)
+    assert float((out.cpu().double() - want).norm() / want.norm()) < 3.7 * 2.0 ** -24
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,d,dv", [(2, 16, 24), (4, 32, 32), (1, 100, 7), (3, 4, 130)])
 def test_decayed_linear_attention_in_chunks(dtype, H, d, dv):
