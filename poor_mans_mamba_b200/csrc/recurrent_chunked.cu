@@ -30,6 +30,7 @@
 // Chunks start at the portion's first token; results do not depend on where a portion is cut beyond
 // rounding.
 #include "recurrence_rules.cuh"
+#include <type_traits>
 
 namespace pmm {
 
@@ -123,7 +124,9 @@ __device__ __forceinline__ Quad quad(const float* p) {  // sixteen bytes
 // its transpose, which lies where q was (its entries wait in registers until q is done).  A row is its sum taken off in one
 // subtraction: a subtraction a term rounds the whole row up to 63 times (error of the states against float64 after 600
 // tokens of weak decays 1.9e-7 at d = 64 to 244, so 1.5e-7, at the same speed).
-// Rows from the chunk's end on are made as zeros, so that the chain kernel needs no count of rows.
+// A chunk of n tokens makes rows up to the next multiple of 16 (chunk_rows), those from n on as zeros; the chain takes as many.
+// All 64 rows of every chunk cost a step of one portion of 512 tokens beside 63 lone ones, 4 heads of 244 x 244, 703 us where
+// 587 us are enough.
 //
 // Bound by the issue of its own instructions; 256 threads and 109 KB at d = 128 put two blocks on an SM, so that one
 // block's barriers and shared-memory latencies are the other's turn and the 256 blocks of 2,048 tokens and 8 heads are one
@@ -132,6 +135,9 @@ __device__ __forceinline__ Quad quad(const float* p) {  // sixteen bytes
 // instruction cache, one block an SM) 96 us, this form 64 us.
 constexpr float kLogDecayMin = -1e4f;  // a token's logarithm to base 2: the power is zero long before, and sums stay finite
 constexpr int kPrepRows = kChunk / 8;  // halves of 8 tokens
+
+// Rows of the operands that a chunk of n tokens fills: the solve's and the chain's steps are whole sixteens.
+__device__ __forceinline__ int chunk_rows(int n) { return (n + 15) & ~15; }
 
 inline size_t delta_prepare_smem(int d) {
   const size_t row = static_cast<size_t>(d) + 4;
@@ -167,7 +173,7 @@ struct CrossPairs {
   int slice, i0, j0;
   float keep[kKeep];
   __device__ __forceinline__ void run(const float* __restrict__ sQ, const float* __restrict__ sK, const float* __restrict__ sKd,
-                                      float* __restrict__ oB, int ds, int d4, int n, int tid) {
+                                      float* __restrict__ oB, int ds, int d4, int n, int rows, int tid) {
     const int tile = tid / kSlices, g = tile / (kSide * kSide), in = tile % (kSide * kSide);
     slice = tid % kSlices;
     i0 = 2 * HALF * g + HALF + 4 * (in / kSide);
@@ -175,7 +181,8 @@ struct CrossPairs {
     Pair acc[32];
 #pragma unroll
     for (int e = 0; e < 32; ++e) acc[e] = 0;
-    for (int c4 = slice; c4 < d4; c4 += kSlices) {
+    const int c_end = i0 < rows ? d4 : 0;  // (a tile behind the last row: zeros, its lanes stay for the sums)
+    for (int c4 = slice; c4 < c_end; c4 += kSlices) {
       Quad kd[4];
 #pragma unroll
       for (int s = 0; s < 4; ++s) kd[s] = quad(sKd + (j0 + s) * ds + 4 * c4);
@@ -232,6 +239,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int kWarps = kPrepThreads / 32;
   const size_t ch = static_cast<size_t>(chunk) * p.H + h;
+  const int rows = chunk_rows(n);
   float* oB = p.B + ch * kChunk * kChunk;
   const bool vec = p.vec_in != 0;
   constexpr float kLog2E = 1.4426950408889634f;
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   // ---- unit-length q and k and the decays' logarithms: a warp per token
   const float a_neg = -expf(p.a_log[h]) * kLog2E;
 #pragma unroll 2
-  for (int i = warp; i < kChunk; i += kWarps) {
+  for (int i = warp; i < rows; i += kWarps) {
     float *rq = sQ + i * ds, *rk = sK + i * ds, *rl = sL + i * ds;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i >= n) {
@@ -281,10 +289,12 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   for (int blk = warp; blk < kPrepRows; blk += kWarps) {  // running sums within 8 tokens
     for (int c = lane; c < d; c += 32) {
       float run = 0.f;
+      if (8 * blk < rows) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        run += sL[(8 * blk + i) * ds + c];
-        sL[(8 * blk + i) * ds + c] = run;
+        for (int i = 0; i < 8; ++i) {
+          run += sL[(8 * blk + i) * ds + c];
+          sL[(8 * blk + i) * ds + c] = run;
+        }
       }
       sT[blk * d + c] = run;
     }
@@ -297,7 +307,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   for (int u = 0; u < kChunk * 8 / kPrepThreads; ++u) {
     const int e = tid + kPrepThreads * u, i = e >> 3, j = (i & ~7) + (e & 7);
     own_a[u] = 0.f;
-    if (j <= i) {
+    if (j <= i && i < rows) {
       const float *qi = sQ + i * ds, *ki = sK + i * ds, *li = sL + i * ds, *kj = sK + j * ds, *lj = sL + j * ds;
       Pair accA = 0, accB = 0;
 #pragma unroll 2
@@ -319,7 +329,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
     *reinterpret_cast<float4*>(at) = make_float4(v.x * f.x, v.y * f.y, v.z * f.z, v.w * f.w);
   };
   auto power = [](const float4& l) { return make_float4(exp2f(l.x), exp2f(l.y), exp2f(l.z), exp2f(l.w)); };
-  for (int i = warp; i < kChunk; i += kWarps) {
+  for (int i = warp; i < rows; i += kWarps) {
     for (int c = 4 * lane; c < d; c += 128) {
       const float4 l = *reinterpret_cast<const float4*>(sL + i * ds + c), t = *reinterpret_cast<const float4*>(sT + (i >> 3) * d + c);
       const float4 k = *reinterpret_cast<const float4*>(sK + i * ds + c);
@@ -345,7 +355,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   // ---- pairs across halves of 8, 16 and 32 tokens; after each, rows reach through the neighbouring half
   auto widen = [&](int half, int first_total) {
     __syncthreads();
-    for (int i = warp; i < kChunk; i += kWarps) {
+    for (int i = warp; i < rows; i += kWarps) {
       const int b = i / half;
       for (int c = 4 * lane; c < d; c += 128) {
         const float4 f = *reinterpret_cast<const float4*>(sT + (first_total + (b ^ 1)) * d + c);
@@ -360,19 +370,23 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
     __syncthreads();
   };
   CrossPairs<8> by8;
-  by8.run(sQ, sK, sL, oB, ds, d4, n, tid);
+  by8.run(sQ, sK, sL, oB, ds, d4, n, rows, tid);
   widen(8, 0);
   CrossPairs<16> by16;
-  by16.run(sQ, sK, sL, oB, ds, d4, n, tid);
-  widen(16, 8);
   CrossPairs<32> by32;
-  by32.run(sQ, sK, sL, oB, ds, d4, n, tid);
-  widen(32, 12);
+  if (rows > 16) {  // (behind the last row the totals are zero, their powers one)
+    by16.run(sQ, sK, sL, oB, ds, d4, n, rows, tid);
+    widen(16, 8);
+  }
+  if (rows > 32) {
+    by32.run(sQ, sK, sL, oB, ds, d4, n, rows, tid);
+    widen(32, 12);
+  }
 
   // ---- what the other launches read; V takes the place of K * exp(L_end - L), A that of q
   float* oQg = p.Qg + ch * kChunk * d;
   float* oKe = p.Ke + ch * kChunk * d;
-  for (int i = warp; i < kChunk; i += kWarps) {
+  for (int i = warp; i < rows; i += kWarps) {
     for (int c = 4 * lane; c < d; c += 128) {
       *reinterpret_cast<float4*>(oQg + i * d + c) = *reinterpret_cast<const float4*>(sQ + i * ds + c);
       *reinterpret_cast<float4*>(oKe + i * d + c) = *reinterpret_cast<const float4*>(sL + i * ds + c);
@@ -380,19 +394,19 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   }
   __syncthreads();
   by8.leave(sAt);
-  by16.leave(sAt);
-  by32.leave(sAt);
+  if (rows > 16) by16.leave(sAt);
+  if (rows > 32) by32.leave(sAt);
 #pragma unroll
   for (int u = 0; u < kChunk * 8 / kPrepThreads; ++u) {
     const int e = tid + kPrepThreads * u, i = e >> 3, j = (i & ~7) + (e & 7);
-    if (j <= i) sAt[j * kChunk + i] = own_a[u];  // (the diagonal's is not read for a result)
+    if (j <= i && i < rows) sAt[j * kChunk + i] = own_a[u];  // (the diagonal's is not read for a result)
   }
 
   // ---- T X = diag(beta) [K * exp L | V] by forward substitution, V's columns d at a time
   const S* gv = static_cast<const S*>(p.v) + static_cast<long long>(t0) * p.ld_v + h * dv;
   for (int v0 = 0; v0 < dv; v0 += d) {
     const int vw = min(d, dv - v0);
-    for (int i = warp; i < kChunk; i += kWarps)
+    for (int i = warp; i < rows; i += kWarps)
       for (int c = lane; c < vw; c += 32) sL[i * ds + c] = i < n ? ldf(gv + static_cast<long long>(i) * p.ld_v + v0 + c) : 0.f;
     __syncthreads();
     const int n_w = v0 == 0 ? d : 0;  // the first pass also solves for W
@@ -403,7 +417,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
       float* to = is_w ? p.W + ch * kChunk * d + c : p.Uv + ch * kChunk * dv + v0 + c;
       const int ld = is_w ? d : dv;
 #pragma unroll 1
-      for (int b0 = 0; b0 < kChunk; b0 += 16) {
+      for (int b0 = 0; b0 < rows; b0 += 16) {
         float in[16];
         Pair r[8];   // what the rows solved before add up to, taken off in one subtraction
 #pragma unroll
@@ -1056,13 +1070,19 @@ __global__ void __launch_bounds__(kChainThreads)
   const int n_chunks = (len + kChunk - 1) / kChunk;
   float* st = p.state + ((static_cast<size_t>(p.slots[seq]) * p.H + h) * d) * dv;
   auto unit = [&](int ci) { return static_cast<size_t>(chunk0 + ci) * p.H + h; };
+  const int n_full = len / kChunk, last_rows = chunk_rows(len - n_full * kChunk);
   auto fetch = [&](int ci) {
     const float *gW = p.W + unit(ci) * kChunk * d, *gKe = p.Ke + unit(ci) * kChunk * d;
     float* dst = sIn + static_cast<size_t>(ci % n_buf) * 2 * kChunk * d;
-#pragma unroll 4
-    for (int e = tid; e < kChunk * d4; e += kChainThreads) {
+    auto copy = [&](int e) {
       cp_async16(dst + 4 * e, gW + 4 * e);
       cp_async16(dst + kChunk * d + 4 * e, gKe + 4 * e);
+    };
+    if (ci < n_full) {
+#pragma unroll 4
+      for (int e = tid; e < kChunk * d4; e += kChainThreads) copy(e);
+    } else {
+      for (int e = tid; e < last_rows * d4; e += kChainThreads) copy(e);
     }
     cp_async_commit();
   };
@@ -1090,13 +1110,16 @@ __global__ void __launch_bounds__(kChainThreads)
     }
   };
   read_ahead(0);
-  for (int ci = 0; ci < n_chunks; ++ci) {
+  // (a sequence's last chunk may hold fewer rows; with their count known when compiling the others' links are 4 % shorter)
+  auto link = [&](int ci, auto full) {
+    constexpr bool FULL = decltype(full)::value;
+    const int rows = FULL ? kChunk : last_rows;
     cp_async_wait<0>();
     __syncthreads();        // W and Ke of this chunk and everyone's rows of S are there; everyone is done with the chunk before
     if (n_buf > 1 && ci + 1 < n_chunks) fetch(ci + 1);
     const float* W = sIn + static_cast<size_t>(ci % n_buf) * 2 * kChunk * d;
     const float* Ke = W + kChunk * d;
-    {
+    if (FULL || 8 * warp < rows) {
       Pair acc[4][4];
 #pragma unroll
       for (int r = 0; r < 4; ++r)
@@ -1156,8 +1179,7 @@ __global__ void __launch_bounds__(kChainThreads)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[0][c] = acc[1][c] = 0;
       if (mine) {
-#pragma unroll 8
-        for (int j = s_slice; j < kChunk; j += 4) {
+        auto add_row = [&](int j) {
           const Quad k = quad(Ke + j * d + 4 * m);
           const float* u = sU + 2 * (j * kChainCols + s_col);
           const Quad u01 = quad(u), u23 = quad(u + 4);
@@ -1167,6 +1189,13 @@ __global__ void __launch_bounds__(kChainThreads)
             acc[0][c] = fma2(k.lo, uu[c], acc[0][c]);
             acc[1][c] = fma2(k.hi, uu[c], acc[1][c]);
           }
+        };
+        if constexpr (FULL) {
+#pragma unroll 8
+          for (int j = s_slice; j < kChunk; j += 4) add_row(j);
+        } else {
+#pragma unroll 4
+          for (int j = s_slice; j < rows; j += 4) add_row(j);
         }
       }
       float v[4][4];
@@ -1208,7 +1237,9 @@ __global__ void __launch_bounds__(kChainThreads)
       __syncthreads();      // everyone is done with the one buffer
       fetch(ci + 1);
     }
-  }
+  };
+  for (int ci = 0; ci < n_full; ++ci) link(ci, std::true_type{});
+  if (n_full < n_chunks) link(n_full, std::false_type{});
   __syncthreads();
   for (int e = tid; e < d * kChainCols; e += kChainThreads) {
     const int r = e / kChainCols, c = e % kChainCols;

@@ -269,6 +269,54 @@ def test_gated_delta_rule_read_out_of_long_keys(d):
     assert float((out.cpu().double() - want).norm() / want.norm()) < 3.7 * 2.0 ** -24
 
 
+def _delta_operands(lens, H, d, dv, dtype=torch.float32):
+    T = sum(lens)
+    q, k, v, a, beta = (rnd(T, n, seed=i).to(DEV, dtype) for i, n in enumerate((H * d, H * d, H * dv, H * d, H)))
+    state = (rnd(len(lens) + 1, H, d, dv, seed=8) * 0.1).to(DEV)
+    cu, _, sl = batch_index(lens, list(range(1, len(lens) + 1)))
+    return q, k, v, a, beta, (rnd(H * d, seed=6) - 1.0).to(DEV), rnd(H, seed=7).to(DEV), state, cu, sl
+
+
+@pytest.mark.parametrize("d,dv", [(64, 64), (128, 40), (244, 8)])
+def test_gated_delta_rule_chunks_that_are_not_full(d, dv):
+    """Portions on both sides of every sixteen rows, alone and behind a full chunk, in one batch: the rows behind a portion's last
+    sixteen are neither made nor read (the scratch is not a number).  Tolerance: float sums of up to 80 tokens and 244 channels
+    in another order, relative to the largest entry."""
+    H, lens = 2, [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 80]
+    q, k, v, a, beta, dt_bias, a_log, state, cu, sl = _delta_operands(lens, H, d, dv)
+    serial, out, want = state.clone(), torch.empty(sum(lens), H * dv, device=DEV), torch.empty(sum(lens), H * dv, device=DEV)
+    scratch = torch.full((K.recurrent_chunked_scratch_floats(lens, H, d, dv, True),), float("nan"), device=DEV)
+    K.recurrent_chunked(q, k, v, state, cu, sl, lens, out, scratch, H, H, d, dv, beta=beta, a=a, dt_bias=dt_bias, a_log=a_log,
+                        unit_eps=1e-6, q_scale=d ** -0.5)
+    K.delta_scan(q, k, v, beta, a, dt_bias, a_log, serial, cu, sl, len(lens), want, H, H, d, dv, 1e-6, d ** -0.5)
+    for x, y in ((out, want), (state, serial)):
+        assert float((x - y).abs().max()) <= 2e-5 * max(1.0, float(y.abs().max()))
+
+
+def test_gated_delta_rule_of_lone_tokens_is_not_a_whole_chunk_each():
+    """Requests with one token beside a prompt portion go through the chunked form with it: what they cost is their rows', not 64
+    rows' (the ratio of a step of lone tokens to one of whole chunks, medians on the device: 0.82 where every chunk's 64 rows are
+    made, 0.51 where 16 are)."""
+    H, d, dv = 4, 244, 64
+    took = {}
+    for n in (1, 64):
+        lens = [n] * 128
+        q, k, v, a, beta, dt_bias, a_log, state, cu, sl = _delta_operands(lens, H, d, dv)
+        out = torch.empty(sum(lens), H * dv, device=DEV)
+        scratch = torch.empty(K.recurrent_chunked_scratch_floats(lens, H, d, dv, True), device=DEV)
+        times = []
+        for _ in range(9):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            K.recurrent_chunked(q, k, v, state, cu, sl, lens, out, scratch, H, H, d, dv, beta=beta, a=a, dt_bias=dt_bias,
+                                a_log=a_log, unit_eps=1e-6, q_scale=d ** -0.5)
+            t1.record()
+            torch.cuda.synchronize()
+            times.append(t0.elapsed_time(t1))
+        took[n] = sorted(times)[4]
+    assert took[1] < 0.65 * took[64], took
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,d,dv", [(2, 16, 24), (4, 32, 32), (1, 100, 7), (3, 4, 130)])
 def test_decayed_linear_attention_in_chunks(dtype, H, d, dv):
