@@ -30,6 +30,7 @@
 // Chunks start at the portion's first token; results do not depend on where a portion is cut beyond
 // rounding.
 #include "recurrence_rules.cuh"
+#include <algorithm>
 #include <type_traits>
 
 namespace pmm {
@@ -54,6 +55,7 @@ struct ChunkArgs {
   float unit_eps, q_scale;
   // per (chunk, head), chunk-major: W [C, d] (delta), Uv [C, dv], B [C, C], Qg [C, d], Ke [C, d], Eg [d]
   float *W, *Uv, *B, *Qg, *Ke, *Eg;
+  int tile0;                            // first column tile of the launch (a grid holds 65,535)
   int with_state;                       // the prepare kernel makes N too (see chunk_state)
   int vec_in;                           // q, k, v (and a) rows and heads start on boundaries of four elements
   float* N;                             // [d, dv] per (chunk, head): see the kernels that use it
@@ -837,7 +839,7 @@ __global__ void __launch_bounds__(kDecayThreads)
   float* sV = sKe + kChunk * d;       // [C][tile]
   pdl_launch_dependents();
   pdl_wait();
-  const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kDecayTile;
+  const int chunk = blockIdx.x, h = blockIdx.y, c0 = (p.tile0 + blockIdx.z) * kDecayTile;
   int seq, t0, n;
   if (!locate_chunk(p.cu, p.n_seq, chunk, &seq, &t0, &n)) return;
   const int tid = threadIdx.x;
@@ -922,7 +924,7 @@ __global__ void __launch_bounds__(kOutThreads)
   const int d = p.d, dv = p.dv;
   pdl_launch_dependents();
   pdl_wait();
-  const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kDecayTile;
+  const int chunk = blockIdx.x, h = blockIdx.y, c0 = (p.tile0 + blockIdx.z) * kDecayTile;
   int seq, t0, n;
   if (!locate_chunk(p.cu, p.n_seq, chunk, &seq, &t0, &n)) return;
   const int tid = threadIdx.x;
@@ -1258,7 +1260,6 @@ template <typename S, int RULE>
 int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   constexpr bool DELTA = RULE == kRuleDelta;
   const int d = a.d, tiles = (a.dv + kDecayTile - 1) / kDecayTile;
-  if (tiles > 65535) return PMM_ERR_BAD_ARGUMENT;
   void (*prep)(ChunkArgs) = nullptr;
   if constexpr (RULE == kRuleWkv) prep = wkv_prepare_kernel<S>;
   else if constexpr (DELTA) prep = delta_prepare_kernel<S>;
@@ -1286,16 +1287,19 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   if (e == cudaSuccess) e = DELTA ? allow(chain, s2) : allow(decay_chunk_state_kernel, s1);
   if (e == cudaSuccess) e = allow(output, s3);
   if (e != cudaSuccess) return static_cast<int>(e);
+  auto for_tiles = [&](auto launch) {
+    for (a.tile0 = 0; a.tile0 < tiles; a.tile0 += 65535) launch(std::min(tiles - a.tile0, 65535));
+  };
   launch_pdl(prep, dim3(n_chunks, a.H), dim3(DELTA ? kPrepThreads : RULE == kRuleWkv ? kWkvThreads : kDecayPrepThreads), sp, stream, a);
   if (DELTA) {
     launch_pdl(chain, dim3((a.dv + kChainCols - 1) / kChainCols, a.H, a.n_seq), dim3(kChainThreads), s2, stream, a, n_buf);
   } else {
     if (!a.with_state)
-      launch_pdl(decay_chunk_state_kernel, dim3(n_chunks, a.H, tiles), dim3(kDecayThreads), s1, stream, a);
+      for_tiles([&](int n) { launch_pdl(decay_chunk_state_kernel, dim3(n_chunks, a.H, n), dim3(kDecayThreads), s1, stream, a); });
     launch_pdl(decay_chunk_scan_kernel, dim3((d * a.dv + kDecayThreads - 1) / kDecayThreads, a.H, a.n_seq),
                dim3(kDecayThreads), 0, stream, a);
   }
-  launch_pdl(output, dim3(n_chunks, a.H, tiles), dim3(kOutThreads), s3, stream, a);
+  for_tiles([&](int n) { launch_pdl(output, dim3(n_chunks, a.H, n), dim3(kOutThreads), s3, stream, a); });
   return launch_status();
 }
 

@@ -365,6 +365,23 @@ def test_chunk_states_in_the_prepare_launch_and_beside_it(d, dv):
     close(state[1], s64, torch.float32, "state", f32=1e-4)
 
 
+def test_decayed_sum_of_more_column_tiles_than_a_grid_is_deep():
+    """65,536 tiles of 64 value columns and one column more: three tokens against the formula, rows and state."""
+    H, n, d, dv = 1, 3, 4, 65536 * 64 + 1
+    q, k = rnd(n, d, seed=1), rnd(n, d, seed=2)
+    v = torch.randn(n, dv, generator=torch.Generator(device=DEV).manual_seed(3), device=DEV)
+    state, out = torch.zeros(1, H, d, dv, device=DEV), torch.full((n, dv), float("nan"), device=DEV)
+    cu, _, sl = batch_index([n], [0])
+    scratch = torch.empty(K.recurrent_chunked_scratch_floats([n], H, d, dv, False), device=DEV)
+    K.recurrent_chunked(q.to(DEV), k.to(DEV), v, state, cu, sl, [n], out, scratch, H, H, d, dv, decay=torch.tensor([0.5], device=DEV))
+    s64 = torch.zeros(d, dv, dtype=torch.float64, device=DEV)
+    for t in range(n):
+        s64 = 0.5 * s64 + P.silu(k[t].double()).to(DEV).unsqueeze(1) * P.silu(v[t].double()).unsqueeze(0)
+        want = (P.silu(q[t].double()).to(DEV).unsqueeze(1) * s64).sum(0)
+        assert float((out[t].double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+    assert float((state[0, 0].double() - s64).abs().max()) <= 1e-5 * float(s64.abs().max())
+
+
 # ----------------------------------------------------------------------------- window attention pieces
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,G,d,dv,rot", [(4, 2, 16, 32, 8), (2, 2, 48, 48, 48), (3, 1, 64, 16, 0), (8, 4, 64, 48, 64)])
