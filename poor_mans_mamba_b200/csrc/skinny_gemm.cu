@@ -21,6 +21,7 @@
 // multipliers, SiLU and adds separate launches, src/ops/cuda_backend.cu:311-338.)
 #include "common.cuh"
 #include <algorithm>
+#include <atomic>
 
 namespace pmm {
 
@@ -550,31 +551,49 @@ inline size_t skinny_head_smem(int MP, int M, int kx) {
          static_cast<size_t>(M) * (kx + 8) * sizeof(bf16) + 3 * 32 * MP * sizeof(float);
 }
 
+// Every call opts in to the same size: were it the call's own, a thread with fewer rows could lower the kernel's limit between
+// another thread's opt-in and its launch, which would then be refused.
+constexpr int kSgMaxSmem = 220 * 1024;
+template <typename F>
+inline cudaError_t sg_opt_in(F kern) {
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgMaxSmem);
+  return e == cudaSuccess ? cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100) : e;
+}
+
+// How many blocks of `smem` bytes are resident on the device at once; 0: the question failed.  The last answer stays in `seen`,
+// device, size and count in one word, so that threads never meet half of one.
+template <typename F>
+inline int sg_resident(F kern, size_t smem, std::atomic<unsigned long long>& seen) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const unsigned long long key = static_cast<unsigned long long>(dev) << 56 | static_cast<unsigned long long>(smem) << 32;
+  const unsigned long long last = seen.load(std::memory_order_relaxed);
+  if (last != 0 && (last >> 32) == (key >> 32)) return static_cast<int>(last & 0xffffffffu);
+  int per_sm = 0, n_sm = 0;
+  if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSgThreads, smem) != cudaSuccess)
+    return 0;
+  seen.store(key | static_cast<unsigned>(per_sm * n_sm), std::memory_order_relaxed);
+  return per_sm * n_sm;
+}
+
 template <int MT, int MODE>
 int launch_skinny(const SkinnyArgsOf<MODE>& a, int k_max, cudaStream_t stream) {
   constexpr int MP = MT * 8;
   const int kx = (min(a.k_slice, k_max) + kSgChunk - 1) / kSgChunk * kSgChunk;
   const size_t smem = MODE == kSgStoreF32 ? skinny_head_smem(MP, a.M, kx) : skinny_smem(MP, kx);
-  if (smem > 220 * 1024) return PMM_ERR_BAD_ARGUMENT;
+  if (smem > kSgMaxSmem) return PMM_ERR_BAD_ARGUMENT;
   auto kern = skinny_gemm_kernel<MT, MODE, false>;
   auto kern_one = skinny_gemm_kernel<MT, MODE, true>;
   for (auto k : {kern, kern_one}) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    const cudaError_t e = sg_opt_in(k);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  // no more blocks than are resident at once; each walks the row tiles bx, bx + gridDim.x, ...
-  static size_t seen_smem = ~size_t(0);
-  static int slots = 0;
-  if (seen_smem != smem) {
-    int per_sm = 0, n_sm = 0, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSgThreads, smem) != cudaSuccess || per_sm < 1)
-      return PMM_ERR_BAD_ARGUMENT;
-    slots = per_sm * n_sm;
-    seen_smem = smem;
-  }
+  // no more blocks than are resident at once; each walks the row tiles bx, bx + gridDim.x, ...  (The head's blocks differ in size
+  // from row count to row count: an answer for each.)
+  static std::atomic<unsigned long long> seen[MODE == kSgStoreF32 ? 8 : 1];
+  const int slots = sg_resident(kern, smem, seen[MODE == kSgStoreF32 ? a.M % 8 : 0]);
+  if (slots < 1) return PMM_ERR_BAD_ARGUMENT;
   const int cols_per_tile = MODE == kSgSwiglu ? 16 : kSgRows;
   const int n_tx = (a.N + cols_per_tile - 1) / cols_per_tile;
   const int gy = (k_max + a.k_slice - 1) / a.k_slice;
@@ -598,8 +617,7 @@ int dispatch_skinny(const SkinnyArgsOf<MODE>& a, int k_max, cudaStream_t stream)
 template <int MT>
 int launch_chain(const SkinnyChain& ch, size_t smem, int grid, cudaStream_t stream) {
   auto kern = skinny_chain_kernel<MT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  cudaError_t e = sg_opt_in(kern);
   if (e != cudaSuccess) return static_cast<int>(e);
   // every block must be resident at once: the barriers wait for all of them
   int per_sm = 0;
@@ -777,7 +795,7 @@ PMM_EXPORT int pmm_skinny_chain(const PmmSkinnyPhase* phases, int n_phases, int 
     const int blocks = ch.gx[p] * ch.gy[p] * ch.gz[p];
     if (blocks > most) most = blocks;
   }
-  if (smem > 220 * 1024) return PMM_ERR_BAD_ARGUMENT;
+  if (smem > pmm::kSgMaxSmem) return PMM_ERR_BAD_ARGUMENT;
   int grid = most < n_sm ? most : n_sm;
   if (grid > 1024) grid = 1024;  // the counter arithmetic allows 3 * 1024 arrivals a launch
   return pmm::launch_chain<2>(ch, smem, grid, stream);

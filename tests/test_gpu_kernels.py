@@ -818,6 +818,37 @@ def test_head_keeps_only_the_rows_that_hold_tokens(M, N, Kd):
     assert bool(torch.isnan(out[:, N:]).all())
 
 
+def test_head_of_two_threads_with_different_rows():
+    """Two host threads launch the head with 1 and 8 rows of 3,072 on streams of their own, as fast as they can: neither may lower what
+    the other's launch was allowed in shared memory between that thread's asking and its launch (which would be refused)."""
+    import threading
+    ops = K()
+    w = torch.randint(-3, 4, (64, 3072), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    launch = ops._fn("pmm_skinny_gemm_f32out")
+    torch.cuda.synchronize()
+    failed, ready = [], threading.Barrier(2)
+
+    def serve(rows):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            x = torch.randint(-3, 4, (rows, 3072), generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).to(DEV)
+            out = torch.empty(rows, 64, device=DEV)
+            want = x.double() @ w.double().t()
+            args = (rows, 64, x.data_ptr(), 3072, w.data_ptr(), 3072, 1.0, 0.0, out.data_ptr(), 64, stream.cuda_stream)
+            ready.wait(30)
+            codes = {launch(*args) for _ in range(20000)}
+            stream.synchronize()
+        if codes != {0} or not torch.equal(out.double(), want):
+            failed.append((rows, codes))
+
+    threads = [threading.Thread(target=serve, args=(n,)) for n in (1, 8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+
+
 @pytest.mark.parametrize("T,N,Kd", [(16, 127, 64), (33, 129, 8), (48, 256, 1024), (49, 136, 328), (63, 8, 1016), (64, 4, 2056), (3, 1, 6152)])
 def test_tcgen05_product_in_clusters(T, N, Kd):
     """Blocks of a cluster share K: none of its boxes for some of them, one, four; tiles of 128 rows (64 + 64) and one beside;
