@@ -31,8 +31,8 @@ constexpr int kSgRows = 32;     // weight rows per block
 constexpr int kSgChunk = 256;   // columns per pipeline stage
 // Pipeline stages: five for up to 32 tokens (K = 1024 is four chunks: all of a block's weights are
 // requested at once); three for 33..64 tokens, whose activations take most of the shared memory; four for the output head of
-// 9..16 rows, where a block walks many tiles and what counts is a second block on the SM (see skinny_smem).
-__host__ __device__ constexpr int sg_stages(int mt, bool head) { return mt > 4 ? 3 : mt == 2 && head ? 4 : 5; }
+// 9..16 rows where that makes room for a second block on the SM (see skinny_head_smem).
+__host__ __device__ constexpr int sg_stages(int mt) { return mt > 4 ? 3 : 5; }
 constexpr int kSgWStride = kSgChunk + 8;
 constexpr int kSgThreads = 256;
 constexpr int kSgPieces = kSgRows * (kSgChunk / 8) / kSgThreads;  // 16-byte pieces per thread and chunk
@@ -99,11 +99,11 @@ __device__ __forceinline__ void sg_mma(float* d, const unsigned* a, unsigned b0,
 }
 
 // What a block needs to know about its place: which slice of K, which product, which row tiles.
-template <int MT, int MODE>
+template <int MT, int MODE, int STAGES = sg_stages(MT)>
 struct SkinnyBlock {
   static constexpr int MP = MT * 8;  // padded tokens
   static constexpr bool kHead = MODE == kSgStoreF32;  // the output head: only the M rows that hold tokens are kept
-  static constexpr int kSgStages = sg_stages(MT, kHead);
+  static constexpr int kSgStages = STAGES;
   static constexpr int kTileCols = MODE == kSgSwiglu ? 16 : kSgRows;  // output columns of a row tile
   using Args = SkinnyArgsOf<MODE>;
   const Args& args;
@@ -188,9 +188,9 @@ struct SkinnyBlock {
   __device__ void finish_tile(float (&acc)[MT][4], int n0) const;
 };
 
-template <int MT, int MODE>
+template <int MT, int MODE, int STAGES>
 template <bool ONE>
-__device__ void SkinnyBlock<MT, MODE>::run() const {
+__device__ void SkinnyBlock<MT, MODE, STAGES>::run() const {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int M = args.M;
   if (total == 0) return;
@@ -343,8 +343,8 @@ __device__ void SkinnyBlock<MT, MODE>::run() const {
 }
 
 // The sums of one row tile -> their place (the next tile's copies are in flight meanwhile).
-template <int MT, int MODE>
-__device__ void SkinnyBlock<MT, MODE>::finish_tile(float (&acc)[MT][4], int n0) const {
+template <int MT, int MODE, int STAGES>
+__device__ void SkinnyBlock<MT, MODE, STAGES>::finish_tile(float (&acc)[MT][4], int n0) const {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int M = args.M;
   const int ft = warp & 1, kh = warp >> 1;
@@ -433,11 +433,11 @@ __device__ void SkinnyBlock<MT, MODE>::finish_tile(float (&acc)[MT][4], int n0) 
 }
 
 // MT: token tiles of 8 (1, 2, 4 or 8 -> up to 8, 16, 32, 64 tokens).
-template <int MT, int MODE, bool ONE>
+template <int MT, int MODE, bool ONE, int STAGES>
 __global__ void __launch_bounds__(kSgThreads) skinny_gemm_kernel(const SkinnyArgsOf<MODE> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch_dependents();
-  const SkinnyBlock<MT, MODE> blk(args, blockIdx.x, gridDim.x, blockIdx.y, blockIdx.z, smem_raw);
+  const SkinnyBlock<MT, MODE, STAGES> blk(args, blockIdx.x, gridDim.x, blockIdx.y, blockIdx.z, smem_raw);
   blk.request_weights();
   pdl_wait();
   blk.template run<ONE>();
@@ -536,20 +536,23 @@ __global__ void __launch_bounds__(kSgThreads) skinny_chain_kernel(const SkinnyCh
     atomicAdd(ch.counter, kChainPerLaunch - static_cast<unsigned long long>(ch.n_phases - 1) * G);
 }
 
-// The head keeps only the M rows that hold tokens and has no norm weights: a block of up to 8 rows whose K is 3,072 takes
-// 93 KB instead of 149 and one of 16 rows whose K is 1,024 (four stages) 107 instead of 128, so that two share an SM and one
-// copies while the other waits at its barriers.  Inside a step, us: one row of 130,049 x 3,072 156 -> 139, 16 rows of
-// 32,784 x 1,024 22 -> 18.  (The layers' products keep whole tiles of rows: blocks as small as one token's let the next
-// launch's blocks in earlier, and a decode step of one request grew from 199 to 204 us, of eight from 909 to 927.)
 inline size_t skinny_smem(int MP, int kx) {
-  return static_cast<size_t>(sg_stages(MP / 8, false)) * kSgRows * kSgWStride * sizeof(bf16) +
+  return static_cast<size_t>(sg_stages(MP / 8)) * kSgRows * kSgWStride * sizeof(bf16) +
          static_cast<size_t>(MP) * (kx + 8) * sizeof(bf16) + 3 * 32 * MP * sizeof(float) +
          static_cast<size_t>(kx + MP) * sizeof(float);
 }
-inline size_t skinny_head_smem(int MP, int M, int kx) {
-  return static_cast<size_t>(sg_stages(MP / 8, true)) * kSgRows * kSgWStride * sizeof(bf16) +
-         static_cast<size_t>(M) * (kx + 8) * sizeof(bf16) + 3 * 32 * MP * sizeof(float);
+// The head keeps only the M rows that hold tokens and has no norm weights, so that two blocks share an SM (113 KB each) up to
+// 4 rows whose K is 3,072 (one row 94 KB, four 112; whole tiles took 149) and 8 whose K is 1,024, and one copies while the
+// other waits at its barriers.  9 to 16 rows give up the fifth stage where four make that room (16 rows of 1,024, 9 of 2,048)
+// and keep it elsewhere.  Us, whole tiles and five stages / only the rows / four stages as well: one row of 130,049 x 3,072
+// 155 / 129, 16 rows of 32,784 x 1,024 22 / / 19, 9 rows of 50,000 x 2,048 54 / / 42, 12 rows of it 55 / 55 / 60, 16 rows of
+// 130,049 x 3,072 188 / 188 / 205.  (The layers' products keep whole tiles of rows: blocks as small as one token's let the next
+// launch's blocks in earlier, and a decode step of one request grew from 199 to 204 us, of eight from 909 to 927.)
+inline size_t skinny_head_smem(int MP, int stages, int M, int kx) {
+  return static_cast<size_t>(stages) * kSgRows * kSgWStride * sizeof(bf16) + static_cast<size_t>(M) * (kx + 8) * sizeof(bf16) +
+         3 * 32 * MP * sizeof(float);
 }
+constexpr size_t kSgTwoBlocks = 113 * 1024;  // of an SM's 228 KB, one of them kept back for each block
 
 // Every call opts in to the same size: were it the call's own, a thread with fewer rows could lower the kernel's limit between
 // another thread's opt-in and its launch, which would then be refused.
@@ -577,14 +580,17 @@ inline int sg_resident(F kern, size_t smem, std::atomic<unsigned long long>& see
   return per_sm * n_sm;
 }
 
-template <int MT, int MODE>
+template <int MT, int MODE, int STAGES = sg_stages(MT)>
 int launch_skinny(const SkinnyArgsOf<MODE>& a, int k_max, cudaStream_t stream) {
   constexpr int MP = MT * 8;
   const int kx = (min(a.k_slice, k_max) + kSgChunk - 1) / kSgChunk * kSgChunk;
-  const size_t smem = MODE == kSgStoreF32 ? skinny_head_smem(MP, a.M, kx) : skinny_smem(MP, kx);
+  const size_t smem = MODE == kSgStoreF32 ? skinny_head_smem(MP, STAGES, a.M, kx) : skinny_smem(MP, kx);
+  if constexpr (MODE == kSgStoreF32 && MT == 2 && STAGES == sg_stages(MT)) {
+    if (skinny_head_smem(MP, STAGES - 1, a.M, kx) <= kSgTwoBlocks) return launch_skinny<MT, MODE, STAGES - 1>(a, k_max, stream);
+  }
   if (smem > kSgMaxSmem) return PMM_ERR_BAD_ARGUMENT;
-  auto kern = skinny_gemm_kernel<MT, MODE, false>;
-  auto kern_one = skinny_gemm_kernel<MT, MODE, true>;
+  auto kern = skinny_gemm_kernel<MT, MODE, false, STAGES>;
+  auto kern_one = skinny_gemm_kernel<MT, MODE, true, STAGES>;
   for (auto k : {kern, kern_one}) {
     const cudaError_t e = sg_opt_in(k);
     if (e != cudaSuccess) return static_cast<int>(e);

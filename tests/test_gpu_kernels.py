@@ -803,10 +803,11 @@ def test_skinny_product_with_float32_output_for_the_head(M, N, Kd):
     assert bool(torch.isnan(out[:, N:]).all())
 
 
-@pytest.mark.parametrize("M,N,Kd", [(1, 12001, 3072), (2, 9601, 1024), (7, 31, 8), (9, 9601, 1024), (11, 70, 1032), (15, 9601, 264), (16, 33, 2048)])
+@pytest.mark.parametrize("M,N,Kd", [(1, 12001, 3072), (2, 9601, 1024), (7, 31, 8), (9, 9601, 1024), (11, 70, 1032), (15, 9601, 264), (16, 33, 2048),
+                                     (9, 9601, 2048), (10, 9601, 2056), (12, 4800, 3072), (16, 4800, 1288)])
 def test_head_keeps_only_the_rows_that_hold_tokens(M, N, Kd):
     """Rows on and off whole tiles of 8 and 16, blocks with one tile of weights and with several, K on and off the chunks of
-    256: small whole numbers, so that the sums are exact, and rows whose neighbours hold infinities."""
+    256, five stages of weights and, where that makes room for a second block, four: small whole numbers, so that the sums are exact, and rows whose neighbours hold infinities."""
     ops = K()
     g = torch.Generator().manual_seed(M + N + Kd)
     xw = torch.full((M + 2, Kd), float("inf"), dtype=torch.bfloat16)
