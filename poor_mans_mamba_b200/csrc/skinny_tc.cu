@@ -87,12 +87,15 @@ __global__ void __launch_bounds__(kStThreads)
   const int share = static_cast<int>(blockIdx.x) - prob * kStCluster * args.groups[0];
   const int kb0 = boxes * share / shares, n_kb = boxes * (share + 1) / shares - kb0;
   constexpr int kTileCols = MODE == kStSwiglu ? kStRows / 2 : kStRows;  // output columns of a block
-  const int n0 = blockIdx.y * kTileCols;
+  const long long tile = static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y;
+  const int n0 = static_cast<int>(tile) * kTileCols;
   const int x_box = args.t_pad * kStKB * 2;
 
   unsigned char* sW = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sX = sW + kStMaxKB * kStWBox;   // [max_kb] boxes of t_pad rows
   float* part = reinterpret_cast<float*>(sW);       // [t_pad][128] partial sums, once the products have read W
+
+  if (tile * kTileCols >= args.N) return;   // (the last z holds fewer tiles; the whole cluster leaves)
 
   if (threadIdx.x == 0) {
     mbar_init(&bar_w, 1);
@@ -264,7 +267,8 @@ int launch_skinny_tc(const CUtensorMap* maps, const SkinnyTcArgs& a, cudaStream_
   if (e != cudaSuccess) return static_cast<int>(e);
   constexpr int kTileCols = MODE == kStSwiglu ? kStRows / 2 : kStRows;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(kStCluster * (a.groups[0] + a.groups[1]), (a.N + kTileCols - 1) / kTileCols);
+  const int tiles = (a.N - 1) / kTileCols + 1, deep = (tiles + 65534) / 65535;
+  cfg.gridDim = dim3(kStCluster * (a.groups[0] + a.groups[1]), (tiles + deep - 1) / deep, deep);
   cfg.blockDim = dim3(kStThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

@@ -876,6 +876,23 @@ def test_tcgen05_product_in_clusters(T, N, Kd):
     assert ops.tc_gemm_status(DEV) == 0
 
 
+def test_tcgen05_product_of_more_tiles_than_a_grid_is_high():
+    """65,536 tiles of 128 rows and one more, each mode that takes such a weight; the products before this form took any number."""
+    ops = K()
+    N, Kd = 65536 * 128 + 1, 8
+    x = torch.randint(-3, 4, (2, Kd), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    w = torch.randint(-3, 4, (N, Kd), generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).to(torch.bfloat16)
+    ref = x.float() @ w.float().t()       # |sums| <= 72: exact in bfloat16
+    out = torch.full((2, (N + 7) // 8 * 8), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.skinny_tc_linear(x, w, out[:, :N])
+    assert torch.equal(out[:, :N].float(), ref) and bool(torch.isnan(out[:, N:]).all())
+    h = torch.ones(2, N, device=DEV)
+    ops.skinny_tc_residual(h, [(x, w, 0.5)])
+    assert torch.equal(h, 1.0 + 0.5 * ref)
+    torch.cuda.synchronize()
+    assert ops.tc_gemm_status(DEV) == 0
+
+
 @pytest.mark.parametrize("T", [1, 17, 40, 64])
 @pytest.mark.parametrize("N,Kd", [(50, 96), (1024, 1000), (4120, 1024), (6000, 512), (304, 72)])
 def test_tcgen05_weight_streaming_product(T, N, Kd):
