@@ -26,11 +26,6 @@ namespace pmm {
 // (`ranked`) where picking them one after the other takes ten exchanges between lanes apiece.  16 experts, 4 chosen in 2
 // of 4 groups, width 1,024, inside a step: 8 tokens 11 -> 4.5 us.
 constexpr int kRouteAhead = 8;   // sixteen-byte pieces of a router row a lane holds before the wait (128 columns each)
-template <int TOK>
-struct RouteShape {
-  static constexpr int kPer = TOK == 1 ? 1 : 2;      // experts a warp makes at a time: several tokens' rows are read once for both
-  static constexpr int kWarps = TOK == 1 ? 16 : 8;
-};
 
 // This lane's place (0: the largest; the lower index wins a tie) among values v[0 .. n - 1], n <= 32, none of them NaN.
 __device__ __forceinline__ int ranked(const float* v, int n, int lane) {
@@ -45,8 +40,8 @@ __device__ __forceinline__ bool all_finite(const float* v, int n, int lane) {
   return n <= 32 && __all_sync(0xffffffffu, lane >= n || fabsf(v[lane]) < INFINITY);
 }
 
-template <typename S, int TOK>
-__global__ void __launch_bounds__(RouteShape<TOK>::kWarps * 32)
+template <typename S, int TOK, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
     moe_route_kernel(const S* __restrict__ x, long long ld_x, const float* __restrict__ w,
                      const float* __restrict__ bias, int* __restrict__ ids, float* __restrict__ weights, int T, int D,
                      int E, int top, int scored, const float* __restrict__ correction, int groups, int keep,
@@ -63,7 +58,8 @@ __global__ void __launch_bounds__(RouteShape<TOK>::kWarps * 32)
   // (gate_w: one more row, whose product goes through a sigmoid into gate_out[t]: a gate per token that reads the
   // router's input, such as a shared expert's)
   const int n_rows = E + (gate_w ? 1 : 0);
-  constexpr int kPer = RouteShape<TOK>::kPer, kRouteWarps = RouteShape<TOK>::kWarps;
+  constexpr int kPer = TOK == 1 ? 1 : 2;  // experts a warp makes at a time: several tokens' rows are read once for both
+  constexpr int kRouteWarps = WARPS;
   auto router_row = [&](int e) { return e < E ? w + static_cast<size_t>(e) * D : gate_w; };
   float4 ahead[kPer][kRouteAhead];
   if (vec) {
@@ -854,18 +850,18 @@ __global__ void __launch_bounds__(256)
 }  // namespace pmm
 
 namespace pmm {
-template <typename S, int TOK>
+template <typename S, int TOK, int WARPS = 8>
 int launch_route(const void* x, long long ld_x, const float* w, const float* bias, int* ids, float* weights, int T, int D,
                  int E, int top, int scored, const float* correction, int groups, int keep, float scale,
                  const float* gate_w, float* gate_out, cudaStream_t stream) {
   const size_t smem = (static_cast<size_t>(TOK) * ((D + 3) & ~3) + static_cast<size_t>(TOK) * E * (scored ? 3 : 1)) * sizeof(float);
   if (smem > 200 * 1024) return PMM_ERR_BAD_ARGUMENT;
-  auto kern = moe_route_kernel<S, TOK>;
+  auto kern = moe_route_kernel<S, TOK, WARPS>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
   }
-  launch_pdl(kern, dim3((T + TOK - 1) / TOK), dim3(RouteShape<TOK>::kWarps * 32), smem, stream, static_cast<const S*>(x), ld_x, w, bias,
+  launch_pdl(kern, dim3((T + TOK - 1) / TOK), dim3(WARPS * 32), smem, stream, static_cast<const S*>(x), ld_x, w, bias,
              ids, weights, T, D, E, top, scored, correction, groups, keep, scale, gate_w, gate_out);
   return launch_status();
 }
@@ -882,16 +878,23 @@ PMM_EXPORT int pmm_moe_route(const void* x, long long ld_x, const float* w, cons
   if (D <= 0 || E <= 0 || top <= 0 || top > E || (gate_w && !gate_out)) return PMM_ERR_BAD_ARGUMENT;
   if (scored && (groups <= 0 || E % groups || keep <= 0 || keep > groups || top > keep * (E / groups)))
     return PMM_ERR_BAD_ARGUMENT;
-  // few tokens: a block each, so that the step's few rows still spread over the GPU; many: four or eight a block (a
-  // block an SM is left), which read the router a quarter or an eighth as often
+  // Few tokens: a block each, of 16 warps while two such blocks an SM are one wave (296 tokens; past it they are two: 300 tokens of
+  // width 2,048, 64 experts 31.7 us), of 8 warps while three are (444; 21.1 us).  More: four or eight tokens a block, which
+  // read the router a quarter or an eighth as often (the same at 511 tokens, a block of 16 warps a token 32.9, four tokens a
+  // block 26.5 us).
+  // Rows too long for that keep a block of 8 warps a token.
+  constexpr int kSms = 148;
   auto room = [&](int tok) { return (static_cast<size_t>(tok) * (((D + 3) & ~3) + 3 * E)) * sizeof(float) <= 96 * 1024; };
   PMM_DISPATCH_DTYPE(dtype, S, {
     if (T >= 1024 && room(8))
       return pmm::launch_route<S, 8>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
                                      gate_w, gate_out, stream);
-    if (T >= 512 && room(4))
+    if (T > 3 * kSms && room(4))
       return pmm::launch_route<S, 4>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
                                      gate_w, gate_out, stream);
+    if (T <= 2 * kSms)
+      return pmm::launch_route<S, 1, 16>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
+                                         gate_w, gate_out, stream);
     return pmm::launch_route<S, 1>(x, ld_x, w, bias, ids, weights, T, D, E, top, scored, correction, groups, keep, scale,
                                    gate_w, gate_out, stream);
   });

@@ -264,3 +264,19 @@ def test_plan_of_many_pairs(A, E):
         assert torch.equal(perm.cpu().long(), torch.sort(ids.long(), stable=True).indices)
         assert offsets.cpu().tolist() == [0] + count.cumsum(0).tolist()
         assert tiles.cpu().tolist() == [0] + ((count + rows - 1) // rows).cumsum(0).tolist()
+
+
+@pytest.mark.parametrize("T", [296, 297, 444, 445])
+@pytest.mark.parametrize("D,E,top", [(132, 16, 4), (64, 40, 3), (30, 8, 2)])
+def test_routes_on_both_sides_of_what_a_block_takes(T, D, E, top):
+    """One token a block of 16 warps, of 8 warps, four tokens a block: small whole numbers, exact logits full of ties."""
+    g = torch.Generator().manual_seed(T + E)
+    x = torch.randint(-2, 3, (T, D), generator=g).float() * (torch.rand(T, D, generator=g) < 4.0 / D)
+    w = torch.randint(-2, 3, (E, D), generator=g).float()
+    z = x @ w.t()
+    want = torch.tensor([sorted(range(E), key=lambda e: (-z[t, e].item(), e))[:top] for t in range(T)])
+    ids = torch.full((T, top), -7, dtype=torch.int32, device=DEV)
+    weights = torch.empty(T, top, device=DEV)
+    K.moe_route(x.to(DEV, torch.bfloat16), w.to(DEV), None, top, ids, weights)
+    assert torch.equal(ids.cpu().long(), want)
+    close(weights, torch.softmax(torch.gather(z.double(), 1, want), 1), torch.float32, "weights", f32=1e-5)
