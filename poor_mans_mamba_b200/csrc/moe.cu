@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "mma_helpers.cuh"
 #include "moe_tile.cuh"
+#include <cmath>
 
 namespace pmm {
 
@@ -671,24 +672,36 @@ __global__ void __launch_bounds__(128)
 // The same product for steps of few pairs (decode steps), where an expert has a handful of rows and the
 // launch is a read of the chosen experts' matrices: tiles of 16 rows, the four warps share the
 // columns, K in slices through a four-stage ring, so that a block keeps three slices in flight.  What it takes is a block's
-// walk along K: 64 columns and slices of 64 for the down product (K is an expert's width); 32 gate and 32 up columns and
-// slices of 128 for the up product, whose K is the model's width: twice the blocks, half the steps (8 tokens, 4 of 16 experts
-// of 256, width 1,024, inside a step: 14.5 us with 64 + 64 columns and slices of 64, 10 us so).
+// walk along K, times the waves of blocks (two on an SM).  64 columns and slices of 64 for the down product, whose K is an
+// expert's width.  The up product, whose K is the model's width, has two forms: NARROW, 32 gate and 32 up columns and slices
+// of 128, walks twice the blocks in 0.4 to 0.6 of the time each (8 tokens, 4 of 16 experts of 256, width 1,024, inside a step: 14.5
+// against 10 us), which loses where a wave becomes two (4 tokens, 6 of 64 experts of 512: 17.0 against 19.0 us; 32
+// tokens 32.5 against 39.7); `few_narrow` decides.
 constexpr int kFewRows = 16, kFewStages = 4;
-template <bool UP>
+template <bool UP, bool NARROW>
 struct FewTile {
-  static constexpr int kCols = UP ? 32 : 64, kK = UP ? 128 : 64, kLd = kK + 8, kBRows = UP ? 2 * kCols : kCols;
+  static constexpr int kCols = NARROW ? 32 : 64, kK = NARROW ? 128 : 64, kLd = kK + 8, kBRows = UP ? 2 * kCols : kCols;
   static constexpr int kStageElems = (kFewRows + kBRows) * kLd;
 };
 
-template <bool UP>
+// Whether the up product of A pairs takes its narrow tiles: waves of blocks, times 5/8 for a narrow one, with the tiles that
+// evenly chosen experts have (the experts met by A draws, and past 8 rows an expert the second tiles of some).
+inline bool few_narrow(int A, int E, int N) {
+  const double met = E * (1.0 - std::pow(1.0 - 1.0 / E, A)) + (A > 8 * E ? A / 32.0 : 0.0);
+  constexpr int kSlots = 2 * 148;
+  auto waves = [&](int cols) { return static_cast<int>(std::ceil(met * ((N + cols - 1) / cols) / kSlots)); };
+  return 5 * waves(32) <= 8 * waves(64);
+}
+
+template <bool UP, bool NARROW>
 __global__ void __launch_bounds__(128)
     moe_gemm_few_kernel(const bf16* __restrict__ a, long long ld_a, const bf16* __restrict__ w,
                         const int* __restrict__ perm, const int* __restrict__ offsets,
                         const int* __restrict__ tile_start, int E, int top, int K, int N, float limit, float alpha,
                         float shift, int ungated, const float* __restrict__ row_w, bf16* __restrict__ out) {
-  constexpr int kCols = FewTile<UP>::kCols, kK = FewTile<UP>::kK, kLd = FewTile<UP>::kLd, BROWS = FewTile<UP>::kBRows;
-  constexpr int kStageElems = FewTile<UP>::kStageElems;
+  using Tile = FewTile<UP, NARROW>;
+  constexpr int kCols = Tile::kCols, kK = Tile::kK, kLd = Tile::kLd, BROWS = Tile::kBRows, kStageElems = Tile::kStageElems;
+  constexpr int NJ = kCols / 32;  // groups of 8 columns a warp (of the gate's and as many of the up matrix's)
   extern __shared__ __align__(16) unsigned char few_smem[];
   bf16* ring = reinterpret_cast<bf16*>(few_smem);
   __shared__ int src_row[kFewRows];
@@ -729,9 +742,9 @@ __global__ void __launch_bounds__(128)
     cp_async_commit();
   };
 
-  float acc[2][4];   // UP: the warp's 8 gate and 8 up columns; else its 16 columns
+  float acc[UP ? 2 * NJ : NJ][4];   // UP: the gate's columns, then the up matrix's
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
+  for (int j = 0; j < (UP ? 2 * NJ : NJ); ++j)
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
 
@@ -749,23 +762,26 @@ __global__ void __launch_bounds__(128)
     const bf16* As = ring + static_cast<size_t>(s % kFewStages) * kStageElems;
     const bf16* Bs = As + kFewRows * kLd;
 #pragma unroll
-    for (int kk = 0; kk < kK; kk += UP ? 32 : 16) {
+    for (int kk = 0; kk < kK; kk += NARROW ? 32 : 16) {
       unsigned af[4], b0, b1, b2, b3;
       ldmatrix_x4(af[0], af[1], af[2], af[3], As + (lane & 15) * kLd + kk + ((lane >> 4) << 3));
-      if (UP) {
+      if (NARROW) {
         // 8 rows of the gate's (the up) matrix x 32 k, in two steps of 16
-        unsigned ag[4], c0, c1, c2, c3;
+        unsigned ag[4];
         ldmatrix_x4(ag[0], ag[1], ag[2], ag[3], As + (lane & 15) * kLd + kk + 16 + ((lane >> 4) << 3));
-        ldmatrix_x4(b0, b1, b2, b3, Bs + (warp * 8 + (lane & 7)) * kLd + kk + ((lane >> 3) << 3));
-        ldmatrix_x4(c0, c1, c2, c3, Bs + (kCols + warp * 8 + (lane & 7)) * kLd + kk + ((lane >> 3) << 3));
-        mma_bf16(acc[0], af, b0, b1);
-        mma_bf16(acc[1], af, c0, c1);
-        mma_bf16(acc[0], ag, b2, b3);
-        mma_bf16(acc[1], ag, c2, c3);
+#pragma unroll
+        for (int part = 0; part < (UP ? 2 : 1); ++part) {
+          ldmatrix_x4(b0, b1, b2, b3, Bs + (part * kCols + warp * 8 + (lane & 7)) * kLd + kk + ((lane >> 3) << 3));
+          mma_bf16(acc[part], af, b0, b1);
+          mma_bf16(acc[part], ag, b2, b3);
+        }
       } else {
-        ldmatrix_x4(b0, b1, b2, b3, Bs + (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * kLd + kk + (((lane >> 3) & 1) << 3));
-        mma_bf16(acc[0], af, b0, b1);
-        mma_bf16(acc[1], af, b2, b3);
+#pragma unroll
+        for (int part = 0; part < (UP ? 2 : 1); ++part) {
+          ldmatrix_x4(b0, b1, b2, b3, Bs + (part * kCols + warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * kLd + kk + (((lane >> 3) & 1) << 3));
+          mma_bf16(acc[part * NJ], af, b0, b1);
+          mma_bf16(acc[part * NJ + NJ - 1], af, b2, b3);
+        }
       }
     }
   }
@@ -778,14 +794,14 @@ __global__ void __launch_bounds__(128)
     if (i >= row1) continue;
     const float rw = (UP && row_w) ? row_w[dst_row[r]] : 1.f;
 #pragma unroll
-    for (int j = 0; j < (UP ? 1 : 2); ++j) {
+    for (int j = 0; j < NJ; ++j) {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const int col = n0 + (UP ? warp * 8 : warp * 16 + j * 8) + c_in + q;
+        const int col = n0 + (warp * NJ + j) * 8 + c_in + q;
         if (col >= N) continue;
         if (UP) {
           out[static_cast<size_t>(i) * N + col] =
-              __float2bfloat16_rn(clamped_glu(rw * acc[0][half * 2 + q], rw * acc[1][half * 2 + q], limit, alpha, shift));
+              __float2bfloat16_rn(clamped_glu(rw * acc[j][half * 2 + q], rw * acc[UP ? NJ + j : j][half * 2 + q], limit, alpha, shift));
         } else {
           const float val = acc[j][half * 2 + q];
           out[static_cast<size_t>(ungated ? i : dst_row[r]) * N + col] = __float2bfloat16_rn(ungated ? relu_squared(val) : val);
@@ -951,27 +967,21 @@ PMM_EXPORT int pmm_moe_gemm(const void* a, long long ld_a, const void* w, const 
         reinterpret_cast<uintptr_t>(w) % 16)
       return PMM_ERR_BAD_ARGUMENT;
     if (tensor_cores == 2) {
-      const int cols = up ? pmm::FewTile<true>::kCols : pmm::FewTile<false>::kCols;
-      const dim3 grid((N + cols - 1) / cols, row_tiles);
-      const size_t smem = static_cast<size_t>(pmm::kFewStages) * sizeof(pmm::bf16) *
-                          (up ? pmm::FewTile<true>::kStageElems : pmm::FewTile<false>::kStageElems);
-      cudaError_t err;
-      if (up) {
-        auto kern = pmm::moe_gemm_few_kernel<true>;
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      auto few = [&](auto kern, int cols, int stage_elems) {
+        const size_t smem = static_cast<size_t>(pmm::kFewStages) * sizeof(pmm::bf16) * stage_elems;
+        const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (err != cudaSuccess) return static_cast<int>(err);
-        pmm::launch_pdl(kern, grid, dim3(128), smem, stream, static_cast<const pmm::bf16*>(a), ld_a,
+        pmm::launch_pdl(kern, dim3((N + cols - 1) / cols, row_tiles), dim3(128), smem, stream, static_cast<const pmm::bf16*>(a), ld_a,
                         static_cast<const pmm::bf16*>(w), perm, offsets, tile_start, E, top, K, N, limit, alpha, shift,
                         ungated, row_w, static_cast<pmm::bf16*>(out));
-      } else {
-        auto kern = pmm::moe_gemm_few_kernel<false>;
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (err != cudaSuccess) return static_cast<int>(err);
-        pmm::launch_pdl(kern, grid, dim3(128), smem, stream, static_cast<const pmm::bf16*>(a), ld_a,
-                        static_cast<const pmm::bf16*>(w), perm, offsets, tile_start, E, top, K, N, limit, alpha, shift,
-                        ungated, row_w, static_cast<pmm::bf16*>(out));
-      }
-      return pmm::launch_status();
+        return pmm::launch_status();
+      };
+      using Down = pmm::FewTile<false, false>;
+      using Narrow = pmm::FewTile<true, true>;
+      using Wide = pmm::FewTile<true, false>;
+      if (!up) return few(pmm::moe_gemm_few_kernel<false, false>, Down::kCols, Down::kStageElems);
+      if (pmm::few_narrow(A, E, N)) return few(pmm::moe_gemm_few_kernel<true, true>, Narrow::kCols, Narrow::kStageElems);
+      return few(pmm::moe_gemm_few_kernel<true, false>, Wide::kCols, Wide::kStageElems);
     }
     const dim3 grid((N + pmm::kMmaCols - 1) / pmm::kMmaCols, row_tiles);
     if (up)

@@ -280,3 +280,26 @@ def test_routes_on_both_sides_of_what_a_block_takes(T, D, E, top):
     K.moe_route(x.to(DEV, torch.bfloat16), w.to(DEV), None, top, ids, weights)
     assert torch.equal(ids.cpu().long(), want)
     close(weights, torch.softmax(torch.gather(z.double(), 1, want), 1), torch.float32, "weights", f32=1e-5)
+
+
+@pytest.mark.parametrize("T,top,E,D,F", [
+    (1, 1, 1, 8, 8), (4, 2, 8, 136, 40), (16, 4, 16, 128, 256),     # narrow tiles of the up product: one wave of them
+    (4, 6, 64, 72, 520), (32, 6, 64, 264, 504), (8, 8, 32, 64, 1096),  # wide: a second wave of narrow ones
+])
+def test_up_product_of_few_pairs_in_both_tiles(T, top, E, D, F):
+    """Widths on and off the tiles of 32 and 64 columns and slices of 64 and 128, experts with none, one and several rows.  Small whole
+    numbers: the products are exact in float, what is left is the gate's arithmetic and the store's rounding."""
+    g = torch.Generator().manual_seed(T * E)
+    x = torch.randint(-1, 2, (T, D), generator=g).to(torch.bfloat16)
+    w = torch.randint(-1, 2, (E, 2 * F, D), generator=g).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    offsets, tiles = (torch.empty(E + 1, dtype=torch.int32, device=DEV) for _ in range(2))
+    perm = torch.empty(T * top, dtype=torch.int32, device=DEV)
+    K.moe_plan(ids.to(DEV), E, "mma_few", offsets, tiles, perm)
+    act = torch.full((T * top, F), float("nan"), dtype=torch.bfloat16, device=DEV)
+    K.moe_gemm(x.to(DEV), w.to(DEV), perm, offsets, tiles, top, True, act, "mma_few", limit=1e4, alpha=1.0)
+    order = perm.cpu().long()
+    rows, experts = order // top, ids.view(-1)[order].long()
+    z = torch.einsum("ad,afd->af", x.double()[rows], w.double()[experts])
+    want = torch.nn.functional.silu(z[:, :F]) * z[:, F:]
+    assert float((act.cpu().double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
