@@ -303,3 +303,18 @@ def test_up_product_of_few_pairs_in_both_tiles(T, top, E, D, F):
     z = torch.einsum("ad,afd->af", x.double()[rows], w.double()[experts])
     want = torch.nn.functional.silu(z[:, :F]) * z[:, F:]
     assert float((act.cpu().double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,D,top,shared", [(1, 8, 1, False), (3, 256, 8, True), (3, 264, 5, True), (1024, 256, 2, False), (1023, 256, 3, True), (2, 260, 2, False), (700, 72, 3, True), (4096, 64, 2, False)])
+def test_weighted_sum_by_the_value_and_by_the_piece(dtype, T, D, top, shared):
+    """Both forms on both sides of their lines (rows of 256 values, 2^18 values in all), rows that are no whole pieces.
+    Tolerance: float sums of at most nine terms, then one rounding to the storage type."""
+    y, w = rnd(T * top, D, seed=1), rnd(T, top, seed=2)
+    s, gate = (rnd(T, D, seed=3), rnd(T, seed=4)) if shared else (None, None)
+    out = torch.full((T, D), float("nan"), dtype=dtype, device=DEV)
+    K.moe_combine(y.to(DEV, dtype), w.to(DEV), s.to(DEV, dtype) if shared else None, out, gate.to(DEV) if shared else None)
+    want = (w.double().unsqueeze(2) * y.double().view(T, top, D)).sum(1)
+    if shared:
+        want = want + gate.double().unsqueeze(1) * s.double()
+    close(out, want, dtype, "weighted sum", f32=2e-6, bf16=2.0 ** -8)
