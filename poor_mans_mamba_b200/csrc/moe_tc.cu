@@ -227,19 +227,22 @@ inline bool moe_make_map(CUtensorMap* map, const void* base, long long rows, lon
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// xs[i, :] = x[perm[i] / top, :]: the token rows in the order of the sorted pairs (16-byte pieces), a warp a row with four
-// reads of a lane in flight (8,192 rows of 1,024 inside a step: 4.3 us, a block a row 8.2).
+// xs[i, :] = x[perm[i] / top, :]: the token rows in the order of the sorted pairs (16-byte pieces), WARPS warps of a block of eight
+// a row, so that a lane has about four reads, all in flight.  Us with 1, 2, 4 and 8 warps a row: 8,192 rows of 1,024 4.3, 4.3,
+// 5.3, 9.0; 8,192 of 2,048 7.3, 6.6, 6.8, 9.3; 16,384 of 4,096 26.2, 24.9, 24.3, 28.5; 6,000 of 8,192 25.1, 19.7, 19.0, 18.4; few rows
+// want more blocks: 2,048 of 1,024 2.7, 2.5, 2.2, 2.7; 560 of 4,096 3.0, 2.5, 2.7, 2.5.
+template <int WARPS>
 __global__ void __launch_bounds__(256)
     moe_gather_rows_kernel(const bf16* __restrict__ x, long long ld_x, const int* __restrict__ perm, int top,
                            bf16* __restrict__ xs, int A, int K) {
   pdl_launch_dependents();
   pdl_wait();
-  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int i = (blockIdx.x * 8 + (threadIdx.x >> 5)) / WARPS;
   if (i >= A) return;
   const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<long long>(perm[i] / top) * ld_x);
   uint4* dst = reinterpret_cast<uint4*>(xs + static_cast<size_t>(i) * K);
 #pragma unroll 4
-  for (int c = threadIdx.x & 31; c < K / 8; c += 32) dst[c] = src[c];
+  for (int c = threadIdx.x % (32 * WARPS); c < K / 8; c += 32 * WARPS) dst[c] = src[c];
 }
 
 }  // namespace pmm
@@ -256,8 +259,15 @@ PMM_EXPORT int pmm_moe_gather_rows(const void* x, long long ld_x, const int* per
   if (A <= 0) return 0;
   if (K <= 0 || K % 8 || ld_x % 8 || top <= 0 || reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(xs) % 16)
     return PMM_ERR_BAD_ARGUMENT;
-  pmm::launch_pdl(pmm::moe_gather_rows_kernel, dim3((A + 7) / 8), dim3(256), 0, stream,
-                  static_cast<const pmm::bf16*>(x), ld_x, perm, top, static_cast<pmm::bf16*>(xs), A, K);
+  auto go = [&](auto kern, int warps) {
+    pmm::launch_pdl(kern, dim3((A + 8 / warps - 1) / (8 / warps)), dim3(256), 0, stream, static_cast<const pmm::bf16*>(x), ld_x, perm,
+                    top, static_cast<pmm::bf16*>(xs), A, K);
+  };
+  const bool many = A >= 4096;  // (fewer rows: more blocks)
+  if (K < (many ? 2048 : 1024)) go(pmm::moe_gather_rows_kernel<1>, 1);
+  else if (many && K < 4096) go(pmm::moe_gather_rows_kernel<2>, 2);
+  else if (K < (many ? 8192 : 4096)) go(pmm::moe_gather_rows_kernel<4>, 4);
+  else go(pmm::moe_gather_rows_kernel<8>, 8);
   return pmm::launch_status();
 }
 

@@ -318,3 +318,15 @@ def test_weighted_sum_by_the_value_and_by_the_piece(dtype, T, D, top, shared):
     if shared:
         want = want + gate.double().unsqueeze(1) * s.double()
     close(out, want, dtype, "weighted sum", f32=2e-6, bf16=2.0 ** -8)
+
+
+@pytest.mark.parametrize("A,top,Kd", [(1, 1, 8), (37, 3, 1016), (37, 3, 1024), (4099, 3, 2040), (4099, 3, 2048), (9, 2, 4088), (4095, 5, 4096), (4097, 5, 4096), (130, 1, 8192)])
+def test_gathered_rows_of_every_width(A, top, Kd):
+    """One, two, four and eight warps a row, the last block's rows among them: the rows as they are."""
+    T = (A + top - 1) // top
+    x = torch.randn(T, Kd + 8, generator=torch.Generator().manual_seed(A)).to(DEV, torch.bfloat16)[:, :Kd]
+    perm = torch.randperm(T * top, generator=torch.Generator().manual_seed(Kd))[:A].to(torch.int32)
+    out = torch.full((A + 1, Kd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    K.moe_gather_rows(x, perm.to(DEV), top, out[:A])
+    assert torch.equal(out[:A].cpu(), x.cpu()[perm.long() // top])
+    assert bool(torch.isnan(out[A]).all())
