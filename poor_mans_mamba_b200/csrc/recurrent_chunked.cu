@@ -906,20 +906,23 @@ __global__ void __launch_bounds__(kDecayThreads)
 
 // The rows of every chunk: [Q * a^(i+1) | B] times [S_0; V], one product whose inner index runs over the d state rows and then
 // the chunk's tokens up to the row's own, 64 rows x 64 columns a block.
-// Bound by the float units and the latency in front of them: a thread makes 8 x 4 results, twelve sixteen-byte reads for four
-// inner indices and 128 multiply-adds (4 x 4: eight for 64), two multiply-adds an instruction, every sum in the order of
-// the inner index.  The operands come in slices of 32 through a ring of three, 48 KB a block, so that four blocks share an SM
-// and the 512 blocks of 2,048 tokens, 8 heads and 128 x 128 states are one wave (whole operands: 80 KB, two blocks, two waves).
-// That size inside a step: 30 -> 27 us (8 x 8 results on two warps a block 29.5: too few warps in flight).
+// Bound by the float units and the latency in front of them: a thread makes ROWS x 4 results, with ROWS = 8 twelve sixteen-byte
+// reads for four inner indices and 128 multiply-adds (4: eight for 64), two multiply-adds an instruction, every sum in the
+// order of the inner index.  The operands come in slices of 32 through a ring of three, 48 KB a block.  Eight rows a thread, four
+// blocks of four warps on an SM, make the 512 blocks of 2,048 tokens, 8 heads and 128 x 128 states one wave (inside a step 30 -> 27
+// us against whole operands of 80 KB); a grid that leaves an SM fewer than four wants the warps: four rows a thread, up to
+// three blocks of eight warps (kOutWave).  The decayed sum with 8 heads of 64 x 128, us with 8 / 4 rows a thread: 37 tokens
+// 21.3 / 20.7, 512 42.7 / 36.5, 1,500 48.8 / 45.3, 2,048 52.3 / 53.5; with 4 heads of 244 x 244 300 tokens 89.8 / 72.5.
 // FOURS: four inner indices are summed by themselves before they enter a result, a quarter more instructions and a quarter
 // of the long sum's roundings (the rows' error against float64 at d = 244 behind a given state 2.8e-7 -> 1.7e-7); chosen for the
 // delta rule's keys from kFoursFrom entries on, which were always summed so.
-constexpr int kOutThreads = 128, kOutK = 32, kOutStages = 3, kFoursFrom = 224;
+constexpr int kOutK = 32, kOutStages = 3, kFoursFrom = 224, kOutWave = 3 * 148;
 constexpr int kOutStage = kChunk * kOutK + kOutK * kDecayTile;  // floats
 
-template <bool FOURS>
-__global__ void __launch_bounds__(kOutThreads)
+template <bool FOURS, int ROWS>
+__global__ void __launch_bounds__(1024 / ROWS)
     decay_chunk_output_kernel(ChunkArgs p) {
+  constexpr int kOutThreads = 1024 / ROWS;  // 64 rows x 64 columns
   extern __shared__ __align__(16) float sm[];
   const int d = p.d, dv = p.dv;
   pdl_launch_dependents();
@@ -952,23 +955,23 @@ __global__ void __launch_bounds__(kOutThreads)
     cp_async_commit();
   };
 
-  // thread: rows i0 .. i0 + 7, columns cc .. cc + 3 (rows at and beyond n hold stale values that are not stored)
-  const int cc = 4 * (tid % 16), i0 = 8 * (tid / 16);
-  Pair acc[8][2];
+  // thread: rows i0 .. i0 + ROWS - 1, columns cc .. cc + 3 (rows at and beyond n hold stale values that are not stored)
+  const int cc = 4 * (tid % 16), i0 = ROWS * (tid / 16);
+  Pair acc[ROWS][2];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0ull;
+  for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0ull;
   // four inner indices from `k` of the slice; with `last`, only those up to last + r enter row r
   auto four = [&](const float* sA, const float* sR, int k, bool whole, int last) {
-    float4 a[8];
+    float4 a[ROWS];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) a[r] = *reinterpret_cast<const float4*>(sA + (i0 + r) * kOutK + k);
+    for (int r = 0; r < ROWS; ++r) a[r] = *reinterpret_cast<const float4*>(sA + (i0 + r) * kOutK + k);
     if constexpr (FOURS) {
       if (whole) {
         Quad b[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) b[q] = quad(sR + (k + q) * kDecayTile + cc);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < ROWS; ++r) {
           const float av[4] = {a[r].x, a[r].y, a[r].z, a[r].w};
           Pair lo = 0ull, hi = 0ull;
 #pragma unroll
@@ -987,7 +990,7 @@ __global__ void __launch_bounds__(kOutThreads)
     for (int q = 0; q < 4; ++q) {
       const Quad b = quad(sR + (k + q) * kDecayTile + cc);
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
+      for (int r = 0; r < ROWS; ++r) {
         if (!whole && k + q > last + r) continue;
         const float av = q == 0 ? a[r].x : q == 1 ? a[r].y : q == 2 ? a[r].z : a[r].w;
         const Pair a2 = pair(av, av);
@@ -1011,13 +1014,13 @@ __global__ void __launch_bounds__(kOutThreads)
       const int last = i0 - (s - n_state) * kOutK;  // of the slice's tokens, the row i0's own
       int k = 0;
       for (; k + 3 <= last && k < kOutK; k += 4) four(sA, sR, k, true, 0);
-      for (; k <= last + 7 && k < kOutK; k += 4) four(sA, sR, k, false, last);
+      for (; k <= last + ROWS - 1 && k < kOutK; k += 4) four(sA, sR, k, false, last);
     }
   }
   if (i0 >= n) return;
   const bool pieces = dv % 4 == 0 && reinterpret_cast<uintptr_t>(p.out) % 16 == 0;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
+  for (int r = 0; r < ROWS; ++r) {
     if (i0 + r >= n) break;
     float* o = p.out + static_cast<size_t>(t0 + i0 + r) * (p.H * dv) + h * dv + c0 + cc;
     const float2 lo = halves(acc[r][0]), hi = halves(acc[r][1]);
@@ -1273,15 +1276,22 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   };
   size_t sp = prepare_smem(d, RULE);
   const size_t with_v = sp + sizeof(float) * kChunk * static_cast<size_t>(a.dv);
-  // (the prepare kernel makes the state's part too where at least two of its blocks share an SM with the values beside the
-  // keys; larger sizes keep the launch of its own, whose blocks split the columns)
-  a.with_state = !DELTA && d % 8 == 0 && a.dv % 8 == 0 && with_v <= 110 * 1024;
+  // The prepare kernel makes the state's part too where at least two of its blocks share an SM with the values beside the
+  // keys and there are blocks for more than half of the SMs; larger sizes and shorter portions keep the launch of its own,
+  // whose blocks split the columns (8 heads of 64 x 128, us so and in the prepare launch: 64 tokens 25 / 36, 300 37 / 37, 800 46 / 40;
+  // time mixing, 16 heads of 64 x 64: 128 tokens 37 / 49, 300 43 / 35).  States of up to 64 x 64 of the decayed sums are too little
+  // work for a launch however few the blocks (4 heads of it, 512 tokens: 33 / 25).
+  const bool blocks_enough = static_cast<long long>(n_chunks) * a.H >= 80 || (RULE != kRuleWkv && d * a.dv <= 64 * 64);
+  a.with_state = !DELTA && d % 8 == 0 && a.dv % 8 == 0 && with_v <= 110 * 1024 && blocks_enough;
   if (a.with_state) sp = with_v;
   const size_t s1 = sizeof(float) * kChunk * (static_cast<size_t>(d) + kDecayTile);
   const size_t s3 = sizeof(float) * kOutStages * kOutStage;
   const int n_buf = delta_chain_smem(d, 2) <= 200 * 1024 ? 2 : 1;
   const size_t s2 = delta_chain_smem(d, n_buf);
-  auto output = DELTA && d >= kFoursFrom ? decay_chunk_output_kernel<true> : decay_chunk_output_kernel<false>;
+  const bool one_wave = static_cast<long long>(n_chunks) * a.H * tiles <= kOutWave;
+  const int out_threads = one_wave ? 1024 / 4 : 1024 / 8;
+  auto output = DELTA && d >= kFoursFrom ? (one_wave ? decay_chunk_output_kernel<true, 4> : decay_chunk_output_kernel<true, 8>)
+                                         : (one_wave ? decay_chunk_output_kernel<false, 4> : decay_chunk_output_kernel<false, 8>);
   auto chain = d == 128 ? delta_chunk_chain_kernel<128> : d == 64 ? delta_chunk_chain_kernel<64> : delta_chunk_chain_kernel<0>;
   cudaError_t e = allow(prep, sp);
   if (e == cudaSuccess) e = DELTA ? allow(chain, s2) : allow(decay_chunk_state_kernel, s1);
@@ -1299,7 +1309,7 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
     launch_pdl(decay_chunk_scan_kernel, dim3((d * a.dv + kDecayThreads - 1) / kDecayThreads, a.H, a.n_seq),
                dim3(kDecayThreads), 0, stream, a);
   }
-  for_tiles([&](int n) { launch_pdl(output, dim3(n_chunks, a.H, n), dim3(kOutThreads), s3, stream, a); });
+  for_tiles([&](int n) { launch_pdl(output, dim3(n_chunks, a.H, n), dim3(out_threads), s3, stream, a); });
   return launch_status();
 }
 

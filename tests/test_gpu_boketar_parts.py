@@ -382,6 +382,29 @@ def test_decayed_sum_of_more_column_tiles_than_a_grid_is_deep():
     assert float((state[0, 0].double() - s64).abs().max()) <= 1e-5 * float(s64.abs().max())
 
 
+@pytest.mark.parametrize("H,lens,d,dv", [(2, [1], 64, 128), (8, [640], 64, 64), (8, [576], 64, 136), (8, [640], 64, 136), (74, [130, 64, 63, 1], 32, 64),
+                                         (75, [130, 64, 63, 1], 32, 64), (16, [1793], 32, 40), (2, [64 * 112], 40, 128)])
+def test_chunk_read_out_and_state_on_both_sides_of_their_grids(H, lens, d, dv):
+    """The read-out with four and eight rows a thread (up to 444 blocks and beyond) and the state's part in the prepare launch (from 80
+    chunks, or small states) and in its own, beside the token-serial kernel.  Tolerance: float sums of up to 7,168 decayed tokens in
+    another order, relative to the largest entry."""
+    T = sum(lens)
+    q, k, v = (rnd(T, H * w, seed=i).to(DEV) for i, w in enumerate((d, d, dv)))
+    decay = torch.linspace(0.6, 0.99, H).to(DEV)
+    cu, _, sl = batch_index(lens, list(range(len(lens))))
+    got = {}
+    for kind in ("chunked", "serial"):
+        state, out = torch.zeros(len(lens), H, d, dv, device=DEV), torch.full((T, H * dv), float("nan"), device=DEV)
+        if kind == "chunked":
+            scratch = torch.full((K.recurrent_chunked_scratch_floats(lens, H, d, dv, False),), float("nan"), device=DEV)
+            K.recurrent_chunked(q, k, v, state, cu, sl, lens, out, scratch, H, H, d, dv, decay=decay)
+        else:
+            K.decay_scan(q, k, v, decay, state, cu, sl, len(lens), out, H, d, dv)
+        got[kind] = (out, state)
+    for x, y in zip(got["chunked"], got["serial"]):
+        assert float((x - y).abs().max()) <= 2e-5 * max(1.0, float(y.abs().max()))
+
+
 # ----------------------------------------------------------------------------- window attention pieces
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,G,d,dv,rot", [(4, 2, 16, 32, 8), (2, 2, 48, 48, 48), (3, 1, 64, 16, 0), (8, 4, 64, 48, 64)])
