@@ -1252,6 +1252,8 @@ __global__ void __launch_bounds__(kChainThreads)
   }
 }
 
+constexpr int kMostSmem = 220 * 1024;
+
 // Largest key sizes: what the blocks that hold a chunk's operands take of shared memory (200 KB and more).
 inline int largest_key(int rule) { return rule == kRuleDelta ? 244 : rule == kRuleWkv ? 280 : 352; }
 
@@ -1271,8 +1273,10 @@ int launch_chunked(ChunkArgs a, int n_chunks, cudaStream_t stream) {
   auto whole = [&](const void* ptr, long long ld) { return reinterpret_cast<uintptr_t>(ptr) % unit == 0 && ld % 4 == 0; };
   a.vec_in = whole(a.q, a.ld_q) && whole(a.k, a.ld_k) && whole(a.v, a.ld_v) && (!DELTA || whole(a.a, a.ld_a)) &&
              (RULE != kRuleWkv || (reinterpret_cast<uintptr_t>(a.a) % 16 == 0 && a.ld_a % 4 == 0 && reinterpret_cast<uintptr_t>(a.dt_bias) % 16 == 0));
+  // (One limit for all calls: were it the call's own, a thread with smaller values could lower it between another thread's
+  // asking and its launch, which would then be refused.)
   auto allow = [](auto kernel, size_t bytes) {
-    return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   };
   size_t sp = prepare_smem(d, RULE);
   const size_t with_v = sp + sizeof(float) * kChunk * static_cast<size_t>(a.dv);

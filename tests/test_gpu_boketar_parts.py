@@ -405,6 +405,40 @@ def test_chunk_read_out_and_state_on_both_sides_of_their_grids(H, lens, d, dv):
         assert float((x - y).abs().max()) <= 2e-5 * max(1.0, float(y.abs().max()))
 
 
+def test_chunked_sums_of_two_threads_with_different_values(monkeypatch):
+    """Two host threads launch the decayed sum with 64 and 128 value columns, whose prepare blocks differ in shared memory, as fast as
+    they can: neither may lower what the other's launch was allowed between that thread's asking and its launch."""
+    import threading
+    H, n, d = 2, 3, 64
+    calls, kept = {}, []
+    for dv in (64, 128):
+        q, k, v = (rnd(n, H * w, seed=w).to(DEV) for w in (d, d, dv))
+        state, out = torch.zeros(1, H, d, dv, device=DEV), torch.empty(n, H * dv, device=DEV)
+        cu, _, sl = batch_index([n], [0])
+        scratch = torch.empty(K.recurrent_chunked_scratch_floats([n], H, d, dv, False), device=DEV)
+        decay = torch.tensor([0.9, 0.5], device=DEV)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream), monkeypatch.context() as m:
+            m.setattr(K, "_call", lambda name, *args: calls.__setitem__(dv, args))
+            K.recurrent_chunked(q, k, v, state, cu, sl, [n], out, scratch, H, H, d, dv, decay=decay)
+        kept.append((q, k, v, state, out, cu, sl, scratch, decay, stream))
+    launch = K._fn("pmm_recurrent_chunked")
+    torch.cuda.synchronize()
+    codes, ready = {}, threading.Barrier(2)
+
+    def serve(dv):
+        ready.wait(30)
+        codes[dv] = {launch(*calls[dv]) for _ in range(10000)}
+
+    threads = [threading.Thread(target=serve, args=(dv,)) for dv in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert codes == {64: {0}, 128: {0}}, codes
+
+
 # ----------------------------------------------------------------------------- window attention pieces
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,G,d,dv,rot", [(4, 2, 16, 32, 8), (2, 2, 48, 48, 48), (3, 1, 64, 16, 0), (8, 4, 64, 48, 64)])
