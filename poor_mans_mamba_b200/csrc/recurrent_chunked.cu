@@ -779,8 +779,9 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // ----------------------------------------------------------------------------------------------
 // The decayed sum has no product with the state inside its chain: S_end = a^n S_0 + N with
-// N = (K * a^(n-1-j))^T V, so the chain over a sequence's chunks is element-wise.  Three launches after
-// the operands', all but the middle one parallel over chunks: (1) N of every chunk; (2) a running
+// N = (K * a^(n-1-j))^T V, so the chain over a sequence's chunks is element-wise.  Three steps after
+// the operands', all but the middle one parallel over chunks: (1) N of every chunk (in the operands' launch where
+// `launch_chunked` finds that better, else in its own); (2) a running
 // pass per state element that leaves every chunk's starting state where its N was; (3) the rows
 // o_i = (q_i a^(i+1))^T S_0 + sum_{j<=i} B_ij v_j of every chunk.
 constexpr int kDecayTile = 64;      // state columns per block in (1) and (3)
@@ -1334,8 +1335,9 @@ PMM_EXPORT long long pmm_recurrent_chunked_scratch(int d, int dv, int rule) {
 }
 
 namespace pmm {
-// the arrays of the scratch; every one starts on a 16-byte boundary where d is a multiple of 4 (the copies in 16 bytes
-// need no more: the d * dv array is read with plain loads)
+// The arrays of the scratch.  Every one starts on a 16-byte boundary, as the 16-byte copies and stores of the kernels need (of N
+// too, whose rows are read in 16 bytes where dv is a multiple of 4): d is a multiple of 4, so every array before another holds a
+// multiple of four floats.
 inline void place_scratch(ChunkArgs& p, float* s, size_t ch, bool delta) {
   const int d = p.d, dv = p.dv;
   p.Ke = s; s += ch * kChunk * d;

@@ -12,8 +12,8 @@
 // W's rows are the M side of the instruction (128), the tokens (rounded up to 16) its N side, so that a block issues 16
 // instructions at most.  The blocks along K of a tile are one thread-block cluster: each leaves its partial sums [token][row]
 // in its shared memory and, behind one cluster barrier, block r adds up the r-th part of the tokens from all of them in
-// the order of K (float) and runs the epilogue, four columns of a row a thread.  Only RESIDUAL products longer than a
-// cluster's 1,024 columns meet in more than one atomic add an element.  97 KB of shared memory a block: two fit an SM, so the
+// the order of K (float) and runs the epilogue, four columns of a row a thread.  RESIDUAL products longer than a cluster's
+// 1,024 columns, and two products in one launch, meet in more than one atomic add an element, whose order is not fixed.  97 KB of shared memory a block: two fit an SM, so the
 // next product's weights are on their way while this one runs.  Clusters of 8 blocks of 128 columns were slower inside a
 // decode step of 64 requests (602 against 543 us).
 // Inside a prompt step of 37 tokens, layers of 1,024 -> 4,120, 1,536 + 512 -> 1,024, 1,024 -> 2 x 2,048 -> 1,024, us from
@@ -24,7 +24,6 @@
 // memory is freed.  No cluster multicast.
 // (reference: linear layers are cublasSgemm calls, src/ops/gpu/linear.cu:3-21.)
 #include "tcgen05.cuh"
-#include <algorithm>
 
 namespace pmm {
 
@@ -44,7 +43,6 @@ enum { kStStore = 0, kStSwiglu = 1, kStResidual = 2, kStGelu = 3 };  // GELU: ST
 struct SkinnyTcArgs {
   int T, N;          // tokens, output columns (SWIGLU: F)
   int t_pad;         // T rounded up to a multiple of 16
-  int n_problems;
   int K[2];
   int groups[2];     // clusters along K of each product
   float scale[2];    // RESIDUAL: factor on y; SWIGLU: gate multiplier
@@ -314,7 +312,6 @@ PMM_EXPORT int pmm_skinny_tc(int mode, int T, int N, const void* x0, long long l
   pmm::SkinnyTcArgs a{};
   a.T = T;
   a.N = N;
-  a.n_problems = w1 ? 2 : 1;
   a.K[0] = K0;
   a.K[1] = w1 ? K1 : 0;
   a.scale[0] = scale0;
@@ -324,7 +321,7 @@ PMM_EXPORT int pmm_skinny_tc(int mode, int T, int N, const void* x0, long long l
   a.h_out = h_out;
   a.status = status;
   a.t_pad = (T + 15) / 16 * 16;
-  for (int p = 0; p < a.n_problems; ++p) {
+  for (int p = 0; p < (w1 ? 2 : 1); ++p) {
     const int boxes = (a.K[p] + pmm::kStKB - 1) / pmm::kStKB, held = pmm::kStCluster * pmm::kStMaxKB;
     a.groups[p] = (boxes + held - 1) / held;
   }

@@ -1611,7 +1611,7 @@ def _skinny_tc_operand(x: Tensor, w: Tensor) -> bool:
 
 def skinny_tc_supported(kind: str, x: Tensor, weight: Tensor, out: Optional[Tensor] = None) -> bool:
     """Whether the tcgen05 weight-streaming product (1..64 tokens) takes these operands; kind is
-    "store", "swiglu" (both keep all of K resident: at most 1,024 columns) or "residual"."""
+    "store", "swiglu" (both end within one cluster of blocks along K: at most 1,024 columns) or "residual"."""
     if not _skinny_tc_operand(x, weight):
         return False
     mode = {"store": 0, "swiglu": 1, "residual": 2}[kind]
@@ -1650,8 +1650,8 @@ def skinny_tc_swiglu(x: Tensor, gate_up: Tensor, gate_mult: float, out: Tensor) 
 
 
 def skinny_tc_residual(h: Tensor, products: Sequence[Tuple[Tensor, Tensor, float]]) -> None:
-    """h[T, N] += sum_i scale_i * (x_i @ w_i^T) for one or two products (tcgen05, up to 64 tokens;
-    float32 atomics, K in slices of at most 1,024 columns)."""
+    """h[T, N] += sum_i scale_i * (x_i @ w_i^T) for one or two products (tcgen05, up to 64 tokens; one float32 atomic add
+    an element for every 1,024 columns of each product, in no fixed order)."""
     if not (1 <= len(products) <= 2):
         raise KernelError("skinny_tc_residual: one or two products")
     _cuda(h)
@@ -2612,8 +2612,8 @@ def recurrent_chunked(q: Tensor, k: Tensor, v: Tensor, state: Tensor, cu: Tensor
                       dt_bias: Optional[Tensor] = None, a_log: Optional[Tensor] = None, unit_eps: float = 0.0,
                       q_scale: float = 1.0) -> None:
     """The recurrences of delta_scan (``decay`` None) and decay_scan (``decay`` given) for prompt portions,
-    in chunks of 64 tokens: one launch prepares every chunk's operands in parallel, a second walks each
-    sequence's chunks in order.  Float arithmetic throughout; same arguments and results (beyond rounding)
+    in chunks of 64 tokens: every chunk's operands in parallel, a walk along each sequence's chunks, every chunk's rows
+    in parallel.  Float arithmetic throughout; same arguments and results (beyond rounding)
     as the token-serial kernels.  ``new_lens``: tokens per sequence (host values)."""
     delta = decay is None
     what = "recurrent_chunked"

@@ -850,7 +850,7 @@ def test_head_of_two_threads_with_different_rows():
     assert not failed, failed
 
 
-@pytest.mark.parametrize("T,N,Kd", [(16, 127, 64), (33, 129, 8), (48, 256, 1024), (49, 136, 328), (63, 8, 1016), (64, 4, 2056), (3, 1, 6152)])
+@pytest.mark.parametrize("T,N,Kd", [(16, 127, 64), (33, 129, 8), (49, 300, 8), (33, 515, 192), (48, 256, 1024), (49, 136, 328), (63, 8, 1016), (64, 4, 2056), (3, 1, 6152)])
 def test_tcgen05_product_in_clusters(T, N, Kd):
     """Blocks of a cluster share K: none of its boxes for some of them, one, four; tiles of 128 rows (64 + 64) and one beside;
     tokens on and off 16; products longer than a cluster in several.  Small whole numbers, so that the sums are exact
@@ -871,7 +871,18 @@ def test_tcgen05_product_in_clusters(T, N, Kd):
         out = torch.full((T, (N + 7) // 8 * 8), float("nan"), dtype=bf, device=DEV)
         ops.skinny_tc_linear(x, w, out[:, :N])
         assert torch.equal(out[:, :N].cpu(), ref.to(bf))
+        ops.skinny_tc_linear(x, w, out[:, :N], gelu=True)     # one rounding of the result beside a float erfc
+        want = torch.nn.functional.gelu(ref)
+        assert float((out[:, :N].cpu().double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
         assert bool(torch.isnan(out[:, N:]).all())
+        F = (N + 1) // 2                                      # 64 gate and 64 up rows a tile, F off whole tiles
+        gu = torch.randint(-3, 4, (2 * F, Kd), generator=g).to(bf).to(DEV)
+        act = torch.full((T, (F + 7) // 8 * 8), float("nan"), dtype=bf, device=DEV)
+        ops.skinny_tc_swiglu(x, gu, 0.25, act[:, :F])
+        both = x.double().cpu() @ gu.double().cpu().t()
+        want = torch.nn.functional.silu(0.25 * both[:, :F]) * both[:, F:]
+        assert float((act[:, :F].cpu().double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+        assert bool(torch.isnan(act[:, F:]).all())
     torch.cuda.synchronize()
     assert ops.tc_gemm_status(DEV) == 0
 
@@ -896,10 +907,9 @@ def test_tcgen05_product_of_more_tiles_than_a_grid_is_high():
 @pytest.mark.parametrize("T", [1, 17, 40, 64])
 @pytest.mark.parametrize("N,Kd", [(50, 96), (1024, 1000), (4120, 1024), (6000, 512), (304, 72)])
 def test_tcgen05_weight_streaming_product(T, N, Kd):
-    """The tcgen05 form of the weight-streaming product (17..64 tokens; fewer work too): store,
-    SwiGLU, and residual accumulation of one and two products with K in slices, at sizes on and
-    off the boxes of 64 columns and tiles of 32 rows, with more row tiles than blocks (a block then
-    walks several tiles through both accumulators), into column slices of wider buffers."""
+    """The tcgen05 form of the weight-streaming product (33..64 tokens; fewer work too): store,
+    SwiGLU, and residual accumulation of one and two products with K over one cluster and several, at sizes on and
+    off the boxes of 64 columns and tiles of 128 rows, into column slices of wider buffers."""
     g = torch.Generator().manual_seed(T * 131 + N + Kd)
     ops = K()
     bf = torch.bfloat16
