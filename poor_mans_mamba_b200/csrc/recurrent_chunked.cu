@@ -130,11 +130,12 @@ __device__ __forceinline__ Quad quad(const float* p) {  // sixteen bytes
 // All 64 rows of every chunk cost a step of one portion of 512 tokens beside 63 lone ones, 4 heads of 244 x 244, 703 us where
 // 587 us are enough.
 //
-// Bound by the issue of its own instructions; 256 threads and 109 KB at d = 128 put two blocks on an SM, so that one
-// block's barriers and shared-memory latencies are the other's turn and the 256 blocks of 2,048 tokens and 8 heads are one
-// wave.  That size, 128 x 128: first form (rows scaled per sub-block of 16 into copies, scalar shared-memory reads, a column
+// Bound by latency on few warps: 256 threads and 109 KB at d = 128 put two blocks on an SM, 3.4 warps a scheduler, which issue in
+// 43 % of the cycles (a warp waits about alike for global reads, shared-memory reads and its own arithmetic; DRAM 3 %).  One
+// block's barriers and reads are the other's turn, and the 256 blocks of 2,048 tokens and 8 heads are one wave.
+// That size, 128 x 128, inside a step: first form (rows scaled per sub-block of 16 into copies, scalar shared-memory reads, a column
 // walking A in shared memory, 157 KB) 160 us, 4 x 4 tiles with the solve's whole column in registers (unrolled past the
-// instruction cache, one block an SM) 96 us, this form 64 us.
+// instruction cache, one block an SM) 96 us, this form 59 us (68 alone with cold caches).
 constexpr float kLogDecayMin = -1e4f;  // a token's logarithm to base 2: the power is zero long before, and sums stay finite
 constexpr int kPrepRows = kChunk / 8;  // halves of 8 tokens
 
@@ -1043,7 +1044,8 @@ __global__ void __launch_bounds__(1024 / ROWS)
 // sum_{j<=i} B_ij u_j of all chunks at once is the decayed sum's (decay_chunk_output_kernel with U as its values).
 // Both products are made in 4 x 4 tiles with the summed index shared by 8 (4) lanes, two multiply-adds an instruction;
 // the next chunk's W and Ke come by asynchronous copies meanwhile.  Bound by the latency of a link (barriers, reads, sums
-// over lanes) on two warps a scheduler.  Measured at 2,048 tokens and 8 heads of 128 x 128 (32 links): 72 us; with
+// over lanes) on two warps a scheduler (37 % of issue slots, a warp every 5.5 cycles).  2,048 tokens and 8 heads of 128 x 128 (32
+// links) inside a step: 70 us (72 alone with cold caches); with
 // the summed index shared by 16 (8) lanes of 512 threads 95 us, in 2 x 2 (4 x 2) tiles shared by two lanes 99 us.
 // (The form S_end = M S_0 + N with M = diag(exp L_end) - Ke^T W reads as many bytes a link, needs a launch of its own for M
 // and N and leaves W S_0 to the read-out: its three launches took 50, 130 and 74 us behind the operands'.)
