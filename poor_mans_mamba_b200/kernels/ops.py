@@ -101,7 +101,7 @@ _SIGNATURES = {
     "pmm_l2_prefetch": [c_void_p, c_void_p, c_int, c_void_p],
     "pmm_attention_tc_supported": [c_int, c_int, c_int, c_int],
     "pmm_attention_tc": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-                         c_void_p, c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                         c_void_p, c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                          c_void_p, c_void_p, c_void_p, c_void_p],
     "pmm_skinny_chain": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p],
     "pmm_flash_decode_attention": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_float,
@@ -1741,17 +1741,29 @@ def attention_tc_supported(n_q_heads: int, n_kv_heads: int, head_dim: int, page_
     return bool(_fn("pmm_attention_tc_supported")(n_q_heads, n_kv_heads, head_dim, page_size))
 
 
+def attention_tc_rows(n_q_heads: int, n_kv_heads: int, head_dim: int, new_lens: Sequence[int]) -> int:
+    """Query rows of a block of `attention_tc`: 64 while blocks of 64 rows all run at once (148 SMs, two blocks an SM at head
+    size 64, one at 128) and the group divides them, else 128, which reads keys and values half as often.  Measured, us, 64 /
+    128 rows: 8 query and 2 key/value heads of 64, 2,048 tokens 21.3 / 28.5, 300 tokens 6.7 / 8.9; 16 and 4 heads 33.7 / 31.2;
+    8,192 tokens 167 / 152; 12 and 2 heads of 128, 1,024 tokens 18.4 / 17.8, 2,048 tokens 46.7 / 30.0."""
+    group = n_q_heads // n_kv_heads
+    if 64 % group:
+        return 128
+    blocks = sum((n * group + 63) // 64 for n in new_lens) * n_kv_heads
+    return 64 if blocks <= 148 * (2 if head_dim == 64 else 1) else 128
+
+
 def attention_tc(q: Tensor, pool: Tensor, block_table: Tensor, positions: Tensor, cu_seqlens: Tensor,
                  new_lens: Sequence[int], out: Tensor, n_q_heads: int, n_kv_heads: int, head_dim: int,
                  softmax_scale: float, window: int = 0, n_splits: int = 1, split_len: int = 0,
                  scratch: Optional[Tensor] = None, split_counter: Optional[Tensor] = None,
                  sink: Optional[Tensor] = None, keep_first: int = 0, lse: Optional[Tensor] = None,
-                 seq_of: Optional[Tensor] = None) -> None:
+                 seq_of: Optional[Tensor] = None, rows: Optional[int] = None) -> None:
     """Causal attention of prompt portions over the paged cache on the fifth-generation tensor cores
-    (TMA tiles straight from the pages, scores and P V in tensor memory, one thread per query row
-    for the softmax).  Same contract as paged_attention with rotated queries and a cache that holds
-    the step's keys already; 128 rows of (token, query head of a group) per block.  ``keep_first`` > 0 behind a
-    window: one key split, ``lse`` scratch and ``seq_of``, as in paged_attention."""
+    (TMA tiles straight from the pages, scores and P V in tensor memory, four threads per two query
+    rows for the softmax).  Same contract as paged_attention with rotated queries and a cache that holds
+    the step's keys already; 64 or 128 ``rows`` of (token, query head of a group) per block (None: `attention_tc_rows`).
+    ``keep_first`` > 0 behind a window: one key split, ``lse`` scratch and ``seq_of``, as in paged_attention."""
     _cuda(q, pool, block_table, positions, cu_seqlens, out, scratch, split_counter)
     T = q.shape[0]
     keep = int(keep_first) if window > 0 else 0
@@ -1768,8 +1780,15 @@ def attention_tc(q: Tensor, pool: Tensor, block_table: Tensor, positions: Tensor
     _i32(block_table, "attention_tc: block_table")
     _i32(positions, "attention_tc: positions")
     _i32(cu_seqlens, "attention_tc: cu_seqlens")
-    per_tile = 128 // (n_q_heads // n_kv_heads)
-    n_tiles = sum((n + per_tile - 1) // per_tile for n in new_lens)
+    group = n_q_heads // n_kv_heads
+    tiles_of = lambda r: sum((n + r // group - 1) // (r // group) for n in new_lens)
+    if rows is None:
+        rows = attention_tc_rows(n_q_heads, n_kv_heads, head_dim, new_lens)
+        if n_splits > 1 and split_counter is not None and split_counter.numel() < tiles_of(rows) * n_kv_heads:
+            rows = 128
+    if rows not in (64, 128):
+        raise KernelError("attention_tc: a block takes 64 or 128 rows")
+    n_tiles = tiles_of(rows)
     part_o = part_ml = counter = None
     if n_splits > 1:
         need = attention_scratch_floats(T, n_q_heads, head_dim, n_splits)
@@ -1786,7 +1805,7 @@ def attention_tc(q: Tensor, pool: Tensor, block_table: Tensor, positions: Tensor
         counter = split_counter.data_ptr()
     _call("pmm_attention_tc", q.data_ptr(), pool.data_ptr(), pool.shape[0], block_table.data_ptr(), block_table.shape[1],
           positions.data_ptr(), cu_seqlens.data_ptr(), out.data_ptr(), part_o, part_ml, float(softmax_scale), int(window),
-          int(split_len), int(n_splits), pool.shape[2], len(new_lens), n_tiles, n_q_heads, n_kv_heads, head_dim, counter,
+          int(split_len), int(n_splits), pool.shape[2], len(new_lens), n_tiles, rows, n_q_heads, n_kv_heads, head_dim, counter,
           _tc_status(q.device).data_ptr(), _ptr(sink), _lse_ptr(lse, T, n_q_heads) if keep > 0 else None, _stream())
     if keep > 0:
         kept_first_merge(q, pool, block_table, positions, seq_of, out, lse, n_q_heads, n_kv_heads, head_dim, softmax_scale,

@@ -449,6 +449,7 @@ class ParallelPreNormBlock(Part):
                 outs = [stream.take_branch() for _ in self.mixers]
             side = self._side_stream(proj.device) if len(self.mixers) > 1 and _PARALLEL_MIXERS else None
             main = torch.cuda.current_stream(proj.device)
+            ctx.beside_mixers = side is not None
             for i, (m, (c0, c1)) in enumerate(zip(self.mixers, self._fused_cols)):
                 def run(i=i, m=m, c0=c0, c1=c1):
                     if joined is not None:
@@ -462,6 +463,7 @@ class ParallelPreNormBlock(Part):
                         run()
                 else:
                     run()
+            ctx.beside_mixers = False
             if side is not None:
                 main.wait_stream(side)
             if joined is not None:

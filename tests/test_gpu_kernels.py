@@ -537,6 +537,57 @@ def test_tcgen05_attention_over_the_paged_cache(Hq, Hkv, page, Dh):
     assert not K().attention_tc_supported(Hq, Hkv, Dh, 16)
 
 
+@pytest.mark.parametrize("Hq,Hkv,Dh", [(8, 2, 64), (2, 2, 64), (64, 1, 64), (8, 1, 128), (10, 2, 64)])
+@pytest.mark.parametrize("window,splits,sink", [(0, 1, False), (100, 1, True), (-96, 1, False), (0, 3, True)])
+def test_tcgen05_attention_rows_of_a_block(Hq, Hkv, Dh, window, splits, sink):
+    """Blocks of 64 and of 128 rows: the same bits (groups that divide 64; others cut a window's keys elsewhere), near the
+    sums in float64, for portions that end on, before and behind the edges of both, behind prefixes off the boxes of 64 keys."""
+    ops, bf, page, group = K(), torch.bfloat16, 64, Hq // Hkv
+    g = torch.Generator().manual_seed(Hq * 100 + Dh + splits)
+    lens, past = [1, 64 // group or 1, 128 // group + 1, 70, 131], [0, 200, 63, 1, 77]
+    T, ends = sum(lens), [n + p for n, p in zip(lens, past)]
+    blocks = [(e + page - 1) // page for e in ends]
+    pool = torch.randn(sum(blocks) + 1, 2, page, Hkv * Dh, generator=g).to(bf)
+    table = torch.full((len(lens), max(blocks)), sum(blocks), dtype=torch.int32)
+    order, used = torch.randperm(sum(blocks), generator=g).int(), 0
+    for i, b in enumerate(blocks):
+        table[i, :b] = order[used:used + b]
+        used += b
+    q = (2 * torch.randn(T, Hq * Dh, generator=g)).to(bf)
+    s = torch.randn(Hq, generator=g) if sink else None
+    pos = torch.cat([torch.arange(p, e) for p, e in zip(past, ends)]).int()
+    cu = torch.tensor([0] + lens).cumsum(0).int()
+    split_len = 128
+    assert max(ends) <= 3 * split_len
+    out = {}
+    for rows in (64, 128):
+        out[rows] = torch.empty(T, Hq * Dh, dtype=bf, device=DEV)
+        scratch = torch.full((ops.attention_scratch_floats(T, Hq, Dh, splits),), float("nan"), device=DEV) if splits > 1 else None
+        counter = torch.zeros(4096, dtype=torch.int32, device=DEV)
+        ops.attention_tc(q.to(DEV), pool.to(DEV), table.to(DEV), pos.to(DEV), cu.to(DEV), lens, out[rows], Hq, Hkv, Dh, Dh ** -0.5,
+                         window=window, n_splits=splits, split_len=split_len if splits > 1 else 0, scratch=scratch,
+                         split_counter=counter, sink=s.to(DEV) if sink else None, rows=rows)
+        assert int(counter.abs().sum()) == 0
+    assert ops.tc_gemm_status(DEV) == 0
+    if 64 % group == 0:
+        assert torch.equal(out[64], out[128])
+    ref = torch.empty(T, Hq, Dh, dtype=torch.float64)
+    for i, n in enumerate(lens):
+        kv = pool[table[i, :blocks[i]].long()].double()
+        keys, vals = (kv[:, j].reshape(-1, Hkv, Dh)[:ends[i]].repeat_interleave(group, 1) for j in (0, 1))
+        at = torch.arange(ends[i])
+        for t in range(int(cu[i]), int(cu[i + 1])):
+            p = int(pos[t])
+            lo = max(0, p - window + 1) if window > 0 else p - p % -window if window < 0 else 0
+            sc = torch.einsum("hd,shd->hs", q[t].double().view(Hq, Dh), keys) * Dh ** -0.5
+            sc = sc.masked_fill(~((at <= p) & (at >= lo)), -math.inf)
+            if sink:
+                sc = torch.cat([sc, s.double()[:, None]], 1)
+            ref[t] = torch.einsum("hs,shd->hd", torch.softmax(sc, 1)[:, :ends[i]], vals)
+    for rows in (64, 128):
+        close(out[rows].view(T, Hq, Dh), ref, bf, what=f"{rows} rows")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tensor_cores", [True, False])
 def test_paged_attention_window(dtype, tensor_cores):
