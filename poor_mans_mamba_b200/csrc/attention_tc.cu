@@ -131,26 +131,6 @@ __device__ __forceinline__ float at_max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// A product issued by the lane for which `lead` is not zero, without a branch: the descriptors stay in uniform registers.
-__device__ __forceinline__ void at_umma(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc,
-                                        unsigned accumulate, unsigned lead) {
-  asm volatile(
-      "{\n\t.reg .pred p, l;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 l, %5, 0;\n\t"
-      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
-      : "memory");
-}
-__device__ __forceinline__ void at_commit(unsigned long long* bar, unsigned lead) {
-  asm volatile(
-      "{\n\t.reg .pred l;\n\t"
-      "setp.ne.b32 l, %1, 0;\n\t"
-      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)), "r"(lead)
-      : "memory");
-}
-
 // Place of a tile among the copies: K_0, K_1, V_0, K_2, V_1, ..., K_{n-1}, V_{n-2}, V_{n-1}, the order of the products.
 __device__ __forceinline__ int at_k_item(int j) { return j == 0 ? 0 : 2 * j - 1; }
 __device__ __forceinline__ int at_v_item(int j, int n) { return j + 1 < n ? 2 * j + 2 : 2 * j + 1; }
@@ -341,10 +321,10 @@ __global__ void __launch_bounds__(at_threads(M), DH == 64 ? 2 : 1)
         const unsigned long long k_desc = ring_desc + static_cast<unsigned>(slot * (kSlot >> 4));
 #pragma unroll
         for (int k = 0; k < DH / 16; ++k)  // 16 head-size columns a step, four steps a sub-tile
-          at_umma(tmem_base, q_desc + (k >> 2) * (kQSub >> 4) + 2 * (k & 3), k_desc + (k >> 2) * (kAtKvSub >> 4) + 2 * (k & 3),
+          umma_f16_lead(tmem_base, q_desc + (k >> 2) * (kQSub >> 4) + 2 * (k & 3), k_desc + (k >> 2) * (kAtKvSub >> 4) + 2 * (k & 3),
                   at_idesc_s(M), k > 0 ? 1u : 0u, lead);
-        at_commit(&bar_s, lead);
-        if (at_k_item(j) + kAtRing < items) at_commit(&bar_empty[slot], lead);  // (nobody waits for the last copies' slots)
+        umma_commit_lead(&bar_s, lead);
+        if (at_k_item(j) + kAtRing < items) umma_commit_lead(&bar_empty[slot], lead);  // (nobody waits for the last copies' slots)
       };
       int code = 0;
       if (wait(&bar_q, 0) && full(0)) {
@@ -378,10 +358,10 @@ __global__ void __launch_bounds__(at_threads(M), DH == 64 ? 2 : 1)
         for (int d = 0; d < NSUB; ++d)  // 64 head-size columns of O an instruction
 #pragma unroll
           for (int k = 0; k < kAtKeys / 16; ++k)
-            at_umma(tmem_base + kOff + d * kAtDhBlock, p_desc + (k / 4) * (kQSub >> 4) + 2 * (k % 4),
+            umma_f16_lead(tmem_base + kOff + d * kAtDhBlock, p_desc + (k / 4) * (kQSub >> 4) + 2 * (k % 4),
                     v_desc + d * (kAtKvSub >> 4) + ((k * 16 * 128) >> 4), at_idesc_o(M), (j > 0 || k > 0) ? 1u : 0u, lead);
-        at_commit(&bar_pv, lead);
-        if (v_item + kAtRing < items) at_commit(&bar_empty[slot], lead);
+        umma_commit_lead(&bar_pv, lead);
+        if (v_item + kAtRing < items) umma_commit_lead(&bar_empty[slot], lead);
       }
       if (code != 0) give_up(code);
     }

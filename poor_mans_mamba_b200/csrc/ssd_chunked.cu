@@ -295,8 +295,8 @@ __global__ void ssd_state_pass_kernel(const float* __restrict__ chunk_state, con
                                       bf16* __restrict__ start_state, float* __restrict__ state,
                                       const int* __restrict__ cu, const int* __restrict__ slots, int H, int PN, int q,
                                       int n_seq, int seqs_per_block, int skip_single) {
-  pdl_launch_dependents();
-  pdl_wait();
+  // (The sequences' bounds are inputs of the step: read before the wait.  The launch behind this one is let go only after it:
+  // then everything before this launch has finished, and that launch may read it without waiting for this one.)
   // four state elements per thread (P*N is a multiple of 4 for every compiled pair)
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   const int h = blockIdx.y, seq0 = blockIdx.z * seqs_per_block;
@@ -311,6 +311,8 @@ __global__ void ssd_state_pass_kernel(const float* __restrict__ chunk_state, con
   __syncthreads();
   int first = 0;
   for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) first += s_first[w];
+  pdl_wait();
+  pdl_launch_dependents();
   if (e >= PN) return;
   // a block takes several sequences in turn when a step holds many (mostly short) ones
   for (int seq = seq0; seq < min(n_seq, seq0 + seqs_per_block); ++seq) {
@@ -334,8 +336,6 @@ __global__ void __launch_bounds__(256)
     ssd_state_pass_multi_kernel(const float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
                                 bf16* __restrict__ start_state, float* __restrict__ state, const int* __restrict__ cu,
                                 const int* __restrict__ slots, int H, int PN, int q, int n_seq) {
-  pdl_launch_dependents();
-  pdl_wait();
   __shared__ int s_multi[256], s_chunks[256];
   __shared__ int s_seq, s_first, s_nc;
   const int tid = threadIdx.x;
@@ -376,6 +376,8 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();  // (behind the wait, as in the kernel above)
   const int e = (blockIdx.x * blockDim.x + tid) * 4;
   if (s_seq < 0 || e >= PN) return;
   ssd_pass_sequence(chunk_state, chunk_decay, start_state, state, slots[s_seq], H, PN, blockIdx.y, e, s_first, s_nc);

@@ -16,16 +16,16 @@
 //                      go out as float.
 //   2. the state pass of ssd_chunked.cu walks the chunks of a sequence in float and hands the
 //      state at every chunk's start on as bfloat16.
-//   3. ssd_tc_output:  one block per (chunk, head, slab of up to 64 head channels), two threads
-//                      per token: G = C B^T (128 x 128, tensor memory) and Y2 = C S^T are issued
-//                      together; every thread reads its row of G, applies the decay, the causal
-//                      mask and delta_j and writes the row of M as a bfloat16 operand into the
-//                      shared memory that held B; Y1 = M x follows (x as it lies in memory,
-//                      MN-major); y = Y1 + exp(cs_i) Y2 + D x, the gate y silu(z) fused.
-// All tiles are brought by 16-byte asynchronous copies into the 128-byte swizzled layout the
-// tensor core reads (rows beyond a short chunk are zero-filled, so they change nothing: their
-// delta is zero).  Any head size that is a multiple of 16 up to 128 and any state size that is a
-// multiple of 16 up to 256 is taken.  All differences of cs are <= 0: no exponential overflows;
+//   3. ssd_tc_output:  one block per chunk and run of units (a unit = a head's slab of up to 64
+//                      channels), four threads per token: G = C B^T (128 x 128, tensor memory) once
+//                      a block; per unit Y2 = C S^T, every thread reads its row of G, applies the
+//                      decay, the causal mask and delta_j and writes the row of M as a bfloat16
+//                      operand into the shared memory that held B, Y1 = M x follows (x as it lies in
+//                      memory, MN-major); y = Y1 + exp(cs_i) Y2 + D x, the gate y silu(z) fused.
+// Tiles come in the 128-byte swizzled layout that the tensor core reads, by 16-byte asynchronous
+// copies (rows beyond a short chunk zero-filled, so they change nothing: their delta is zero) or,
+// in phase 3, by TMA where they are whole tiles of 64 columns.  Any head size that is a multiple of 16 up to 128 and any state
+// size that is a multiple of 16 up to 256 is taken.  All differences of cs are <= 0: no exponential overflows;
 // delta, cs and every accumulator are float.  Every mbarrier wait is bounded (status codes
 // 31..33 in *status; the block then skips its output, frees its tensor memory and returns).
 #include "tcgen05.cuh"
@@ -204,7 +204,6 @@ __global__ void __launch_bounds__(kTState)
                         float* __restrict__ chunk_decay, float* __restrict__ chunk_dt, int H, int P, int N, int G,
                         int slabs_per_group, int tmem_cols, int skip_single, int* __restrict__ status) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bar;
   __shared__ unsigned s_tmem;
@@ -219,6 +218,7 @@ __global__ void __launch_bounds__(kTState)
   int seq_tokens;
   if (!tq_locate(cu, n_seq, c, t0, len, seq_tokens, s_loc)) return;
   if (skip_single && seq_tokens == 1) return;  // lone tokens of a mixed step are the token-serial kernel's
+  pdl_wait();  // (the sequences' bounds are inputs of the step)
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = tiles;                 // [128 tokens][128 channels]: two atoms of 64 channels
   unsigned char* sB = tiles + 2 * kTSub;     // [128 tokens][N]: one atom per 64 state columns
@@ -390,12 +390,26 @@ __global__ void __launch_bounds__(kTState)
 }
 
 // ----------------------------------------------------------------------------- phase 3
-// grid (chunks, H * (P / PB)); 512 threads: threads t, t + 128, t + 256 and t + 384 share token t of
-// the chunk (= tensor-memory lane t) and split its columns.  The chunk's B rows and the slab's
-// start-state rows lie one after the other in shared memory as ONE K-major operand of 128 + PB
-// rows, so G = C B^T and Y2 = C S^T are one product.  Tensor memory: G columns 0..127, Y2
-// columns 128..128+PB, Y1 columns 192..192+PB.
+// grid (chunks, groups * blocks a group); a block takes `per_block` units of one chunk and one group, a unit being a head's
+// slab of PB channels.  C and B of the chunk are brought once and G = C B^T is made once; then unit by unit the start state's
+// rows, x and the gate's input arrive while the unit before is worked on: Y2 = C S^T is issued, M made from G for the unit's
+// head (slabs of one head share it), Y1 = M x issued, and the rows y go out.  512 threads: threads t, t + 128, t + 256 and
+// t + 384 share token t of the chunk (= tensor-memory lane t) and split its columns; warp 16 issues the products.  Tensor
+// memory: G columns 0..127, Y2 columns 128..128+PB, Y1 columns 192..192+PB.
+// Everything but the start states was finished before the state pass was let go (it lets this launch go behind its own
+// wait), so C, B, x, the decays and G are there before this launch's wait.
+// What bounds it: a unit is a chain of two products, an exponential per entry of M's lower half and two per output, about
+// 2,400 clocks.  One block a unit (two blocks an SM, C and B brought and G made for every head) took 19.5 us at 24 heads of
+// 64 x 128 and 2,048 tokens and 56 us at 48 heads of 128 x 256 and 1,024 tokens.
 constexpr int kTOut = 512;
+constexpr int kTOutAll = kTOut + 32;
+
+__host__ __device__ constexpr int tq_state_bytes(int nb, int PB) { return nb * PB * 128; }
+// The second stage of the start states lies behind M in B's place where it fits there.
+__host__ __device__ constexpr bool tq_second_in_b(int nb, int PB) { return (nb - 2) * kTSub >= tq_state_bytes(nb, PB); }
+__host__ __device__ constexpr size_t tq_output_smem(int nb, int PB) {
+  return 1024 + static_cast<size_t>(nb + (nb > 2 ? nb : 2)) * kTSub + tq_state_bytes(nb, PB) * (tq_second_in_b(nb, PB) ? 1 : 2) + 3 * kTSub;
+}
 
 // Calls f(row, piece) for the 16-byte pieces tid, tid + 512, ... of `rows` rows of `cpr` pieces.
 template <typename F>
@@ -409,262 +423,394 @@ __device__ __forceinline__ void tq_pieces(int tid, int rows, int cpr, F f) {
   }
 }
 
-__global__ void __launch_bounds__(kTOut, 2)
-    ssd_tc_output_kernel(const bf16* __restrict__ xbc, int ld_xbc, const float* __restrict__ chunk_dt,
+// A lone token (a decoding request in a mixed step): y[p] = (C.B) delta x[p] + exp(cs_0) C.S[p] + D x[p] for the channels
+// col0 .. col0 + PB - 1 of head h, a warp per channel.
+__device__ __forceinline__ void tq_lone_output(const bf16* __restrict__ xbc, int ld_xbc, const float* __restrict__ dtp, float Dh1, int t0,
+                                               const bf16* __restrict__ start, bf16* __restrict__ y, int I, int g, int G, int N,
+                                               size_t col0, int PB, const bf16* __restrict__ z_raw, long long ld_z, float z_scale,
+                                               const float* __restrict__ z_bias, int warp, int lane) {
+  const float d0 = dtp[0], e0 = tq_ex2(dtp[kTQ]);
+  const bf16* rowp = xbc + static_cast<size_t>(t0) * ld_xbc;
+  const bf16* bp = rowp + I + g * N;
+  const bf16* cp = bp + G * N;
+  float cb = 0.f;
+  float cv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (lane * 8 < N) {
+    const uint4 cq = *reinterpret_cast<const uint4*>(cp + lane * 8), bq = *reinterpret_cast<const uint4*>(bp + lane * 8);
+    const unsigned cw[4] = {cq.x, cq.y, cq.z, cq.w}, bw[4] = {bq.x, bq.y, bq.z, bq.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 cf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&cw[e]));
+      const float2 bf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bw[e]));
+      cv[2 * e] = cf.x, cv[2 * e + 1] = cf.y;
+      cb += cf.x * bf.x + cf.y * bf.y;
+    }
+  }
+  cb = warp_sum(cb);
+  constexpr int kW = kTOut / 32;
+  for (int pbase = warp; pbase < PB; pbase += 4 * kW) {  // four channels of this warp at a time: their loads go out together
+    uint4 sq[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int p = pbase + u * kW;
+      sq[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (p < PB && lane * 8 < N) sq[u] = *reinterpret_cast<const uint4*>(start + static_cast<size_t>(p) * N + lane * 8);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int p = pbase + u * kW;
+      if (p >= PB) break;  // the same in every lane
+      const unsigned sw[4] = {sq[u].x, sq[u].y, sq[u].z, sq[u].w};
+      float acc = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 sf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&sw[e]));
+        acc += cv[2 * e] * sf.x + cv[2 * e + 1] * sf.y;
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) {
+        const float xv = __bfloat162float(rowp[col0 + p]);
+        float v = cb * d0 * xv + e0 * acc + Dh1 * xv;
+        if (z_raw) {
+          const float zv = __bfloat162float(z_raw[static_cast<long long>(t0) * ld_z + col0 + p]);
+          v *= silu_fast(zv * z_scale + (z_bias ? z_bias[col0 + p] : 0.f));
+        }
+        y[static_cast<size_t>(t0) * I + col0 + p] = __float2bfloat16_rn(v);
+      }
+    }
+  }
+}
+
+template <bool kTma>
+__global__ void __launch_bounds__(kTOutAll, 1)
+    ssd_tc_output_kernel(const __grid_constant__ CUtensorMap map_xbc, const __grid_constant__ CUtensorMap map_start,
+                         const __grid_constant__ CUtensorMap map_z, const bf16* __restrict__ xbc, int ld_xbc, const float* __restrict__ chunk_dt,
                          const float* __restrict__ d_skip, const int* __restrict__ cu, int n_seq,
-                         const bf16* __restrict__ start_state, bf16* __restrict__ y, int H, int P, int N, int G, int PB,
-                         const bf16* __restrict__ z_raw, long long ld_z, float z_scale, const float* __restrict__ z_bias,
-                         int z_vec, int skip_single, int* __restrict__ status) {
+                         const bf16* __restrict__ start_state, bf16* __restrict__ y, int H, int P, int N, int G, int PB_any,
+                         int per_block, const bf16* __restrict__ z_raw, long long ld_z, float z_scale,
+                         const float* __restrict__ z_bias, int z_vec, int skip_single, int* __restrict__ status) {
   pdl_launch_dependents();
-  pdl_wait();
+  const int PB = kTma ? 64 : PB_any;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long bar1, bar2;
+  __shared__ __align__(8) unsigned long long bar_g, bar_y, bar_cb, bar_x[2], bar_s[2], bar_z;
   __shared__ unsigned s_tmem;
   __shared__ int s_abort;
-  __shared__ float s_delta[kTQ], s_csl[kTQ];  // delta_j and cs_j * log2(e)
+  __shared__ __align__(16) float s_dt[2][2 * kTQ];  // per stage: delta_j, then cs_j * log2(e)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int row = tid & (kTQ - 1), part = tid >> 7, rw = warp & 3;
+  const bool worker = tid < kTOut;  // (warp 16 issues the products)
   const int c = blockIdx.x;
   int t0, len;
   __shared__ int s_loc[36];
   int seq_tokens;
   if (!tq_locate(cu, n_seq, c, t0, len, seq_tokens, s_loc)) return;
   if (skip_single && seq_tokens == 1) return;  // lone tokens of a mixed step are the token-serial kernel's
-  const int slabs = P / PB;
-  const int h = blockIdx.y / slabs, p0 = (blockIdx.y % slabs) * PB;
-  const int I = H * P, g = h / (H / G);
-  const int nb = (N + 63) / 64;
-  const int bs_sub = (kTQ + PB) * 128;  // bytes of one 64-column block of the [B ; S] operand
-  unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* sC = tiles;                                  // [128 tokens][N], K-major; later M [128][128]
-  unsigned char* sBS = sC + (nb > 2 ? nb : 2) * kTSub;        // [128 tokens + PB channels][N], K-major; later z [128][PB]
-  unsigned char* sX = sBS + nb * bs_sub;                      // [128 tokens][PB], MN-major; later y, in place
-  const size_t col0 = static_cast<size_t>(h) * P + p0;
+  const int slabs = P / PB, heads = H / G, group_units = heads * slabs;
+  const int group_blocks = (group_units + per_block - 1) / per_block;
+  const int g = blockIdx.y / group_blocks;
+  const int unit0 = static_cast<int>(blockIdx.y % group_blocks) * per_block, n_units = min(per_block, group_units - unit0);
+  const int I = H * P;
+  auto head_of = [&](int k) { return g * heads + (unit0 + k) / slabs; };
+  auto col_of = [&](int k) { return static_cast<size_t>(g * heads * P) + static_cast<size_t>(unit0 + k) * PB; };
 
   if (len == 1) {
-    // A lone token: y[p] = (C.B) delta x[p] + exp(cs_0) C.S[p] + D x[p], a warp per channel.
-    const float* dtp = chunk_dt + (static_cast<size_t>(c) * H + h) * (2 * kTQ);
-    const float d0 = dtp[0], e0 = tq_ex2(dtp[kTQ]), Dh1 = d_skip[h];
-    const bf16* rowp = xbc + static_cast<size_t>(t0) * ld_xbc;
-    const bf16* bp = rowp + I + g * N;
-    const bf16* cp = bp + G * N;
-    float cb = 0.f;
-    float cv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (lane * 8 < N) {
-      const uint4 cq = *reinterpret_cast<const uint4*>(cp + lane * 8), bq = *reinterpret_cast<const uint4*>(bp + lane * 8);
-      const unsigned cw[4] = {cq.x, cq.y, cq.z, cq.w}, bw[4] = {bq.x, bq.y, bq.z, bq.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 cf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&cw[e]));
-        const float2 bf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bw[e]));
-        cv[2 * e] = cf.x, cv[2 * e + 1] = cf.y;
-        cb += cf.x * bf.x + cf.y * bf.y;
+    pdl_wait();
+    if (worker)
+      for (int k = 0; k < n_units; ++k) {
+        const int h = head_of(k);
+        tq_lone_output(xbc, ld_xbc, chunk_dt + (static_cast<size_t>(c) * H + h) * (2 * kTQ), d_skip[h], t0,
+                       start_state + (static_cast<size_t>(c) * I + col_of(k)) * N, y, I, g, G, N, col_of(k), PB, z_raw, ld_z, z_scale,
+                       z_bias, warp, lane);
       }
-    }
-    cb = warp_sum(cb);
-    constexpr int kW = kTOut / 32;
-    for (int pbase = warp; pbase < PB; pbase += 4 * kW) {  // four channels of this warp at a time: their loads go out together
-      uint4 sq[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int p = pbase + u * kW;
-        sq[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (p < PB && lane * 8 < N)
-          sq[u] = *reinterpret_cast<const uint4*>(start_state + (static_cast<size_t>(c) * I + col0 + p) * N + lane * 8);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int p = pbase + u * kW;
-        if (p >= PB) break;  // the same in every lane
-        const unsigned sw[4] = {sq[u].x, sq[u].y, sq[u].z, sq[u].w};
-        float acc = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 sf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&sw[e]));
-          acc += cv[2 * e] * sf.x + cv[2 * e + 1] * sf.y;
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) {
-          const float xv = __bfloat162float(rowp[col0 + p]);
-          float v = cb * d0 * xv + e0 * acc + Dh1 * xv;
-          if (z_raw) {
-            const float zv = __bfloat162float(z_raw[static_cast<long long>(t0) * ld_z + col0 + p]);
-            v *= silu_fast(zv * z_scale + (z_bias ? z_bias[col0 + p] : 0.f));
-          }
-          y[static_cast<size_t>(t0) * I + col0 + p] = __float2bfloat16_rn(v);
-        }
-      }
-    }
     return;
   }
 
+  const int nb = (N + 63) / 64;
+  const int s_sub = PB * 128;  // bytes of one 64-column block of the start state's rows
+  unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* sC = tiles;                                // [128 tokens][N], K-major
+  unsigned char* sB = sC + nb * kTSub;                      // [128 tokens][N], K-major; later M [128][128]
+  unsigned char* sX = sB + (nb > 2 ? nb : 2) * kTSub;       // two stages of [128 tokens][PB], MN-major; later y, in place
+  unsigned char* sZ = sX + 2 * kTSub;                       // [128 tokens][PB]
+  unsigned char* sS0 = sZ + kTSub;                          // [PB channels][N], K-major
+  unsigned char* sS1 = tq_second_in_b(nb, PB) ? sB + 2 * kTSub : sS0 + tq_state_bytes(nb, PB);
+
   if (tid == 0) {
-    mbar_init(&bar1, 1);
-    mbar_init(&bar2, 1);
+    mbar_init(&bar_g, 1);
+    mbar_init(&bar_y, 1);
+    mbar_init(&bar_cb, 1);
+    mbar_init(&bar_x[0], 1);
+    mbar_init(&bar_x[1], 1);
+    mbar_init(&bar_s[0], 1);
+    mbar_init(&bar_s[1], 1);
+    mbar_init(&bar_z, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  tq_pieces(tid, kTQ, N / 8, [&](int j, int ck) {
-    const bool ok = j < len;
-    const size_t src = ok ? static_cast<size_t>(t0 + j) * ld_xbc + I + g * N + ck * 8 : 0;
-    tq_cp16(sBS + (ck >> 3) * bs_sub + tq_swz(j, ck & 7), xbc + src, ok);
-    tq_cp16(sC + (ck >> 3) * kTSub + tq_swz(j, ck & 7), xbc + src + (ok ? G * N : 0), ok);
-  });
-  {
-    const bf16* src = start_state + (static_cast<size_t>(c) * I + col0) * N;
-    tq_pieces(tid, PB, N / 8, [&](int p, int ck) {
-      tq_cp16(sBS + (ck >> 3) * bs_sub + tq_swz(kTQ + p, ck & 7), src + static_cast<size_t>(p) * N + ck * 8, true);
+  auto copy_x = [&](int k) {  // x and the decays of unit k into its stage
+    unsigned char* dst = sX + (k & 1) * kTSub;
+    const size_t col = col_of(k);
+    tq_pieces(tid, kTQ, PB / 8, [&](int j, int ck) {
+      const bool ok = j < len;
+      tq_cp16(dst + tq_swz(j, ck), xbc + (ok ? static_cast<size_t>(t0 + j) * ld_xbc + col + ck * 8 : 0), ok);
     });
-  }
-  tq_pieces(tid, kTQ, PB / 8, [&](int j, int ck) {
-    const bool ok = j < len;
-    tq_cp16(sX + tq_swz(j, ck), xbc + (ok ? static_cast<size_t>(t0 + j) * ld_xbc + col0 + ck * 8 : 0), ok);
-  });
-  if (tid < kTQ) {  // delta_j and cs_j log2(e), as phase 1 left them
-    const float* dtp = chunk_dt + (static_cast<size_t>(c) * H + h) * (2 * kTQ);
-    s_delta[tid] = dtp[tid];
-    s_csl[tid] = dtp[kTQ + tid];
-  }
-  const float Dh = d_skip[h];
-  tq_cp_wait();
-  fence_proxy_async();
-  const unsigned tmem_base = tq_tmem_alloc(&s_tmem, 256, warp);  // includes the __syncthreads after the copies
-
-  if (tid == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const unsigned idesc = tq_idesc(kTQ + PB, false);
-    for (int k = 0; k < N / 16; ++k)  // [G | Y2] = C [B ; S]^T, K = the state columns
-      umma_f16(tmem_base, umma_desc(sC + (k >> 2) * kTSub) + 2 * (k & 3), umma_desc(sBS + (k >> 2) * bs_sub) + 2 * (k & 3),
-               idesc, k > 0 ? 1u : 0u);
-    umma_commit(&bar1);
-  }
-  volatile int* abort_flag = &s_abort;
-  const unsigned lane_base = tmem_base + (static_cast<unsigned>(rw * 32) << 16);
-  bool ok = mbar_wait(&bar1, 0, abort_flag);
-  ok = __all_sync(0xffffffffu, ok);
-  if (!ok && lane == 0) {
-    if (!*abort_flag) atomicExch(status, 32);
-    s_abort = 1;
-  }
-  const float csl_i = s_csl[row];
-  unsigned char* sZ = sBS;
-  if (ok) {
-    // C, B and S have been read.  The gate's inputs of the chunk come into B's place while M is made.
-    if (z_raw && z_vec) {
-      tq_pieces(tid, kTQ, PB / 8, [&](int j, int ck) {
-        const bool in = j < len;
-        tq_cp16(sZ + tq_swz(j, ck), z_raw + (in ? static_cast<long long>(t0 + j) * ld_z + col0 + ck * 8 : 0), in);
-      });
-    }
-    // M[i][j] = G[i][j] exp(cs_i - cs_j) delta_j for j <= i, as the A operand of Y1 = M x, in C's
-    // place; this thread's 32 columns
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    unsigned char* sM = sC;
-    const int jc = part;
-    if (jc <= rw) {  // the warp's rows reach this block of 32 columns
-      unsigned v[32];
-      tmem_ld32(lane_base + jc * 32, v);
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-      for (int c8 = 0; c8 < 4; ++c8) {
-        float m[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int j = jc * 32 + c8 * 8 + e;
-          m[e] = j <= row ? __uint_as_float(v[c8 * 8 + e]) * tq_ex2(csl_i - s_csl[j]) * s_delta[j] : 0.f;
-        }
-        uint4 pk;
-        pk.x = tq_pack(m[0], m[1]);
-        pk.y = tq_pack(m[2], m[3]);
-        pk.z = tq_pack(m[4], m[5]);
-        pk.w = tq_pack(m[6], m[7]);
-        const int ck = jc * 4 + c8;
-        *reinterpret_cast<uint4*>(sM + (ck >> 3) * kTSub + tq_swz(row, ck & 7)) = pk;
+    if (tid < kTQ / 2)
+      tq_cp16(&s_dt[k & 1][tid * 4], chunk_dt + (static_cast<size_t>(c) * H + head_of(k)) * (2 * kTQ) + tid * 4, true);
+  };
+  auto copy_s = [&](int k) {
+    unsigned char* dst = (k & 1) ? sS1 : sS0;
+    const bf16* src = start_state + (static_cast<size_t>(c) * I + col_of(k)) * N;
+    tq_pieces(tid, PB, N / 8, [&](int p, int ck) {
+      tq_cp16(dst + (ck >> 3) * s_sub + tq_swz(p, ck & 7), src + static_cast<size_t>(p) * N + ck * 8, true);
+    });
+  };
+  auto commit = [&]() { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+  // (whole tiles of 64 columns) one lane of warp 16 asks for them; rows beyond the chunk bring what lies there: a row of C reaches
+  // only its own output, a row of B only entries of M that are set to zero, and x's rows are zeroed below
+  const unsigned dt_bytes = 2 * kTQ * sizeof(float);
+  auto tma_x = [&](int k) {
+    unsigned long long* bar = &bar_x[k & 1];
+    mbar_expect_tx(bar, kTSub + dt_bytes);
+    tma_load_2d(sX + (k & 1) * kTSub, &map_xbc, static_cast<int>(col_of(k)), t0, bar);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(s_dt[k & 1])),
+                 "l"(chunk_dt + (static_cast<size_t>(c) * H + head_of(k)) * (2 * kTQ)), "r"(dt_bytes), "r"(smem_u32(bar))
+                 : "memory");
+  };
+  auto tma_s = [&](int k) {
+    unsigned long long* bar = &bar_s[k & 1];
+    unsigned char* dst = (k & 1) ? sS1 : sS0;
+    mbar_expect_tx(bar, tq_state_bytes(nb, 64));
+    for (int b = 0; b < nb; ++b) tma_load_2d(dst + b * s_sub, &map_start, b * 64, c * I + static_cast<int>(col_of(k)), bar);
+  };
+  auto tma_z = [&](int k) {
+    mbar_expect_tx(&bar_z, kTSub);
+    tma_load_2d(sZ, &map_z, static_cast<int>(col_of(k)), t0, &bar_z);
+  };
+  const bool gate_tile = z_raw && z_vec;
+  if (kTma) {
+    __syncthreads();  // the barriers
+    if (tid == kTOut) {
+      mbar_expect_tx(&bar_cb, 2 * nb * kTSub);
+      for (int b = 0; b < nb; ++b) {
+        tma_load_2d(sB + b * kTSub, &map_xbc, I + g * N + b * 64, t0, &bar_cb);
+        tma_load_2d(sC + b * kTSub, &map_xbc, I + (G + g) * N + b * 64, t0, &bar_cb);
       }
-    } else {
-#pragma unroll
-      for (int c8 = 0; c8 < 4; ++c8) {
-        const int ck = jc * 4 + c8;
-        *reinterpret_cast<uint4*>(sM + (ck >> 3) * kTSub + tq_swz(row, ck & 7)) = make_uint4(0u, 0u, 0u, 0u);
-      }
+      tma_x(0);
+      if (gate_tile) tma_z(0);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  } else if (worker) {
+    tq_pieces(tid, kTQ, N / 8, [&](int j, int ck) {
+      const bool ok = j < len;
+      const size_t src = ok ? static_cast<size_t>(t0 + j) * ld_xbc + I + g * N + ck * 8 : 0;
+      tq_cp16(sB + (ck >> 3) * kTSub + tq_swz(j, ck & 7), xbc + src, ok);
+      tq_cp16(sC + (ck >> 3) * kTSub + tq_swz(j, ck & 7), xbc + src + (ok ? G * N : 0), ok);
+    });
+    commit();
+    copy_x(0);
+    commit();
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     fence_proxy_async();
   }
-  tq_cp_wait();  // the gate's inputs
-  __syncthreads();
-  if (tid == 0 && !s_abort) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const unsigned idesc_y1 = tq_idesc(PB, true);
-    const unsigned long long x_desc = umma_desc(sX);
-#pragma unroll
-    for (int k = 0; k < kTQ / 16; ++k)
-      umma_f16(tmem_base + 192, umma_desc(sC + (k >> 2) * kTSub) + 2 * (k & 3), x_desc + ((k * 16 * 128) >> 4), idesc_y1,
-               k > 0 ? 1u : 0u);
-    umma_commit(&bar2);
-  }
-  if (ok) {
-    ok = mbar_wait(&bar2, 0, abort_flag);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok && lane == 0) {
-      if (!*abort_flag) atomicExch(status, 33);
-      s_abort = 1;
-    }
-  }
-  if (ok) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const float e_i = tq_ex2(csl_i);
-    const bool row_ok = row < len;
-    for (int pc = part; pc < PB / 16; pc += 4) {
-      unsigned y1[16], y2[16];
-      tmem_ld16(lane_base + 192 + pc * 16, y1);
-      tmem_ld16(lane_base + 128 + pc * 16, y2);
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int ck = pc * 2 + hf;
-        uint4* cell = reinterpret_cast<uint4*>(sX + tq_swz(row, ck));  // x in, y out: the product has read x
-        const uint4 xq = *cell;
-        const unsigned xw[4] = {xq.x, xq.y, xq.z, xq.w};
-        unsigned zw[4] = {0u, 0u, 0u, 0u};
-        if (z_raw) {
-          if (z_vec) {
-            const uint4 zq = *reinterpret_cast<const uint4*>(sZ + tq_swz(row, ck));
-            zw[0] = zq.x, zw[1] = zq.y, zw[2] = zq.z, zw[3] = zq.w;
-          } else if (row_ok) {  // rows of z that do not start on 16-byte boundaries
-            const bf16* zp = z_raw + static_cast<long long>(t0 + row) * ld_z + col0 + ck * 8;
-#pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2)
-              zw[e2] = static_cast<unsigned>(__bfloat16_as_ushort(zp[2 * e2])) |
-                       (static_cast<unsigned>(__bfloat16_as_ushort(zp[2 * e2 + 1])) << 16);
-          }
-        }
-        unsigned out[4];
-#pragma unroll
-        for (int e2 = 0; e2 < 4; ++e2) {
-          const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xw[e2]));
-          const int e = hf * 8 + e2 * 2;
-          float v0 = __uint_as_float(y1[e]) + e_i * __uint_as_float(y2[e]) + Dh * xv.x;
-          float v1 = __uint_as_float(y1[e + 1]) + e_i * __uint_as_float(y2[e + 1]) + Dh * xv.y;
-          if (z_raw) {  // gate fused: y * silu(z), z = z_raw * z_scale + z_bias
-            const float2 zv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[e2]));
-            const size_t ch = col0 + ck * 8 + e2 * 2;
-            v0 *= silu_fast(zv.x * z_scale + (z_bias ? z_bias[ch] : 0.f));
-            v1 *= silu_fast(zv.y * z_scale + (z_bias ? z_bias[ch + 1] : 0.f));
-          }
-          out[e2] = tq_pack(v0, v1);
-        }
-        *cell = make_uint4(out[0], out[1], out[2], out[3]);
+  const unsigned tmem_base = tq_tmem_alloc(&s_tmem, 256, warp);  // includes the __syncthreads after the copies
+  volatile int* abort_flag = &s_abort;
+  bool ok = true;
+  auto wait_all = [&](unsigned long long* bar, unsigned parity, int code) {  // the same answer in a warp
+    if (!__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag))) {
+      if (lane == 0) {
+        if (!*abort_flag) atomicExch(status, code);
+        s_abort = 1;
       }
+      ok = false;
+    }
+    return ok;
+  };
+  const unsigned lead = lane == 0 ? 1u : 0u;
+  const unsigned long long c_desc = umma_desc(sC), b_desc = umma_desc(sB);
+  if (warp == kTOut / 32 && (!kTma || wait_all(&bar_cb, 0, 32))) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    for (int k = 0; k < N / 16; ++k)  // G = C B^T, K = the state columns
+      umma_f16_lead(tmem_base, c_desc + (k >> 2) * (kTSub >> 4) + 2 * (k & 3), b_desc + (k >> 2) * (kTSub >> 4) + 2 * (k & 3),
+                    tq_idesc(kTQ, false), k > 0 ? 1u : 0u, lead);
+    umma_commit_lead(&bar_g, lead);
+  }
+  pdl_wait();  // the start states come from the launch before this one
+  if (kTma) {
+    if (tid == kTOut) tma_s(0);
+  } else if (worker) {
+    copy_s(0);
+    commit();
+  }
+  wait_all(&bar_g, 0, 32);
+  const unsigned lane_base = tmem_base + (static_cast<unsigned>(rw * 32) << 16);
+  unsigned char* sM = sB;
+  int made = -1;  // the head whose M lies there
+  for (int k = 0; k < n_units; ++k) {
+    const int st = k & 1, h = head_of(k);
+    const size_t col0 = col_of(k);
+    const float Dh = d_skip[h];
+    if (kTma) {
+      wait_all(&bar_x[st], (k >> 1) & 1, 33);
+      if (len < kTQ) {  // x's rows beyond the chunk belong to others: zero times what they hold is not always zero
+        if (worker)
+          for (int i = tid; i < (kTQ - len) * 8; i += kTOut)
+            *reinterpret_cast<uint4*>(sX + st * kTSub + tq_swz(len + (i >> 3), i & 7)) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
+      }
+      if (warp == kTOut / 32) wait_all(&bar_s[st], (k >> 1) & 1, 33);
+    } else if (worker) {
+      if (z_raw && z_vec)
+        tq_pieces(tid, kTQ, PB / 8, [&](int j, int ck) {
+          const bool in = j < len;
+          tq_cp16(sZ + tq_swz(j, ck), z_raw + (in ? static_cast<long long>(t0 + j) * ld_z + col0 + ck * 8 : 0), in);
+        });
+      commit();
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the unit's state rows, x and decays
+      fence_proxy_async();
+    }
+    if (!kTma) __syncthreads();
+    if (warp == kTOut / 32) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const unsigned long long s_desc = umma_desc(st ? sS1 : sS0);
+      for (int i = 0; i < N / 16; ++i)  // Y2 = C S^T
+        umma_f16_lead(tmem_base + 128, c_desc + (i >> 2) * (kTSub >> 4) + 2 * (i & 3), s_desc + (i >> 2) * (s_sub >> 4) + 2 * (i & 3),
+                      tq_idesc(PB, false), i > 0 ? 1u : 0u, lead);
+    }
+    const float* s_delta = s_dt[st];
+    const float* s_csl = s_dt[st] + kTQ;
+    const float csl_i = s_csl[row];
+    if (worker) {
+      if (!kTma) {
+        if (k + 1 < n_units) {  // the next unit's, while this one is worked on
+          copy_s(k + 1);
+          copy_x(k + 1);
+        }
+        commit();
+      }
+      // M[i][j] = G[i][j] exp(cs_i - cs_j) delta_j for j <= i, as the A operand of Y1 = M x, in B's place; this thread's 32 columns
+      if (h != made) {
+        const int jc = part;
+        if (jc <= rw) {  // the warp's rows reach this block of 32 columns
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          unsigned v[32];
+          tmem_ld32(lane_base + jc * 32, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+          for (int c8 = 0; c8 < 4; ++c8) {
+            float m[8];
+#pragma unroll
+            for (int e = 0; e < 8; e += 4) {
+              const int j = jc * 32 + c8 * 8 + e;
+              const float4 cs4 = *reinterpret_cast<const float4*>(s_csl + j), de4 = *reinterpret_cast<const float4*>(s_delta + j);
+              const float cs[4] = {cs4.x, cs4.y, cs4.z, cs4.w}, de[4] = {de4.x, de4.y, de4.z, de4.w};
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                m[e + q] = j + q <= row ? __uint_as_float(v[c8 * 8 + e + q]) * tq_ex2(csl_i - cs[q]) * de[q] : 0.f;
+            }
+            uint4 pk;
+            pk.x = tq_pack(m[0], m[1]);
+            pk.y = tq_pack(m[2], m[3]);
+            pk.z = tq_pack(m[4], m[5]);
+            pk.w = tq_pack(m[6], m[7]);
+            const int ck = jc * 4 + c8;
+            *reinterpret_cast<uint4*>(sM + (ck >> 3) * kTSub + tq_swz(row, ck & 7)) = pk;
+          }
+        } else if (made < 0) {  // (zeros stay)
+#pragma unroll
+          for (int c8 = 0; c8 < 4; ++c8) {
+            const int ck = jc * 4 + c8;
+            *reinterpret_cast<uint4*>(sM + (ck >> 3) * kTSub + tq_swz(row, ck & 7)) = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        fence_proxy_async();
+      }
+      if (!kTma) asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the gate's inputs
+    }
+    made = h;
+    __syncthreads();
+    if (s_abort) break;  // (the same in every thread: the waits that raise it lie between the barriers of a round)
+    if (warp == kTOut / 32) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const unsigned long long m_desc = umma_desc(sM), x_desc = umma_desc(sX + st * kTSub);
+#pragma unroll
+      for (int i = 0; i < kTQ / 16; ++i)
+        umma_f16_lead(tmem_base + 192, m_desc + (i >> 2) * (kTSub >> 4) + 2 * (i & 3), x_desc + ((i * 16 * 128) >> 4), tq_idesc(PB, true),
+                      i > 0 ? 1u : 0u, lead);
+      umma_commit_lead(&bar_y, lead);
+      if (kTma && k + 1 < n_units && lane == 0) {  // the next unit's (the rows of the unit before have left that stage)
+        tma_s(k + 1);
+        tma_x(k + 1);
+      }
+      __syncwarp();
+    }
+    wait_all(&bar_y, k & 1, 33);
+    if (kTma && gate_tile && worker) wait_all(&bar_z, k & 1, 33);
+    unsigned char* xt = sX + st * kTSub;
+    if (ok && worker) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const float e_i = tq_ex2(csl_i);
+      const bool row_ok = row < len;
+      for (int pc = part; pc < PB / 16; pc += 4) {
+        unsigned y1[16], y2[16];
+        tmem_ld16(lane_base + 192 + pc * 16, y1);
+        tmem_ld16(lane_base + 128 + pc * 16, y2);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          const int ck = pc * 2 + hf;
+          uint4* cell = reinterpret_cast<uint4*>(xt + tq_swz(row, ck));  // x in, y out: the product has read x
+          const uint4 xq = *cell;
+          const unsigned xw[4] = {xq.x, xq.y, xq.z, xq.w};
+          unsigned zw[4] = {0u, 0u, 0u, 0u};
+          if (z_raw) {
+            if (z_vec) {
+              const uint4 zq = *reinterpret_cast<const uint4*>(sZ + tq_swz(row, ck));
+              zw[0] = zq.x, zw[1] = zq.y, zw[2] = zq.z, zw[3] = zq.w;
+            } else if (row_ok) {  // rows of z that do not start on 16-byte boundaries
+              const bf16* zp = z_raw + static_cast<long long>(t0 + row) * ld_z + col0 + ck * 8;
+#pragma unroll
+              for (int e2 = 0; e2 < 4; ++e2)
+                zw[e2] = static_cast<unsigned>(__bfloat16_as_ushort(zp[2 * e2])) |
+                         (static_cast<unsigned>(__bfloat16_as_ushort(zp[2 * e2 + 1])) << 16);
+            }
+          }
+          unsigned out[4];
+#pragma unroll
+          for (int e2 = 0; e2 < 4; ++e2) {
+            const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xw[e2]));
+            const int e = hf * 8 + e2 * 2;
+            float v0 = __uint_as_float(y1[e]) + e_i * __uint_as_float(y2[e]) + Dh * xv.x;
+            float v1 = __uint_as_float(y1[e + 1]) + e_i * __uint_as_float(y2[e + 1]) + Dh * xv.y;
+            if (z_raw) {  // gate fused: y * silu(z), z = z_raw * z_scale + z_bias
+              const float2 zv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[e2]));
+              const size_t ch = col0 + ck * 8 + e2 * 2;
+              v0 *= silu_fast(zv.x * z_scale + (z_bias ? z_bias[ch] : 0.f));
+              v1 *= silu_fast(zv.y * z_scale + (z_bias ? z_bias[ch + 1] : 0.f));
+            }
+            out[e2] = tq_pack(v0, v1);
+          }
+          *cell = make_uint4(out[0], out[1], out[2], out[3]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    }
+    if (kTma) fence_proxy_async();  // (a copy may take the place of what was read and written here)
+    __syncthreads();
+    if (s_abort) break;
+    if (kTma && gate_tile && k + 1 < n_units && tid == kTOut) tma_z(k + 1);
+    if (worker) {  // the finished rows go out in whole lines
+      tq_pieces(tid, len, PB / 8, [&](int j, int ck) {
+        *reinterpret_cast<uint4*>(y + static_cast<size_t>(t0 + j) * I + col0 + ck * 8) =
+            *reinterpret_cast<const uint4*>(xt + tq_swz(j, ck));
+      });
     }
   }
-  __syncthreads();
-  if (!s_abort) {  // the finished rows go out in whole lines
-    tq_pieces(tid, len, PB / 8, [&](int j, int ck) {
-      *reinterpret_cast<uint4*>(y + static_cast<size_t>(t0 + j) * I + col0 + ck * 8) =
-          *reinterpret_cast<const uint4*>(sX + tq_swz(j, ck));
-    });
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (kTma && s_abort && tid == kTOut) {
+    // copies that were asked for still write into this block's shared memory: a bounded time for them to land
+    for (unsigned i = 0; i < kSpinLimit / 4; ++i) __nanosleep(32);
   }
   tq_tmem_free(tmem_base, 256, warp);
 }
@@ -688,8 +834,8 @@ PMM_EXPORT int pmm_ssd_tc_supported(int P, int N) {
 PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long long ld_dt, float dt_scale,
                           const float* dt_shift, const float* a_log, const float* d_skip, float* state, const int* cu,
                           const int* slots, void* y, float* chunk_state, float* chunk_decay, float* chunk_dt,
-                          void* start_state, int n_seq, int n_chunks, int H, int P, int N, int G, const void* z_raw, long long ld_z,
-                          float z_scale, const float* z_bias, int skip_single, int n_multi, int* status,
+                          void* start_state, int n_seq, int n_tokens, int n_chunks, int H, int P, int N, int G, const void* z_raw,
+                          long long ld_z, float z_scale, const float* z_bias, int skip_single, int n_multi, int* status,
                           cudaStream_t stream) {
   using namespace pmm;
   if (n_seq <= 0 || n_chunks <= 0) return 0;
@@ -707,7 +853,30 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
   int tmem_cols = 32;
   while (tmem_cols < N) tmem_cols *= 2;
   const size_t smem1 = 1024 + 2 * kTSub + static_cast<size_t>(nb + (nb & 1)) * kTSub;
-  const size_t smem3 = 1024 + static_cast<size_t>(nb > 2 ? nb : 2) * kTSub + static_cast<size_t>(nb) * (kTQ + PB) * 128 + kTSub;
+  const size_t smem3 = tq_output_smem(nb, PB);
+  // Phase 3: as many units a block as keep the blocks within one an SM
+  const int group_units = (H / G) * (P / PB);
+  const int sms = 148;
+  const int per_block = min(group_units, static_cast<int>((static_cast<long long>(n_chunks) * G * group_units + sms - 1) / sms));
+  const int group_blocks = (group_units + per_block - 1) / per_block;
+  // Whole tiles of 64 columns come by TMA: a unit's copies took its 512 threads 2,800 clocks of issue, of about 7,500.
+  const bool tma = PB == 64 && N % 64 == 0 && n_tokens > 0;
+  CUtensorMap map_xbc{}, map_start{}, map_z{};
+  if (tma) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return PMM_ERR_BAD_ARGUMENT;
+    auto tiles_of = [&](CUtensorMap* map, const void* base, long long cols, long long rows, long long ld, unsigned box_rows) {
+      const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+      const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
+      const cuuint32_t box[2] = {64, box_rows}, elem[2] = {1, 1};
+      return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    const long long I = static_cast<long long>(H) * P;
+    if (!tiles_of(&map_xbc, xbc, I + 2LL * G * N, n_tokens, ld_xbc, kTQ) || !tiles_of(&map_start, start_state, N, n_chunks * I, N, 64) ||
+        (z_vec && !tiles_of(&map_z, z_raw, I, n_tokens, ld_z, kTQ)))
+      return PMM_ERR_BAD_ARGUMENT;
+  }
   static size_t set1 = 0, set3 = 0;  // the opt-in to large shared memory, raised when a larger shape comes
   if (smem1 > set1) {
     cudaError_t e = cudaFuncSetAttribute(ssd_tc_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem1));
@@ -715,7 +884,9 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
     set1 = smem1;
   }
   if (smem3 > set3) {
-    cudaError_t e = cudaFuncSetAttribute(ssd_tc_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem3));
+    cudaError_t e = cudaFuncSetAttribute(ssd_tc_output_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem3));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(ssd_tc_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem3));
     if (e != cudaSuccess) return static_cast<int>(e);
     set3 = smem3;
   }
@@ -727,8 +898,9 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
   int rc = launch_ssd_state_pass(chunk_state, chunk_decay, static_cast<bf16*>(start_state), state, cu, slots, n_seq, H,
                                  P * N, kTQ, skip_single, n_multi, stream);
   if (rc != 0) return rc;
-  launch_pdl(ssd_tc_output_kernel, dim3(n_chunks, H * (P / PB)), dim3(kTOut), smem3, stream, xb, ld_xbc,
+  launch_pdl(tma ? ssd_tc_output_kernel<true> : ssd_tc_output_kernel<false>, dim3(n_chunks, G * group_blocks), dim3(kTOutAll), smem3,
+             stream, map_xbc, map_start, map_z, xb, ld_xbc,
              static_cast<const float*>(chunk_dt), d_skip, cu, n_seq, static_cast<const bf16*>(start_state),
-             static_cast<bf16*>(y), H, P, N, G, PB, static_cast<const bf16*>(z_raw), ld_z, z_scale, z_bias, z_vec, skip_single, status);
+             static_cast<bf16*>(y), H, P, N, G, PB, per_block, static_cast<const bf16*>(z_raw), ld_z, z_scale, z_bias, z_vec, skip_single, status);
   return launch_status();
 }

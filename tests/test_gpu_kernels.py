@@ -274,6 +274,38 @@ def test_ssd_tcgen05_scan(H, Pd, N, G, gated):
     assert float(state[1].abs().sum()) == 0.0
 
 
+@pytest.mark.parametrize("H,Pd,N,G,lens", [(24, 64, 128, 1, [700, 129, 260]), (24, 128, 256, 1, [257, 400]), (24, 128, 64, 2, [640, 127]),
+                                           (40, 48, 80, 1, [513, 128]), (16, 64, 192, 1, [1300]), (2, 64, 128, 1, [2048, 100]),
+                                           (24, 64, 128, 1, [64] * 9)])
+def test_ssd_tcgen05_scan_keeps_to_its_rows(H, Pd, N, G, lens):
+    """Several heads and slabs a block, sequences that end on, before and behind a chunk, few and many of them: near the serial
+    kernel, states too, and the same bits beside a sequence of infinities and NaN whose rows follow in the same tiles."""
+    dtype = torch.bfloat16
+    g = torch.Generator().manual_seed(H + Pd + N)
+    I, conv_dim, n_all = H * Pd, H * Pd + 2 * G * N, sum(lens) + 70
+    xbc, z = (q(torch.randn(n_all, w, generator=g), dtype) for w in (conv_dim, I))
+    dt = q(torch.randn(n_all, H, generator=g), dtype)
+    a_log, d_skip, shift = (v.to(DEV) for v in (torch.rand(H, generator=g) * 2, torch.randn(H, generator=g), torch.randn(H, generator=g) - 3.0))
+    start = torch.randn(len(lens) + 2, H, Pd, N, generator=g)
+    new_lens = list(lens) + [70]
+    cu, slots = i32([0] + torch.tensor(new_lens).cumsum(0).tolist()), i32(list(range(len(new_lens))))
+    got, states = {}, {}
+    for other in (0.0, math.inf, math.nan):
+        x = xbc.clone()
+        x[sum(lens):] = x[sum(lens):] * other if other == 0.0 else other
+        state, out = start.clone().to(DEV), torch.empty(n_all, I, dtype=dtype, device=DEV)
+        scratch = torch.full((K().ssd_tc_scratch_floats(new_lens, H, Pd, N),), float("nan"), device=DEV)
+        K().ssm_scan_tc(x.to(DEV), dt.to(DEV), 1.0, shift, a_log, d_skip, state, cu, slots, new_lens, out, G, scratch, gate=(z.to(DEV), 1.0, None))
+        got[other], states[other] = out[:sum(lens)].cpu(), state[:len(lens)].cpu()
+    assert K().tc_gemm_status(DEV) == 0
+    want, ref = start.clone().to(DEV), torch.empty(n_all, I, dtype=dtype, device=DEV)
+    K().ssm_scan_seq(xbc.to(DEV), dt.to(DEV), 1.0, shift, a_log, d_skip, want, cu, slots, len(new_lens), ref, G, gate=(z.to(DEV), 1.0, None))
+    close(got[0.0], ref[:sum(lens)], dtype, what="outputs")
+    close(states[0.0], want[:len(lens)], dtype, what="states")
+    for other in (math.inf, math.nan):
+        assert torch.equal(got[other], got[0.0]) and torch.equal(states[other], states[0.0])
+
+
 def test_ssd_tcgen05_scan_refuses_other_sizes():
     assert not K().ssd_tc_supported(20, 24) and not K().ssd_tc_supported(64, 272) and not K().ssd_tc_supported(144, 64)
     assert K().ssd_tc_supported(112, 16)
