@@ -7,7 +7,7 @@
 // the chunk and S the state at the chunk's start:
 //   y_i   = sum_{j<=i} (C_i.B_j) exp(cs_i-cs_j) delta_j x_j  +  exp(cs_i) (C_i . S)  +  D x_i
 //   S_end = exp(cs_last) S  +  sum_j exp(cs_last-cs_j) delta_j x_j B_j^T
-// Three launches:
+// Three launches, or two (1 and 2 as one walk, ssd_tc_walk, where that is shorter):
 //   1. ssd_tc_state:   one block per (chunk, 128 channels of x): the local term of S_end as ONE
 //                      product  D[channel, n] = sum_j (w_j x_j[channel]) B_j[n].  Both operands are
 //                      the chunk's rows as they lie in memory (tokens = the K dimension, so both
@@ -389,6 +389,331 @@ __global__ void __launch_bounds__(kTState)
   tq_tmem_free(tmem_base, tmem_cols, warp);
 }
 
+// ----------------------------------------------------------------------------- phases 1 and 2 in one walk
+// grid (slabs of 128 channels * blocks of NB state columns, sequences): a block walks the chunks of one sequence with its part
+// of the state in registers.  Per chunk: the local term as in phase 1 (x scaled by w_j in shared memory, one product with K =
+// the tokens), the state before the chunk out as bfloat16, S <- exp(cs_last) S + local as in the state pass: the same sums
+// in the same order, without the local terms (float, written and read once) and the second launch between them.
+// 512 threads scale and fold: warps w, w + 4, w + 8, w + 12 share the tensor-memory lanes (= channels) 32 (w % 4) ... and split the
+// NB columns; warp 16 asks for the tiles (TMA), issues the products (two accumulators) and sends the start states off, so
+// that the product of a chunk runs while the chunk behind it is scaled.  The decays of up to 16 (chunk, head)s are made
+// at a time by all warps.
+constexpr int kTWalk = 512;
+constexpr int kTWalkAll = kTWalk + 32;
+constexpr int kTWalkDecays = 16;  // (chunk, head)s whose decays lie in shared memory
+__host__ __device__ constexpr int tq_walk_stages(int NB) { return NB == 64 ? 3 : 2; }
+__host__ __device__ constexpr int tq_walk_stage(int NB) { return 2 * kTSub + NB * 256; }  // x, then 128 rows of NB columns of B
+__host__ __device__ constexpr size_t tq_walk_smem(int NB) {  // ..., two tiles of start states [128 channels][NB], the decays
+  return 1024 + static_cast<size_t>(tq_walk_stages(NB)) * tq_walk_stage(NB) + 2 * NB * 256 + 2 * kTWalkDecays * kTQ * sizeof(float);
+}
+
+template <int NB>
+__global__ void __launch_bounds__(kTWalkAll, 1)
+    ssd_tc_walk_kernel(const __grid_constant__ CUtensorMap map_xbc, const __grid_constant__ CUtensorMap map_out,
+                       const bf16* __restrict__ xbc, int ld_xbc, const bf16* __restrict__ dt_raw, long long ld_dt, float dt_scale,
+                       const float* __restrict__ dt_shift, const float* __restrict__ a_log, const int* __restrict__ cu,
+                       const int* __restrict__ slots, float* __restrict__ state, float* __restrict__ chunk_dt,
+                       bf16* __restrict__ start_state, int H, int P, int N, int G, int slabs_per_group, int skip_single,
+                       int* __restrict__ status) {
+  constexpr int kCols = NB / 4;        // state columns a thread
+  constexpr int kBSub = NB / 64;       // sub-tiles of B, and of a tile of start states
+  constexpr int kStages = tq_walk_stages(NB);
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long bar_in[kStages], bar_scaled[2], bar_mma[2], bar_out[2];
+  __shared__ unsigned s_tmem;
+  __shared__ int s_abort, s_first[kTWalkAll / 32];
+  __shared__ float s_tot[kTWalkDecays][4];  // per (chunk, head): the sums of delta * A of four groups of 32 tokens
+  __shared__ float s_decay[kTWalkDecays];
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int seq = blockIdx.y;
+  // the sequence and its chunks (inputs of the step, read before the wait)
+  const int t_begin = cu[seq], n_tok = cu[seq + 1] - t_begin;
+  if (n_tok <= 0 || (skip_single && n_tok == 1)) return;
+  const int nc = (n_tok + kTQ - 1) / kTQ;
+  int mine = 0;
+  for (int q = tid; q < seq; q += kTWalkAll) mine += (cu[q + 1] - cu[q] + kTQ - 1) / kTQ;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if (lane == 0) s_first[warp] = mine;
+  const int col_blocks = N / NB;
+  const int slab_id = blockIdx.x / col_blocks, n0 = (blockIdx.x % col_blocks) * NB;
+  const int I = H * P, g = slab_id / slabs_per_group, slab = slab_id % slabs_per_group;
+  const int ch_per_group = (H / G) * P;
+  const int ch0 = g * ch_per_group + slab * kTQ;
+  const int n_ch = min(kTQ, ch_per_group - slab * kTQ);
+  const int head0 = ch0 / P;
+  const int n_heads = (ch0 + n_ch - 1) / P - head0 + 1;  // <= 8: a head has at least 16 channels
+  const int span = kTWalkDecays / n_heads;               // chunks whose decays are made at a time
+  unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  auto stage = [&](int k) { return tiles + (k % kStages) * tq_walk_stage(NB); };
+  unsigned char* sOut = tiles + kStages * tq_walk_stage(NB);
+  float* s_w = reinterpret_cast<float*>(sOut + 2 * NB * 256);  // [(chunk, head)][token]: exp(cs_last - cs_j) * delta_j
+  float* s_delta = s_w + kTWalkDecays * kTQ;
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < kStages; ++i) mbar_init(&bar_in[i], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar_scaled[i], kTWalk / 32);
+      mbar_init(&bar_mma[i], 1);
+      mbar_init(&bar_out[i], kTWalk / 32);
+    }
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  pdl_wait();
+  const unsigned tmem_base = tq_tmem_alloc(&s_tmem, 2 * NB, warp);  // includes a __syncthreads
+  volatile int* abort_flag = &s_abort;
+  auto wait_all = [&](unsigned long long* bar, unsigned parity) {  // the same answer in a warp
+    if (__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag))) return true;
+    if (lane == 0) {
+      if (!*abort_flag) atomicExch(status, 31);
+      s_abort = 1;
+    }
+    return false;
+  };
+  int first = 0;  // chunks of the sequences before this one
+  for (int w = 0; w < kTWalkAll / 32; ++w) first += s_first[w];
+  const bool whole = n_ch == kTQ;  // the slab's start states go out as one tile (else a thread writes its own)
+
+  if (warp == kTWalk / 32) {
+    // ---------------------------------------------------------------- tiles and products
+    auto request = [&](int k) {
+      unsigned char* dst = stage(k);
+      unsigned long long* bar = &bar_in[k % kStages];
+      const int t0 = t_begin + k * kTQ;
+      mbar_expect_tx(bar, tq_walk_stage(NB));
+      tma_load_2d(dst, &map_xbc, ch0, t0, bar);
+      tma_load_2d(dst + kTSub, &map_xbc, ch0 + 64, t0, bar);  // (columns behind the slab's channels: rows of the product nobody reads)
+#pragma unroll
+      for (int b = 0; b < kBSub; ++b) tma_load_2d(dst + (2 + b) * kTSub, &map_xbc, I + g * N + n0 + b * 64, t0, bar);
+    };
+    if (lane < min(kStages, nc)) request(lane);
+    __syncwarp();
+    auto send = [&](int k) {  // the states before chunk k
+      if (!wait_all(&bar_out[k & 1], (k >> 1) & 1)) return false;
+      if (lane == 0) {
+#pragma unroll
+        for (int b = 0; b < kBSub; ++b)
+          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n" ::"l"(
+                           reinterpret_cast<unsigned long long>(&map_out)),
+                       "r"(smem_u32(sOut + (k & 1) * (NB * 256) + b * kTSub)), "r"(n0 + b * 64), "r"((first + k) * I + ch0)
+                       : "memory");
+        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+      }
+      __syncwarp();
+      return true;
+    };
+    const unsigned lead = lane == 0 ? 1u : 0u;
+    constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (static_cast<unsigned>(NB >> 3) << 17) |
+                               (static_cast<unsigned>(kTQ >> 4) << 24);  // A and B both MN-major
+    bool ok = true;
+    for (int k = 0; k < nc && ok; ++k) {
+      if (!wait_all(&bar_scaled[k & 1], (k >> 1) & 1)) break;
+      // (the states before chunk k - 2 have left their tile: who waits for this product may write it)
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const unsigned long long a_desc = umma_desc_mn(stage(k), kTSub), b_desc = umma_desc_mn(stage(k) + 2 * kTSub, kTSub);
+#pragma unroll
+      for (int i = 0; i < kTQ / 16; ++i)  // 16 tokens further = 16 rows of 128 bytes in both operands
+        umma_f16_lead(tmem_base + (k & 1) * NB, a_desc + ((i * 16 * 128) >> 4), b_desc + ((i * 16 * 128) >> 4), idesc, i > 0 ? 1u : 0u, lead);
+      umma_commit_lead(&bar_mma[k & 1], lead);
+      // a stage takes its next chunk once its product has finished: of three stages the one of chunk k - 1, of two this one
+      const int done = kStages == 3 ? k - 1 : k;
+      if (done >= 0 && done + kStages < nc) {
+        ok = wait_all(&bar_mma[done & 1], (done >> 1) & 1);
+        if (ok && lane == 0) request(done + kStages);
+        __syncwarp();
+      }
+      if (k > 0 && whole) ok = ok && send(k - 1);
+    }
+    if (whole && ok) send(nc - 1);
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+  } else {
+    // ---------------------------------------------------------------- scaling and folding
+    const int rw = warp & 3, part = warp >> 2, row = rw * 32 + lane;
+    const unsigned lane_base = tmem_base + (static_cast<unsigned>(rw * 32) << 16);
+    const bool row_ok = row < n_ch;
+    const int my_head = row_ok ? (ch0 + row) / P - head0 : 0;
+    const int col = n0 + part * kCols;
+    float* sp = state + (static_cast<size_t>(slots[seq]) * I + ch0 + row) * N + col;
+    float S[kCols];
+#pragma unroll
+    for (int i = 0; i < kCols; i += 4) {
+      const float4 v = row_ok ? *reinterpret_cast<const float4*>(sp + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[i] = v.x, S[i + 1] = v.y, S[i + 2] = v.z, S[i + 3] = v.w;
+    }
+    auto sync_workers = [&]() { asm volatile("bar.sync 1, 512;\n" ::: "memory"); };
+    // delta, cs and w of chunks k0 .. k0 + span - 1, every head of the slab: a warp per 32 tokens of a (chunk, head), four at a time
+    auto make_decays = [&](int k0) {
+      const int tasks = min(span, nc - k0) * n_heads * 4;
+      sync_workers();  // (what lay there has been used)
+#pragma unroll 1
+      for (int base = warp; base < tasks; base += 4 * (kTWalk / 32)) {
+        float delta[4], incl[4], raw[4], shift[4], al[4];
+        bool in[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {  // (the loads of all four before anything waits for one)
+          const int task = min(base + u * (kTWalk / 32), tasks - 1), item = task >> 2, tok = (task & 3) * 32 + lane;
+          const int kk = item / n_heads, t = (k0 + kk) * kTQ + tok, h = head0 + (item - kk * n_heads);
+          in[u] = t < n_tok;
+          raw[u] = __bfloat162float(dt_raw[static_cast<long long>(t_begin + min(t, n_tok - 1)) * ld_dt + h]);
+          shift[u] = dt_shift[h];
+          al[u] = a_log[h];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          delta[u] = in[u] ? softplus_f(raw[u] * dt_scale + shift[u]) : 0.f;
+          incl[u] = delta[u] * -expf(al[u]);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float up = __shfl_up_sync(0xffffffffu, incl[u], o);
+            if (lane >= o) incl[u] += up;
+          }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int task = base + u * (kTWalk / 32), item = task >> 2, tok = (task & 3) * 32 + lane;
+          if (task < tasks) {
+            s_delta[item * kTQ + tok] = delta[u];
+            s_w[item * kTQ + tok] = incl[u];
+            if (lane == 31) s_tot[item][task & 3] = incl[u];
+          }
+        }
+      }
+      sync_workers();
+#pragma unroll 1
+      for (int base = warp; base < tasks; base += 4 * (kTWalk / 32))
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int task = base + u * (kTWalk / 32), item = task >> 2, tok = (task & 3) * 32 + lane;
+          if (task < tasks) {
+            const int kk = item / n_heads, k = k0 + kk, h = head0 + (item - kk * n_heads);
+            const float* tot = s_tot[item];
+            const float delta = s_delta[item * kTQ + tok];
+            float cs = s_w[item * kTQ + tok];
+            for (int w = 0; w < (task & 3); ++w) cs += tot[w];
+            const float last = (tot[0] + tot[1]) + (tot[2] + tot[3]);
+            s_w[item * kTQ + tok] = expf(last - cs) * delta;
+            if (tok == 0) s_decay[item] = expf(last);
+            if (n0 == 0 && h * P >= ch0) {  // the head begins in this slab
+              float* dtp = chunk_dt + (static_cast<size_t>(first + k) * H + h) * (2 * kTQ);
+              dtp[tok] = delta;
+              dtp[kTQ + tok] = cs * kLog2e;
+            }
+          }
+        }
+      sync_workers();
+    };
+    float decay = 0.f, lone_w = 0.f;  // of the chunk that is folded in next
+    auto fold = [&](int k) {  // chunk k: the state before it out, its local term in
+      const int c = first + k, len = min(kTQ, n_tok - k * kTQ);
+      unsigned char* out = sOut + (k & 1) * (NB * 256);
+      bf16* dst = start_state + (static_cast<size_t>(c) * I + ch0 + row) * N + col;
+      wait_all(&bar_mma[k & 1], (k >> 1) & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      unsigned v[16];
+      tmem_ld16(lane_base + (k & 1) * NB + part * kCols, v);
+#pragma unroll
+      for (int i = 0; i < kCols; i += 8) {
+        const uint4 p = make_uint4(tq_pack(S[i], S[i + 1]), tq_pack(S[i + 2], S[i + 3]), tq_pack(S[i + 4], S[i + 5]), tq_pack(S[i + 6], S[i + 7]));
+        const int ck = (part * kCols + i) >> 3;
+        if (whole)
+          *reinterpret_cast<uint4*>(out + (ck >> 3) * kTSub + tq_swz(row, ck & 7)) = p;
+        else if (row_ok)
+          *reinterpret_cast<uint4*>(dst + i) = p;
+      }
+      if (whole) {
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_out[k & 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < kCols; i += 16) {
+        if (i > 0) tmem_ld16(lane_base + (k & 1) * NB + part * kCols + i, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        if (len > 1) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) S[i + e] = fmaf(S[i + e], decay, __uint_as_float(v[e]));
+        }
+      }
+      if (len == 1) {  // one token: S_local[ch][n] = delta x[ch] B[n], not through bfloat16 operands
+        const bf16* rowp = xbc + static_cast<size_t>(t_begin + k * kTQ) * ld_xbc;
+        const float xv = row_ok ? __bfloat162float(rowp[ch0 + row]) * lone_w : 0.f;
+#pragma unroll
+        for (int i = 0; i < kCols; ++i) S[i] = fmaf(S[i], decay, __fmul_rn(xv, __bfloat162float(rowp[I + g * N + col + i])));
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    };
+    // this thread's pieces of x: 16 bytes (8 channels of one head) of every 32nd token
+    const int ck = tid & 15, j0 = tid >> 4;
+    const bool piece_ok = ck * 8 < n_ch;
+    const int piece_head = piece_ok ? (ch0 + ck * 8) / P - head0 : 0;
+    const int piece_off = (ck >> 3) * kTSub + tq_swz(j0, ck & 7);  // (32 tokens further: 4,096 bytes)
+    // (a wait that gave up does not leave the loop: the warps meet at named barriers, and the waits behind it end at once)
+    int at = span;  // the chunk's place among those whose decays lie there
+    for (int k = 0; k < nc; ++k) {
+      const int len = min(kTQ, n_tok - k * kTQ);
+      if (at == span) {
+        make_decays(k);
+        at = 0;
+      }
+      const float* w_row = s_w + (at * n_heads + piece_head) * kTQ + j0;
+      const float next_decay = s_decay[at * n_heads + my_head], next_w = s_w[(at * n_heads + my_head) * kTQ];
+      ++at;
+      wait_all(&bar_in[k % kStages], (k / kStages) & 1);
+      unsigned char* sA = stage(k);
+      if (piece_ok) {
+        uint4 in[4];
+        float w[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          in[r] = *reinterpret_cast<const uint4*>(sA + piece_off + r * 4096);
+          w[r] = w_row[32 * r];
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const unsigned rw4[4] = {in[r].x, in[r].y, in[r].z, in[r].w};
+          unsigned o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rw4[e]));
+            o[e] = j0 + 32 * r < len ? tq_pack(f.x * w[r], f.y * w[r]) : 0u;  // (rows beyond the chunk belong to others: zero, whatever they hold)
+          }
+          *reinterpret_cast<uint4*>(sA + piece_off + r * 4096) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+      }
+      if (len < kTQ)
+        for (int i = tid; i < (kTQ - len) * kBSub * 8; i += kTWalk) {
+          const int j = len + i / (kBSub * 8), cb = i % (kBSub * 8);
+          *reinterpret_cast<uint4*>(sA + (2 + (cb >> 3)) * kTSub + tq_swz(j, cb & 7)) = make_uint4(0u, 0u, 0u, 0u);
+        }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_scaled[k & 1]);
+      // The launch behind this one is let go with the last chunk: behind the wait, so that it may read what came before this
+      // one, and late, so that its blocks do not hold the SMs that other streams' launches could use.
+      if (k == nc - 1) pdl_launch_dependents();
+      if (k > 0) fold(k - 1);
+      decay = next_decay, lone_w = next_w;
+    }
+    fold(nc - 1);
+    if (row_ok && !*abort_flag) {
+#pragma unroll
+      for (int i = 0; i < kCols; i += 4) *reinterpret_cast<float4*>(sp + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+    }
+  }
+  if (s_abort && tid == kTWalk) {
+    // copies that were asked for still write into this block's shared memory: a bounded time for them to land
+    for (unsigned i = 0; i < kSpinLimit / 4; ++i) __nanosleep(32);
+  }
+  tq_tmem_free(tmem_base, 2 * NB, warp);
+}
+
 // ----------------------------------------------------------------------------- phase 3
 // grid (chunks, groups * blocks a group); a block takes `per_block` units of one chunk and one group, a unit being a head's
 // slab of PB channels.  C and B of the chunk are brought once and G = C B^T is made once; then unit by unit the start state's
@@ -396,8 +721,8 @@ __global__ void __launch_bounds__(kTState)
 // head (slabs of one head share it), Y1 = M x issued, and the rows y go out.  512 threads: threads t, t + 128, t + 256 and
 // t + 384 share token t of the chunk (= tensor-memory lane t) and split its columns; warp 16 issues the products.  Tensor
 // memory: G columns 0..127, Y2 columns 128..128+PB, Y1 columns 192..192+PB.
-// Everything but the start states was finished before the state pass was let go (it lets this launch go behind its own
-// wait), so C, B, x, the decays and G are there before this launch's wait.
+// C, B, x and the gate's input were finished before the launch before this one (which lets this one go behind its own wait):
+// they are brought and G is made before this launch's wait.
 // What bounds it: a unit is a chain of two products, an exponential per entry of M's lower half and two per output, about
 // 2,400 clocks.  One block a unit (two blocks an SM, C and B brought and G made for every head) took 19.5 us at 24 heads of
 // 64 x 128 and 2,048 tokens and 56 us at 48 heads of 128 x 256 and 1,024 tokens.
@@ -572,17 +897,17 @@ __global__ void __launch_bounds__(kTOutAll, 1)
   const unsigned dt_bytes = 2 * kTQ * sizeof(float);
   auto tma_x = [&](int k) {
     unsigned long long* bar = &bar_x[k & 1];
-    mbar_expect_tx(bar, kTSub + dt_bytes);
+    mbar_expect_tx(bar, kTSub);
     tma_load_2d(sX + (k & 1) * kTSub, &map_xbc, static_cast<int>(col_of(k)), t0, bar);
+  };
+  auto tma_s = [&](int k) {  // the start state's rows and the decays
+    unsigned long long* bar = &bar_s[k & 1];
+    unsigned char* dst = (k & 1) ? sS1 : sS0;
+    mbar_expect_tx(bar, tq_state_bytes(nb, 64) + dt_bytes);
+    for (int b = 0; b < nb; ++b) tma_load_2d(dst + b * s_sub, &map_start, b * 64, c * I + static_cast<int>(col_of(k)), bar);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(s_dt[k & 1])),
                  "l"(chunk_dt + (static_cast<size_t>(c) * H + head_of(k)) * (2 * kTQ)), "r"(dt_bytes), "r"(smem_u32(bar))
                  : "memory");
-  };
-  auto tma_s = [&](int k) {
-    unsigned long long* bar = &bar_s[k & 1];
-    unsigned char* dst = (k & 1) ? sS1 : sS0;
-    mbar_expect_tx(bar, tq_state_bytes(nb, 64));
-    for (int b = 0; b < nb; ++b) tma_load_2d(dst + b * s_sub, &map_start, b * 64, c * I + static_cast<int>(col_of(k)), bar);
   };
   auto tma_z = [&](int k) {
     mbar_expect_tx(&bar_z, kTSub);
@@ -658,7 +983,7 @@ __global__ void __launch_bounds__(kTOutAll, 1)
             *reinterpret_cast<uint4*>(sX + st * kTSub + tq_swz(len + (i >> 3), i & 7)) = make_uint4(0u, 0u, 0u, 0u);
         fence_proxy_async();
       }
-      if (warp == kTOut / 32) wait_all(&bar_s[st], (k >> 1) & 1, 33);
+      wait_all(&bar_s[st], (k >> 1) & 1, 33);
     } else if (worker) {
       if (z_raw && z_vec)
         tq_pieces(tid, kTQ, PB / 8, [&](int j, int ck) {
@@ -827,6 +1152,7 @@ PMM_EXPORT int pmm_ssd_tc_supported(int P, int N) {
 // n_chunks*H*256 floats, start_state n_chunks*H*P*N bfloat16 (16-byte aligned); n_chunks = sum over
 // sequences of ceil(new tokens / 128).
 // z_raw (or nullptr): the gate's input [T, ld_z], y <- y * silu(z_raw * z_scale + z_bias).
+// n_tokens: rows of xbc (and z_raw); longest: about the tokens of the longest sequence (a choice of form hangs on it, not a result).
 // skip_single: sequences that bring exactly one token are left alone (state and y): in a mixed step
 // the token-serial kernel takes them (pmm_ssm_scan_seq with one_token = 2); n_multi is then the
 // number of sequences that bring more than one token (0: not known).
@@ -834,7 +1160,7 @@ PMM_EXPORT int pmm_ssd_tc_supported(int P, int N) {
 PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long long ld_dt, float dt_scale,
                           const float* dt_shift, const float* a_log, const float* d_skip, float* state, const int* cu,
                           const int* slots, void* y, float* chunk_state, float* chunk_decay, float* chunk_dt,
-                          void* start_state, int n_seq, int n_tokens, int n_chunks, int H, int P, int N, int G, const void* z_raw,
+                          void* start_state, int n_seq, int n_tokens, int longest, int n_chunks, int H, int P, int N, int G, const void* z_raw,
                           long long ld_z, float z_scale, const float* z_bias, int skip_single, int n_multi, int* status,
                           cudaStream_t stream) {
   using namespace pmm;
@@ -854,15 +1180,24 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
   while (tmem_cols < N) tmem_cols *= 2;
   const size_t smem1 = 1024 + 2 * kTSub + static_cast<size_t>(nb + (nb & 1)) * kTSub;
   const size_t smem3 = tq_output_smem(nb, PB);
+  const int sms = 148;
   // Phase 3: as many units a block as keep the blocks within one an SM
   const int group_units = (H / G) * (P / PB);
-  const int sms = 148;
   const int per_block = min(group_units, static_cast<int>((static_cast<long long>(n_chunks) * G * group_units + sms - 1) / sms));
   const int group_blocks = (group_units + per_block - 1) / per_block;
   // Whole tiles of 64 columns come by TMA: a unit's copies took its 512 threads 2,800 clocks of issue, of about 7,500.
-  const bool tma = PB == 64 && N % 64 == 0 && n_tokens > 0;
-  CUtensorMap map_xbc{}, map_start{}, map_z{};
-  if (tma) {
+  const bool tiles64 = N % 64 == 0 && n_tokens > 0, tma = PB == 64 && tiles64;
+  // Phases 1 and 2 in one walk where its blocks all run at once and it is the shorter one: a walk takes a chunk after the other,
+  // the two launches write and read the local terms.  Measured, us: 24 heads of 64 x 128, walk / both: one chunk 9.0 / 10.3 and a launch's
+  // latency, 5 sequences of up to 3 chunks 12.4 / 18.8, one sequence of 4 chunks 13.2 / 11.3 (the whole chain 21.0 / 20.7), of 16 chunks 33 /
+  // 20; 48 heads of 128 x 256, 8 chunks 29 / 53.
+  const int walkers = (n_multi > 0 && skip_single ? n_multi : n_seq) * G * slabs_per_group;
+  const int NB = walkers * (N / 64) <= sms ? 64 : N % 128 == 0 && walkers * (N / 128) <= sms ? 128 : 0;
+  const double walk_us = NB == 64 ? 7.6 + 1.45 * ((longest + kTQ - 1) / kTQ) : 9.0 + 2.5 * ((longest + kTQ - 1) / kTQ);
+  const double both_us = 11.0 + 0.88e-6 * 4.0 * n_chunks * H * P * N;
+  const bool walk = tiles64 && NB > 0 && walk_us < both_us;
+  CUtensorMap map_xbc{}, map_start{}, map_z{}, map_out{};
+  if (tma || walk) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return PMM_ERR_BAD_ARGUMENT;
     auto tiles_of = [&](CUtensorMap* map, const void* base, long long cols, long long rows, long long ld, unsigned box_rows) {
@@ -873,10 +1208,12 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
     const long long I = static_cast<long long>(H) * P;
-    if (!tiles_of(&map_xbc, xbc, I + 2LL * G * N, n_tokens, ld_xbc, kTQ) || !tiles_of(&map_start, start_state, N, n_chunks * I, N, 64) ||
-        (z_vec && !tiles_of(&map_z, z_raw, I, n_tokens, ld_z, kTQ)))
+    if (!tiles_of(&map_xbc, xbc, I + 2LL * G * N, n_tokens, ld_xbc, kTQ) || (tma && !tiles_of(&map_start, start_state, N, n_chunks * I, N, 64)) ||
+        (walk && !tiles_of(&map_out, start_state, N, n_chunks * I, N, kTQ)) ||
+        (tma && z_vec && !tiles_of(&map_z, z_raw, I, n_tokens, ld_z, kTQ)))
       return PMM_ERR_BAD_ARGUMENT;
   }
+  if (longest < 0) return PMM_ERR_BAD_ARGUMENT;
   static size_t set1 = 0, set3 = 0;  // the opt-in to large shared memory, raised when a larger shape comes
   if (smem1 > set1) {
     cudaError_t e = cudaFuncSetAttribute(ssd_tc_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem1));
@@ -892,12 +1229,21 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
   }
   const bf16* xb = static_cast<const bf16*>(xbc);
   const bf16* dtb = static_cast<const bf16*>(dt_raw);
+  if (walk) {
+    auto kern = NB == 64 ? ssd_tc_walk_kernel<64> : ssd_tc_walk_kernel<128>;
+    const size_t smem2 = tq_walk_smem(NB);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem2));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    launch_pdl(kern, dim3(G * slabs_per_group * (N / NB), n_seq), dim3(kTWalkAll), smem2, stream, map_xbc, map_out, xb, ld_xbc, dtb, ld_dt, dt_scale,
+               dt_shift, a_log, cu, slots, state, chunk_dt, static_cast<bf16*>(start_state), H, P, N, G, slabs_per_group, skip_single, status);
+  } else {
   launch_pdl(ssd_tc_state_kernel, dim3(n_chunks, G * slabs_per_group), dim3(kTState), smem1, stream, xb, ld_xbc, dtb, ld_dt,
              dt_scale, dt_shift, a_log, cu, n_seq, chunk_state, chunk_decay, chunk_dt, H, P, N, G, slabs_per_group, tmem_cols,
              skip_single, status);
   int rc = launch_ssd_state_pass(chunk_state, chunk_decay, static_cast<bf16*>(start_state), state, cu, slots, n_seq, H,
                                  P * N, kTQ, skip_single, n_multi, stream);
   if (rc != 0) return rc;
+  }
   launch_pdl(tma ? ssd_tc_output_kernel<true> : ssd_tc_output_kernel<false>, dim3(n_chunks, G * group_blocks), dim3(kTOutAll), smem3,
              stream, map_xbc, map_start, map_z, xb, ld_xbc,
              static_cast<const float*>(chunk_dt), d_skip, cu, n_seq, static_cast<const bf16*>(start_state),

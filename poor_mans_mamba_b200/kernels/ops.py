@@ -61,7 +61,7 @@ _SIGNATURES = {
                         c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_float, c_void_p, c_void_p],
     "pmm_ssd_tc_supported": [c_int, c_int],
     "pmm_ssd_tc": [c_void_p, c_int, c_void_p, c_longlong, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                   c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                   c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                    c_longlong, c_float, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "pmm_gated_norm": [c_void_p, c_void_p, c_longlong, c_float, c_void_p, c_void_p, c_float, c_int,
                        c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -915,9 +915,12 @@ def ssm_scan_tc(xbc: Tensor, dt_raw: Tensor, dt_scale: float, dt_shift: Tensor, 
     n_multi = getattr(new_lens, "multi", None)  # lengths given as bounds carry the bound with them
     if n_multi is None:
         n_multi = sum(1 for n in new_lens if n > 1)
+        longest = max(new_lens, default=0)
+    else:  # half as long again as the lengths' mean
+        longest = -(-3 * sum(new_lens) // (2 * max(n_multi, 1)))
     _call("pmm_ssd_tc", xbc.data_ptr(), ld_x, dt_raw.data_ptr(), ld_dt, float(dt_scale), dt_shift.data_ptr(),
           a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), cu.data_ptr(), slots.data_ptr(), out.data_ptr(),
-          chunk_state, chunk_decay, chunk_dt, start_state, len(new_lens), xbc.shape[0], n_chunks, H, P, N, n_groups, zp, ld_z, zs, zb,
+          chunk_state, chunk_decay, chunk_dt, start_state, len(new_lens), xbc.shape[0], longest, n_chunks, H, P, N, n_groups, zp, ld_z, zs, zb,
           int(bool(skip_single)), n_multi if skip_single else 0,
           _tc_status(xbc.device).data_ptr(), _stream())
 

@@ -276,7 +276,7 @@ def test_ssd_tcgen05_scan(H, Pd, N, G, gated):
 
 @pytest.mark.parametrize("H,Pd,N,G,lens", [(24, 64, 128, 1, [700, 129, 260]), (24, 128, 256, 1, [257, 400]), (24, 128, 64, 2, [640, 127]),
                                            (40, 48, 80, 1, [513, 128]), (16, 64, 192, 1, [1300]), (2, 64, 128, 1, [2048, 100]),
-                                           (24, 64, 128, 1, [64] * 9)])
+                                           (24, 64, 128, 1, [64] * 9), (5, 48, 64, 1, [300, 40]), (16, 16, 64, 2, [129, 1, 127])])
 def test_ssd_tcgen05_scan_keeps_to_its_rows(H, Pd, N, G, lens):
     """Several heads and slabs a block, sequences that end on, before and behind a chunk, few and many of them: near the serial
     kernel, states too, and the same bits beside a sequence of infinities and NaN whose rows follow in the same tiles."""
