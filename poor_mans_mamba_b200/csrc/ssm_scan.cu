@@ -143,12 +143,14 @@ __global__ void __launch_bounds__(kScanRows* kScanTpr)
     t0 = cu[s];
     t1 = cu[s + 1];
   }
+  float* srow = state + ((static_cast<size_t>(slot) * H + h) * P + (row_ok ? p : 0)) * N;
+  // the state's row is asked for into L2 while the launch before this one runs (a hint: the row is read behind the wait)
+  if (row_ok && lane_n * 32 < N && t1 > t0) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(srow + lane_n * 32));
   pdl_wait();
   if (t1 <= t0) return;
   if (one_token == 2 && t1 - t0 != 1) return;  // only the lone tokens of a mixed step
 
   float4 st[NV];
-  float* srow = state + ((static_cast<size_t>(slot) * H + h) * P + (row_ok ? p : 0)) * N;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int q = lane_n + i * kScanTpr;

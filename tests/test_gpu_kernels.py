@@ -311,6 +311,25 @@ def test_ssd_tcgen05_scan_refuses_other_sizes():
     assert K().ssd_tc_supported(112, 16)
 
 
+@pytest.mark.parametrize("C", [4, 252, 260, 1792])
+@pytest.mark.parametrize("taps,biased,act", [(2, False, True), (3, True, False), (4, True, True)])
+def test_conv1d_decode_four_channels_a_thread(C, taps, biased, act):
+    """The same bits, windows too, whether the rows start on 8-byte boundaries (four channels a thread) or not (one)."""
+    bf, g, n = torch.bfloat16, torch.Generator().manual_seed(C + taps), 5
+    rand = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    pre, w, pre_b, b = rand(C), rand(C, taps), rand(C) if biased else None, rand(C) if biased else None
+    slots, window, vals = i32([3, 0, 6, 2, 5]), rand(7, taps - 1, C), rand(n, C).to(bf)
+    got = []
+    for shift in (0, 1):
+        x, win, out = torch.zeros(n, C + 4, dtype=bf, device=DEV), window.clone(), torch.empty(n, C, dtype=bf, device=DEV)
+        x[:, shift:shift + C] = vals
+        for _ in range(2):
+            K().conv1d_decode(x[:, shift:shift + C], pre, pre_b, w, b, win, slots, out, activation=act)
+        got.append((out, win))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert torch.equal(got[0][1][[1, 4]], window[[1, 4]])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("mode", ["gate", "gate_then_norm", "norm_then_gate"])
 def test_gated_norm(dtype, mode):
