@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(at_threads(M), DH == 64 ? 2 : 1)
   }
   const size_t q_base = static_cast<size_t>(tok0) * Hq * DH;
   pdl_wait();
+  pdl_written(q);
   uint4 q_piece[DH / 16];
   if (warp > 1) {
 #pragma unroll

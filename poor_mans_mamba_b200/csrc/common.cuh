@@ -133,6 +133,18 @@ inline int launch_status() { return static_cast<int>(cudaGetLastError()); }
 // pdl_launch_dependents() lets the next kernel of the stream start its own preamble early.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// In a kernel with code before its wait: what is read through a `const T* __restrict__` parameter counts as never written, so
+// the compiler may move such a load above pdl_wait().  Called behind the wait for every such parameter that earlier
+// launches write, this makes the pointer a value that is only known there.
+template <typename T>
+__device__ __forceinline__ void pdl_written(T* __restrict__& p) {
+  asm volatile("" : "+l"(p)::"memory");
+}
+template <typename T, typename... More>
+__device__ __forceinline__ void pdl_written(T* __restrict__& p, More&... more) {
+  pdl_written(p);
+  pdl_written(more...);
+}
 
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(64)
   const float4 ps = ldf4(pre_scale + c), pb = pre_bias ? ldf4(pre_bias + c) : zero, cb = bias ? ldf4(bias + c) : zero;
   float* win = window + static_cast<size_t>(slots[s]) * L * C + c;
   pdl_wait();
+  pdl_written(x);
   const float4 raw = ldf4(x + static_cast<long long>(s) * ldx + c);
   float4 hist[L];
 #pragma unroll

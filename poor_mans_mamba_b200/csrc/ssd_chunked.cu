@@ -313,6 +313,7 @@ __global__ void ssd_state_pass_kernel(const float* __restrict__ chunk_state, con
   for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) first += s_first[w];
   pdl_wait();
   pdl_launch_dependents();
+  pdl_written(chunk_state, chunk_decay);
   if (e >= PN) return;
   // a block takes several sequences in turn when a step holds many (mostly short) ones
   for (int seq = seq0; seq < min(n_seq, seq0 + seqs_per_block); ++seq) {
@@ -378,6 +379,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   pdl_wait();
   pdl_launch_dependents();  // (behind the wait, as in the kernel above)
+  pdl_written(chunk_state, chunk_decay);
   const int e = (blockIdx.x * blockDim.x + tid) * 4;
   if (s_seq < 0 || e >= PN) return;
   ssd_pass_sequence(chunk_state, chunk_decay, start_state, state, slots[s_seq], H, PN, blockIdx.y, e, s_first, s_nc);

@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(kTState)
   if (!tq_locate(cu, n_seq, c, t0, len, seq_tokens, s_loc)) return;
   if (skip_single && seq_tokens == 1) return;  // lone tokens of a mixed step are the token-serial kernel's
   pdl_wait();  // (the sequences' bounds are inputs of the step)
+  pdl_written(xbc, dt_raw);
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = tiles;                 // [128 tokens][128 channels]: two atoms of 64 channels
   unsigned char* sB = tiles + 2 * kTSub;     // [128 tokens][N]: one atom per 64 state columns
@@ -463,6 +464,7 @@ __global__ void __launch_bounds__(kTWalkAll, 1)
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   pdl_wait();
+  pdl_written(xbc, dt_raw);
   const unsigned tmem_base = tq_tmem_alloc(&s_tmem, 2 * NB, warp);  // includes a __syncthreads
   volatile int* abort_flag = &s_abort;
   auto wait_all = [&](unsigned long long* bar, unsigned parity) {  // the same answer in a warp
@@ -842,6 +844,7 @@ __global__ void __launch_bounds__(kTOutAll, 1)
 
   if (len == 1) {
     pdl_wait();
+    pdl_written(chunk_dt, start_state);
     if (worker)
       for (int k = 0; k < n_units; ++k) {
         const int h = head_of(k);
@@ -961,6 +964,7 @@ __global__ void __launch_bounds__(kTOutAll, 1)
     umma_commit_lead(&bar_g, lead);
   }
   pdl_wait();  // the start states come from the launch before this one
+  pdl_written(chunk_dt, start_state);
   if (kTma) {
     if (tid == kTOut) tma_s(0);
   } else if (worker) {

@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(kScanRows* kScanTpr)
   // the state's row is asked for into L2 while the launch before this one runs (a hint: the row is read behind the wait)
   if (row_ok && lane_n * 32 < N && t1 > t0) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(srow + lane_n * 32));
   pdl_wait();
+  pdl_written(xbc, dt_raw, z_raw);
   if (t1 <= t0) return;
   if (one_token == 2 && t1 - t0 != 1) return;  // only the lone tokens of a mixed step
 
