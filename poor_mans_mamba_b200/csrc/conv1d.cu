@@ -87,7 +87,8 @@ __global__ void conv1d_window_update_kernel(const S* __restrict__ x, long long l
 // and a strip of tokens.  All rows of the strip (and the K-1 before it) and the tokens' places
 // in their sequences are requested before anything is computed, so the strip costs two memory
 // round trips (short strips: the kernel needs many threads to hide its arithmetic); the K-1 previous inputs then slide through registers.  At the first token of a
-// sequence the history comes from the request's window.
+// sequence the history comes from the request's window.  (Strips of 8 read constants and history half as often, but at 168
+// registers fewer threads run: 2,048 x 1,792 8.2 instead of 7.0 us.)
 constexpr int kConvStrip = 4;
 
 template <int K>
@@ -98,21 +99,13 @@ __global__ void __launch_bounds__(128)
                           const int* __restrict__ seq_of, const int* __restrict__ cu,
                           const int* __restrict__ slots, __nv_bfloat16* __restrict__ y, int T, int C, int act) {
   pdl_launch_dependents();
-  pdl_wait();
   constexpr int L = K - 1;
   constexpr int R = kConvStrip + L;
   const int c0 = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   const int t_begin = blockIdx.x * kConvStrip;
   if (c0 >= C || t_begin >= T) return;
   const int n_tok = min(T - t_begin, kConvStrip);
-
-  uint4 raw[R];  // rows t_begin - L .. t_begin + strip - 1
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int t = t_begin - L + i;
-    raw[i] = (t >= 0 && t < T) ? *reinterpret_cast<const uint4*>(x + static_cast<long long>(t) * ldx + c0)
-                               : make_uint4(0u, 0u, 0u, 0u);
-  }
+  // (constants, and the tokens' places in their sequences, which are inputs of the step, are read before the wait)
   int seq[kConvStrip], j[kConvStrip];
 #pragma unroll
   for (int i = 0; i < kConvStrip; ++i) seq[i] = i < n_tok ? seq_of[t_begin + i] : 0;
@@ -136,6 +129,15 @@ __global__ void __launch_bounds__(128)
     load8(w_t + static_cast<size_t>(k) * C, col);
 #pragma unroll
     for (int i = 0; i < 8; ++i) wk[i][k] = col[i];
+  }
+  pdl_wait();
+  pdl_written(x);
+  uint4 raw[R];  // rows t_begin - L .. t_begin + strip - 1
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int t = t_begin - L + i;
+    raw[i] = (t >= 0 && t < T) ? *reinterpret_cast<const uint4*>(x + static_cast<long long>(t) * ldx + c0)
+                               : make_uint4(0u, 0u, 0u, 0u);
   }
   auto unpack = [&](const uint4& r, float* v) {
     const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&r);
@@ -283,9 +285,8 @@ PMM_EXPORT int pmm_conv1d_fwd(const void* x, long long ldx, const float* pre_sca
     dim3 vgrid((T + pmm::kConvStrip - 1) / pmm::kConvStrip, (C / 8 + 127) / 128);
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     __nv_bfloat16* yb = static_cast<__nv_bfloat16*>(y);
-    if (K == 2) pmm::launch_pdl(pmm::conv1d_fwd_vec_kernel<2>, vgrid, dim3(128), 0, stream, xb, ldx, pre_scale, pre_bias, w_t, bias, window, seq_of, cu, slots, yb, T, C, act);
-    if (K == 3) pmm::launch_pdl(pmm::conv1d_fwd_vec_kernel<3>, vgrid, dim3(128), 0, stream, xb, ldx, pre_scale, pre_bias, w_t, bias, window, seq_of, cu, slots, yb, T, C, act);
-    if (K == 4) pmm::launch_pdl(pmm::conv1d_fwd_vec_kernel<4>, vgrid, dim3(128), 0, stream, xb, ldx, pre_scale, pre_bias, w_t, bias, window, seq_of, cu, slots, yb, T, C, act);
+    auto kern = K == 2 ? pmm::conv1d_fwd_vec_kernel<2> : K == 3 ? pmm::conv1d_fwd_vec_kernel<3> : pmm::conv1d_fwd_vec_kernel<4>;
+    pmm::launch_pdl(kern, vgrid, dim3(128), 0, stream, xb, ldx, pre_scale, pre_bias, w_t, bias, window, seq_of, cu, slots, yb, T, C, act);
     return pmm::launch_status();
   }
   dim3 grid(T, (C + 127) / 128);
