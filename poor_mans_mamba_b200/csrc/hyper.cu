@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(256)
                        const float* __restrict__ mix, const float* __restrict__ out_w,
                        const float* __restrict__ in_w, const float* __restrict__ norm_w, float eps,
                        S* __restrict__ normed, const int* __restrict__ rows, int D) {
-  extern __shared__ float u_row[];
+  extern __shared__ __align__(16) float u_row[];
   __shared__ float red[32];
   __shared__ float s_mix[kMaxLanes * kMaxLanes], s_out[kMaxLanes], s_in[kMaxLanes];
   pdl_launch_dependents();
@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(256)
     s_in[threadIdx.x] = in_w ? in_w[threadIdx.x] : 0.f;
   }
   pdl_wait();
+  pdl_written(y);
   __syncthreads();
   const int r = blockIdx.x;
   const int t = rows ? rows[r] : r;
@@ -78,8 +79,8 @@ __global__ void __launch_bounds__(256)
         }
       }
       if (y) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) yv[e] = ldf(y + static_cast<size_t>(t) * D + d + e);
+        const float4 v = ldf4(y + static_cast<size_t>(t) * D + d);
+        yv[0] = v.x, yv[1] = v.y, yv[2] = v.z, yv[3] = v.w;
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) element(d + e, xo[e], yv[e], xn[e]);
@@ -108,6 +109,13 @@ __global__ void __launch_bounds__(256)
   if (!normed) return;
   const float total = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(total / static_cast<float>(D) + eps);
+  if (VEC) {  // (a thread's own four values of the row)
+    for (int d = threadIdx.x * 4; d < D; d += blockDim.x * 4) {
+      const float4 u = *reinterpret_cast<const float4*>(u_row + d), w = ldf4(norm_w + d);
+      stf4(normed + static_cast<size_t>(r) * D + d, make_float4(u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w));
+    }
+    return;
+  }
   for (int d = threadIdx.x; d < D; d += blockDim.x)
     stf(normed + static_cast<size_t>(r) * D + d, u_row[d] * inv * norm_w[d]);
 }
@@ -227,7 +235,9 @@ PMM_EXPORT int pmm_hc_mix_norm(const float* x_in, long long in_lane_stride, floa
   if (smem > 200 * 1024) return PMM_ERR_BAD_ARGUMENT;
   // 16-byte accesses where every row of every lane starts on such a boundary
   const bool vec = D % 4 == 0 && reinterpret_cast<uintptr_t>(x_in) % 16 == 0 && in_lane_stride % 4 == 0 &&
-                   (!x_out || (reinterpret_cast<uintptr_t>(x_out) % 16 == 0 && out_lane_stride % 4 == 0));
+                   (!x_out || (reinterpret_cast<uintptr_t>(x_out) % 16 == 0 && out_lane_stride % 4 == 0)) &&
+                   reinterpret_cast<uintptr_t>(y) % 16 == 0 && reinterpret_cast<uintptr_t>(norm_w) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(normed) % 16 == 0;
   PMM_DISPATCH_DTYPE(dtype, S, PMM_DISPATCH_DTYPE(y_dtype, Y, {
     auto kern = vec ? (n_lanes <= 2 ? pmm::hc_mix_norm_kernel<S, Y, true, 2>
                                     : n_lanes <= 4 ? pmm::hc_mix_norm_kernel<S, Y, true, 4> : pmm::hc_mix_norm_kernel<S, Y, true, 8>)

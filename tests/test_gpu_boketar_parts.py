@@ -58,6 +58,24 @@ def test_lanes_mix_and_norm(dtype, n, D):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("D", [4, 1020, 1024, 2052])
+def test_lanes_rows_on_and_off_their_boundaries(dtype, D):
+    """Four values at a time where a row of the sublayer's result starts on a 16-byte boundary, one where it does not."""
+    n, T = 2, 9
+    x, y = rnd(n, T, D, seed=1), rnd(T, D, seed=2).to(dtype)
+    mix, ow, iw, nw = rnd(n, n, seed=3), rnd(n, seed=4), rnd(n, seed=5), rnd(D, seed=6) + 1.0
+    new = torch.einsum("st,sij->tij", mix.double(), x.double()) + ow.double().view(n, 1, 1) * y.double()
+    want = P.norm_plain(torch.einsum("s,sij->ij", iw.double(), new), nw.double(), 1e-5)
+    for shift in (0, 1):
+        flat = torch.zeros(T * D + 1, dtype=dtype, device=DEV)
+        flat[shift:shift + T * D] = y.reshape(-1).to(DEV)
+        lanes, out = x.to(DEV).clone(), torch.empty(T, D, dtype=dtype, device=DEV)
+        K.hc_mix_norm(lanes, lanes, flat[shift:shift + T * D].view(T, D), mix.reshape(-1).to(DEV), ow.to(DEV), iw.to(DEV), nw.to(DEV), 1e-5, out)
+        close(lanes, new, torch.float32, "lanes")
+        close(out, want, dtype, "normed")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_normed_sum_of_branches(dtype):
     T, D = 5, 72
     a, b, wa, wb = rnd(T, D, seed=1, scale=3.0), rnd(T, D, seed=2, scale=0.1), rnd(D, seed=3), rnd(D, seed=4)
