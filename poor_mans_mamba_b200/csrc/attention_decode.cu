@@ -84,13 +84,12 @@ __device__ __forceinline__ unsigned cluster_addr(unsigned smem_addr, unsigned ra
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster_f32(unsigned addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(addr), "f"(v) : "memory");
-}
-// Arrival on a barrier of another block of the cluster; this thread's earlier writes into that
-// block's shared memory are visible to whoever has waited for the barrier.
-__device__ __forceinline__ void mbar_arrive_remote(unsigned cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_bar) : "memory");
+// Two floats into another block's shared memory, counted (8 bytes) on a barrier of that block: whoever has waited for all its
+// bytes sees them.  (Plain stores and an arrival that released them took 3,700 clocks from the last part to the wait's end.)
+__device__ __forceinline__ void st_async_f32x2(unsigned addr, float x, float y, unsigned cluster_bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(addr),
+               "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(cluster_bar)
+               : "memory");
 }
 // Bounded wait on a barrier of this block on which other blocks of the cluster arrive.
 __device__ __forceinline__ bool mbar_wait_cluster(unsigned long long* bar, unsigned parity, volatile int* abort_flag) {
@@ -127,7 +126,7 @@ __global__ void __launch_bounds__(kDaThreads)
   __shared__ __align__(8) unsigned long long bar_full[NSTAGE], bar_empty[NSTAGE], bar_parts;
   __shared__ int s_bt[kDaBtCap];
   __shared__ __align__(16) bf16 s_new_k[DH], s_new_v[DH];
-  __shared__ float s_wm[4][16], s_wl[4][16], s_M[16], s_L[16];
+  __shared__ float s_wm[4][16], s_wl[4][16], s_M[16], s_L[16], s_pw[16][kDaClusterMax];
   __shared__ int s_abort, s_last;
 
   // Positions and block tables are inputs of the step, written before its first kernel: they are
@@ -157,9 +156,10 @@ __global__ void __launch_bounds__(kDaThreads)
       mbar_init(&bar_full[s], 1);
       mbar_init(&bar_empty[s], 4);
     }
-    mbar_init(&bar_parts, 128 * (a.n_splits > 1 ? a.n_splits - 1 : 1));
+    mbar_init(&bar_parts, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    if (a.clustered && z == 0) mbar_expect_tx(&bar_parts, static_cast<unsigned>(da_parts_bytes(DH, G, a.n_splits)));  // the others' parts
   }
   __syncthreads();
   // (clustered) every block has its barrier ready before another block arrives on it: the arrival
@@ -226,27 +226,50 @@ __global__ void __launch_bounds__(kDaThreads)
   // byte offset of 16-byte piece c (0 .. Dh/8-1) of row r inside a tile
   auto piece = [&](int r, int c) { return (c >> 3) * BOX + r * 128 + (((c & 7) ^ (r & 7)) << 4); };
 
+  // A thread rotates the same pair of every row that it takes: its angle's cosine and sine are made before the wait.
+  constexpr int kRowsPass = 128 / HALF;      // rows the threads take at a time
+  const int pair = tid % HALF, row_in_pass = tid / HALF;
+  float cs = 1.f, sn = 0.f;
+  if (a.inv_freq) {
+    const float ang = static_cast<float>(pos) * a.inv_freq[pair];
+    cs = cosf(ang);
+    sn = sinf(ang);
+  }
+  auto rotated = [&](float x1, float x2, float& o1, float& o2) {
+    o1 = x1;
+    o2 = x2;
+    if (a.inv_freq) {
+      o1 = x1 * cs - x2 * sn;
+      o2 = x2 * cs + x1 * sn;
+    }
+  };
   pdl_wait();  // the projections come from the kernel before this one
+  // all of this thread's loads go out together: its pairs of the query rows, and of the new key and value
+  bf16 q1[16 / kRowsPass], q2[16 / kRowsPass];
+#pragma unroll
+  for (int u = 0; u < 16 / kRowsPass; ++u) {
+    const int r = u * kRowsPass + row_in_pass;
+    q1[u] = q2[u] = __float2bfloat16_rn(0.f);
+    if (n_tiles > 0 && r < G) {
+      const bf16* src = a.q + static_cast<long long>(seq) * a.ldq + (hk * G + r) * DH;
+      q1[u] = src[pair];
+      q2[u] = src[pair + HALF];
+    }
+  }
   if (stores_new) {
     const int page = bt[pos / page_size];
     bf16* k_dst = a.pool + (static_cast<size_t>(page) * 2 * page_size + pos % page_size) * kv_dim + hk * DH;
     bf16* v_dst = k_dst + static_cast<size_t>(page_size) * kv_dim;
     const bf16* ksrc = a.k + static_cast<long long>(seq) * a.ldk + hk * DH;
     const bf16* vsrc = a.v + static_cast<long long>(seq) * a.ldv + hk * DH;
-    for (int i = tid; i < HALF; i += 128) {
-      const float x1 = __bfloat162float(ksrc[i]) * a.k_scale, x2 = __bfloat162float(ksrc[i + HALF]) * a.k_scale;
-      float o1 = x1, o2 = x2;
-      if (a.inv_freq) {
-        const float ang = static_cast<float>(pos) * a.inv_freq[i];
-        const float c = cosf(ang), sn = sinf(ang);
-        o1 = x1 * c - x2 * sn;
-        o2 = x2 * c + x1 * sn;
-      }
+    if (tid < HALF) {  // (pair == tid)
+      float o1, o2;
+      rotated(__bfloat162float(ksrc[tid]) * a.k_scale, __bfloat162float(ksrc[tid + HALF]) * a.k_scale, o1, o2);
       const bf16 b1 = __float2bfloat16_rn(o1), b2 = __float2bfloat16_rn(o2);
-      k_dst[i] = b1;
-      k_dst[i + HALF] = b2;
-      s_new_k[i] = b1;
-      s_new_k[i + HALF] = b2;
+      k_dst[tid] = b1;
+      k_dst[tid + HALF] = b2;
+      s_new_k[tid] = b1;
+      s_new_k[tid + HALF] = b2;
     }
     for (int i = tid; i < DH; i += 128) {
       const bf16 b = __float2bfloat16_rn(__bfloat162float(vsrc[i]) * a.v_scale);
@@ -255,23 +278,13 @@ __global__ void __launch_bounds__(kDaThreads)
     }
   }
   if (n_tiles > 0) {  // the query rows, scaled and rotated; rows beyond the group are zero
-    for (int idx = tid; idx < 16 * HALF; idx += 128) {
-      const int r = idx / HALF, i = idx % HALF;
+#pragma unroll
+    for (int u = 0; u < 16 / kRowsPass; ++u) {
+      const int r = u * kRowsPass + row_in_pass;
       float o1 = 0.f, o2 = 0.f;
-      if (r < G) {
-        const bf16* src = a.q + static_cast<long long>(seq) * a.ldq + (hk * G + r) * DH;
-        const float x1 = __bfloat162float(src[i]) * a.q_scale, x2 = __bfloat162float(src[i + HALF]) * a.q_scale;
-        o1 = x1;
-        o2 = x2;
-        if (a.inv_freq) {
-          const float ang = static_cast<float>(pos) * a.inv_freq[i];
-          const float c = cosf(ang), sn = sinf(ang);
-          o1 = x1 * c - x2 * sn;
-          o2 = x2 * c + x1 * sn;
-        }
-      }
-      sQ[r * QSTRIDE + i] = __float2bfloat16_rn(o1);
-      sQ[r * QSTRIDE + i + HALF] = __float2bfloat16_rn(o2);
+      if (r < G) rotated(__bfloat162float(q1[u]) * a.q_scale, __bfloat162float(q2[u]) * a.q_scale, o1, o2);
+      sQ[r * QSTRIDE + pair] = __float2bfloat16_rn(o1);
+      sQ[r * QSTRIDE + pair + HALF] = __float2bfloat16_rn(o2);
     }
   }
   sync_compute();
@@ -293,12 +306,13 @@ __global__ void __launch_bounds__(kDaThreads)
   const int row_v = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3);
   const float scale_log2 = a.scale_log2;
 
-  for (int it = 0; it < n_tiles; ++it) {
+  // Tile `it` is there, its rows outside the key range are zero and the new token's row is in it; false: a wait gave up.
+  auto arrived = [&](int it) {
     const int s = it % NSTAGE, base = first_tile + it * KT;
     const bool landed = mbar_wait(&bar_full[s], (it / NSTAGE) & 1, abort_flag);
     if (!landed) {  // (every warp waits on the same barrier: all of them leave)
       if (lane == 0) give_up(31);
-      break;
+      return false;
     }
     unsigned char* tK = sK + s * TILE;
     unsigned char* tV = sV + s * TILE;
@@ -319,20 +333,43 @@ __global__ void __launch_bounds__(kDaThreads)
       }
       sync_compute();
     }
+    return true;
+  };
+  // the scores of this warp's 16 keys of tile `it`
+  auto scores = [&](int it, float (&sc)[2][4]) {
+    const unsigned char* tK = sK + (it % NSTAGE) * TILE;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < KS_Q; ++ks) {
+      unsigned b0, b1, b2, b3;
+      ldmatrix_x4(b0, b1, b2, b3,
+                  tK + (ks >> 2) * BOX + row_k * 128 + (((((ks & 3) << 1) + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+      mma_bf16(sc[0], qf[ks], b0, b1);
+      mma_bf16(sc[1], qf[ks], b2, b3);
+    }
+  };
+  // The scores of a tile are made ahead of the softmax of the tile before it: two chains of dependent steps side by side
+  // (a tile is 16 keys a warp, bound by the chain: 1,200 clocks one after the other).
+  float ahead[2][4];
+  bool there = n_tiles > 0 && arrived(0);
+  if (there) scores(0, ahead);
+  for (int it = 0; it < n_tiles && there; ++it) {
+    const int s = it % NSTAGE, base = first_tile + it * KT;
+    const int next = min(it + 1, n_tiles - 1);  // (behind the last tile its own scores once more: no branch around them)
+    if (next > it) there = arrived(next);
+    unsigned char* tV = sV + s * TILE;
 
     const int kbase = base + warp * 16;
-    if (kbase < k_end && kbase + 16 > k_begin) {  // some of this warp's keys are wanted
+    if (!(kbase < k_end && kbase + 16 > k_begin)) {
+      scores(next, ahead);
+    } else {  // some of this warp's keys are wanted
       float sc[2][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int ks = 0; ks < KS_Q; ++ks) {
-        unsigned b0, b1, b2, b3;
-        ldmatrix_x4(b0, b1, b2, b3,
-                    tK + (ks >> 2) * BOX + row_k * 128 + (((((ks & 3) << 1) + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
-        mma_bf16(sc[0], qf[ks], b0, b1);
-        mma_bf16(sc[1], qf[ks], b2, b3);
-      }
+        for (int e = 0; e < 4; ++e) sc[i][e] = ahead[i][e];
+      scores(next, ahead);
       unsigned bv[NT_O / 2][4];  // the V fragments travel while the softmax is computed
 #pragma unroll
       for (int np = 0; np < NT_O / 2; ++np)
@@ -464,16 +501,14 @@ __global__ void __launch_bounds__(kDaThreads)
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // every block's tiles are done
     if (z > 0) {
       const unsigned dst = cluster_addr(smem_u32(sParts), 0) + static_cast<unsigned>((z - 1) * G * PW) * 4u;
-      for (int i = tid; i < G * DH; i += 128) {
-        const int r = i / DH, d = i % DH;
-        const float sum = (sO[r * SO + d] + sO[(16 + r) * SO + d]) + (sO[(32 + r) * SO + d] + sO[(48 + r) * SO + d]);
-        st_cluster_f32(dst + static_cast<unsigned>(r * PW + d) * 4u, sum);
-        if (d == 0) {
-          st_cluster_f32(dst + static_cast<unsigned>(r * PW + DH) * 4u, s_M[r]);
-          st_cluster_f32(dst + static_cast<unsigned>(r * PW + DH + 1) * 4u, s_L[r]);
-        }
+      const unsigned bar = cluster_addr(smem_u32(&bar_parts), 0);
+      for (int i = tid; i < G * (DH / 2); i += 128) {  // (rows of a part begin on 8-byte boundaries)
+        const int r = i / (DH / 2), d = (i % (DH / 2)) * 2;
+        const float s0 = (sO[r * SO + d] + sO[(16 + r) * SO + d]) + (sO[(32 + r) * SO + d] + sO[(48 + r) * SO + d]);
+        const float s1 = (sO[r * SO + d + 1] + sO[(16 + r) * SO + d + 1]) + (sO[(32 + r) * SO + d + 1] + sO[(48 + r) * SO + d + 1]);
+        st_async_f32x2(dst + static_cast<unsigned>(r * PW + d) * 4u, s0, s1, bar);
       }
-      mbar_arrive_remote(cluster_addr(smem_u32(&bar_parts), 0));  // releases this thread's writes above
+      if (tid < G) st_async_f32x2(dst + static_cast<unsigned>(tid * PW + DH) * 4u, s_M[tid], s_L[tid], bar);
       return;
     }
     // block 0: its own part is in sO / s_M / s_L; the others arrive in sParts
@@ -481,18 +516,27 @@ __global__ void __launch_bounds__(kDaThreads)
       if (lane == 0) give_up(33);
       return;
     }
+    // the weight of every part of every row, a thread each (16 lanes share a row)
+    for (int r0 = 0; r0 < G; r0 += 8) {
+      const int r = r0 + (tid >> 4), p = tid & 15;
+      float m = -CUDART_INF_F;
+      if (r < G && p < n_splits) m = p == 0 ? s_M[r] : sParts[((p - 1) * G + r) * PW + DH];
+      float mx = m;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (r < G) s_pw[r][p] = exp2f(m - ((mx == -CUDART_INF_F) ? 0.f : mx));  // (-inf - 0 -> 0: a part without keys)
+    }
+    sync_compute();
     for (int i = tid; i < G * (DH / 2); i += 128) {  // a thread per (row, two columns)
       const int r = i / (DH / 2), d = (i % (DH / 2)) * 2;
-      float mx = s_M[r];
-      for (int p = 0; p < n_splits - 1; ++p) mx = fmaxf(mx, sParts[(p * G + r) * PW + DH]);
-      const float mu = (mx == -CUDART_INF_F) ? 0.f : mx;
-      float w = exp2f(s_M[r] - mu);  // (-inf - 0 -> 0: a part without keys)
+      float w = s_pw[r][0];
       float tot = w * s_L[r];
       float a0 = w * ((sO[r * SO + d] + sO[(16 + r) * SO + d]) + (sO[(32 + r) * SO + d] + sO[(48 + r) * SO + d]));
       float a1 = w * ((sO[r * SO + d + 1] + sO[(16 + r) * SO + d + 1]) + (sO[(32 + r) * SO + d + 1] + sO[(48 + r) * SO + d + 1]));
+#pragma unroll 5
       for (int p = 0; p < n_splits - 1; ++p) {
         const float* part = sParts + (p * G + r) * PW;
-        w = exp2f(part[DH] - mu);
+        w = s_pw[r][p + 1];
         tot += w * part[DH + 1];
         a0 += w * part[d];
         a1 += w * part[d + 1];
