@@ -13,6 +13,12 @@
 // The four warps share every tile, warp w taking its keys 16w .. 16w+15 (own running maximum and
 // sum, merged at the end), so a tile is used up quickly and the ring stays ahead.
 //
+// A block is a chain of short steps, so what can be ahead of the wait for the projections is (the first tiles, the angle of
+// a thread's pair), all loads behind it go out together, a tile's scores are made beside the softmax of the tile before,
+// and the key splits' parts reach the first block of their cluster by st.async, weighted by a thread each.  One after the
+// other, with an arrival per thread that released plain remote stores, us before / now: 8 requests of 2,048 (8 query, 2
+// key/value heads of 64) 8.1 / 7.0, 1 of 700 5.9 / 5.0, 8 of 1,000 with one head of 128 for 8 queries 10.3 / 7.7; the same bits.
+//
 // As in the cp.async form the block scales and rotates its query rows itself, and the block whose
 // key range holds the new position rotates the new key, writes key and value into the cache page
 // and patches them into its tile once that has landed (the copy may have read the page before the

@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(64)
   float4 hist[L];
 #pragma unroll
   for (int k = 0; k < L; ++k) hist[k] = ldf4(win + static_cast<size_t>(k) * C);
-  const float4 v_new = make_float4(raw.x * ps.x + pb.x, raw.y * ps.y + pb.y, raw.z * ps.z + pb.z, raw.w * ps.w + pb.w);
+  auto scaled = [](float v, float m, float b) { return __fadd_rn(__fmul_rn(v, m), b); };  // (as the form above rounds: not fused)
+  const float4 v_new = make_float4(scaled(raw.x, ps.x, pb.x), scaled(raw.y, ps.y, pb.y), scaled(raw.z, ps.z, pb.z), scaled(raw.w, ps.w, pb.w));
 #pragma unroll
   for (int k = 1; k < L; ++k) stf4(win + static_cast<size_t>(k - 1) * C, hist[k]);
   stf4(win + static_cast<size_t>(L - 1) * C, v_new);
