@@ -10,7 +10,8 @@
 // of 64-wide K slices (A: one box of 128 sorted rows; B: two boxes of 128 weight rows of the tile's
 // expert out of the stacked matrix), one thread issues tcgen05.mma (M = 128, N = 256, K = 16) into
 // tensor memory, four epilogue warps read the accumulator a lane quarter each, apply the
-// activation and store whole row pieces.  Rows of a tile that lie beyond the expert's last row are
+// activation and store whole row pieces, put together in the stages (16 bytes to each of 32 rows at a time before: the same
+// four stages, down product 15.8 -> 12.2 us at 8,192 pairs, 256 -> 1,024).  Rows of a tile that lie beyond the expert's last row are
 // computed (they belong to the next expert, or are zero past the end) and not stored; weight rows
 // beyond the expert's block are loaded and their columns not stored.  Every mbarrier wait is
 // bounded; a wait that gives up records a code in *status and the block leaves.  No cluster
@@ -25,35 +26,34 @@ using bf16 = __nv_bfloat16;
 constexpr int kGM = 128;         // rows per tile
 constexpr int kGN = 256;         // accumulator columns per tile
 constexpr int kGK = 64;          // K per stage: one 128-byte swizzle row of bfloat16
-constexpr int kGStages = 4;
 constexpr int kGThreads = 192;   // warp 0: TMA producer, warp 1: tensor memory and MMA, warps 2..5: epilogue
 constexpr int kGABytes = kGM * kGK * 2;  // 16 KB
 constexpr int kGBBytes = kGN * kGK * 2;  // 32 KB
-constexpr size_t kGSmem = static_cast<size_t>(kGStages) * (kGABytes + kGBBytes) + 1024 /*alignment*/;
+constexpr size_t moe_tc_smem(int stages) { return static_cast<size_t>(stages) * (kGABytes + kGBBytes) + 1024 /*alignment*/; }
 constexpr unsigned kGIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kGN >> 3) << 17) | ((kGM >> 4) << 24);
 
-template <bool UP>
-__global__ void __launch_bounds__(kGThreads)
+template <bool UP, int STAGES>
+__global__ void __launch_bounds__(kGThreads, STAGES > 2 ? 1 : 2)
     moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                   const int* __restrict__ perm, const int* __restrict__ offsets, const int* __restrict__ tile_start, int E,
                   int K, int N, float limit, float alpha, float shift, int ungated,
                   const float* __restrict__ row_w, void* __restrict__ out, int* __restrict__ status) {
   pdl_launch_dependents();
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long bar_full[kGStages], bar_empty[kGStages], bar_accum;
+  __shared__ __align__(8) unsigned long long bar_full[STAGES], bar_empty[STAGES], bar_accum;
   __shared__ unsigned s_tmem_base;
   __shared__ int s_abort;
 
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = tiles;
-  unsigned char* sB = tiles + kGStages * kGABytes;
+  unsigned char* sB = tiles + STAGES * kGABytes;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.y * (UP ? kGN / 2 : kGN);      // first output column of the tile
   const int k_blocks = (K + kGK - 1) / kGK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kGStages; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&bar_full[s], 1);
       mbar_init(&bar_empty[s], 1);
     }
@@ -61,6 +61,9 @@ __global__ void __launch_bounds__(kGThreads)
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  // (tensor memory behind the wait: a block that holds some never waits for one that may still need some)
+  pdl_wait();
+  pdl_written(perm, offsets, tile_start, row_w);
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem_base)), "r"(kGN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -71,7 +74,6 @@ __global__ void __launch_bounds__(kGThreads)
   const unsigned tmem_base = s_tmem_base;
   volatile int* abort_flag = &s_abort;
 
-  pdl_wait();  // (barriers and tensor memory are set up while the kernel before this one still runs)
   int e = 0, row0 = 0, row1 = 0;
   const bool found = moe_tile(blockIdx.x, offsets, tile_start, E, kGM, e, row0, row1);  // the same in every warp
   const int w_row = e * (UP ? 2 * N : N) + n0;           // first weight row of the tile in the stacked matrix
@@ -83,8 +85,8 @@ __global__ void __launch_bounds__(kGThreads)
     if (lane == 0) {
       int issued = 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
-        const int s = kb % kGStages;
-        const unsigned use = kb / kGStages;
+        const int s = kb % STAGES;
+        const unsigned use = kb / STAGES;
         if (!mbar_wait(&bar_empty[s], (use & 1) ^ 1, abort_flag)) {
           if (!*abort_flag) atomicExch(status, 11);
           s_abort = 1;
@@ -98,9 +100,9 @@ __global__ void __launch_bounds__(kGThreads)
       }
       if (s_abort) {
         // copies already requested still write into this block's shared memory: wait for them
-        for (int kb = issued > kGStages ? issued - kGStages : 0; kb < issued; ++kb) {
-          const int s = kb % kGStages;
-          for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&bar_full[s], (kb / kGStages) & 1); ++i) {
+        for (int kb = issued > STAGES ? issued - STAGES : 0; kb < issued; ++kb) {
+          const int s = kb % STAGES;
+          for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&bar_full[s], (kb / STAGES) & 1); ++i) {
           }
         }
       }
@@ -110,8 +112,8 @@ __global__ void __launch_bounds__(kGThreads)
     if (lane == 0) {
       bool ok = true;
       for (int kb = 0; kb < k_blocks && ok; ++kb) {
-        const int s = kb % kGStages;
-        if (!mbar_wait(&bar_full[s], (kb / kGStages) & 1, abort_flag)) {
+        const int s = kb % STAGES;
+        if (!mbar_wait(&bar_full[s], (kb / STAGES) & 1, abort_flag)) {
           if (!*abort_flag) atomicExch(status, 12);
           s_abort = 1;
           ok = false;
@@ -139,9 +141,26 @@ __global__ void __launch_bounds__(kGThreads)
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const int i = row0 + quad * 32 + lane;  // this thread's row among the sorted pairs
       const bool row_ok = i < row1;
+      // A thread holds 64 columns of a row; rows go out through the stages (all products have read them), 128 bytes at a time
+      // and four rows a store, where a thread's own stores touched 32 lines with 16 bytes each.
+      unsigned char* mine = tiles + quad * (32 * 128);
+      auto stage_piece = [&](int ck, const uint4& v) {
+        *reinterpret_cast<uint4*>(mine + lane * 128 + ((ck ^ (lane & 7)) << 4)) = v;
+      };
+      auto rows_out = [&](int out_row, int col) {  // out_row: where this thread's row goes; col: the first of 64 columns
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = k * 4 + (lane >> 3), ck = lane & 7;
+          const int to = __shfl_sync(0xffffffffu, out_row, r);
+          if (row0 + quad * 32 + r < row1 && col + ck * 8 < N)  // N is a multiple of 8
+            *reinterpret_cast<uint4*>(static_cast<bf16*>(out) + static_cast<size_t>(to) * N + col + ck * 8) =
+                *reinterpret_cast<const uint4*>(mine + r * 128 + ((ck ^ (r & 7)) << 4));
+        }
+        __syncwarp();
+      };
       const unsigned lane_base = tmem_base + (static_cast<unsigned>(quad * 32) << 16);
       if (UP) {
-        bf16* dst_row = static_cast<bf16*>(out) + static_cast<size_t>(row_ok ? i : 0) * N;
         const float rw = (row_w && row_ok) ? row_w[perm[i]] : 1.f;  // the pair's input is rw * x
 #pragma unroll 1
         for (int c = 0; c < kGN / 64; ++c) {
@@ -149,57 +168,49 @@ __global__ void __launch_bounds__(kGThreads)
           tmem_ld32(lane_base + c * 32, g);
           tmem_ld32(lane_base + kGN / 2 + c * 32, u);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-          if (row_ok) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              const int col = n0 + c * 32 + j;
-              if (col < N) {  // N is a multiple of 8
-                uint4 pack;
-                __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pack);
+          for (int j = 0; j < 32; j += 8) {
+            uint4 pack;
+            __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pack);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  float r[2];
+            for (int q = 0; q < 4; ++q) {
+              float r[2];
 #pragma unroll
-                  for (int h = 0; h < 2; ++h) {
-                    const float gv = fminf(rw * __uint_as_float(g[j + 2 * q + h]), limit);
-                    const float uv = fminf(fmaxf(rw * __uint_as_float(u[j + 2 * q + h]), -limit), limit);
-                    r[h] = __fdividef(gv, 1.f + __expf(-alpha * gv)) * (uv + shift);
-                  }
-                  p2[q] = __floats2bfloat162_rn(r[0], r[1]);
-                }
-                *reinterpret_cast<uint4*>(dst_row + col) = pack;
+              for (int h = 0; h < 2; ++h) {
+                const float gv = fminf(rw * __uint_as_float(g[j + 2 * q + h]), limit);
+                const float uv = fminf(fmaxf(rw * __uint_as_float(u[j + 2 * q + h]), -limit), limit);
+                r[h] = __fdividef(gv, 1.f + __expf(-alpha * gv)) * (uv + shift);
               }
+              p2[q] = __floats2bfloat162_rn(r[0], r[1]);
             }
+            stage_piece((c & 1) * 4 + (j >> 3), pack);
           }
+          if (c & 1) rows_out(i, n0 + (c >> 1) * 64);
         }
       } else {
         // (ungated experts' up product: rows stay in the order of the sorted pairs, values become max(z, 0)^2)
-        bf16* dst_row = static_cast<bf16*>(out) + static_cast<size_t>(row_ok ? (ungated ? i : perm[i]) : 0) * N;
+        const int out_row = row_ok ? (ungated ? i : perm[i]) : 0;
 #pragma unroll 1
         for (int q = 0; q < kGN / 32; ++q) {
           unsigned v[32];
           tmem_ld32(lane_base + q * 32, v);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-          if (row_ok) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              const int col = n0 + q * 32 + j;
-              if (col < N) {  // N is a multiple of 8
-                uint4 pack;
-                __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pack);
+          for (int j = 0; j < 32; j += 8) {
+            uint4 pack;
+            __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pack);
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                  float v0 = __uint_as_float(v[j + 2 * h]), v1 = __uint_as_float(v[j + 2 * h + 1]);
-                  if (ungated) {
-                    v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
-                    v0 *= v0, v1 *= v1;
-                  }
-                  p2[h] = __floats2bfloat162_rn(v0, v1);
-                }
-                *reinterpret_cast<uint4*>(dst_row + col) = pack;
+            for (int h = 0; h < 4; ++h) {
+              float v0 = __uint_as_float(v[j + 2 * h]), v1 = __uint_as_float(v[j + 2 * h + 1]);
+              if (ungated) {
+                v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
+                v0 *= v0, v1 *= v1;
               }
+              p2[h] = __floats2bfloat162_rn(v0, v1);
             }
+            stage_piece((q & 1) * 4 + (j >> 3), pack);
           }
+          if (q & 1) rows_out(out_row, n0 + (q >> 1) * 64);
         }
       }
     }
@@ -291,19 +302,20 @@ PMM_EXPORT int pmm_moe_tc_gemm(const void* a, long long ld_a, const void* w, con
   const int cols_per_block = up ? pmm::kGN / 2 : pmm::kGN;
   dim3 grid(row_tiles, (N + cols_per_block - 1) / cols_per_block);
   if (grid.y > 65535) return PMM_ERR_BAD_ARGUMENT;
-  cudaError_t err;
-  if (up) {
-    auto kern = pmm::moe_tc_kernel<true>;
-    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pmm::kGSmem));
+  // A block of four stages, one an SM, while about one tile an SM is expected (half a ragged tile an expert; the plan is on the
+  // device): its products wait for copies less.  Beyond, two blocks of two stages share an SM, one's epilogue beside the
+  // other's products.  Us with four / two stages, up and down: 8,192 pairs, 16 experts, 1,024 -> 256 -> 1,024 11.2 / 15.5
+  // (144 tiles) and 12.2 / 8.9 (288); 16,384 pairs 19.6 / 17.1 and 22.0 / 15.3; 12,288 pairs, 64 experts,
+  // 2,048 -> 1,408 -> 2,048 247 / 233 and 138 / 122; 2,048 pairs, 16 experts 9.7 / 12.3 and 6.0 / 6.4.
+  const bool few = static_cast<long long>(A / pmm::kGM + (E < A ? E : A) / 2) * grid.y <= 148;
+  auto run = [&](auto kern, int stages) -> int {
+    const size_t smem = pmm::moe_tc_smem(stages);
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
-    pmm::launch_pdl(kern, grid, dim3(pmm::kGThreads), pmm::kGSmem, stream, map_a, map_w, perm, offsets, tile_start, E, K, N,
-                    limit, alpha, shift, ungated, row_w, out, status);
-  } else {
-    auto kern = pmm::moe_tc_kernel<false>;
-    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pmm::kGSmem));
-    if (err != cudaSuccess) return static_cast<int>(err);
-    pmm::launch_pdl(kern, grid, dim3(pmm::kGThreads), pmm::kGSmem, stream, map_a, map_w, perm, offsets, tile_start, E, K, N,
-                    limit, alpha, shift, ungated, row_w, out, status);
-  }
-  return pmm::launch_status();
+    pmm::launch_pdl(kern, grid, dim3(pmm::kGThreads), smem, stream, map_a, map_w, perm, offsets, tile_start, E, K, N, limit,
+                    alpha, shift, ungated, row_w, out, status);
+    return pmm::launch_status();
+  };
+  if (few) return up ? run(pmm::moe_tc_kernel<true, 4>, 4) : run(pmm::moe_tc_kernel<false, 4>, 4);
+  return up ? run(pmm::moe_tc_kernel<true, 2>, 2) : run(pmm::moe_tc_kernel<false, 2>, 2);
 }

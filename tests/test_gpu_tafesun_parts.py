@@ -330,3 +330,37 @@ def test_gathered_rows_of_every_width(A, top, Kd):
     K.moe_gather_rows(x, perm.to(DEV), top, out[:A])
     assert torch.equal(out[:A].cpu(), x.cpu()[perm.long() // top])
     assert bool(torch.isnan(out[A]).all())
+
+
+@pytest.mark.parametrize("T,E,top,Kd,N", [(130, 5, 2, 64, 8), (130, 3, 3, 192, 200), (3000, 5, 2, 192, 1000), (2500, 40, 4, 320, 264), (4000, 1, 1, 64, 1288)])
+def test_tcgen05_products_of_few_and_many_tiles(T, E, top, Kd, N):
+    """One block and two blocks an SM, fewer and more slices of K than stages, columns that end inside a store's 64: small
+    whole numbers, so that plain and squared sums are exact up to the rounding to bfloat16 (2^-9 of a value, exp's and the
+    quotient's errors far below), and nothing is stored behind the last row."""
+    g = torch.Generator().manual_seed(T + E)
+    a = torch.randint(-1, 2, (T * top, Kd), generator=g).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    if E > 4:
+        ids[ids == E - 2] = 0   # an expert without pairs
+    A = T * top
+    offsets, tiles = (torch.empty(E + 1, dtype=torch.int32, device=DEV) for _ in range(2))
+    perm = torch.empty(A, dtype=torch.int32, device=DEV)
+    K.moe_plan(ids.to(DEV), E, "tcgen05", offsets, tiles, perm)
+    order = perm.cpu().long()
+    experts = ids.view(-1)[order].long()
+    for form, up, ungated, rows_w in (("down", False, False, N), ("ungated", True, True, N), ("gated", True, False, 2 * N)):
+        w = torch.randint(-1, 2, (E, rows_w, Kd), generator=g).to(torch.bfloat16)
+        z = torch.zeros(A, rows_w, dtype=torch.float64)
+        for e in range(E):
+            z[experts == e] = (a.float()[experts == e] @ w[e].float().t()).double()   # (exact: whole numbers below 2^24)
+        out = torch.full((A + 1, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        K.moe_tc_gemm(a.to(DEV), w.to(DEV), perm, offsets, tiles, up, out[:A], limit=1e4, alpha=1.0, ungated=ungated)
+        assert K.tc_gemm_status(out.device) == 0
+        if form == "down":
+            want = torch.empty_like(z)
+            want[order] = z
+        else:
+            want = z.clamp_min(0).square() if ungated else torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+        err = (out[:A].cpu().double() - want).abs()
+        assert bool((err <= 2.0 ** -8 * want.abs() + 1e-6).all()), form
+        assert bool(torch.isnan(out[A]).all())
