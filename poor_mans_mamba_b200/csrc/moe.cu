@@ -25,16 +25,55 @@ namespace pmm {
 // A chain of reads and reductions, bound by their latency: a warp's first router rows are read before the wait for the
 // kernel before this one (they are weights), and up to 32 experts are ranked by one lane each against all others at once
 // (`ranked`) where picking them one after the other takes ten exchanges between lanes apiece.  16 experts, 4 chosen in 2
-// of 4 groups, width 1,024, inside a step: 8 tokens 11 -> 4.5 us.
+// of 4 groups, width 1,024, inside a step: 8 tokens 11 -> 4.5 us.  Of many tokens' 19,000 clocks 3,900 went to rows read one
+// piece after the other behind an integer division, 5,000 to 80 exchanges a warp for its 16 sums and 4,000 to the ranking's
+// chain: a row's pieces are read together, sums over lanes are halved as they are exchanged (`warp_sums`, the same
+// order), the ranking's reads go out eight at a time.  Alone, us: 2,048 tokens 10.4 -> 8.0, 4,096 20.2 -> 15.5, 512 6.5 -> 5.7; 8,192
+// of width 2,048, 32 experts 97 -> 83.  What is left most is the products' reads of the rows from shared memory.
 constexpr int kRouteAhead = 8;   // sixteen-byte pieces of a router row a lane holds before the wait (128 columns each)
 
 // This lane's place (0: the largest; the lower index wins a tie) among values v[0 .. n - 1], n <= 32, none of them NaN.
 __device__ __forceinline__ int ranked(const float* v, int n, int lane) {
   const float mine = lane < n ? v[lane] : -INFINITY;
   int rank = 0;
-#pragma unroll 8
-  for (int e = 0; e < n; ++e) rank += (v[e] > mine || (v[e] == mine && e < lane)) ? 1 : 0;
+  for (int e0 = 0; e0 < n; e0 += 8) {  // eight reads in flight
+    float o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = v[min(e0 + k, n - 1)];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) rank += (e0 + k < n && (o[k] > mine || (o[k] == mine && e0 + k < lane))) ? 1 : 0;
+  }
   return rank;
+}
+// v[0] + v[1] + ... + v[n - 1] in this order, eight reads in flight.
+__device__ __forceinline__ float sum_in_order(const float* v, int n) {
+  float sum = 0.f;
+  for (int j0 = 0; j0 < n; j0 += 8) {
+    float o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = v[min(j0 + k, n - 1)];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (j0 + k < n) sum += o[k];
+  }
+  return sum;
+}
+// The sums over a warp's lanes of N values each (a power of two, up to 32): lane l gets that of value l / (32 / N), added in
+// warp_sum's order, for N + log2(32 / N) exchanges instead of 5 N.
+template <int N>
+__device__ __forceinline__ float warp_sums(const float (&v)[N], int lane, int o = 16) {
+  if constexpr (N == 1) {
+    float sum = v[0];
+    for (; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+  } else {
+    const bool high = lane & o;
+    float half[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i)
+      half[i] = (high ? v[N / 2 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, high ? v[i] : v[N / 2 + i], o);
+    return warp_sums(half, lane, o >> 1);
+  }
 }
 // Whether one lane an expert can rank them: the picks of a row with NaN or infinite entries are left to the serial form.
 __device__ __forceinline__ bool all_finite(const float* v, int n, int lane) {
@@ -71,14 +110,18 @@ __global__ void __launch_bounds__(WARPS * 32)
         if (warp * kPer + q < n_rows && lane * 4 + 128 * k < D)
           ahead[q][k] = *reinterpret_cast<const float4*>(router_row(warp * kPer + q) + lane * 4 + 128 * k);
   }
+  // (weights and divisions of the ranking, ahead of the wait as well)
+  const float correction0 = scored && correction && lane < E ? correction[lane] : 0.f;
+  const int per = scored && groups > 1 ? E / groups : 1, lane_group = scored && groups > 1 ? lane / per : 0;
   pdl_wait();
+  pdl_written(x);
   if ((D & 3) == 0 && ld_x % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (4 * sizeof(S)) == 0) {
-    const int D4 = D / 4;
-    for (int i = threadIdx.x; i < TOK * D4; i += blockDim.x) {
-      const int r = i / D4, c = 4 * (i - r * D4);
-      *reinterpret_cast<float4*>(rows + r * Dpad + c) =
-          r < nt ? ldf4(x + static_cast<long long>(t0 + r) * ld_x + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    constexpr int kParts = WARPS / TOK;  // warps a row
+    const int r = warp / kParts, part = warp % kParts;
+    const S* from = x + static_cast<long long>(t0 + min(r, nt - 1)) * ld_x;
+#pragma unroll 8
+    for (int c = 4 * (part * 32 + lane); c < D; c += 128 * kParts)
+      *reinterpret_cast<float4*>(rows + r * Dpad + c) = r < nt ? ldf4(from + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   } else {
     for (int r = 0; r < TOK; ++r)
       for (int i = threadIdx.x; i < Dpad; i += blockDim.x)
@@ -131,18 +174,17 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
       }
     }
+    float of_lane[kPer * TOK];
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int e = e0 + q;
-      if (q >= n_here) break;
+    for (int q = 0; q < kPer; ++q)
 #pragma unroll
-      for (int r = 0; r < TOK; ++r) {
-        const float sum = warp_sum(acc[q][r]);
-        if (lane == 0) {
-          if (e < E) logits[r * E + e] = sum + (bias ? bias[e] : 0.f);
-          else if (r < nt) gate_out[t0 + r] = 1.f / (1.f + expf(-sum));
-        }
-      }
+      for (int r = 0; r < TOK; ++r) of_lane[q * TOK + r] = acc[q][r];
+    const float sum = warp_sums(of_lane, lane);
+    constexpr int kLanes = 32 / (kPer * TOK);  // that hold the same sum
+    const int q = lane / kLanes / TOK, r = lane / kLanes % TOK, e = e0 + q;
+    if (lane % kLanes == 0 && q < n_here) {
+      if (e < E) logits[r * E + e] = sum + (bias ? bias[e] : 0.f);
+      else if (r < nt) gate_out[t0 + r] = 1.f / (1.f + expf(-sum));
     }
   }
   __syncthreads();
@@ -172,24 +214,31 @@ __global__ void __launch_bounds__(WARPS * 32)
         for (int e = lane; e < E; e += 32) {
           const float sv = sc[e] * zinv;
           sc[e] = sv;
-          z[e] = sv + (correction ? correction[e] : 0.f);
+          z[e] = sv + (e < 32 ? correction0 : correction ? correction[e] : 0.f);
         }
       } else {
         for (int e = lane; e < E; e += 32) {
           const float sv = 1.f / (1.f + expf(-z[e]));
           sc[e] = sv;
-          z[e] = sv + (correction ? correction[e] : 0.f);
+          z[e] = sv + (e < 32 ? correction0 : correction ? correction[e] : 0.f);
         }
       }
       __syncwarp();
       const bool at_once = all_finite(z, E, lane);
       if (groups > 1) {
-        const int per = E / groups;
         for (int g = lane; g < groups; g += 32) {
           float a = -INFINITY, b = -INFINITY;  // the largest and the second largest
-          for (int e = g * per; e < (g + 1) * per; ++e) {
-            const float v = z[e];
-            if (v > a) { b = a; a = v; } else if (v > b) { b = v; }
+          for (int e0 = 0; e0 < per; e0 += 8) {  // eight reads in flight
+            float o[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) o[k] = z[g * per + min(e0 + k, per - 1)];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const float v = o[k];
+              if (e0 + k < per) {
+                if (v > a) { b = a; a = v; } else if (v > b) { b = v; }
+              }
+            }
           }
           gs[g] = (per > 1 && scored != 2) ? a + b : a;
         }
@@ -219,7 +268,7 @@ __global__ void __launch_bounds__(WARPS * 32)
           __syncwarp();
         }
         for (int e = lane; e < E; e += 32)
-          if (gs[e / per] != INFINITY) z[e] = -INFINITY;
+          if (gs[e < 32 ? lane_group : e / per] != INFINITY) z[e] = -INFINITY;
         __syncwarp();
       }
       if (at_once) {
@@ -228,8 +277,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         __syncwarp();
         if (chosen) z[place] = sc[lane];  // the chosen scores in their order
         __syncwarp();
-        float denom = 0.f;
-        for (int j = 0; j < top; ++j) denom += z[j];
+        const float denom = sum_in_order(z, top);
         const float inv = scored >= 2 ? scale : scale / (denom + 1e-20f);
         if (chosen) {
           ids[static_cast<size_t>(t0 + r) * top + place] = lane;
@@ -277,8 +325,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       __syncwarp();
       if (chosen) z[place] = p;
       __syncwarp();
-      float denom = 0.f;
-      for (int j = 0; j < top; ++j) denom += z[j];
+      const float denom = sum_in_order(z, top);
       const float inv = 1.f / denom;
       if (chosen) {
         ids[static_cast<size_t>(t0 + r) * top + place] = lane;
