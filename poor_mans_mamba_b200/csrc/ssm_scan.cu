@@ -151,11 +151,13 @@ __global__ void __launch_bounds__(kScanRows* kScanTpr)
   if (t1 <= t0) return;
   if (one_token == 2 && t1 - t0 != 1) return;  // only the lone tokens of a mixed step
 
+  // read once and written once a step: streaming accesses, so that states go out of the caches before weights and activations do
+  // (decode steps, us: 36 layers, 8 requests 872 -> 862; 8 layers, 64 requests 532 -> 527, 1 request 187 -> 187)
   float4 st[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int q = lane_n + i * kScanTpr;
-    st[i] = (row_ok && q < n4) ? scan_ld4(srow + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    st[i] = (row_ok && q < n4) ? __ldcs(reinterpret_cast<const float4*>(srow + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 
   for (int t = t0; t < t1; ++t) {
@@ -199,7 +201,7 @@ __global__ void __launch_bounds__(kScanRows* kScanTpr)
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int q = lane_n + i * kScanTpr;
-      if (q < n4) *reinterpret_cast<float4*>(srow + 4 * q) = st[i];
+      if (q < n4) __stcs(reinterpret_cast<float4*>(srow + 4 * q), st[i]);
     }
   }
 }
