@@ -30,7 +30,7 @@
 // (reference src/ops/gpu/attention.cu:4-40 and :44-105), keys lo..pos, lo from the window.
 // Several key splits of a (sequence, head) are merged without a second launch.  Up to 16 splits run
 // as one thread-block cluster: every block writes its (maximum, sum, unnormalised output) into the
-// first block's shared memory and arrives on a barrier there; the first block merges and stores.
+// first block's shared memory, where a barrier counts their bytes; the first block merges and stores.
 // More splits (or results too large for that buffer) go through global memory and a counter: the
 // block that finishes the last split merges them.
 // Every mbarrier wait is bounded; a wait that gives up writes a code (31: a tile never landed,
