@@ -724,7 +724,8 @@ __global__ void __launch_bounds__(kTWalkAll, 1)
 // t + 384 share token t of the chunk (= tensor-memory lane t) and split its columns; warp 16 issues the products.  Tensor
 // memory: G columns 0..127, Y2 columns 128..128+PB, Y1 columns 192..192+PB.
 // C, B, x and the gate's input were finished before the launch before this one (which lets this one go behind its own wait):
-// they are brought and G is made before this launch's wait.
+// they are brought and G is made before this launch's wait.  The start states and the tokens' steps and decays (chunk_dt) are not:
+// the walk, directly before this launch, writes both, so they are read behind the wait only.
 // What bounds it: a unit is a chain of two products, an exponential per entry of M's lower half and two per output, about
 // 2,400 clocks.  One block a unit (two blocks an SM, C and B brought and G made for every head) took 19.5 us at 24 heads of
 // 64 x 128 and 2,048 tokens and 56 us at 48 heads of 128 x 256 and 1,024 tokens.
@@ -877,22 +878,22 @@ __global__ void __launch_bounds__(kTOutAll, 1)
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  auto copy_x = [&](int k) {  // x and the decays of unit k into its stage
+  auto copy_x = [&](int k) {  // x of unit k into its stage
     unsigned char* dst = sX + (k & 1) * kTSub;
     const size_t col = col_of(k);
     tq_pieces(tid, kTQ, PB / 8, [&](int j, int ck) {
       const bool ok = j < len;
       tq_cp16(dst + tq_swz(j, ck), xbc + (ok ? static_cast<size_t>(t0 + j) * ld_xbc + col + ck * 8 : 0), ok);
     });
-    if (tid < kTQ / 2)
-      tq_cp16(&s_dt[k & 1][tid * 4], chunk_dt + (static_cast<size_t>(c) * H + head_of(k)) * (2 * kTQ) + tid * 4, true);
   };
-  auto copy_s = [&](int k) {
+  auto copy_s = [&](int k) {  // its start states, steps and decays (results of the launch before: behind the wait)
     unsigned char* dst = (k & 1) ? sS1 : sS0;
     const bf16* src = start_state + (static_cast<size_t>(c) * I + col_of(k)) * N;
     tq_pieces(tid, PB, N / 8, [&](int p, int ck) {
       tq_cp16(dst + (ck >> 3) * s_sub + tq_swz(p, ck & 7), src + static_cast<size_t>(p) * N + ck * 8, true);
     });
+    if (tid < kTQ / 2)
+      tq_cp16(&s_dt[k & 1][tid * 4], chunk_dt + (static_cast<size_t>(c) * H + head_of(k)) * (2 * kTQ) + tid * 4, true);
   };
   auto commit = [&]() { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
   // (whole tiles of 64 columns) one lane of warp 16 asks for them; rows beyond the chunk bring what lies there: a row of C reaches
