@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128)
     for (int i = 0; i < 8; ++i) wk[i][k] = col[i];
   }
   pdl_wait();
-  pdl_written(x);
+  pdl_written(x, window);
   uint4 raw[R];  // rows t_begin - L .. t_begin + strip - 1
 #pragma unroll
   for (int i = 0; i < R; ++i) {

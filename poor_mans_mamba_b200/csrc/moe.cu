@@ -371,6 +371,7 @@ __global__ void __launch_bounds__(1024)
   pdl_launch_dependents();
   for (int e = threadIdx.x; e < E; e += blockDim.x) plan_counts[e] = 0;
   pdl_wait();
+  pdl_written(ids);
   __syncthreads();
   for (int i = threadIdx.x; i < A; i += blockDim.x) {
     const int e = ids[i];
@@ -436,6 +437,7 @@ __global__ void __launch_bounds__(1024)
   for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) plan_hist[i] = 0;
   __syncthreads();
   pdl_wait();
+  pdl_written(ids);
   const int e = blockIdx.x;
   const int run = (A + 1023) / 1024;  // a thread owns a run of consecutive pairs
   const int i0 = min(A, static_cast<int>(threadIdx.x) * run), i1 = min(A, i0 + run);

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(kSideThreads)
     es[idx] = r < nt ? ldf(table + static_cast<long long>(tokens[t0 + r]) * ld_table + col0 + j) : 0.f;
   }
   pdl_wait();
+  pdl_written(a, b);
   // x = h + sa * a + sb * b; the rows of a short last block that have no token are zero
   if (VEC) {
     const int per_row = D >> 2;
@@ -286,6 +287,7 @@ __global__ void __launch_bounds__(kSideMmaThreads)  // (64 registers for two blo
     es[idx] = r < nt ? ldf(table + static_cast<long long>(tokens[t0 + r]) * ld_table + col0 + j) : 0.f;
   }
   pdl_wait();
+  pdl_written(a, b);
   const int per_row = D >> 2;
 #pragma unroll 4
   for (int idx = threadIdx.x; idx < kSideMmaTok * per_row; idx += kSideMmaThreads) {

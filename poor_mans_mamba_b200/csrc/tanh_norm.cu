@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256)
   const float al = alpha ? alpha[0] : 0.f;      // constants of the model: read before the wait
   const float pal = post_alpha ? post_alpha[0] : 0.f;
   pdl_wait();
+  pdl_written(a, b);
   const int r = blockIdx.x;
   const size_t src = static_cast<size_t>(rows ? rows[r] : r) * D;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < D; i += gridDim.y * blockDim.x) {

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(kMixThreads)
   for (int s = 0; s < kMixMax; ++s)  // (the mixes' weights are constants: read before the wait)
     if (s < n_mixes && c < D) PF::load(mu + static_cast<size_t>(s) * D + c, m[s]);
   pdl_wait();
+  pdl_written(x);
   if (c >= D) return;
   const int t_begin = blockIdx.x * tokens, t_end = min(T, t_begin + tokens);
   float before[VEC];

@@ -91,3 +91,27 @@ def test_results_of_a_launch_are_read_behind_the_wait(name, body):
     """What a kernel marks as written by the launches before it, it does not touch before it has waited for them."""
     ahead = ahead_of_wait(body)
     assert [p for p in sorted(marked(body)) if uses(ahead, p)] == []
+
+
+# Weights, and inputs of the step that are written before its first launch: no launch's result, so on neither side of a wait.
+CONSTANT = {"w", "w_t", "bias", "norm_w", "gate_w", "w_gate", "w_proj", "w_proj_t", "mix", "in_w", "out_w", "post_w", "post_b", "post_alpha", "alpha", "sink", "mu",
+            "correction", "pre_scale", "pre_bias", "dt_shift", "a_log", "d_skip", "z_bias", "table",
+            "cu", "slots", "seq_of", "positions", "block_table", "rows", "tokens"}
+# Read by asynchronous copies only (the compiler leaves them where they stand), or finished before the launch before let this one go.
+OTHERWISE = {"attention_mma.cu:flash_paged_kernel": {"q", "pool"}, "ssd_tc.cu:ssd_tc_output_kernel": {"xbc", "z_raw"}}
+
+
+def works_ahead(body):
+    """Whether a kernel has code, not only declarations, ahead of its wait."""
+    if not uses(body, "pdl_wait"):
+        return False
+    ahead = re.sub(r"(extern\s+)?__shared__[^;]*;|constexpr[^;]*;|using[^;]*;", "", ahead_of_wait(body))
+    return re.search(r"\b(if|for|while)\b|__syncthreads|\bldf|\w\[", ahead) is not None
+
+
+@pytest.mark.parametrize("name,params,body", [pytest.param(n, p, b, id=n) for n, p, b in KERNELS if works_ahead(b)])
+def test_results_of_a_launch_are_marked_behind_the_wait(name, params, body):
+    """The compiler may move what is read through a `const T* __restrict__` parameter above the wait once there is code in front
+    of it: every such parameter is a constant of the step or is marked."""
+    pointers = re.findall(r"\bconst\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params)
+    assert [p for p in pointers if p not in CONSTANT | marked(body) | OTHERWISE.get(name, set())] == []
