@@ -33,9 +33,10 @@
 // first block's shared memory, where a barrier counts their bytes; the first block merges and stores.
 // More splits (or results too large for that buffer) go through global memory and a counter: the
 // block that finishes the last split merges them.
-// Every mbarrier wait is bounded; a wait that gives up writes a code (31: a tile never landed,
-// 32: a stage never came free, 33: another block's result never came) to *status, and the step's
-// results are discarded by the host.
+// Every mbarrier wait is bounded.  A warp whose wait gives up raises the block's flag and walks on
+// like the others, so that all meet at the block's barriers; the flag is read behind one, and they
+// leave together.  It writes a code (31: a tile never landed, 32: a stage never came free, 33:
+// another block's result never came) to *status, and the step's results are discarded by the host.
 #include "mma_helpers.cuh"
 #include "tcgen05.cuh"
 #include <math_constants.h>
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kDaThreads)
       int issued = first;
       for (int j = first; j < n_tiles; ++j) {
         int ok = 1;
-        if (lane == 0) ok = mbar_wait(&bar_empty[j % NSTAGE], ((j / NSTAGE) & 1) ^ 1, abort_flag) ? 1 : 0;
+        if (lane == 0) ok = mbar_wait(&bar_empty[j % NSTAGE], ((j / NSTAGE) & 1) ^ 1, abort_flag) && !*abort_flag ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) {
           if (lane == 0) give_up(32);
@@ -312,14 +313,11 @@ __global__ void __launch_bounds__(kDaThreads)
   const int row_v = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3);
   const float scale_log2 = a.scale_log2;
 
-  // Tile `it` is there, its rows outside the key range are zero and the new token's row is in it; false: a wait gave up.
+  // Behind this tile `it` is there, its rows outside the key range are zero and the new token's row is in it.  (A wait that gave
+  // up goes on like the others, which may have seen the tile: all meet at the barriers, and the block's result is dropped.)
   auto arrived = [&](int it) {
     const int s = it % NSTAGE, base = first_tile + it * KT;
-    const bool landed = mbar_wait(&bar_full[s], (it / NSTAGE) & 1, abort_flag);
-    if (!landed) {  // (every warp waits on the same barrier: all of them leave)
-      if (lane == 0) give_up(31);
-      return false;
-    }
+    if (!mbar_wait(&bar_full[s], (it / NSTAGE) & 1, abort_flag)) give_up(31);
     unsigned char* tK = sK + s * TILE;
     unsigned char* tV = sV + s * TILE;
     const bool last = it == n_tiles - 1;
@@ -339,7 +337,6 @@ __global__ void __launch_bounds__(kDaThreads)
       }
       sync_compute();
     }
-    return true;
   };
   // the scores of this warp's 16 keys of tile `it`
   auto scores = [&](int it, float (&sc)[2][4]) {
@@ -358,12 +355,14 @@ __global__ void __launch_bounds__(kDaThreads)
   // The scores of a tile are made ahead of the softmax of the tile before it: two chains of dependent steps side by side
   // (a tile is 16 keys a warp, bound by the chain: 1,200 clocks one after the other).
   float ahead[2][4];
-  bool there = n_tiles > 0 && arrived(0);
-  if (there) scores(0, ahead);
-  for (int it = 0; it < n_tiles && there; ++it) {
+  if (n_tiles > 0) {
+    arrived(0);
+    scores(0, ahead);
+  }
+  for (int it = 0; it < n_tiles; ++it) {
     const int s = it % NSTAGE, base = first_tile + it * KT;
     const int next = min(it + 1, n_tiles - 1);  // (behind the last tile its own scores once more: no branch around them)
-    if (next > it) there = arrived(next);
+    if (next > it) arrived(next);
     unsigned char* tV = sV + s * TILE;
 
     const int kbase = base + warp * 16;
@@ -436,7 +435,7 @@ __global__ void __launch_bounds__(kDaThreads)
     __syncwarp();
     if (lane == 0) mbar_arrive(&bar_empty[s]);  // this warp is done with the stage
   }
-  sync_compute();  // every warp is done with the ring (it is reused below)
+  sync_compute();  // every warp is done with the ring (it is reused below), and has raised the flag if a wait of its own gave up
   if (a.clustered) {
     // Second round of the cluster barrier: this block's tiles are done (all of them have landed and
     // been used: nothing writes into its ring any more).  Behind it the first block's V ring takes
@@ -518,12 +517,10 @@ __global__ void __launch_bounds__(kDaThreads)
       return;
     }
     // block 0: its own part is in sO / s_M / s_L; the others arrive in sParts
-    if (!mbar_wait_cluster(&bar_parts, 0, abort_flag)) {
-      if (lane == 0) give_up(33);
-      return;
-    }
+    const bool sent = __all_sync(0xffffffffu, mbar_wait_cluster(&bar_parts, 0, abort_flag));
+    if (!sent && lane == 0) give_up(33);
     // the weight of every part of every row, a thread each (16 lanes share a row)
-    for (int r0 = 0; r0 < G; r0 += 8) {
+    for (int r0 = 0; r0 < (sent ? G : 0); r0 += 8) {
       const int r = r0 + (tid >> 4), p = tid & 15;
       float m = -CUDART_INF_F;
       if (r < G && p < n_splits) m = p == 0 ? s_M[r] : sParts[((p - 1) * G + r) * PW + DH];
@@ -533,6 +530,7 @@ __global__ void __launch_bounds__(kDaThreads)
       if (r < G) s_pw[r][p] = exp2f(m - ((mx == -CUDART_INF_F) ? 0.f : mx));  // (-inf - 0 -> 0: a part without keys)
     }
     sync_compute();
+    if (*abort_flag) return;  // (some warp's wait gave up)
     for (int i = tid; i < G * (DH / 2); i += 128) {  // a thread per (row, two columns)
       const int r = i / (DH / 2), d = (i % (DH / 2)) * 2;
       float w = s_pw[r][0];

@@ -115,3 +115,17 @@ def test_results_of_a_launch_are_marked_behind_the_wait(name, params, body):
     of it: every such parameter is a constant of the step or is marked."""
     pointers = re.findall(r"\bconst\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params)
     assert [p for p in pointers if p not in CONSTANT | marked(body) | OTHERWISE.get(name, set())] == []
+
+
+@pytest.mark.parametrize("name,body", [pytest.param(n, b, id=n) for n, _, b in KERNELS if re.search(r"auto sync_\w+ = \[&\]\(\) \{ asm", b)])
+def test_a_wait_that_gives_up_leaves_no_barrier_to_the_others(name, body):
+    """Where the warps of a part of the block meet at a barrier of their own, a warp whose bounded wait gave up walks on with them:
+    it leaves neither a loop nor the kernel on its own wait's answer, which the other warps' need not share."""
+    body = body[re.search(r"auto sync_\w+ = \[&\]\(\) \{ asm", body).start():]
+    answers = re.findall(r"\b(\w+) = (?:__all_sync\(0xffffffffu, )?mbar_wait\w*\(", body)
+    failed = r"if \(!(?:mbar_wait\w*\(|" + "|".join(rf"{a}\b" for a in answers + ["wait_all"]) + ")"
+    for m in re.finditer(failed, body):
+        then = closing(body, body.index("(", m.start()), "()") + 1
+        rest = body[then:].lstrip()
+        end = closing(rest, 0) if rest.startswith("{") else rest.index(";")
+        assert not re.search(r"\b(return|break)\b", rest[:end]), body[m.start():then]
