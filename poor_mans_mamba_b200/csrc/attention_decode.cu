@@ -39,6 +39,7 @@
 // another block's result never came) to *status, and the step's results are discarded by the host.
 #include "mma_helpers.cuh"
 #include "tcgen05.cuh"
+#include <atomic>
 #include <math_constants.h>
 
 namespace pmm {
@@ -631,14 +632,11 @@ int launch_decode_attention(const CUtensorMap& map, DecodeAttnArgs a, int n_seq,
   const size_t parts = a.n_splits > 1 ? (da_parts_bytes(DH, G, a.n_splits) + 15) / 16 * 16 : 0;
   a.clustered = a.n_splits > 1 && a.n_splits <= kDaClusterMax && parts <= kDaPartsMax ? 1 : 0;
   const size_t smem = da_smem(DH);  // (the results of a cluster's blocks go into the first block's idle V ring)
-  static bool attrs_set = false;
-  if (!attrs_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    attrs_set = true;
-  }
+  // (attributes hold for the current device: set at every call)
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return static_cast<int>(e);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(n_seq, a.Hkv, a.n_splits);
   cfg.blockDim = dim3(kDaThreads);
@@ -655,15 +653,24 @@ int launch_decode_attention(const CUtensorMap& map, DecodeAttnArgs a, int n_seq,
     attrs[1].val.clusterDim.y = 1;
     attrs[1].val.clusterDim.z = a.n_splits;
     cfg.numAttrs = 2;
-    // a cluster this large may not find room (shared memory, blocks of one GPC): then through the counter
-    static signed char fits[kDaClusterMax + 1] = {};  // per cluster size: 0 not asked yet, 1 fits, -1 does not
-    if (fits[a.n_splits] == 0) {
+    // A cluster this large may not find room (shared memory, blocks of one GPC): then through the counter.  The answers for one
+    // device stay in one word, two bits a cluster size (0 not asked yet, 1 fits, 2 does not) below the device, so that threads never meet half of one.
+    static std::atomic<unsigned long long> seen{0};
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    const unsigned long long device = static_cast<unsigned long long>(dev) << 48;
+    unsigned long long answers = seen.load(std::memory_order_relaxed);
+    if (answers >> 48 != device >> 48) answers = device;
+    unsigned fits = static_cast<unsigned>(answers >> (2 * a.n_splits)) & 3u;
+    if (fits == 0) {
       int n = 0;
       const bool ok = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
       if (!ok) (void)cudaGetLastError();
-      fits[a.n_splits] = ok ? 1 : -1;
+      fits = ok ? 1u : 2u;
+      seen.store(answers | static_cast<unsigned long long>(fits) << (2 * a.n_splits), std::memory_order_relaxed);
     }
-    if (fits[a.n_splits] < 0) {
+    if (fits == 2u) {
       a.clustered = 0;
       cfg.numAttrs = 1;
     }

@@ -743,13 +743,10 @@ PMM_EXPORT int pmm_skinny_chain(const PmmSkinnyPhase* phases, int n_phases, int 
                                 int* status, cudaStream_t stream) {
   if (M <= 0 || n_phases <= 0) return 0;
   if (n_phases > pmm::kChainPhases || M > 16 || !counter || !status) return PMM_ERR_BAD_ARGUMENT;
-  static int n_sm = 0;
-  if (n_sm == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0)
-      return PMM_ERR_BAD_ARGUMENT;
-  }
+  int dev = 0, n_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0)
+    return PMM_ERR_BAD_ARGUMENT;
   pmm::SkinnyChain ch{};
   ch.n_phases = n_phases;
   ch.counter = counter;

@@ -197,6 +197,8 @@ __device__ __forceinline__ void tq_tmem_free(unsigned base, int cols, int warp) 
 // and, for phase 3, delta_j and cs_j log2(e) of the chunk's tokens.
 constexpr int kTState = 512;
 
+__host__ __device__ constexpr size_t tq_state_smem(int nb) { return 1024 + 2 * kTSub + static_cast<size_t>(nb + (nb & 1)) * kTSub; }
+
 __global__ void __launch_bounds__(kTState)
     ssd_tc_state_kernel(const bf16* __restrict__ xbc, int ld_xbc, const bf16* __restrict__ dt_raw, long long ld_dt,
                         float dt_scale, const float* __restrict__ dt_shift, const float* __restrict__ a_log,
@@ -1183,7 +1185,7 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
     return PMM_ERR_BAD_ARGUMENT;
   int tmem_cols = 32;
   while (tmem_cols < N) tmem_cols *= 2;
-  const size_t smem1 = 1024 + 2 * kTSub + static_cast<size_t>(nb + (nb & 1)) * kTSub;
+  const size_t smem1 = tq_state_smem(nb);
   const size_t smem3 = tq_output_smem(nb, PB);
   const int sms = 148;
   // Phase 3: as many units a block as keep the blocks within one an SM
@@ -1219,38 +1221,33 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
       return PMM_ERR_BAD_ARGUMENT;
   }
   if (longest < 0) return PMM_ERR_BAD_ARGUMENT;
-  static size_t set1 = 0, set3 = 0;  // the opt-in to large shared memory, raised when a larger shape comes
-  if (smem1 > set1) {
-    cudaError_t e = cudaFuncSetAttribute(ssd_tc_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem1));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    set1 = smem1;
-  }
-  if (smem3 > set3) {
-    cudaError_t e = cudaFuncSetAttribute(ssd_tc_output_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem3));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ssd_tc_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem3));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    set3 = smem3;
-  }
+  // the opt-in to large shared memory holds for the current device: asked for at every call, always for the largest shape, so
+  // that a call on another device or thread never finds less than it needs
+  auto opt_in = [](const void* kern, size_t most) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
+  };
+  auto output = tma ? ssd_tc_output_kernel<true> : ssd_tc_output_kernel<false>;
+  cudaError_t e = opt_in(reinterpret_cast<const void*>(output), tq_output_smem(4, 64));
+  if (e == cudaSuccess && !walk) e = opt_in(reinterpret_cast<const void*>(ssd_tc_state_kernel), tq_state_smem(4));
+  if (e != cudaSuccess) return static_cast<int>(e);
   const bf16* xb = static_cast<const bf16*>(xbc);
   const bf16* dtb = static_cast<const bf16*>(dt_raw);
   if (walk) {
     auto kern = NB == 64 ? ssd_tc_walk_kernel<64> : ssd_tc_walk_kernel<128>;
     const size_t smem2 = tq_walk_smem(NB);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem2));
+    e = opt_in(reinterpret_cast<const void*>(kern), smem2);
     if (e != cudaSuccess) return static_cast<int>(e);
     launch_pdl(kern, dim3(G * slabs_per_group * (N / NB), n_seq), dim3(kTWalkAll), smem2, stream, map_xbc, map_out, xb, ld_xbc, dtb, ld_dt, dt_scale,
                dt_shift, a_log, cu, slots, state, chunk_dt, static_cast<bf16*>(start_state), H, P, N, G, slabs_per_group, skip_single, status);
   } else {
-  launch_pdl(ssd_tc_state_kernel, dim3(n_chunks, G * slabs_per_group), dim3(kTState), smem1, stream, xb, ld_xbc, dtb, ld_dt,
-             dt_scale, dt_shift, a_log, cu, n_seq, chunk_state, chunk_decay, chunk_dt, H, P, N, G, slabs_per_group, tmem_cols,
-             skip_single, status);
-  int rc = launch_ssd_state_pass(chunk_state, chunk_decay, static_cast<bf16*>(start_state), state, cu, slots, n_seq, H,
-                                 P * N, kTQ, skip_single, n_multi, stream);
-  if (rc != 0) return rc;
+    launch_pdl(ssd_tc_state_kernel, dim3(n_chunks, G * slabs_per_group), dim3(kTState), smem1, stream, xb, ld_xbc, dtb, ld_dt,
+               dt_scale, dt_shift, a_log, cu, n_seq, chunk_state, chunk_decay, chunk_dt, H, P, N, G, slabs_per_group, tmem_cols,
+               skip_single, status);
+    int rc = launch_ssd_state_pass(chunk_state, chunk_decay, static_cast<bf16*>(start_state), state, cu, slots, n_seq, H,
+                                   P * N, kTQ, skip_single, n_multi, stream);
+    if (rc != 0) return rc;
   }
-  launch_pdl(tma ? ssd_tc_output_kernel<true> : ssd_tc_output_kernel<false>, dim3(n_chunks, G * group_blocks), dim3(kTOutAll), smem3,
-             stream, map_xbc, map_start, map_z, xb, ld_xbc,
+  launch_pdl(output, dim3(n_chunks, G * group_blocks), dim3(kTOutAll), smem3, stream, map_xbc, map_start, map_z, xb, ld_xbc,
              static_cast<const float*>(chunk_dt), d_skip, cu, n_seq, static_cast<const bf16*>(start_state),
              static_cast<bf16*>(y), H, P, N, G, PB, per_block, static_cast<const bf16*>(z_raw), ld_z, z_scale, z_bias, z_vec, skip_single, status);
   return launch_status();

@@ -129,3 +129,11 @@ def test_a_wait_that_gives_up_leaves_no_barrier_to_the_others(name, body):
         rest = body[then:].lstrip()
         end = closing(rest, 0) if rest.startswith("{") else rest.index(";")
         assert not re.search(r"\b(return|break)\b", rest[:end]), body[m.start():then]
+
+
+def test_no_state_of_a_launcher_outlives_a_call():
+    """Attributes, residency and SM counts belong to the current device, and calls come from several threads: what a launcher keeps
+    for the calls after it is one atomic word that names its device, or the address of a driver function."""
+    for path in sorted(glob.glob(os.path.join(CSRC_DIR, "*.cu*"))):
+        for line in re.findall(r"^\s*static\s+[^;({]*[;={\[]", source(path), flags=re.M):
+            assert re.search(r"static (constexpr|std::atomic<|EncodeTiledFn )", line), f"{os.path.basename(path)}: {line.strip()}"
