@@ -1744,15 +1744,17 @@ def attention_tc_supported(n_q_heads: int, n_kv_heads: int, head_dim: int, page_
     return bool(_fn("pmm_attention_tc_supported")(n_q_heads, n_kv_heads, head_dim, page_size))
 
 
-def attention_tc_rows(n_q_heads: int, n_kv_heads: int, head_dim: int, new_lens: Sequence[int]) -> int:
-    """Query rows of a block of `attention_tc`: 64 while blocks of 64 rows all run at once (148 SMs, two blocks an SM at head
-    size 64, one at 128) and the group divides them, else 128, which reads keys and values half as often.  Measured, us, 64 /
-    128 rows: 8 query and 2 key/value heads of 64, 2,048 tokens 21.3 / 28.5, 300 tokens 6.7 / 8.9; 16 and 4 heads 33.7 / 31.2;
-    8,192 tokens 167 / 152; 12 and 2 heads of 128, 1,024 tokens 18.4 / 17.8, 2,048 tokens 46.7 / 30.0."""
+def attention_tc_rows(n_q_heads: int, n_kv_heads: int, head_dim: int, new_lens: Sequence[int], n_splits: int = 1) -> int:
+    """Query rows of a block of `attention_tc`: 64 while blocks of 64 rows, one for each of `n_splits` key ranges, all run at
+    once (148 SMs, two blocks an SM at head size 64, one at 128) and the group divides them, else 128, which reads keys and
+    values half as often.  Measured, us, 64 / 128 rows: 8 query and 2 key/value heads of 64, 2,048 tokens 21.3 / 28.5, 300
+    tokens 6.7 / 8.9; 16 and 4 heads 33.7 / 31.2; 8,192 tokens 167 / 152; 12 and 2 heads of 128, 1,024 tokens 18.4 / 17.8,
+    2,048 tokens 46.7 / 30.0.  Behind a context, 8 and 2 heads: 64 tokens behind 4,000 in 16 ranges 31.6 / 39.8 at 128, 512
+    behind 15,000 in 4 ranges 101 / 71 at 128 and 57 / 62 at 64; 32 and 8 heads of 128, 256 behind 15,000 166 / 117."""
     group = n_q_heads // n_kv_heads
     if 64 % group:
         return 128
-    blocks = sum((n * group + 63) // 64 for n in new_lens) * n_kv_heads
+    blocks = sum((n * group + 63) // 64 for n in new_lens) * n_kv_heads * n_splits
     return 64 if blocks <= 148 * (2 if head_dim == 64 else 1) else 128
 
 
@@ -1786,7 +1788,7 @@ def attention_tc(q: Tensor, pool: Tensor, block_table: Tensor, positions: Tensor
     group = n_q_heads // n_kv_heads
     tiles_of = lambda r: sum((n + r // group - 1) // (r // group) for n in new_lens)
     if rows is None:
-        rows = attention_tc_rows(n_q_heads, n_kv_heads, head_dim, new_lens)
+        rows = attention_tc_rows(n_q_heads, n_kv_heads, head_dim, new_lens, n_splits)
         if n_splits > 1 and split_counter is not None and split_counter.numel() < tiles_of(rows) * n_kv_heads:
             rows = 128
     if rows not in (64, 128):

@@ -39,3 +39,17 @@ def test_prompt_ranges():
     n, length = a.plan_splits_tc([256], 8192)                         # few rows, long context: cut the keys
     assert n > 1 and length % 64 == 0 and n * length >= 8192
     assert a.plan_splits([8192], 8192, torch.bfloat16) == (1, 0)
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (16, 4, 64), (8, 2, 128), (16, 2, 128), (32, 8, 128)])
+@pytest.mark.parametrize("tokens", [64, 100, 256, 512, 1024])
+@pytest.mark.parametrize("past", [0, 1000, 4000, 15000])
+def test_low_blocks_of_prompt_attention_run_at_once(heads, kv_heads, head_dim, tokens, past):
+    """Blocks of 64 rows only where all of them, those of every key range, are resident: a second wave of them reads keys and
+    values twice as often as blocks of 128 rows for nothing."""
+    from poor_mans_mamba_b200.kernels import ops as K
+    from poor_mans_mamba_b200.parts.attention import plan_key_splits_tc
+    n, _ = plan_key_splits_tc(heads, kv_heads, 0, [tokens], 1 << (tokens + past - 1).bit_length())
+    rows = K.attention_tc_rows(heads, kv_heads, head_dim, [tokens], n)
+    blocks = -(-tokens * heads // kv_heads // 64) * kv_heads * n
+    assert rows == (64 if blocks <= 148 * (2 if head_dim == 64 else 1) else 128)
