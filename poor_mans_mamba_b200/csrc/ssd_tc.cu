@@ -7,7 +7,7 @@
 // the chunk and S the state at the chunk's start:
 //   y_i   = sum_{j<=i} (C_i.B_j) exp(cs_i-cs_j) delta_j x_j  +  exp(cs_i) (C_i . S)  +  D x_i
 //   S_end = exp(cs_last) S  +  sum_j exp(cs_last-cs_j) delta_j x_j B_j^T
-// Three launches, or two (1 and 2 as one walk, ssd_tc_walk, where that is shorter):
+// Three launches, or two (1 and 2 as one walk, ssd_tc_walk_kernel, where the caller asks for it):
 //   1. ssd_tc_state:   one block per (chunk, 128 channels of x): the local term of S_end as ONE
 //                      product  D[channel, n] = sum_j (w_j x_j[channel]) B_j[n].  Both operands are
 //                      the chunk's rows as they lie in memory (tokens = the K dimension, so both
@@ -1159,7 +1159,8 @@ PMM_EXPORT int pmm_ssd_tc_supported(int P, int N) {
 // n_chunks*H*256 floats, start_state n_chunks*H*P*N bfloat16 (16-byte aligned); n_chunks = sum over
 // sequences of ceil(new tokens / 128).
 // z_raw (or nullptr): the gate's input [T, ld_z], y <- y * silu(z_raw * z_scale + z_bias).
-// n_tokens: rows of xbc (and z_raw); longest: about the tokens of the longest sequence (a choice of form hangs on it, not a result).
+// n_tokens: rows of xbc (and z_raw).  walk_cols: 0 for phases 1 and 2 as two launches, 64 or 128 for the walk with blocks of so
+// many state columns (N a multiple of them).
 // skip_single: sequences that bring exactly one token are left alone (state and y): in a mixed step
 // the token-serial kernel takes them (pmm_ssm_scan_seq with one_token = 2); n_multi is then the
 // number of sequences that bring more than one token (0: not known).
@@ -1167,7 +1168,7 @@ PMM_EXPORT int pmm_ssd_tc_supported(int P, int N) {
 PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long long ld_dt, float dt_scale,
                           const float* dt_shift, const float* a_log, const float* d_skip, float* state, const int* cu,
                           const int* slots, void* y, float* chunk_state, float* chunk_decay, float* chunk_dt,
-                          void* start_state, int n_seq, int n_tokens, int longest, int n_chunks, int H, int P, int N, int G, const void* z_raw,
+                          void* start_state, int n_seq, int n_tokens, int walk_cols, int n_chunks, int H, int P, int N, int G, const void* z_raw,
                           long long ld_z, float z_scale, const float* z_bias, int skip_single, int n_multi, int* status,
                           cudaStream_t stream) {
   using namespace pmm;
@@ -1194,15 +1195,9 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
   const int group_blocks = (group_units + per_block - 1) / per_block;
   // Whole tiles of 64 columns come by TMA: a unit's copies took its 512 threads 2,800 clocks of issue, of about 7,500.
   const bool tiles64 = N % 64 == 0 && n_tokens > 0, tma = PB == 64 && tiles64;
-  // Phases 1 and 2 in one walk where its blocks all run at once and it is the shorter one: a walk takes a chunk after the other,
-  // the two launches write and read the local terms.  Measured, us: 24 heads of 64 x 128, walk / both: one chunk 9.0 / 10.3 and a launch's
-  // latency, 5 sequences of up to 3 chunks 12.4 / 18.8, one sequence of 4 chunks 13.2 / 11.3 (the whole chain 21.0 / 20.7), of 16 chunks 33 /
-  // 20; 48 heads of 128 x 256, 8 chunks 29 / 53.
-  const int walkers = (n_multi > 0 && skip_single ? n_multi : n_seq) * G * slabs_per_group;
-  const int NB = walkers * (N / 64) <= sms ? 64 : N % 128 == 0 && walkers * (N / 128) <= sms ? 128 : 0;
-  const double walk_us = NB == 64 ? 7.6 + 1.45 * ((longest + kTQ - 1) / kTQ) : 9.0 + 2.5 * ((longest + kTQ - 1) / kTQ);
-  const double both_us = 11.0 + 0.88e-6 * 4.0 * n_chunks * H * P * N;
-  const bool walk = tiles64 && NB > 0 && walk_us < both_us;
+  const int NB = walk_cols;
+  const bool walk = NB > 0;
+  if (walk && ((NB != 64 && NB != 128) || !tiles64 || N % NB)) return PMM_ERR_BAD_ARGUMENT;
   CUtensorMap map_xbc{}, map_start{}, map_z{}, map_out{};
   if (tma || walk) {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -1220,7 +1215,6 @@ PMM_EXPORT int pmm_ssd_tc(const void* xbc, int ld_xbc, const void* dt_raw, long 
         (tma && z_vec && !tiles_of(&map_z, z_raw, I, n_tokens, ld_z, kTQ)))
       return PMM_ERR_BAD_ARGUMENT;
   }
-  if (longest < 0) return PMM_ERR_BAD_ARGUMENT;
   // the opt-in to large shared memory holds for the current device: asked for at every call, always for the largest shape, so
   // that a call on another device or thread never finds less than it needs
   auto opt_in = [](const void* kern, size_t most) {

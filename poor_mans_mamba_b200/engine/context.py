@@ -20,13 +20,17 @@ class LengthBounds(list):
     of more than one token.  The true lengths are in ``cu_seqlens`` on the device and some of them
     may be zero (a cut with empty sequences needs no more blocks than one without: the bound
     floor((total - k) / c) + k does not fall as k grows); only parts that say
-    `accepts_length_bounds` are ever given this."""
+    `accepts_length_bounds` are ever given this.  ``at_hand``: the true lengths of the step that it
+    was made for (None: not told).  No launch may be sized by them; a choice between forms that all
+    serve every cut may hang on them where the mixer names it (`Mixer.length_choice`), which puts it
+    into the recording's key."""
 
-    def __init__(self, total: int, count: int):
+    def __init__(self, total: int, count: int, at_hand: Optional[List[int]] = None):
         if count < 2 or total < count:
             raise ValueError("length bounds need at least two sequences and a token for each")
         super().__init__([total - (count - 1)] + [1] * (count - 1))
         self.multi = count
+        self.at_hand = at_hand
 
 
 @dataclass

@@ -36,6 +36,7 @@ class Model:
         self.layers = []
         self._fetch_ahead = os.environ.get("PMM_FETCH_AHEAD", "1") == "1"
         self._fetch_lists: Dict[int, tuple] = {}
+        self._length_choices: Optional[list] = None
         for ls in spec.layers:
             factory = _REGISTRIES["arrangement"].get(ls.arrangement)
             if factory is None:
@@ -199,6 +200,13 @@ class Model:
         Mixer.accepts_length_bounds); an arrangement that does not say so does not."""
         return self.dtype is not None and all(
             getattr(layer, "accepts_length_bounds", lambda d, p: False)(self.dtype, page_size) for layer in self.layers)
+
+    def length_choices(self, new_lens) -> tuple:
+        """Which forms the mixers' launches take for these lengths (see Mixer.length_choice), asked once for mixers of equal sizes."""
+        if self._length_choices is None:
+            self._length_choices = list(dict.fromkeys(
+                c for layer in self.layers for c in getattr(layer, "length_choices", list)() if c is not None))
+        return tuple(choice(new_lens, *sizes) for choice, *sizes in self._length_choices)
 
     @staticmethod
     def _join(ctx: StepContext, device) -> None:

@@ -234,7 +234,8 @@ class ModelRunner:
         sees the padded batch with `LengthBounds` in place of the tokens per sequence, so every
         launch has the shape the key gives it and the recording serves every cut of the real
         tokens; the real rows' results are what they are without the padding (rows and sequences do
-        not mix)."""
+        not mix).  (Where a mixer's launches take one of several forms by the lengths at hand, `step`
+        adds the forms to the key.)"""
         T, n_seq = sum(new_lens), len(new_lens)
         if T < _STEP_GRAPH_SMALL_FROM or max(new_lens) == 1 or not _ROUNDED_STEP_GRAPHS:
             return None
@@ -419,13 +420,19 @@ class ModelRunner:
         # fixed chunk size) gets a recording of its own the third time: it saves the padding.
         large = rounded is not None or T >= _STEP_GRAPH_MIN_TOKENS  # rounded shapes have at least that many tokens
         shapes = self._step_graphs if large else self._small_step_graphs
-        key, padded, record = self._choose_form(shapes, exact_key, rounded[0] if rounded is not None else None)
+        rounded_key = None
+        if rounded is not None:
+            rounded_key, pad_lens, rows_b, kv_b = rounded
+            lens_g = LengthBounds(T + sum(pad_lens), len(new_lens) + len(pad_lens), new_lens + pad_lens)
+            # the forms that its mixers' launches take are part of the shape: those that it came with first go unmarked
+            forms = self.model.length_choices(lens_g)
+            if self._shape_seen.setdefault(("forms",) + rounded_key, forms) != forms:
+                rounded_key += forms
+        key, padded, record = self._choose_form(shapes, exact_key, rounded_key)
         if padded:
-            _, pad_lens, rows_b, kv_b = rounded
             spare = cache.spare_slot
             seqs_g = seqs + [(np.zeros(n, dtype=np.int32), 0, spare, None) for n in pad_lens]
             rows_g = rows + rows[:1] * (rows_b - n_rows)
-            lens_g = LengthBounds(T + sum(pad_lens), len(seqs_g))
             total, fill, context = self._layout(seqs_g, rows_g, groups, widths, kv_b, lens_g)
         else:
             total, fill, context = self._layout(seqs, rows, groups, widths, kv_len, new_lens)

@@ -877,13 +877,39 @@ def ssd_tc_scratch_floats(new_lens: Sequence[int], n_heads: int, d_head: int, d_
             + ((per_state + 1) // 2 + 3) // 4 * 4)
 
 
+def ssd_tc_walk_columns(new_lens: Sequence[int], n_heads: int, d_head: int, d_state: int, n_groups: int,
+                        skip_single: bool = False) -> int:
+    """The form of `ssm_scan_tc` for these lengths: 0 for local terms and state pass as two launches, else the state columns (64
+    or 128) of a block of the walk that does both.
+
+    A walk takes the longest sequence chunk by chunk; the two launches write and read every chunk's local terms, and cost the more
+    the more sequences there are to look through, empty ones too.  The walk is taken where all its blocks run at once and it is
+    the shorter by two straight lines, in us, fitted to the whole scan (walk / two launches).  24 heads of 64 x 128: one sequence
+    of 1, 3, 4, 6, 16 chunks 12.6 / 15.4, 15.4 / 16.2, 16.6 / 16.4, 21.0 / 16.9, 41.5 / 30.0; five of up to 3 chunks 23.9 / 34.5;
+    1,000 tokens beside three sequences of 60 27.0 / 24.2; given as bounds of 8 sequences, 1,536 tokens, all in one 38.7 / 36.5,
+    in two halves 29.5 / 36.9; of 32 sequences, 2,048 in one 55.8 / 69.8.  40 heads of 64 x 256: 4 and 16 chunks 21.7 / 25.6, 51.0
+    / 54.1.  48 of 128 x 256 (128 columns): 1, 8, 16 chunks 20.1 / 26.8, 48.0 / 62.5, 78.0 / 112.  Of 398 timed cases the lines
+    miss ten, by 0.5 to 2.5 us."""
+    slabs = n_groups * -(-(n_heads // n_groups * d_head) // 128)
+    lens = getattr(new_lens, "at_hand", None) or new_lens   # (bounds that are not told of a step: their one long sequence)
+    taken = [n for n in lens if n > (1 if skip_single else 0)]
+    cols = next((c for c in (64, 128) if d_state % c == 0 and 0 < len(taken) * slabs * (d_state // c) <= 148), 0)
+    if cols == 0:
+        return 0
+    steps, chunks = -(-max(taken) // SSD_TC_CHUNK), sum(-(-n // SSD_TC_CHUNK) for n in taken)
+    walk_us = 7.6 + 1.45 * steps if cols == 64 else 9.0 + 2.5 * steps
+    both_us = 7.2 + 0.8 * len(new_lens) + 0.025 * d_state + 0.45e-6 * 4 * chunks * n_heads * d_head * d_state
+    return cols if walk_us < both_us else 0
+
+
 def ssm_scan_tc(xbc: Tensor, dt_raw: Tensor, dt_scale: float, dt_shift: Tensor, a_log: Tensor, d_skip: Tensor,
                 state: Tensor, cu: Tensor, slots: Tensor, new_lens: Sequence[int], out: Tensor, n_groups: int,
-                scratch: Tensor, gate=None, skip_single: bool = False) -> None:
+                scratch: Tensor, gate=None, skip_single: bool = False, walk_cols: Optional[int] = None) -> None:
     """The Mamba2 recurrence over prompt portions in chunks of 128 tokens on the tcgen05 tensor
     cores (bfloat16 activations); same contract as ssm_scan_seq.  ``scratch``: float32, at least
     ssd_tc_scratch_floats(...) elements.  ``skip_single``: sequences that bring exactly one token are
-    left alone (their rows of ``out`` and their states): ssm_scan_seq(only_single=True) takes them."""
+    left alone (their rows of ``out`` and their states): ssm_scan_seq(only_single=True) takes them.
+    ``walk_cols``: the form, 0, 64 or 128 (None: `ssd_tc_walk_columns`)."""
     _cuda(xbc, dt_raw, dt_shift, a_log, d_skip, state, cu, slots, out, scratch)
     if not (state.dtype == torch.float32 and state.dim() == 4 and state.is_contiguous()):
         raise KernelError("ssm_scan: state must be contiguous float32 [slots, H, P, N]")
@@ -915,12 +941,13 @@ def ssm_scan_tc(xbc: Tensor, dt_raw: Tensor, dt_scale: float, dt_shift: Tensor, 
     n_multi = getattr(new_lens, "multi", None)  # lengths given as bounds carry the bound with them
     if n_multi is None:
         n_multi = sum(1 for n in new_lens if n > 1)
-        longest = max(new_lens, default=0)
-    else:  # half as long again as the lengths' mean
-        longest = -(-3 * sum(new_lens) // (2 * max(n_multi, 1)))
+    if walk_cols is None:
+        walk_cols = ssd_tc_walk_columns(new_lens, H, P, N, n_groups, skip_single)
+    if walk_cols and not (walk_cols in (64, 128) and N % walk_cols == 0):
+        raise KernelError(f"ssm_scan_tc: a block of the walk takes 64 or 128 state columns that divide {N}, got {walk_cols}")
     _call("pmm_ssd_tc", xbc.data_ptr(), ld_x, dt_raw.data_ptr(), ld_dt, float(dt_scale), dt_shift.data_ptr(),
           a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), cu.data_ptr(), slots.data_ptr(), out.data_ptr(),
-          chunk_state, chunk_decay, chunk_dt, start_state, len(new_lens), xbc.shape[0], longest, n_chunks, H, P, N, n_groups, zp, ld_z, zs, zb,
+          chunk_state, chunk_decay, chunk_dt, start_state, len(new_lens), xbc.shape[0], int(walk_cols), n_chunks, H, P, N, n_groups, zp, ld_z, zs, zb,
           int(bool(skip_single)), n_multi if skip_single else 0,
           _tc_status(xbc.device).data_ptr(), _stream())
 

@@ -234,6 +234,12 @@ class Mixer(Part):
         rounded shapes are then recorded once and replayed whatever the cut (see ModelRunner)."""
         return False
 
+    def length_choice(self) -> Optional[tuple]:
+        """(function, its further arguments): function(new_lens, *arguments) is which of several forms this mixer's launches take
+        for the lengths at hand, those of a `LengthBounds` among them; None: no form hangs on them.  A step recorded under a
+        rounded shape is replayed only for steps of the same choices."""
+        return None
+
 
 class FeedForward(Part):
     """forward(x, ctx, out): x [T, D] normalised activations, out [T, D]."""

@@ -419,6 +419,10 @@ class ParallelPreNormBlock(Part):
         """See Mixer.accepts_length_bounds: norms and feed-forwards go row by row, the mixers decide."""
         return not self._input_maps() and all(m.accepts_length_bounds(dtype, page_size) for m in self.mixers)
 
+    def length_choices(self) -> List[Optional[tuple]]:
+        """See Mixer.length_choice."""
+        return [m.length_choice() for m in self.mixers]
+
     def joins_side_stream(self, ctx) -> bool:
         """Whether this layer may start while ``ctx.unjoined_stream`` still works (a weight fetch that
         an earlier layer of the same kind left running: nothing this layer does depends on it)."""

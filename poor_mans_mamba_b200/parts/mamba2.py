@@ -192,6 +192,10 @@ class Mamba2Mixer(Mixer):
         # leave when there is none; the convolution and the lone tokens' scan go by token or sequence
         return _TC_SCAN and dtype == torch.bfloat16 and K.ssd_tc_supported(self.d_head, self.d_state)
 
+    def length_choice(self) -> Optional[tuple]:
+        # (lengths given as bounds hold sequences of one token: those are left to the lone tokens' scan)
+        return K.ssd_tc_walk_columns, self.n_heads, self.d_head, self.d_state, self.n_groups, True
+
     def pre_output(self, proj: Tensor, ctx, cache, into: Optional[Tensor] = None, scale: float = 1.0) -> Tensor:
         """``into``/``scale`` (gated norm only): the result times ``scale`` goes into that column block."""
         T = proj.shape[0]
@@ -234,7 +238,7 @@ class Mamba2Mixer(Mixer):
             if lone:
                 # The two scans touch different sequences (their states, their rows of y).  The lone
                 # tokens' scan is a read and write of their states at the memory's rate, the chunked one
-                # a chain of three tensor-core launches: they run side by side (parallel branches of a
+                # a chain of two or three tensor-core launches: they run side by side (parallel branches of a
                 # captured step).
                 side = branches.branch_stream(xbc.device, "lone")
                 with branches.fork(here, side):

@@ -306,6 +306,48 @@ def test_ssd_tcgen05_scan_keeps_to_its_rows(H, Pd, N, G, lens):
         assert torch.equal(got[other], got[0.0]) and torch.equal(states[other], states[0.0])
 
 
+@pytest.mark.parametrize("H,Pd,N,G,lens", [(24, 64, 128, 1, [300, 1, 129, 90]), (5, 48, 64, 1, [257, 128, 40]), (40, 64, 256, 1, [500, 2]),
+                                           (16, 16, 128, 2, [130, 1, 127])])
+def test_ssd_tcgen05_scan_forms(H, Pd, N, G, lens):
+    """Local terms and state pass as two launches and as a walk, whichever a step's lengths would choose: near the serial kernel, the
+    same bits with exact lengths and with bounds (a sequence more, empty), lone tokens taken or left alone."""
+    from poor_mans_mamba_b200.engine.context import LengthBounds
+    dtype, T, I = torch.bfloat16, sum(lens), H * Pd
+    g = torch.Generator().manual_seed(H + Pd + N)
+    xbc, z = (q(torch.randn(T, w, generator=g), dtype).to(DEV) for w in (I + 2 * G * N, I))
+    dt = q(torch.randn(T, H, generator=g), dtype).to(DEV)
+    a_log, d_skip, shift = (v.to(DEV) for v in (torch.rand(H, generator=g) * 2, torch.randn(H, generator=g), torch.randn(H, generator=g) - 3.0))
+    start = torch.randn(len(lens) + 1, H, Pd, N, generator=g)
+    cu, slots = i32([0] + torch.tensor(lens + [0]).cumsum(0).tolist()), i32(list(range(len(lens) + 1)))
+    want, ref = start.clone().to(DEV), torch.empty(T, I, dtype=dtype, device=DEV)
+    K().ssm_scan_seq(xbc, dt, 1.0, shift, a_log, d_skip, want, cu, slots, len(lens), ref, G, gate=(z, 1.0, None))
+    lone = [i for i, n in enumerate(lens) if n == 1]
+    rows = torch.ones(T, dtype=torch.bool)
+    for i in lone:
+        rows[int(cu[i])] = False
+    first = {}
+    for cols in [c for c in (0, 64, 128) if c == 0 or N % c == 0]:
+        for new_lens in (lens, LengthBounds(T, len(lens) + 1)):
+            for skip in (False, True):
+                state, out = start.clone().to(DEV), torch.full((T, I), 7.0, dtype=dtype, device=DEV)
+                scratch = torch.full((K().ssd_tc_scratch_floats(new_lens, H, Pd, N),), float("nan"), device=DEV)
+                K().ssm_scan_tc(xbc, dt, 1.0, shift, a_log, d_skip, state, cu, slots, new_lens, out, G, scratch, gate=(z, 1.0, None),
+                                skip_single=skip, walk_cols=cols)
+                assert K().tc_gemm_status(DEV) == 0
+                out, state = out.cpu(), state.cpu()
+                assert torch.equal(state[len(lens)], start[len(lens)])
+                if skip:
+                    assert torch.equal(state[lone], start[lone]) and bool((out[~rows] == 7.0).all())
+                    state[lone], out[~rows] = want.cpu()[lone], ref.cpu()[~rows]
+                close(out, ref, dtype, what=f"outputs, {cols} columns")
+                close(state, want, dtype, what=f"states, {cols} columns")
+                if skip not in first:
+                    first[skip] = (out, state)
+                assert torch.equal(out, first[skip][0]) and torch.equal(state, first[skip][1]), (cols, type(new_lens), skip)
+    with pytest.raises(K().KernelError):
+        K().ssm_scan_tc(xbc, dt, 1.0, shift, a_log, d_skip, want, cu, slots, lens, ref, G, scratch, walk_cols=N + 64)
+
+
 def test_ssd_tcgen05_scan_refuses_other_sizes():
     assert not K().ssd_tc_supported(20, 24) and not K().ssd_tc_supported(64, 272) and not K().ssd_tc_supported(144, 64)
     assert K().ssd_tc_supported(112, 16)
