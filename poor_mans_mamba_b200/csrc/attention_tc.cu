@@ -658,18 +658,20 @@ __global__ void __launch_bounds__(at_threads(M), DH == 64 ? 2 : 1)
 }  // namespace pmm
 
 // Whether the tcgen05 attention takes this shape: head size 64 or 128, up to 64 query heads per
-// key/value head (a tile holds floor(128 / group) tokens; with a group size that does not divide
-// 128 its last rows stay empty), pages that hold whole boxes of 64 keys.
+// key/value head (a tile of `rows` rows, 64 or 128, holds floor(rows / group) tokens; with a group
+// size that does not divide them its last rows stay empty), pages that hold whole boxes of 64 keys.
 PMM_EXPORT int pmm_attention_tc_supported(int Hq, int Hkv, int Dh, int page_size) {
   if (Hkv <= 0 || Hq % Hkv) return 0;
   const int G = Hq / Hkv;
   return ((Dh == 64 || Dh == 128) && G <= 64 && page_size > 0 && page_size % pmm::kAtBox == 0) ? 1 : 0;
 }
 
-// q [T, Hq*64] rotated queries; pool [n_pages + spare, 2, page_size, Hkv*64]; n_tiles = sum over
-// sequences of ceil(new tokens / (128 / G)).  Several key splits need part_o / part_ml and
-// split_counter (n_tiles * Hkv ints, zero between calls; at most 64 splits, split_len a multiple
-// of 64).  status: one int, stays 0 unless a bounded wait gave up.
+// q [T, Hq*Dh] rotated queries; pool [n_pages + spare, 2, page_size, Hkv*Dh]; rows: 64 or 128 (token,
+// query head of a group) rows a block; n_tiles = sum over sequences of ceil(new tokens / floor(rows /
+// G)), or more (surplus blocks leave).  Several key splits need part_o / part_ml and split_counter
+// (n_tiles * Hkv ints, zero between calls; at most 64 splits, split_len a multiple of 64).  positions,
+// cu and block_table are read ahead of the wait: see launch_pdl.  status: one int, stays 0 unless a
+// bounded wait gave up.
 PMM_EXPORT int pmm_attention_tc(const void* q, const void* pool, long long pool_pages, const int* block_table,
                                 int max_blocks, const int* positions, const int* cu, void* out, float* part_o,
                                 float* part_ml, float scale, int window, int split_len, int n_splits, int page_size,

@@ -128,8 +128,12 @@ inline int launch_status() { return static_cast<int>(cudaGetLastError()); }
 
 // Programmatic dependent launch.  A kernel started with launch_pdl may begin while the kernel
 // before it on the stream is still running; pdl_wait() inside it returns once that kernel has
-// finished and its writes are visible, so everything a kernel does before pdl_wait() must not
-// touch memory that other kernels write (reading constant weights is fine).
+// finished and its writes are visible, so what a kernel reads before pdl_wait() must not be another
+// kernel's result: weights, and the step's inputs (positions, sequence bounds, slots, block tables),
+// which a copy brings before the step's first launch.  One exception: results that were finished
+// before the launch before this one passed its own wait, where that launch lets this one go behind
+// that wait (ssd_tc_output_kernel reads the convolution's rows so, never what the launch directly
+// before it writes).
 // pdl_launch_dependents() lets the next kernel of the stream start its own preamble early.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -5,6 +5,12 @@ that is not on a CUDA device, a size a kernel cannot take, or a missing library 
 Matrix products go to the library (cuBLAS through ``torch.mm``), as the reference sends
 its linear layers to ``cublasSgemm`` (src/ops/gpu/linear.cu:3-21); in float32 the
 reduced-precision matrix mode is switched off for the call.
+
+What is not a tensor of activations must be there before the launch ahead of a call starts: kernels
+begin while the launch before them on the stream is still running, and weights, positions, sequence
+bounds (``cu``), ``seq_of``, ``slots``, block tables, rows and tokens are read before they wait for
+it.  A copy, any torch operation or a step's upload ahead of its first launch is in time; a kernel of
+this library that wrote them directly before the call would not be (none does).
 """
 from __future__ import annotations
 
@@ -699,6 +705,7 @@ def conv1d_fwd(x: Tensor, pre_scale: Tensor, pre_bias: Optional[Tensor], weight:
                bias: Optional[Tensor], window: Tensor, seq_of: Tensor, cu: Tensor, slots: Tensor,
                out: Tensor, weight_t: Optional[Tensor] = None, activation: bool = True) -> None:
     """Causal depthwise conv + SiLU (``activation`` False: the conv alone) over all tokens of the step; reads the windows.
+    Constants, ``seq_of`` and ``cu`` are read early (see the module's head).
     ``weight_t`` is the tap-major copy [K, C] of ``weight`` [C, K]; with it bfloat16 inputs take
     the vector kernel."""
     _cuda(x, pre_scale, pre_bias, weight, bias, window, seq_of, cu, slots, out, weight_t)
@@ -734,7 +741,7 @@ def conv1d_decode(x: Tensor, pre_scale: Tensor, pre_bias: Optional[Tensor], weig
                   bias: Optional[Tensor], window: Tensor, slots: Tensor, out: Tensor,
                   activation: bool = True) -> None:
     """Conv + SiLU (``activation`` False: the conv alone) + window shift for a step in which every
-    sequence brings one token."""
+    sequence brings one token.  Constants and ``slots`` are read early (see the module's head)."""
     _cuda(x, pre_scale, pre_bias, weight, bias, window, slots, out)
     ld = _rows_view(x, "conv1d: x")
     n_seq = x.shape[0]
@@ -909,7 +916,8 @@ def ssm_scan_tc(xbc: Tensor, dt_raw: Tensor, dt_scale: float, dt_shift: Tensor, 
     cores (bfloat16 activations); same contract as ssm_scan_seq.  ``scratch``: float32, at least
     ssd_tc_scratch_floats(...) elements.  ``skip_single``: sequences that bring exactly one token are
     left alone (their rows of ``out`` and their states): ssm_scan_seq(only_single=True) takes them.
-    ``walk_cols``: the form, 0, 64 or 128 (None: `ssd_tc_walk_columns`)."""
+    ``walk_cols``: the form, 0, 64 or 128 (None: `ssd_tc_walk_columns`).  ``cu`` and ``slots`` are read early (see the module's
+    head)."""
     _cuda(xbc, dt_raw, dt_shift, a_log, d_skip, state, cu, slots, out, scratch)
     if not (state.dtype == torch.float32 and state.dim() == 4 and state.is_contiguous()):
         raise KernelError("ssm_scan: state must be contiguous float32 [slots, H, P, N]")
@@ -1795,7 +1803,8 @@ def attention_tc(q: Tensor, pool: Tensor, block_table: Tensor, positions: Tensor
     (TMA tiles straight from the pages, scores and P V in tensor memory, four threads per two query
     rows for the softmax).  Same contract as paged_attention with rotated queries and a cache that holds
     the step's keys already; 64 or 128 ``rows`` of (token, query head of a group) per block (None: `attention_tc_rows`).
-    ``keep_first`` > 0 behind a window: one key split, ``lse`` scratch and ``seq_of``, as in paged_attention."""
+    ``keep_first`` > 0 behind a window: one key split, ``lse`` scratch and ``seq_of``, as in paged_attention.
+    ``positions``, ``cu_seqlens`` and ``block_table`` are read early (see the module's head)."""
     _cuda(q, pool, block_table, positions, cu_seqlens, out, scratch, split_counter)
     T = q.shape[0]
     keep = int(keep_first) if window > 0 else 0
