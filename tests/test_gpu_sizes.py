@@ -191,3 +191,25 @@ def test_steps_of_33_to_64_tokens_take_the_tcgen05_products(h64, monkeypatch):
         H.check_rows(out[i], ref, "bfloat16", f"h64 steps of 33..64 tokens seq {i}")
     assert K.tc_gemm_status("cuda:0") == 0
     assert calls["swiglu"] == 5 * 2 and calls["residual"] == 5 * 2 * 2  # five such steps, two layers
+
+
+def test_rounded_steps_are_recorded_for_each_form_of_the_scan(h64):
+    """One long portion beside short ones and three portions of a third, the same rounded shape: the first takes the scan's two
+    launches, the second its walk, each from a recording of its own; every wanted row against the plain implementation."""
+    from poor_mans_mamba_b200.engine import StepEntry
+    d, seqs, refs = h64
+    runner = H.make_runner(d, "bfloat16", page_size=64, num_pages=40, num_slots=4)
+    runner.enable_graphs(max_seq_len=1024)
+    for rnd in range(5):
+        for what, cut in (("long", ((0, 690 - rnd), (0, 30 + rnd), (0, 48))), ("thirds", ((444, 256 - rnd), (0, 256), (0, 256 + rnd)))):
+            ids = [(what, i, rnd) for i in range(3)]
+            if cut[0][0]:
+                runner.step([StepEntry(ids[0], seqs[0][:cut[0][0]], [])])
+            logits = runner.step([StepEntry(r, s[p:p + n], [n - 1]) for r, s, (p, n) in zip(ids, seqs, cut)]).float().cpu()
+            for i, (p, n) in enumerate(cut):
+                H.check_rows(logits[i:i + 1], refs[i][p + n - 1:p + n], "bfloat16", f"{what} round {rnd} request {i}")
+            for r in ids:
+                runner.finish(r)
+    runner.check_kernels(wait=True)
+    shape = ("rounded", 768, 4, 4, 1024)
+    assert shape in runner._step_graphs and shape + (64,) in runner._step_graphs, list(runner._step_graphs)
